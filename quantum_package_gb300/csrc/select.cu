@@ -33,6 +33,14 @@
 // generic i_H_j (slater_rules.irp.f:478-570) with a as the first
 // determinant.
 //
+// Few of the staged selectors are connected to an entry, so the tile is also
+// kept transposed: one bit per selector for each virtual orbital and each k.
+// An entry finds its connected selectors with a few AND / OR per 32 selectors
+// and visits those alone.  Testing every selector against every entry
+// instead bound the kernel by integer issue: the call over 8 generators,
+// 2,000 selectors and 10.1M entries (14a+14b in 80 MOs) took 18.8 ms and
+// takes 12.5 ms this way.
+//
 // Banned determinants.  a is dropped when it is in the wave function
 // (device hash set of psi_det) or within a double excitation of an earlier
 // generator, so that every external determinant is counted once, by the
@@ -59,7 +67,9 @@ namespace {
 
 constexpr int SBLK = 256;
 constexpr int SEL_TILE = 16384;    // FP64 numerators per CTA at most (128 KB of shared memory)
-constexpr int SEL_DTILE = 256;     // selectors staged per filtering pass
+constexpr int SEL_DTILE = 256;     // selectors staged per pass (one word of 32 per warp of the CTA)
+constexpr int SEL_DWORDS = SEL_DTILE / 32;
+static_assert(SEL_DWORDS == SBLK / 32 && SBLK <= SEL_DTILE, "each warp transposes one word of staged selectors");
 constexpr int SEL_MAXST = 8;       // states
 constexpr int SEL_MAXFG = 2048;    // earlier generators kept per item in shared memory (else read from the global list)
 
@@ -190,52 +200,68 @@ __global__ void __launch_bounds__(SBLK) k_sel_lists(const u64* dets, const int* 
   if (mode == 0 && threadIdx.x == 0) cnt[l] = base_s;
 }
 
+__device__ __forceinline__ bool has_orb(const u64* d, int nint, int spin, int orb) {
+  return (d[spin * nint + ((orb - 1) >> 6)] >> ((orb - 1) & 63)) & 1ull;
+}
+
 // build_fock_tmp (Fock_diag.irp.f:1-98) of every listed generator:
 // f[l][s][i], i = 1..n_mo, and f[l][s][n_mo + 1] = <g|H|g>
+// One CTA per generator, a thread per (spin, orbital): each f keeps the order of
+// its sum (one thread per generator walked all of them: 443 us for 8
+// generators of 28 electrons in 80 orbitals, 12 us now).
 template <int NINT>
-__global__ void k_sel_fock(DevTables t, const u64* dets, const int* gens, int n_list, double* fock) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(SBLK) k_sel_fock(DevTables t, const u64* dets, const int* gens, int n_list,
+                                                   double* fock) {
+  __shared__ int occ[2][QPGPU_MAX_MO];
+  __shared__ int no[2];
+  __shared__ double part[2 * QPGPU_MAX_MO];  // shares of <g|H|g>
+  const int l = blockIdx.x;
   if (l >= n_list) return;
   const int n = t.n, st = n + 2;
   const u64* d = dets + (int64_t)gens[l] * 2 * NINT;
   double* f = fock + (int64_t)l * 2 * st;
-  for (int i = 0; i < 2 * st; ++i) f[i] = 0.0;
-  int occ[2][QPGPU_MAX_MO];
-  int no[2] = {0, 0};
-  for (int s = 0; s < 2; ++s)
+  if (threadIdx.x < 2) {
+    const int s = threadIdx.x;
+    int c = 0;
     for (int w = 0; w < NINT; ++w)
-      for (u64 x = d[s * NINT + w]; x; x &= x - 1) occ[s][no[s]++] = ctz64(x) + 1 + 64 * w;
-  double e0 = 0.0;
-  for (int s = 0; s < 2; ++s) {
-    const int o = 1 - s;
-    for (int ii = 0; ii < no[s]; ++ii) {
-      const int i = occ[s][ii];
-      f[s * st + i] += tab2(t.h, n, i, i);
-      e0 += tab2(t.h, n, i, i);
+      for (u64 x = d[s * NINT + w]; x; x &= x - 1) occ[s][c++] = ctz64(x) + 1 + 64 * w;
+    no[s] = c;
+  }
+  __syncthreads();
+  for (int x = threadIdx.x; x < 2 * n; x += SBLK) {
+    const int s = x / n, o = 1 - s, i = x % n + 1;
+    double v = 0.0, e = 0.0;
+    if (has_orb(d, NINT, s, i)) {
+      v = tab2(t.h, n, i, i);
+      e = tab2(t.h, n, i, i);
       for (int jj = 0; jj < no[s]; ++jj) {
         const int j = occ[s][jj];
         if (i == j) continue;
-        f[s * st + i] += tab2(t.ja, n, i, j);
-        e0 += 0.5 * tab2(t.ja, n, i, j);
+        v += tab2(t.ja, n, i, j);
+        e += 0.5 * tab2(t.ja, n, i, j);
       }
       for (int jj = 0; jj < no[o]; ++jj) {
         const int j = occ[o][jj];
-        f[s * st + i] += tab2(t.jj, n, i, j);
-        if (s == 0) e0 += tab2(t.jj, n, i, j);
+        v += tab2(t.jj, n, i, j);
+        if (s == 0) e += tab2(t.jj, n, i, j);
       }
     }
-  }
-  for (int s = 0; s < 2; ++s) {
-    const int o = 1 - s;
-    for (int i = 1; i <= n; ++i) {
-      if (f[s * st + i] != 0.0) continue;
-      f[s * st + i] += tab2(t.h, n, i, i);
-      for (int jj = 0; jj < no[s]; ++jj) f[s * st + i] += tab2(t.ja, n, i, occ[s][jj]);
-      for (int jj = 0; jj < no[o]; ++jj) f[s * st + i] += tab2(t.jj, n, i, occ[o][jj]);
+    if (v == 0.0) {  // empty orbitals (the reference tests the sum, not the occupation)
+      v += tab2(t.h, n, i, i);
+      for (int jj = 0; jj < no[s]; ++jj) v += tab2(t.ja, n, i, occ[s][jj]);
+      for (int jj = 0; jj < no[o]; ++jj) v += tab2(t.jj, n, i, occ[o][jj]);
     }
+    f[s * st + i] = v;
+    part[x] = e;
   }
-  f[n + 1] = e0;
-  f[st + n + 1] = e0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double e0 = 0.0;
+    for (int x = 0; x < 2 * n; ++x) e0 += part[x];
+    f[0] = f[st] = 0.0;
+    f[n + 1] = e0;
+    f[st + n + 1] = e0;
+  }
 }
 
 // <a|H|D>, generic path (degree from the words; a is the first determinant)
@@ -258,9 +284,6 @@ __device__ __forceinline__ double ihj(const DevTables& t, const u64* a, const u6
   return 0.0;
 }
 
-__device__ __forceinline__ bool has_orb(const u64* d, int nint, int spin, int orb) {
-  return (d[spin * nint + ((orb - 1) >> 6)] >> ((orb - 1) & 63)) & 1ull;
-}
 __device__ __forceinline__ void set_orb(u64* d, int nint, int spin, int orb, bool on) {
   const u64 b = 1ull << ((orb - 1) & 63);
   u64& w = d[spin * nint + ((orb - 1) >> 6)];
@@ -282,12 +305,13 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
   __shared__ u64 sdet[SEL_DTILE][2 * NINT];
   __shared__ int sidx[SEL_DTILE];
   __shared__ unsigned char sk[SEL_DTILE];
+  __shared__ unsigned shas[SEL_DWORDS][2][QPGPU_MAX_MO];  // staged selectors that hold a virtual orbital of g
+  __shared__ unsigned skm[SEL_DWORDS][3];                 // staged selectors with k = 0, 1, 2
   __shared__ int vir[2][QPGPU_MAX_MO];
   __shared__ int nvir[2];
   __shared__ int fgen[SEL_MAXFG];
   __shared__ int nfg;
   __shared__ int wsum[SBLK / 32];
-  __shared__ int nsel_s;
   const SelItem it = A.items[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nst = A.n_st, n = A.t.n;
@@ -333,81 +357,121 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
   __syncthreads();
   const int sp1 = it.kind == IT_AB ? 0 : it.spin;  // spin of particle 1
   const int sp2 = it.kind == IT_AB ? 1 : it.spin;  // spin of particle 2
-  auto particles = [&](int e, int& p1, int& p2) {
+  const bool two = it.kind != IT_SINGLE;
+  // positions of an entry's particles in vir[sp1], vir[sp2]
+  auto entry = [&](int e, int& v1, int& v2) {
     if (it.kind == IT_SINGLE) {
-      p1 = vir[it.spin][e];
-      p2 = 0;
+      v1 = e;
+      v2 = 0;
     } else if (it.kind == IT_SAME) {
-      int i1, i2;
-      tri_decode(e, i1, i2);
-      p1 = vir[it.spin][i1];
-      p2 = vir[it.spin][i2];
+      tri_decode(e, v1, v2);
     } else {
       const int nb = nvir[1];
-      p1 = vir[0][e / nb];
-      p2 = vir[1][e % nb];
+      v1 = e / nb;
+      v2 = e - v1 * nb;
     }
   };
   const int64_t i0 = A.ilist_off[it.gl], i1 = A.ilist_off[it.gl + 1];
-  for (int64_t base = i0; base < i1; base += SEL_DTILE) {
-    // stage the selectors of this pass with k = |mask \ D| <= 2, in order
-    if (tid == 0) nsel_s = 0;
-    __syncthreads();
-    for (int sub = 0; sub < SEL_DTILE; sub += SBLK) {
-      const int64_t q = base + sub + tid;
+  int64_t base = i0;
+  while (base < i1) {
+    // stage the next selectors with k = |mask \ D| <= 2, in order: blocks of
+    // SBLK candidates as long as what they keep fits the tile
+    int ns = 0;
+    while (base < i1) {
+      const int64_t q = base + tid;
       int D = -1, k = 3;
+      u64 dd[2 * NINT];
       if (q < i1) {
         D = A.ilist[q];
-        const u64* dd = A.dets + (int64_t)D * 2 * NINT;
         k = 0;
 #pragma unroll
-        for (int w = 0; w < 2 * NINT; ++w) k += popc64(mask[w] & ~dd[w]);
+        for (int w = 0; w < 2 * NINT; ++w) {
+          dd[w] = A.dets[(int64_t)D * 2 * NINT + w];
+          k += popc64(mask[w] & ~dd[w]);
+        }
       }
       const bool keep = k <= 2;
       const unsigned bal = __ballot_sync(0xffffffffu, keep);
       if (lane == 0) wsum[warp] = __popc(bal);
       __syncthreads();
-      int pos = nsel_s;
-      for (int w = 0; w < warp; ++w) pos += wsum[w];
-      pos += __popc(bal & ((1u << lane) - 1));
+      int before = 0, total = 0;
+#pragma unroll
+      for (int w = 0; w < SBLK / 32; ++w) {
+        before += w < warp ? wsum[w] : 0;
+        total += wsum[w];
+      }
+      __syncthreads();
+      if (ns + total > SEL_DTILE) break;  // this block opens the next tile
       if (keep) {
-        const u64* dd = A.dets + (int64_t)D * 2 * NINT;
+        const int pos = ns + before + __popc(bal & ((1u << lane) - 1));
 #pragma unroll
         for (int w = 0; w < 2 * NINT; ++w) sdet[pos][w] = dd[w];
         sidx[pos] = D;
         sk[pos] = (unsigned char)k;
       }
-      __syncthreads();
-      if (tid == 0) {
-        int tot = 0;
-        for (int w = 0; w < SBLK / 32; ++w) tot += wsum[w];
-        nsel_s += tot;
-      }
-      __syncthreads();
+      ns += total;
+      base += SBLK;
     }
-    const int ns = nsel_s;
-    // every thread: its entries against the staged selectors, in order
+    __syncthreads();
+    const int nw = (ns + 31) >> 5;
+    // transposed tile: warp w turns selectors 32 w .. 32 w + 31 into one word
+    // per virtual orbital and one per k
+    if (warp < nw) {
+      const int j = warp * 32 + lane;
+      const bool live = j < ns;
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        u64 x[NINT];
+#pragma unroll
+        for (int w = 0; w < NINT; ++w) x[w] = live ? sdet[j][s * NINT + w] : 0ull;
+        for (int v = 0; v < nvir[s]; ++v) {
+          const int o = vir[s][v] - 1;
+          u64 xw = x[0];
+          if (NINT == 2 && o >= 64) xw = x[NINT - 1];
+          const unsigned bal = __ballot_sync(0xffffffffu, (xw >> (o & 63)) & 1ull);
+          if (lane == 0) shas[warp][s][v] = bal;
+        }
+      }
+      const int k = live ? sk[j] : 3;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const unsigned bal = __ballot_sync(0xffffffffu, k == q);
+        if (lane == 0) skm[warp][q] = bal;
+      }
+    }
+    __syncthreads();
+    // every thread: its entries against their connected selectors, in order.
+    // deg = k + [p1 not in D] + [p2 not in D] is 1 or 2 for 32 selectors at a
+    // time (deg 0: a = D, in the wave function)
     for (int e = tid; e < ne; e += SBLK) {
-      int p1, p2;
-      particles(it.e0 + e, p1, p2);
+      int v1, v2;
+      entry(it.e0 + e, v1, v2);
       u64 a[2 * NINT];
 #pragma unroll
       for (int w = 0; w < 2 * NINT; ++w) a[w] = mask[w];
-      set_orb(a, NINT, sp1, p1, true);
-      if (it.kind != IT_SINGLE) set_orb(a, NINT, sp2, p2, true);
+      set_orb(a, NINT, sp1, vir[sp1][v1], true);
+      if (two) set_orb(a, NINT, sp2, vir[sp2][v2], true);
       double* m = tile + (size_t)e * nst;
-      for (int j = 0; j < ns; ++j) {
-        const u64* dd = sdet[j];
-        int deg = sk[j] + (has_orb(dd, NINT, sp1, p1) ? 0 : 1);
-        if (it.kind != IT_SINGLE) deg += has_orb(dd, NINT, sp2, p2) ? 0 : 1;
-        if (deg > 2 || deg == 0) continue;  // deg 0: a = D, in the wave function
+      double m0 = m[0];
+      int w = -1;
+      unsigned bits = 0;
+      while (true) {
+        while (bits == 0 && ++w < nw) {
+          const unsigned h1 = shas[w][sp1][v1], h2 = two ? shas[w][sp2][v2] : 0xffffffffu;
+          bits = (skm[w][0] & ~(h1 & h2)) | (skm[w][1] & (h1 | h2)) | (skm[w][2] & h1 & h2);
+        }
+        if (bits == 0) break;
+        const int j = w * 32 + __ffs(bits) - 1;
+        bits &= bits - 1;
         u64 Dw[2 * NINT];
 #pragma unroll
-        for (int w = 0; w < 2 * NINT; ++w) Dw[w] = dd[w];
+        for (int x = 0; x < 2 * NINT; ++x) Dw[x] = sdet[j][x];
         const double h = ihj<NINT>(A.t, a, Dw);
         const double* cD = A.coef + (int64_t)sidx[j] * nst;
-        for (int s = 0; s < nst; ++s) m[s] = fma(__ldg(&cD[s]), h, m[s]);
+        m0 = fma(__ldg(&cD[0]), h, m0);
+        for (int s = 1; s < nst; ++s) m[s] = fma(__ldg(&cD[s]), h, m[s]);
       }
+      m[0] = m0;
     }
     __syncthreads();
   }
@@ -424,13 +488,14 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
     double sabs = 0.0;
     for (int s = 0; s < nst; ++s) sabs += fabs(m[s]);
     if (sabs == 0.0) continue;
-    int p1, p2;
-    particles(it.e0 + e, p1, p2);
+    int v1, v2;
+    entry(it.e0 + e, v1, v2);
+    const int p1 = vir[sp1][v1], p2 = two ? vir[sp2][v2] : 0;
     u64 a[2 * NINT];
 #pragma unroll
     for (int w = 0; w < 2 * NINT; ++w) a[w] = mask[w];
     set_orb(a, NINT, sp1, p1, true);
-    if (it.kind != IT_SINGLE) set_orb(a, NINT, sp2, p2, true);
+    if (two) set_orb(a, NINT, sp2, p2, true);
     bool banned = in_wf<NINT>(A, a);
     if (nfg <= SEL_MAXFG) {
       for (int f = 0; f < nfg && !banned; ++f) banned = exc_deg<NINT>(a, A.dets + (int64_t)fgen[f] * 2 * NINT) <= 2;
@@ -470,7 +535,11 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
       pt[s] += ev;
       mine = fmin(ev, mine);
     }
-    const unsigned long long slot = atomicAdd(A.n_cand, 1ull);
+    // one atomic for the lanes that are here together
+    const unsigned grp = __activemask();
+    unsigned long long slot = 0;
+    if (lane == __ffs(grp) - 1) slot = atomicAdd(A.n_cand, (unsigned long long)__popc(grp));
+    slot = __shfl_sync(grp, slot, __ffs(grp) - 1) + __popc(grp & ((1u << lane) - 1));
     if (slot < A.cap) {
       A.cand_val[slot] = mine;
 #pragma unroll
@@ -490,13 +559,20 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
   }
 }
 
-// pt2[s] = sum over items, in order
-__global__ void k_sel_pt2(const double* part, int64_t n_items, int nst, double* pt2) {
-  const int s = threadIdx.x;
-  if (s >= nst) return;
+// pt2[s] = sum over items: one CTA per state, strided partial sums combined in
+// thread order (one thread walking 3,248 items waited 193 us on its loads)
+__global__ void __launch_bounds__(SBLK) k_sel_pt2(const double* part, int64_t n_items, int nst, double* pt2) {
+  __shared__ double red[SBLK];
+  const int s = blockIdx.x;
   double acc = 0.0;
-  for (int64_t i = 0; i < n_items; ++i) acc += part[i * nst + s];
-  pt2[s] = acc;
+  for (int64_t i = threadIdx.x; i < n_items; i += SBLK) acc += part[i * nst + s];
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  for (int o = SBLK / 2; o > 0; o >>= 1) {
+    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) pt2[s] = red[0];
 }
 
 // ascending order of doubles as unsigned keys
@@ -613,7 +689,7 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   k_hash_insert<NI><<<hb, 256, 0, st>>>(dets, N, (int*)d_slot.p, hcap - 1);                                     \
   k_sel_lists<NI><<<n_list, SBLK, 0, st>>>(dets, dg, n_list, n_sel, 0, 0, (int64_t*)d_icnt.p, nullptr, nullptr); \
   k_sel_lists<NI><<<n_list, SBLK, 0, st>>>(dets, dg, n_list, n_sel, 1, 0, (int64_t*)d_fcnt.p, nullptr, nullptr); \
-  k_sel_fock<NI><<<(n_list + 63) / 64, 64, 0, st>>>(c->tab, dets, dg, n_list, (double*)d_fock.p);
+  k_sel_fock<NI><<<n_list, SBLK, 0, st>>>(c->tab, dets, dg, n_list, (double*)d_fock.p);
   if (nint == 1) {
     QP_SEL_NINT(1)
   } else {
@@ -696,7 +772,7 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
     if (buf_size == 0 || hcnt[1] <= cap) break;
     cap = hcnt[1];  // every candidate counted: run once more with room for all of them
   }
-  k_sel_pt2<<<1, 32, 0, st>>>((const double*)d_part.p, n_items, n_st, (double*)d_pt2.p);
+  k_sel_pt2<<<n_st, SBLK, 0, st>>>((const double*)d_part.p, n_items, n_st, (double*)d_pt2.p);
   QP_CUDA(c, cudaMemcpyAsync(pt2, d_pt2.p, n_st * sizeof(double), cudaMemcpyDeviceToHost, st));
   if (per_gen) {
     std::vector<double> part((size_t)n_items * n_st);
