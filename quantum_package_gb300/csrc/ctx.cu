@@ -103,19 +103,21 @@ __device__ void export_pair(const DevTables& t, const u64* alpha, const u64* bet
     da += popc64(di[w] ^ dj[w]);
     db += popc64(di[NINT + w] ^ dj[NINT + w]);
   }
+  u64 E[2 * NINT];
+  det_parity<NINT>(di, E);
   int c, neg = 0, x4[4] = {0, 0, 0, 0};
   double s2;
   if (db == 0) {
     c = (da == 2) ? 1 : 3;
-    if (c == 1) h_mono_spin<NINT>(t, di, dj, 1, x4, &neg);
-    else h_double_spin<NINT>(t, di, dj, x4, &neg);
+    if (c == 1) h_mono_spin<NINT>(t, di, dj, E, 1, x4, &neg);
+    else h_double_spin<NINT>(t, di, dj, E, x4, &neg);
   } else if (da == 0) {
     c = (db == 2) ? 2 : 4;
-    if (c == 2) h_mono_spin<NINT>(t, di, dj, 2, x4, &neg);
-    else h_double_spin<NINT>(t, di + NINT, dj + NINT, x4, &neg);
+    if (c == 2) h_mono_spin<NINT>(t, di, dj, E, 2, x4, &neg);
+    else h_double_spin<NINT>(t, di + NINT, dj + NINT, E + NINT, x4, &neg);
   } else {
     c = 5;
-    h_double_ab<NINT>(t, di, dj, &s2, x4, &neg);
+    h_double_ab<NINT>(t, di, dj, E, &s2, x4, &neg);
   }
   out.I[o] = order[k];
   out.J[o] = order[jp];

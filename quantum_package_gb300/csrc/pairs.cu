@@ -30,6 +30,7 @@
 #include <cub/cub.cuh>
 
 #include "qpgpu_internal.cuh"
+#include "sigma_device.cuh"
 
 namespace {
 
@@ -109,20 +110,6 @@ constexpr int MODE_COUNT = 0, MODE_FILL = 1;
 
 __device__ __forceinline__ bool dsel(const BuildArgs& a, int64_t k) {
   return k >= a.row_lo && k < a.row_hi && ((k - a.row_first) % a.row_step) == 0;
-}
-
-// acc[st] += h * u[j][st] (j bilinear position; dacc_t: alpha-major position)
-__device__ __forceinline__ void dacc_t(const BuildArgs& a, double h, int64_t q, double (&acc)[8]) {
-  const double* uj = a.uT + q * a.nst;
-#pragma unroll
-  for (int st = 0; st < 8; ++st)
-    if (st < a.nst) acc[st] = fma(h, __ldg(uj + st), acc[st]);
-}
-__device__ __forceinline__ void dacc(const BuildArgs& a, double h, int64_t j, double (&acc)[8]) {
-  const double* uj = a.u + j * a.nst;
-#pragma unroll
-  for (int st = 0; st < 8; ++st)
-    if (st < a.nst) acc[st] = fma(h, __ldg(uj + st), acc[st]);
 }
 
 // ---- class A: same beta column, alpha singles / doubles -------------------
@@ -320,8 +307,10 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
             J[w] = ca[w];
             J[NINT + w] = cb[w];
           }
+          u64 E[2 * NINT];
+          det_parity<NINT>(my, E);
           double s2;
-          h_double_ab<NINT>(a.t, my, J, &s2, nullptr, nullptr);
+          h_double_ab<NINT>(a.t, my, J, E, &s2, nullptr, nullptr);
           const int64_t so = sout + scnt + __popc(sbal & lt);
           if (so < a.s2ptr[k + 1]) {
             a.s2col[so] = jpos;
@@ -634,56 +623,133 @@ __global__ void __launch_bounds__(BLK) k_same_keyed(BuildArgs a) {
   }
 }
 
+// A warp's list of pairs put off until 32 of them are there (shared memory):
+// the rare, long branches of an element kernel then run with all lanes busy.
+constexpr int DEFER = 64;
+struct Deferred {
+  int* q;  // DEFER entries of this warp
+  int n;
+  // lanes with `on` append x; true when 32 or more are waiting
+  __device__ __forceinline__ bool push(bool on, int x, unsigned lt) {
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (on) q[n + __popc(m & lt)] = x;
+    n += __popc(m);
+    __syncwarp();
+    return n >= 32;
+  }
+  // the last up to 32 entries, one per lane (-1: none)
+  __device__ __forceinline__ int pop(int lane) {
+    const int m = min(n, 32);
+    n -= m;
+    const int x = lane < m ? q[n + lane] : -1;
+    __syncwarp();
+    return x;
+  }
+};
+
 // FP64 / FP32 elements of the stored pairs, after the fill pass has written
 // their columns: one warp per row, lanes over the row's pairs, so that the
 // dependent integral loads of 32 pairs are in flight at once (the fill's
 // scanning thread would evaluate its row's pairs one after the other).  The
-// class of a pair follows from the two determinants' strings, and each class
-// calls the same Slater routine with the same arguments as the scans do, so
-// the values are bit-identical.
+// columns are ascending, so the same-beta partners are one run (the row's own
+// beta column); same-alpha partners are told by their alpha id, and only the
+// string that differs is read.  Each class calls the same Slater routine with
+// the same arguments as the scans do, so the values are bit-identical.
+// Same-alpha pairs and single excitations (whose sums over the holes and
+// particles against the reference take several times a double's loads) are
+// deferred until 32 of a kind are there: with them inline almost every trip
+// paid for all branches.  991M pairs at 1e6 determinants: 35.4 -> 30.8 ms.
 template <int NINT>
 __global__ void __launch_bounds__(BLK) k_pair_values(BuildArgs a) {
+  __shared__ int s_q[BLK / 32][2][DEFER];
   const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
   const int64_t warp = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5;
   const int64_t nwarp = ((int64_t)gridDim.x * BLK) >> 5;
+  Deferred same_alpha{s_q[threadIdx.x >> 5][0], 0}, mono{s_q[threadIdx.x >> 5][1], 0};
   for (int64_t k = warp; k < a.N; k += nwarp) {
-    u64 my[2 * NINT];
-    const int bi = a.cols[k];
+    u64 my[2 * NINT], E[2 * NINT];
+    const int bi = a.cols[k], ai = a.rows[k];
+    const int cs = a.col_loc[bi], ce = a.col_loc[bi + 1];
 #pragma unroll
     for (int w = 0; w < NINT; ++w) {
       my[w] = a.alpha_pos[k * NINT + w];
       my[NINT + w] = a.beta[(int64_t)bi * NINT + w];
     }
-    const int64_t e1 = a.rowptr[k + 1];
-    for (int64_t e = a.rowptr[k] + lane; e < e1; e += 32) {
-      const int j = a.colidx[e];
+    det_parity<NINT>(my, E);
+    const int64_t e0 = a.rowptr[k];
+    const int n = (int)(a.rowptr[k + 1] - e0);
+    auto put = [&](int x, double v) {
+      a.val64[e0 + x] = v;
+      a.val32[e0 + x] = (float)v;
+    };
+    auto do_mono = [&](int x) {  // one string differs, by one electron
+      if (x < 0) return;
+      const int j = a.colidx[e0 + x];
+      const bool beta = j < cs || j >= ce;
       u64 J[2 * NINT];
-      const int bj = a.cols[j];
-      bool samea = true, sameb = true;
-      int da = 0, db = 0;
+      const int bj = beta ? a.cols[j] : bi;
 #pragma unroll
       for (int w = 0; w < NINT; ++w) {
-        J[w] = a.alpha_pos[(int64_t)j * NINT + w];
-        J[NINT + w] = a.beta[(int64_t)bj * NINT + w];
-        samea &= J[w] == my[w];
-        sameb &= J[NINT + w] == my[NINT + w];
-        da += popc64(my[w] ^ J[w]);
-        db += popc64(my[NINT + w] ^ J[NINT + w]);
+        J[w] = beta ? my[w] : a.alpha_pos[(int64_t)j * NINT + w];
+        J[NINT + w] = beta ? a.beta[(int64_t)bj * NINT + w] : my[NINT + w];
       }
-      double v;
-      if (sameb)  // class A (same beta column)
-        v = (da == 2) ? h_mono_spin<NINT>(a.t, my, J, 1, nullptr, nullptr)
-                      : h_double_spin<NINT>(a.t, my, J, nullptr, nullptr);
-      else if (samea)  // class B (same alpha row)
-        v = (db == 2) ? h_mono_spin<NINT>(a.t, my, J, 2, nullptr, nullptr)
-                      : h_double_spin<NINT>(a.t, my + NINT, J + NINT, nullptr, nullptr);
-      else {  // class C (alpha single x beta single)
-        double s2;
-        v = h_double_ab<NINT>(a.t, my, J, &s2, nullptr, nullptr);
+      put(x, h_mono_spin<NINT>(a.t, my, J, E, beta ? 2 : 1, nullptr, nullptr));
+    };
+    auto do_same_alpha = [&](int x) -> bool {  // true: a single
+      if (x < 0) return false;
+      const int bj = a.cols[a.colidx[e0 + x]];
+      u64 J[NINT];
+      int d = 0;
+#pragma unroll
+      for (int w = 0; w < NINT; ++w) {
+        J[w] = a.beta[(int64_t)bj * NINT + w];
+        d += popc64(my[NINT + w] ^ J[w]);
       }
-      a.val64[e] = v;
-      a.val32[e] = (float)v;
+      if (d == 2) return true;
+      put(x, h_double_spin<NINT>(a.t, my + NINT, J, E + NINT, nullptr, nullptr));
+      return false;
+    };
+    for (int x0 = 0; x0 < n; x0 += 32) {
+      const int x = x0 + lane;
+      const bool in = x < n;
+      const int j = in ? a.colidx[e0 + x] : -1;
+      bool is_b = false, is_mono = false;
+      if (in && j >= cs && j < ce) {  // same beta column
+        u64 J[NINT];
+        int d = 0;
+#pragma unroll
+        for (int w = 0; w < NINT; ++w) {
+          J[w] = a.alpha_pos[(int64_t)j * NINT + w];
+          d += popc64(my[w] ^ J[w]);
+        }
+        is_mono = d == 2;
+        if (!is_mono) put(x, h_double_spin<NINT>(a.t, my, J, E, nullptr, nullptr));
+      } else if (in) {
+        is_b = a.rows[j] == ai;  // same alpha row
+        if (!is_b) {             // alpha single x beta single
+          const int bj = a.cols[j];
+          u64 J[2 * NINT];
+#pragma unroll
+          for (int w = 0; w < NINT; ++w) {
+            J[w] = a.alpha_pos[(int64_t)j * NINT + w];
+            J[NINT + w] = a.beta[(int64_t)bj * NINT + w];
+          }
+          double s2;
+          put(x, h_double_ab<NINT>(a.t, my, J, E, &s2, nullptr, nullptr));
+        }
+      }
+      if (mono.push(is_mono, x, lt)) do_mono(mono.pop(lane));
+      if (same_alpha.push(is_b, x, lt)) {
+        const int y = same_alpha.pop(lane);
+        if (mono.push(do_same_alpha(y), y, lt)) do_mono(mono.pop(lane));
+      }
     }
+    {
+      const int y = same_alpha.pop(lane);
+      if (mono.push(do_same_alpha(y), y, lt)) do_mono(mono.pop(lane));
+    }
+    do_mono(mono.pop(lane));
   }
 }
 
@@ -943,96 +1009,120 @@ __global__ void k_alpha_major(const double* u, const int* t_order, double* uT, i
 // k_pair_values (same routines, same arguments), multiplied by the partner's
 // coefficients (same-alpha partners, tagged with their alpha-major position,
 // read from the alpha-major copy uT, where a row's partners are contiguous),
-// and the lanes are combined in a fixed butterfly order.
-template <int NINT>
+// and the lanes are combined in a fixed order.  The fill wrote the row's
+// same-beta partners, then its same-alpha partners, then the alpha x beta
+// ones, so each class has a loop of its own, a same-spin partner reads only
+// the string it does not share with the row, and the single excitations of
+// both same-spin classes are deferred until 32 are there (k_pair_values).
+// NP: states padded to a power of two, so that the sums stay in registers.
+// 2e5 determinants in 120 MOs, 2 states: 7.4 -> 4.1 ms with the register-only
+// Slater routines, the loops per class and the deferred singles.
+template <int NINT, int NP>
 __global__ void __launch_bounds__(BLK, 3) k_pair_sigma(BuildArgs a, const int* __restrict__ pc) {
+  __shared__ int s_q[BLK / 32][DEFER];
   const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
   const int64_t warp = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5;
   const int64_t nwarp = ((int64_t)gridDim.x * BLK) >> 5;
+  const int nst = a.nst;
+  Deferred mono{s_q[threadIdx.x >> 5], 0};
   for (int64_t k = a.row_lo + warp; k < a.row_hi; k += nwarp) {
     if (((k - a.row_first) % a.row_step) != 0) continue;
-    u64 my[2 * NINT];
+    u64 my[2 * NINT], E[2 * NINT];
     const int bi = a.cols[k];
 #pragma unroll
     for (int w = 0; w < NINT; ++w) {
       my[w] = a.alpha_pos[k * NINT + w];
       my[NINT + w] = a.beta[(int64_t)bi * NINT + w];
     }
-    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, sacc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const int64_t e0 = a.rowptr[k], e1 = a.rowptr[k + 1];
-    // the fill wrote the row's same-beta partners, then its same-alpha
-    // partners, then the alpha x beta ones: a same-spin partner shares one
-    // string with the row, so only its other string is read
-    const int64_t eA = e0 + a.cntA[k], eB = eA + a.cntB[k];
-    for (int64_t e = e0 + lane; e < e1; e += 32) {
-      const unsigned cj = (unsigned)pc[e - a.col_base];
+    det_parity<NINT>(my, E);
+    double acc[NP], sacc[NP];
+#pragma unroll
+    for (int st = 0; st < NP; ++st) acc[st] = sacc[st] = 0.0;
+    auto add = [&](double (&s)[NP], double v, const double* uj) {
+#pragma unroll
+      for (int st = 0; st < NP; ++st)
+        if (st < nst) s[st] = fma(v, __ldg(uj + st), s[st]);
+    };
+    const int64_t e0 = a.rowptr[k];
+    const int* prow = pc + (e0 - a.col_base);
+    const int n = (int)(a.rowptr[k + 1] - e0), nA = a.cntA[k], nB = nA + a.cntB[k];
+    auto do_mono = [&](int x) {
+      if (x < 0) return;
+      const bool beta = x >= nA;
+      const int q = (int)((unsigned)prow[x] & ~QP_TAG_T);
+      const u64* str = beta ? a.beta_tpos : a.alpha_pos;
+      u64 J[2 * NINT];
+#pragma unroll
+      for (int w = 0; w < NINT; ++w) {
+        const u64 y = str[(int64_t)q * NINT + w];
+        J[w] = beta ? my[w] : y;
+        J[NINT + w] = beta ? y : my[NINT + w];
+      }
+      const double v = h_mono_spin<NINT>(a.t, my, J, E, beta ? 2 : 1, nullptr, nullptr);
+      add(acc, v, (beta ? a.uT : a.u) + (int64_t)q * nst);
+    };
+    for (int x0 = 0; x0 < nB; x0 += 32) {  // same-spin partners (beta column, then alpha row)
+      const int x = x0 + lane;
+      bool is_mono = false;
+      if (x < nB) {
+        const bool beta = x >= nA;
+        const int q = (int)((unsigned)prow[x] & ~QP_TAG_T);
+        const u64* str = beta ? a.beta_tpos : a.alpha_pos;
+        u64 I[NINT], J[NINT], Es[NINT];
+        int d = 0;
+#pragma unroll
+        for (int w = 0; w < NINT; ++w) {
+          J[w] = str[(int64_t)q * NINT + w];
+          I[w] = beta ? my[NINT + w] : my[w];
+          Es[w] = beta ? E[NINT + w] : E[w];
+          d += popc64(I[w] ^ J[w]);
+        }
+        is_mono = d == 2;
+        if (!is_mono)
+          add(acc, h_double_spin<NINT>(a.t, I, J, Es, nullptr, nullptr), (beta ? a.uT : a.u) + (int64_t)q * nst);
+      }
+      if (mono.push(is_mono, x, lt)) do_mono(mono.pop(lane));
+    }
+    for (int x = nB + lane; x < n; x += 32) {  // alpha single x beta single
+      const unsigned cj = (unsigned)prow[x];
       const bool via_t = (cj & QP_TAG_T) != 0;
       const int q = (int)(cj & ~QP_TAG_T);
+      const int j = via_t ? a.t_order[q] : q;
+      const int bj = a.cols[j];
       u64 J[2 * NINT];
-      bool samea, sameb;
-      int da = 0, db = 0, j = q;
-      if (e < eA) {  // same beta column: q is the partner's bilinear position
-        samea = false;
-        sameb = true;
 #pragma unroll
-        for (int w = 0; w < NINT; ++w) {
-          J[w] = a.alpha_pos[(int64_t)q * NINT + w];
-          J[NINT + w] = my[NINT + w];
-          da += popc64(my[w] ^ J[w]);
-        }
-      } else if (e < eB) {  // same alpha row: q is the partner's alpha-major position
-        samea = true;
-        sameb = false;
-#pragma unroll
-        for (int w = 0; w < NINT; ++w) {
-          J[w] = my[w];
-          J[NINT + w] = a.beta_tpos[(int64_t)q * NINT + w];
-          db += popc64(my[NINT + w] ^ J[NINT + w]);
-        }
-      } else {
-        j = via_t ? a.t_order[q] : q;
-        const int bj = a.cols[j];
-        samea = sameb = false;
-#pragma unroll
-        for (int w = 0; w < NINT; ++w) {
-          J[w] = a.alpha_pos[(int64_t)j * NINT + w];
-          J[NINT + w] = a.beta[(int64_t)bj * NINT + w];
-        }
+      for (int w = 0; w < NINT; ++w) {
+        J[w] = a.alpha_pos[(int64_t)j * NINT + w];
+        J[NINT + w] = a.beta[(int64_t)bj * NINT + w];
       }
-      double v, s2 = 0.0;
-      if (sameb)
-        v = (da == 2) ? h_mono_spin<NINT>(a.t, my, J, 1, nullptr, nullptr)
-                      : h_double_spin<NINT>(a.t, my, J, nullptr, nullptr);
-      else if (samea)
-        v = (db == 2) ? h_mono_spin<NINT>(a.t, my, J, 2, nullptr, nullptr)
-                      : h_double_spin<NINT>(a.t, my + NINT, J + NINT, nullptr, nullptr);
-      else
-        v = h_double_ab<NINT>(a.t, my, J, &s2, nullptr, nullptr);
-      if (via_t) {
-        dacc_t(a, v, q, acc);
-        if (s2 != 0.0) dacc_t(a, s2, q, sacc);
-      } else {
-        dacc(a, v, j, acc);
-        if (s2 != 0.0) dacc(a, s2, j, sacc);
-      }
+      double s2;
+      const double v = h_double_ab<NINT>(a.t, my, J, E, &s2, nullptr, nullptr);
+      const double* uj = (via_t ? a.uT : a.u) + (int64_t)q * nst;
+      add(acc, v, uj);
+      if (s2 != 0.0) add(sacc, s2, uj);
     }
-#pragma unroll
-    for (int st = 0; st < 8; ++st) {
-      if (st >= a.nst) break;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        acc[st] += __shfl_xor_sync(0xffffffffu, acc[st], o);
-        sacc[st] += __shfl_xor_sync(0xffffffffu, sacc[st], o);
-      }
+    __syncwarp();
+    do_mono(mono.pop(lane));
+    constexpr int SH = 5 - qpsig::Pow2<NP>::lg;
+    const double hv = qpsig::reduce_scatter64<NP>(acc, lane);
+    const double sv = qpsig::reduce_scatter64<NP>(sacc, lane);
+    const int st = lane >> SH;
+    if ((lane & ((1 << SH) - 1)) == 0 && st < nst) {
+      const double uk = a.u[k * nst + st];
+      a.v[k * nst + st] = hv + a.hdiag[k] * uk;
+      a.s[k * nst + st] = sv + a.sdiag[k] * uk;
     }
-    if (lane == 0) {
-      const double hd = a.hdiag[k], sd = a.sdiag[k];
-      for (int st = 0; st < a.nst; ++st) {
-        const double uk = a.u[k * a.nst + st];
-        a.v[k * a.nst + st] = acc[st] + hd * uk;
-        a.s[k * a.nst + st] = sacc[st] + sd * uk;
-      }
-    }
+  }
+}
+
+template <int NINT>
+void launch_pair_sigma(const BuildArgs& a, const int* pc, unsigned grid, cudaStream_t st) {
+  switch (qp_pad_states(a.nst)) {
+    case 1: k_pair_sigma<NINT, 1><<<grid, BLK, 0, st>>>(a, pc); break;
+    case 2: k_pair_sigma<NINT, 2><<<grid, BLK, 0, st>>>(a, pc); break;
+    case 4: k_pair_sigma<NINT, 4><<<grid, BLK, 0, st>>>(a, pc); break;
+    default: k_pair_sigma<NINT, 8><<<grid, BLK, 0, st>>>(a, pc); break;
   }
 }
 
@@ -1087,7 +1177,7 @@ int sigma_direct_t(qpgpu_ctx* c, double* v, double* s, const double* u, const do
       if (marks) qp_mark(c, "direct: scan B");
       k_class_c<NINT, MODE_FILL><<<gC, BLK, 0, st>>>(a);
       if (marks) qp_mark(c, "direct: scan C");
-      k_pair_sigma<NINT><<<nblocks((hi - lo) * 32, BLK), BLK, 0, st>>>(a, c->d_direct_cols);
+      launch_pair_sigma<NINT>(a, c->d_direct_cols, gK, st);
       if (marks) qp_mark(c, "direct: elements");
     }
     clo = chi;

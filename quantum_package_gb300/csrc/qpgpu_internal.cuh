@@ -44,10 +44,16 @@ __host__ __device__ inline long long pair_idx(long long i, long long j) {
 }
 
 #ifdef __CUDACC__
+// bielec_integrals_index of two 1-based orbitals / pairs in 32 bits: n_mo <= 128
+// keeps the packed index below 3.5e7
+__device__ __forceinline__ unsigned pair_idx32(unsigned i, unsigned j) {
+  const unsigned p = min(i, j), r = max(i, j);
+  return p + ((r * r - r) >> 1);
+}
 // <ij|kl> physicist = (ik|jl) chemist  (get_mo_bielec_integral,
 // src/Integrals_Bielec/map_integrals.irp.f:383-413; dense-cache path)
 __device__ __forceinline__ double get_int(const DevTables& t, int i, int j, int k, int l) {
-  return __ldg(&t.eri[pair_idx(pair_idx(i, k), pair_idx(j, l)) - 1]);
+  return __ldg(&t.eri[pair_idx32(pair_idx32(i, k), pair_idx32(j, l)) - 1]);
 }
 __device__ __forceinline__ double tab2(const double* a, int n, int i, int j) {
   return __ldg(&a[(i - 1) + (size_t)(j - 1) * n]);
@@ -59,75 +65,126 @@ __device__ __forceinline__ double tab3(const double* a, int n, int x, int y, int
 __device__ __forceinline__ int popc64(u64 x) { return __popcll(x); }
 __device__ __forceinline__ int ctz64(u64 x) { return __ffsll((long long)x) - 1; }
 
-// Electrons of det1 strictly between orbitals low < high (1-based), the nperm
-// term of get_mono/double_excitation_spin (slater_rules.irp.f:2837-2860,2954-2969)
+// The routines below keep every string in registers: no word is picked by a
+// run-time index (that puts the string in local memory), and the electrons
+// between two orbitals come from a parity word formed once per determinant
+// instead of a masked count per pair.
+
+// lowest / highest set orbital (0-based) of a non-empty string
 template <int NINT>
-__device__ __forceinline__ int nperm_between(const u64* det1, int low, int high) {
-  int j = (low - 1) >> 6, n = ((low - 1) & 63) + 1;
-  int k = (high - 1) >> 6, m = ((high - 1) & 63) + 1;
-  int np = 0;
-  if (j == k) {
-    u64 mask = ((1ull << (m - 1)) - 1ull) & (0ull - (1ull << n));
-    np += popc64(det1[j] & mask);
-  } else {
-    np += popc64(det1[k] & ((1ull << (m - 1)) - 1ull));
-    if (n < 64) np += popc64(det1[j] & (0ull - (1ull << n)));
+__device__ __forceinline__ int lowest_orb(const u64* x) {
+  if constexpr (NINT == 1) return ctz64(x[0]);
+  else return x[0] ? ctz64(x[0]) : 64 + ctz64(x[NINT - 1]);
+}
+template <int NINT>
+__device__ __forceinline__ int highest_orb(const u64* x) {
+  if constexpr (NINT == 1) return 63 - __clzll((long long)x[0]);
+  else return x[NINT - 1] ? 127 - __clzll((long long)x[NINT - 1]) : 63 - __clzll((long long)x[0]);
+}
+template <int NINT>
+__device__ __forceinline__ int orb_bit(const u64* x, int b) {
+  u64 w = x[0];
+  if constexpr (NINT == 2) w = b < 64 ? x[0] : x[NINT - 1];
+  return (int)(w >> (b & 63)) & 1;
+}
+// E: bit b of the NINT words = parity of the electrons of d below orbital b
+template <int NINT>
+__device__ __forceinline__ void prefix_parity(const u64* d, u64* E) {
+  u64 carry = 0;
 #pragma unroll
-    for (int i = 0; i < NINT; ++i)
-      if (i > j && i < k) np += popc64(det1[i]);
+  for (int w = 0; w < NINT; ++w) {
+    u64 x = d[w];
+#pragma unroll
+    for (int o = 1; o < 64; o <<= 1) x ^= x << o;
+    E[w] = x ^ d[w] ^ carry;
+    carry ^= 0ull - (x >> 63);
   }
+}
+// the same for both spins of a determinant (alpha words, then beta words)
+template <int NINT>
+__device__ __forceinline__ void det_parity(const u64* det, u64* E) {
+  prefix_parity<NINT>(det, E);
+  prefix_parity<NINT>(det + NINT, E + NINT);
+}
+// parity of the electrons of d strictly between hole h (occupied in d) and
+// particle p (empty in d), 0-based: the nperm term of
+// get_mono/double_excitation_spin (slater_rules.irp.f:2837-2860,2954-2969).
+// The parities below h and p differ by those electrons and, when h < p, by h
+// itself.
+template <int NINT>
+__device__ __forceinline__ int move_parity(const u64* E, int h, int p) {
+  return orb_bit<NINT>(E, h) ^ orb_bit<NINT>(E, p) ^ (h < p ? 1 : 0);
+}
+
+// get_mono_excitation_spin, slater_rules.irp.f:2913-2987 (hole in d1, particle
+// in d2, 1-based); E = prefix_parity of d1
+template <int NINT>
+__device__ __forceinline__ int mono_exc_spin(const u64* d1, const u64* d2, const u64* E, int* hole, int* part) {
+  u64 hw[NINT], pw[NINT];
+#pragma unroll
+  for (int l = 0; l < NINT; ++l) {
+    hw[l] = d1[l] & ~d2[l];
+    pw[l] = d2[l] & ~d1[l];
+  }
+  const int h = lowest_orb<NINT>(hw), p = lowest_orb<NINT>(pw);
+  *hole = h + 1;
+  *part = p + 1;
+  return move_parity<NINT>(E, h, p);  // 1 => phase -1
+}
+
+// get_double_excitation_spin, slater_rules.irp.f:2783-2911 (holes/particles
+// ascending, 1-based); E = prefix_parity of d1
+template <int NINT>
+__device__ __forceinline__ int double_exc_spin(const u64* d1, const u64* d2, const u64* E, int* h, int* p) {
+  u64 hw[NINT], pw[NINT];
+#pragma unroll
+  for (int l = 0; l < NINT; ++l) {
+    hw[l] = d1[l] & ~d2[l];
+    pw[l] = d2[l] & ~d1[l];
+  }
+  const int h0 = lowest_orb<NINT>(hw), h1 = highest_orb<NINT>(hw);
+  const int p0 = lowest_orb<NINT>(pw), p1 = highest_orb<NINT>(pw);
+  int np = move_parity<NINT>(E, h0, p0) ^ move_parity<NINT>(E, h1, p1);
+  const int a = min(h0, p0), b = max(h0, p0);
+  const int c = min(h1, p1), d = max(h1, p1);
+  if (c > a && c < b && d > b) np ^= 1;
+  h[0] = h0 + 1;
+  h[1] = h1 + 1;
+  p[0] = p0 + 1;
+  p[1] = p1 + 1;
   return np;
 }
 
-// get_mono_excitation_spin, slater_rules.irp.f:2913-2987 (hole in d1, particle in d2)
-template <int NINT>
-__device__ __forceinline__ int mono_exc_spin(const u64* d1, const u64* d2, int* hole, int* part) {
-  int h = 0, p = 0;
+// h +- the terms tab(x, h, p) of the orbitals in X, ascending: four loads in
+// flight at a time, added in order
+template <int NINT, bool ADD>
+__device__ __forceinline__ double add_terms(double hij, const double* tab, int n, const u64* X, int h, int p) {
+  u64 x[NINT];
 #pragma unroll
-  for (int l = 0; l < NINT; ++l) {
-    u64 tmp = d1[l] ^ d2[l];
-    u64 particle = tmp & d2[l];
-    u64 hl = tmp & d1[l];
-    if (particle) p = ctz64(particle) + 1 + 64 * l;
-    if (hl) h = ctz64(hl) + 1 + 64 * l;
-  }
-  *hole = h;
-  *part = p;
-  int low = h < p ? h : p, high = h < p ? p : h;
-  return nperm_between<NINT>(d1, low, high) & 1;  // 1 => phase -1
-}
-
-// get_double_excitation_spin, slater_rules.irp.f:2783-2911 (holes/particles ascending)
-template <int NINT>
-__device__ __forceinline__ int double_exc_spin(const u64* d1, const u64* d2, int* h, int* p) {
-  int ih = 0, ip = 0;
-  h[0] = h[1] = p[0] = p[1] = 0;
+  for (int w = 0; w < NINT; ++w) x[w] = X[w];
+  const double* col = tab + (size_t)n * ((h - 1) + (size_t)n * (p - 1));
+  while (true) {
+    double v[4];
+    int k = 0;
 #pragma unroll
-  for (int l = 0; l < NINT; ++l) {
-    u64 tmp = d1[l] ^ d2[l];
-    u64 particle = tmp & d2[l];
-    u64 hl = tmp & d1[l];
-    while (particle) {
-      if (ip < 2) p[ip] = ctz64(particle) + 1 + 64 * l;
-      ++ip;
-      particle &= particle - 1;
+    for (int q = 0; q < 4; ++q) {
+      bool any = x[0] != 0;
+      if constexpr (NINT == 2) any = any || x[NINT - 1] != 0;
+      v[q] = 0.0;
+      if (any) {
+        v[q] = __ldg(col + lowest_orb<NINT>(x));
+        if constexpr (NINT == 2) {
+          if (x[0] == 0) x[NINT - 1] &= x[NINT - 1] - 1;
+        }
+        x[0] &= x[0] - 1;  // 0 stays 0
+        k = q + 1;
+      }
     }
-    while (hl) {
-      if (ih < 2) h[ih] = ctz64(hl) + 1 + 64 * l;
-      ++ih;
-      hl &= hl - 1;
-    }
-  }
-  int np = 0;
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    int low = h[i] < p[i] ? h[i] : p[i], high = h[i] < p[i] ? p[i] : h[i];
-    np += nperm_between<NINT>(d1, low, high);
+    for (int q = 0; q < 4; ++q)
+      if (q < k) hij = ADD ? __dadd_rn(hij, v[q]) : __dsub_rn(hij, v[q]);
+    if (k < 4) return hij;
   }
-  int a = min(h[0], p[0]), b = max(h[0], p[0]);
-  int c = min(h[1], p[1]), d = max(h[1], p[1]);
-  if (c > a && c < b && d > b) np += 1;
-  return np & 1;
 }
 
 // get_mono_excitation_from_fock, src/Determinants/mono_excitations.irp.f:97-155
@@ -145,34 +202,30 @@ __device__ __forceinline__ double mono_from_fock(const DevTables& t, const u64* 
       hole[s][i] = diff & t.ref_cs[s * NINT + i];
       partcl[s][i] = diff & det1[s * NINT + i];
     }
+  u64 hs[NINT], ps[NINT];  // holes and particles of the excitation's spin
+#pragma unroll
+  for (int i = 0; i < NINT; ++i) {
+    hs[i] = spin == 1 ? hole[0][i] : hole[1][i];
+    ps[i] = spin == 1 ? partcl[0][i] : partcl[1][i];
+  }
   double hij = tab2(t.fock, n, h, p);
   // holes: direct terms (alpha then beta), exchange terms (same spin)
-#pragma unroll
-  for (int s = 0; s < 2; ++s)
-#pragma unroll
-    for (int w = 0; w < NINT; ++w)
-      for (u64 x = hole[s][w]; x; x &= x - 1) hij = __dsub_rn(hij, tab3(t.bc, n, ctz64(x) + 1 + 64 * w, h, p));
-#pragma unroll
-  for (int w = 0; w < NINT; ++w)
-    for (u64 x = hole[spin - 1][w]; x; x &= x - 1) hij = __dadd_rn(hij, tab3(t.bx, n, ctz64(x) + 1 + 64 * w, h, p));
+  hij = add_terms<NINT, false>(hij, t.bc, n, hole[0], h, p);
+  hij = add_terms<NINT, false>(hij, t.bc, n, hole[1], h, p);
+  hij = add_terms<NINT, true>(hij, t.bx, n, hs, h, p);
   // particles: direct terms, exchange terms
-#pragma unroll
-  for (int s = 0; s < 2; ++s)
-#pragma unroll
-    for (int w = 0; w < NINT; ++w)
-      for (u64 x = partcl[s][w]; x; x &= x - 1) hij = __dadd_rn(hij, tab3(t.bc, n, ctz64(x) + 1 + 64 * w, h, p));
-#pragma unroll
-  for (int w = 0; w < NINT; ++w)
-    for (u64 x = partcl[spin - 1][w]; x; x &= x - 1) hij = __dsub_rn(hij, tab3(t.bx, n, ctz64(x) + 1 + 64 * w, h, p));
+  hij = add_terms<NINT, true>(hij, t.bc, n, partcl[0], h, p);
+  hij = add_terms<NINT, true>(hij, t.bc, n, partcl[1], h, p);
+  hij = add_terms<NINT, false>(hij, t.bx, n, ps, h, p);
   return neg ? -hij : hij;
 }
 
-// i_H_j_double_spin, slater_rules.irp.f:3008-3035 (si, sj: spin strings)
+// i_H_j_double_spin, slater_rules.irp.f:3008-3035 (si, sj: spin strings, E = prefix_parity of si)
 template <int NINT>
-__device__ __forceinline__ double h_double_spin(const DevTables& t, const u64* si, const u64* sj, int* exc4,
-                                                int* neg_out) {
+__device__ __forceinline__ double h_double_spin(const DevTables& t, const u64* si, const u64* sj, const u64* E,
+                                                int* exc4, int* neg_out) {
   int h[2], p[2];
-  int neg = double_exc_spin<NINT>(si, sj, h, p);
+  int neg = double_exc_spin<NINT>(si, sj, E, h, p);
   double v = __dsub_rn(get_int(t, h[0], h[1], p[0], p[1]), get_int(t, h[0], h[1], p[1], p[0]));
   if (exc4) { exc4[0] = h[0]; exc4[1] = p[0]; exc4[2] = h[1]; exc4[3] = p[1]; }
   if (neg_out) *neg_out = neg;
@@ -187,11 +240,11 @@ __device__ __forceinline__ double h_double_spin(const DevTables& t, const u64* s
 // reverse excitation J->I that get_s2 uses equals that of I->J: the electrons
 // strictly between hole and particle are the same in I and J.)
 template <int NINT>
-__device__ __forceinline__ double h_double_ab(const DevTables& t, const u64* ki, const u64* kj, double* s2,
-                                              int* exc4, int* neg_out) {
+__device__ __forceinline__ double h_double_ab(const DevTables& t, const u64* ki, const u64* kj, const u64* E,
+                                              double* s2, int* exc4, int* neg_out) {
   int ha, pa, hb, pb;
-  int na = mono_exc_spin<NINT>(ki, kj, &ha, &pa);
-  int nb = mono_exc_spin<NINT>(ki + NINT, kj + NINT, &hb, &pb);
+  int na = mono_exc_spin<NINT>(ki, kj, E, &ha, &pa);
+  int nb = mono_exc_spin<NINT>(ki + NINT, kj + NINT, E + NINT, &hb, &pb);
   int neg = na ^ nb;
   double v = get_int(t, ha, hb, pa, pb);
   *s2 = (pa == hb && pb == ha) ? (neg ? 1.0 : -1.0) : 0.0;
@@ -200,12 +253,19 @@ __device__ __forceinline__ double h_double_ab(const DevTables& t, const u64* ki,
   return neg ? -v : v;
 }
 
-// i_H_j_mono_spin, slater_rules.irp.f:2989-3006 (ki, kj: (nint,2))
+// i_H_j_mono_spin, slater_rules.irp.f:2989-3006 (ki, kj: (nint,2), E = det_parity of ki)
 template <int NINT>
-__device__ __forceinline__ double h_mono_spin(const DevTables& t, const u64* ki, const u64* kj, int spin,
-                                              int* exc4, int* neg_out) {
+__device__ __forceinline__ double h_mono_spin(const DevTables& t, const u64* ki, const u64* kj, const u64* E,
+                                              int spin, int* exc4, int* neg_out) {
   int h, p;
-  int neg = mono_exc_spin<NINT>(ki + (spin - 1) * NINT, kj + (spin - 1) * NINT, &h, &p);
+  u64 si[NINT], sj[NINT], Es[NINT];
+#pragma unroll
+  for (int w = 0; w < NINT; ++w) {
+    si[w] = spin == 1 ? ki[w] : ki[NINT + w];
+    sj[w] = spin == 1 ? kj[w] : kj[NINT + w];
+    Es[w] = spin == 1 ? E[w] : E[NINT + w];
+  }
+  int neg = mono_exc_spin<NINT>(si, sj, Es, &h, &p);
   if (exc4) { exc4[0] = h; exc4[1] = p; exc4[2] = 0; exc4[3] = 0; }
   if (neg_out) *neg_out = neg;
   return mono_from_fock<NINT>(t, ki, h, p, spin, neg);

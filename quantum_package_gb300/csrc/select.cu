@@ -264,9 +264,9 @@ __global__ void __launch_bounds__(SBLK) k_sel_fock(DevTables t, const u64* dets,
   }
 }
 
-// <a|H|D>, generic path (degree from the words; a is the first determinant)
+// <a|H|D>, generic path (degree from the words; a is the first determinant, E = det_parity of a)
 template <int NINT>
-__device__ __forceinline__ double ihj(const DevTables& t, const u64* a, const u64* D) {
+__device__ __forceinline__ double ihj(const DevTables& t, const u64* a, const u64* D, const u64* E) {
   int da = 0, db = 0;
 #pragma unroll
   for (int w = 0; w < NINT; ++w) {
@@ -274,20 +274,24 @@ __device__ __forceinline__ double ihj(const DevTables& t, const u64* a, const u6
     db += popc64(a[NINT + w] ^ D[NINT + w]);
   }
   if (da + db == 4) {
-    if (da == 4) return h_double_spin<NINT>(t, a, D, nullptr, nullptr);
-    if (db == 4) return h_double_spin<NINT>(t, a + NINT, D + NINT, nullptr, nullptr);
+    if (da == 4) return h_double_spin<NINT>(t, a, D, E, nullptr, nullptr);
+    if (db == 4) return h_double_spin<NINT>(t, a + NINT, D + NINT, E + NINT, nullptr, nullptr);
     double s2;
-    return h_double_ab<NINT>(t, a, D, &s2, nullptr, nullptr);
+    return h_double_ab<NINT>(t, a, D, E, &s2, nullptr, nullptr);
   }
-  if (da + db == 2) return h_mono_spin<NINT>(t, a, D, da == 2 ? 1 : 2, nullptr, nullptr);
+  if (da + db == 2) return h_mono_spin<NINT>(t, a, D, E, da == 2 ? 1 : 2, nullptr, nullptr);
   if (da + db == 0) return diag_h<NINT>(t, a);
   return 0.0;
 }
 
-__device__ __forceinline__ void set_orb(u64* d, int nint, int spin, int orb, bool on) {
+// every word is written, so the determinant stays in registers
+template <int NINT>
+__device__ __forceinline__ void set_orb(u64* d, int spin, int orb, bool on) {
   const u64 b = 1ull << ((orb - 1) & 63);
-  u64& w = d[spin * nint + ((orb - 1) >> 6)];
-  w = on ? (w | b) : (w & ~b);
+  const int at = spin * NINT + ((orb - 1) >> 6);
+#pragma unroll
+  for (int w = 0; w < 2 * NINT; ++w)
+    if (w == at) d[w] = on ? (d[w] | b) : (d[w] & ~b);
 }
 
 // triangular entry e -> (i1 < i2)
@@ -320,13 +324,13 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
 #pragma unroll
   for (int w = 0; w < 2 * NINT; ++w) mask[w] = gd[w];
   if (it.kind == IT_SINGLE) {
-    set_orb(mask, NINT, it.spin, it.h1, false);
+    set_orb<NINT>(mask, it.spin, it.h1, false);
   } else if (it.kind == IT_SAME) {
-    set_orb(mask, NINT, it.spin, it.h1, false);
-    set_orb(mask, NINT, it.spin, it.h2, false);
+    set_orb<NINT>(mask, it.spin, it.h1, false);
+    set_orb<NINT>(mask, it.spin, it.h2, false);
   } else {
-    set_orb(mask, NINT, 0, it.h1, false);
-    set_orb(mask, NINT, 1, it.h2, false);
+    set_orb<NINT>(mask, 0, it.h1, false);
+    set_orb<NINT>(mask, 1, it.h2, false);
   }
   if (tid < 2) {
     int c = 0;
@@ -449,8 +453,10 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
       u64 a[2 * NINT];
 #pragma unroll
       for (int w = 0; w < 2 * NINT; ++w) a[w] = mask[w];
-      set_orb(a, NINT, sp1, vir[sp1][v1], true);
-      if (two) set_orb(a, NINT, sp2, vir[sp2][v2], true);
+      set_orb<NINT>(a, sp1, vir[sp1][v1], true);
+      if (two) set_orb<NINT>(a, sp2, vir[sp2][v2], true);
+      u64 E[2 * NINT];
+      det_parity<NINT>(a, E);
       double* m = tile + (size_t)e * nst;
       double m0 = m[0];
       int w = -1;
@@ -466,7 +472,7 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
         u64 Dw[2 * NINT];
 #pragma unroll
         for (int x = 0; x < 2 * NINT; ++x) Dw[x] = sdet[j][x];
-        const double h = ihj<NINT>(A.t, a, Dw);
+        const double h = ihj<NINT>(A.t, a, Dw, E);
         const double* cD = A.coef + (int64_t)sidx[j] * nst;
         m0 = fma(__ldg(&cD[0]), h, m0);
         for (int s = 1; s < nst; ++s) m[s] = fma(__ldg(&cD[s]), h, m[s]);
@@ -494,8 +500,8 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
     u64 a[2 * NINT];
 #pragma unroll
     for (int w = 0; w < 2 * NINT; ++w) a[w] = mask[w];
-    set_orb(a, NINT, sp1, p1, true);
-    if (two) set_orb(a, NINT, sp2, p2, true);
+    set_orb<NINT>(a, sp1, p1, true);
+    if (two) set_orb<NINT>(a, sp2, p2, true);
     bool banned = in_wf<NINT>(A, a);
     if (nfg <= SEL_MAXFG) {
       for (int f = 0; f < nfg && !banned; ++f) banned = exc_deg<NINT>(a, A.dets + (int64_t)fgen[f] * 2 * NINT) <= 2;
