@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "qpgpu_internal.cuh"
@@ -491,11 +492,15 @@ __global__ void k_bcopy_block(const BProb* __restrict__ probs, int nsd, const in
 constexpr int SMALL = 8 * BMAXM * BMAXS;  // doubles of per-problem small storage
 constexpr int O_H = 0, O_S = 512, O_G = 1024, O_RI = 1536, O_Y = 2048, O_G0 = 2560, O_SKIP = 3072;
 
-template <class T>
-void bfree(T*& p) {
-  if (p) cudaFree(p);
-  p = nullptr;
-}
+struct GraphCache {
+  std::vector<cudaGraphExec_t> g;
+  void clear() {
+    for (auto e : g)
+      if (e) cudaGraphExecDestroy(e);
+    g.clear();
+  }
+  ~GraphCache() { clear(); }
+};
 
 }  // namespace
 
@@ -510,6 +515,14 @@ struct qpgpu_batch {
   unsigned long long* d_counter = nullptr;
   int sm_count = 0;  // multiprocessors of the problems' device (set at create)
   int tuned_warps = 0, tuned_bps = 0;  // launch shape of the persistent sigma
+  // Davidson storage of all problems (one allocation) and the graphs that
+  // refer to it, kept for the next call with the same block shape: 117
+  // cudaMalloc / cudaFree pairs and 14 graph instantiations took 5 of the
+  // 35 ms of a 16-problem call
+  char* slab = nullptr;
+  size_t slab_bytes = 0;
+  int slab_nsd = 0, slab_itermax = 0;
+  GraphCache ga, gb;
   double tune_ms = 0.0;
 };
 
@@ -560,15 +573,6 @@ struct BDav {
   BStepPar* step = nullptr;
   int* mper = nullptr;      // [np] basis size of each problem's last Ritz step
   int* copyf = nullptr;     // [np] re-contract flags
-  std::vector<void*> owned;
-  ~BDav() {
-    bfree(part);
-    bfree(small);
-    bfree(step);
-    bfree(mper);
-    bfree(copyf);
-    for (void* p : owned) cudaFree(p);
-  }
 };
 
 void bgram(BDav& D, int asel, int a0, int nbA, int bsel, int bb, int out_off, const int* skip) {
@@ -640,14 +644,6 @@ void segment_b(BDav& D, int b, double sz2sz, int64_t maxN) {
   blin(D, L, 0, (b + 1) * nsd, nullptr, O_Y, 0, nullptr, 0, maxN);
   k_bstep<<<dim3(D.ncta_max, B->np), BBLK, 0, B->st>>>(B->d, D.step, nsd, b + 1, sz2sz, D.part, D.ncta_max);
 }
-
-struct GraphCache {
-  std::vector<cudaGraphExec_t> g;
-  ~GraphCache() {
-    for (auto e : g)
-      if (e) cudaGraphExecDestroy(e);
-  }
-};
 
 // capture `fn` on the batch stream once and replay it afterwards
 template <class F>
@@ -722,6 +718,9 @@ int qpgpu_batch_create(qpgpu_ctx* const* ctxs, int n, qpgpu_batch** out) {
 int qpgpu_batch_destroy(qpgpu_batch* B) {
   if (!B) return QPGPU_ERR_ARG;
   cudaStreamSynchronize(B->st);
+  B->ga.clear();
+  B->gb.clear();
+  cudaFree(B->slab);
   cudaFree(B->d);
   cudaFree(B->d_counter);
   cudaStreamDestroy(B->st);
@@ -763,37 +762,53 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
   D.itermax = itermax;
   D.ncta_max = 1;
   for (auto& p : B->h) D.ncta_max = std::max(D.ncta_max, p.ncta);
-  // per-problem Davidson storage
-  for (int p = 0; p < np; ++p) {
-    BProb& P = B->h[p];
-    const size_t blk = (size_t)P.N * nsd;
-    double *U, *W, *S, *R, *pv, *ps;
-    float* u32;
-    if (cudaMalloc((void**)&U, blk * itermax * 8) != cudaSuccess ||
-        cudaMalloc((void**)&W, blk * itermax * 8) != cudaSuccess ||
-        cudaMalloc((void**)&S, blk * itermax * 8) != cudaSuccess || cudaMalloc((void**)&R, blk * 8) != cudaSuccess ||
-        cudaMalloc((void**)&u32, blk * 4 + 16) != cudaSuccess ||
-        cudaMalloc((void**)&pv, (size_t)P.n_items * nsd * 8 + 16) != cudaSuccess ||
-        cudaMalloc((void**)&ps, (size_t)P.n_items * nsd * 8 + 16) != cudaSuccess) {
-      cudaGetLastError();
-      return bfail(B, QPGPU_ERR_NOMEM, "batch Davidson storage does not fit on the device");
-    }
-    for (void* x : {(void*)U, (void*)W, (void*)S, (void*)R, (void*)u32, (void*)pv, (void*)ps}) D.owned.push_back(x);
-    P.U = U;
-    P.W = W;
-    P.S = S;
-    P.R = R;
-    P.u32 = u32;
-    P.pv = pv;
-    P.ps = ps;
-    P.nst = n_states[p];
-    P.active = 1;
+  // Davidson storage of the problems: pieces of one allocation (256-byte
+  // aligned), sized in a first pass and handed out in a second
+  if (B->slab_nsd != nsd || B->slab_itermax != itermax) {
+    B->ga.clear();
+    B->gb.clear();
   }
-  QB_CUDA(B, cudaMalloc((void**)&D.part, (size_t)np * D.ncta_max * 512 * 8));
-  QB_CUDA(B, cudaMalloc((void**)&D.small, (size_t)np * SMALL * 8));
-  QB_CUDA(B, cudaMalloc((void**)&D.step, (size_t)np * sizeof(BStepPar)));
-  QB_CUDA(B, cudaMalloc((void**)&D.mper, (size_t)np * sizeof(int)));
-  QB_CUDA(B, cudaMalloc((void**)&D.copyf, (size_t)np * sizeof(int)));
+  for (int pass = 0; pass < 2; ++pass) {
+    size_t off = 0;
+    auto take = [&](auto*& p, size_t bytes) {
+      p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(reinterpret_cast<uintptr_t>(B->slab) + off);
+      off += (bytes + 255) & ~(size_t)255;
+    };
+    for (int p = 0; p < np; ++p) {
+      BProb& P = B->h[p];
+      const size_t blk = (size_t)P.N * nsd;
+      take(P.U, blk * itermax * 8);
+      take(P.W, blk * itermax * 8);
+      take(P.S, blk * itermax * 8);
+      take(P.R, blk * 8);
+      take(P.u32, blk * 4 + 16);
+      take(P.pv, (size_t)P.n_items * nsd * 8 + 16);
+      take(P.ps, (size_t)P.n_items * nsd * 8 + 16);
+      P.nst = n_states[p];
+      P.active = 1;
+    }
+    take(D.part, (size_t)np * D.ncta_max * 512 * 8);
+    take(D.small, (size_t)np * SMALL * 8);
+    take(D.step, (size_t)np * sizeof(BStepPar));
+    take(D.mper, (size_t)np * sizeof(int));
+    take(D.copyf, (size_t)np * sizeof(int));
+    if (pass == 0 && B->slab_bytes < off) {
+      B->ga.clear();
+      B->gb.clear();
+      cudaFree(B->slab);
+      B->slab = nullptr;
+      B->slab_bytes = 0;
+      if (cudaMalloc((void**)&B->slab, off) != cudaSuccess) {
+        cudaGetLastError();
+        return bfail(B, QPGPU_ERR_NOMEM, "batch Davidson storage does not fit on the device");
+      }
+      B->slab_bytes = off;
+    }
+  }
+  B->slab_nsd = nsd;
+  B->slab_itermax = itermax;
+  B->ga.g.resize(2 * itermax, nullptr);
+  B->gb.g.resize(itermax, nullptr);
   QB_CUDA(B, cudaMemsetAsync(D.small, 0, (size_t)np * SMALL * 8, st));
   QB_CUDA(B, cudaMemcpyAsync(B->d, B->h.data(), np * sizeof(BProb), cudaMemcpyHostToDevice, st));
   // guesses -> block 0 (bilinear order)
@@ -847,9 +862,6 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
   std::vector<std::vector<double>> lam(np, std::vector<double>(mmax)), s2v = lam;
   std::vector<int> mper(np, 0), copyf(np, 0), conv(np, 0), iters(np, 0);
   std::vector<double> res((size_t)np * BMAXS, 0.0);
-  GraphCache ga, gb;
-  ga.g.assign(2 * itermax, nullptr);
-  gb.g.assign(itermax, nullptr);
   cudaEvent_t t_start, t_end;
   cudaEventCreate(&t_start);
   cudaEventCreate(&t_end);
@@ -862,7 +874,7 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
       const int b = iter - 1;
       shift2 = nsd * iter;
       const int prec = (mixed && iter > 1) ? QPGPU_FP32 : QPGPU_FP64;
-      int rc = replay(B, ga.g[2 * b + (prec == QPGPU_FP32)], [&] { segment_a(D, b, prec, maxN); });
+      int rc = replay(B, B->ga.g[2 * b + (prec == QPGPU_FP32)], [&] { segment_a(D, b, prec, maxN); });
       if (rc) return rc;
       ++launches;
       ++n_iter;
@@ -926,7 +938,7 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
       QB_CUDA(B, cudaMemcpy2DAsync(D.small + O_Y, SMALL * 8, ystage.data(), 512 * 8, 512 * 8, np,
                                    cudaMemcpyHostToDevice, st));
       QB_CUDA(B, cudaMemcpyAsync(D.step, sp.data(), np * sizeof(BStepPar), cudaMemcpyHostToDevice, st));
-      rc = replay(B, gb.g[b], [&] { segment_b(D, b, sz2sz[0], maxN); });
+      rc = replay(B, B->gb.g[b], [&] { segment_b(D, b, sz2sz[0], maxN); });
       if (rc) return rc;
       QB_CUDA(B, cudaMemcpyAsync(parts.data(), D.part, parts.size() * 8, cudaMemcpyDeviceToHost, st));
       QB_CUDA(B, cudaStreamSynchronize(st));

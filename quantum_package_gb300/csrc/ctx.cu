@@ -185,6 +185,44 @@ int ensure_work(qpgpu_ctx* c, size_t bytes) {
 
 }  // namespace
 
+cudaError_t qp_pool_alloc(qpgpu_ctx* c, void** p, size_t bytes) {
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+  if (e != cudaSuccess) {  // cached blocks may hold the memory that is missing
+    cudaGetLastError();
+    cudaStreamSynchronize(c->stream);
+    cudaMemPoolTrimTo(c->pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+  }
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
+
+void qp_pool_free(qpgpu_ctx* c, void* p) {
+  if (p) cudaFreeAsync(p, c->stream);
+}
+
+void qp_pool_idle(qpgpu_ctx* c) {
+  int cur = -1;
+  if (cudaGetDevice(&cur) == cudaSuccess && cur != c->device) cudaSetDevice(c->device);
+  cudaDeviceSynchronize();
+  if (cur >= 0 && cur != c->device) cudaSetDevice(cur);
+}
+
+size_t qp_pool_cached(qpgpu_ctx* c) {
+  uint64_t used = 0, reserved = 0;
+  if (cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
+      cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess)
+    return 0;
+  return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
+void qp_pool_trim(qpgpu_ctx* c) {
+  uint64_t used = 0;
+  if (cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return;
+  const uint64_t spare = std::max<uint64_t>(used / 2, 64ull << 20);
+  if (qp_pool_cached(c) > spare) cudaMemPoolTrimTo(c->pool, (size_t)(used + spare));
+}
+
 void qp_report_marks(qpgpu_ctx* c) {
   if (!c->profile || c->marks.size() < 2) return;
   cudaEventSynchronize(c->marks.back().second);
@@ -242,6 +280,21 @@ int qpgpu_create(int n_mo, int n_alpha, int n_beta, int n_int, qpgpu_ctx** out) 
     delete c;
     return QPGPU_ERR_CUDA;
   }
+  {
+    cudaMemPoolProps pp{};
+    pp.allocType = cudaMemAllocationTypePinned;
+    pp.location.type = cudaMemLocationTypeDevice;
+    pp.location.id = c->device;
+    uint64_t keep = UINT64_MAX;  // qp_pool_trim decides what goes back, not every synchronisation
+    if (cudaMemPoolCreate(&c->pool, &pp) != cudaSuccess ||
+        cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaGetLastError();
+      if (c->pool) cudaMemPoolDestroy(c->pool);
+      cudaStreamDestroy(c->stream);
+      delete c;
+      return QPGPU_ERR_CUDA;
+    }
+  }
   *out = c;
   return QPGPU_OK;
 }
@@ -250,8 +303,8 @@ int qpgpu_destroy(qpgpu_ctx* c) {
   if (!c) return QPGPU_ERR_ARG;
   {
     Lock l(c->mu);
-    cudaStreamSynchronize(c->stream);
-    c->items.free_all();
+    qp_pool_idle(c);
+    c->items.free_all(c);
     qp_free_dressing(c);
     qp_free_pairs(c);
     qp_free_dets(c);
@@ -263,6 +316,8 @@ int qpgpu_destroy(qpgpu_ctx* c) {
     dev_free(c->d_direct_ut);
     dev_free(c->d_flag);
     dev_free(c->d_tc_scratch);
+    cudaStreamSynchronize(c->stream);
+    cudaMemPoolDestroy(c->pool);
     cudaStreamDestroy(c->stream);
   }
   delete c;
@@ -325,7 +380,8 @@ int qpgpu_set_integrals(qpgpu_ctx* c, const double* h, const double* eri) {
     for (int j = 0; j < i; ++j)
       if (h[i + (size_t)j * n] != h[j + (size_t)i * n])
         return qpgpu_fail(c, QPGPU_ERR_ARG, "h_pq must be symmetric");
-  c->items.free_all();
+  qp_pool_idle(c);
+  c->items.free_all(c);
   qp_free_dressing(c);
   qp_free_pairs(c);
   qp_free_dets(c);
@@ -397,7 +453,9 @@ int qpgpu_set_dets(qpgpu_ctx* c, const uint64_t* psi_det, int64_t n_det) {
         return qpgpu_fail(c, QPGPU_ERR_ARG, "determinant " + std::to_string(k) + " has a wrong electron count");
     }
   }
-  c->items.free_all();
+  qp_pool_idle(c);
+  PoolTrim trim{c};
+  c->items.free_all(c);
   qp_free_dressing(c);
   qp_free_pairs(c);
   qp_free_dets(c);
@@ -405,7 +463,7 @@ int qpgpu_set_dets(qpgpu_ctx* c, const uint64_t* psi_det, int64_t n_det) {
   cudaEvent_t e0, e1;
   QP_CUDA(c, cudaEventCreate(&e0));
   QP_CUDA(c, cudaEventCreate(&e1));
-  QP_CUDA(c, dev_alloc(&c->d_dets, (size_t)n_det * 2 * nint));
+  QP_CUDA(c, pool_alloc(c, &c->d_dets, (size_t)n_det * 2 * nint));
   QP_CUDA(c, cudaMemcpyAsync(c->d_dets, psi_det, (size_t)n_det * 2 * nint * 8, cudaMemcpyHostToDevice, st));
   QP_CUDA(c, cudaEventRecord(e0, st));
   qp_mark(c, "start");
@@ -426,7 +484,7 @@ int qpgpu_set_dets(qpgpu_ctx* c, const uint64_t* psi_det, int64_t n_det) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) {
-    c->items.free_all();
+    c->items.free_all(c);
     qp_free_pairs(c);
     qp_free_dets(c);
     return rc;
@@ -584,6 +642,7 @@ int qpgpu_u0_h_u0(qpgpu_ctx* c, double* e_0, const double* u0, int n_st, int64_t
   const int64_t N = c->N;
   const size_t cols = (size_t)N * n_st;
   Lock l(c->mu);
+  PoolTrim trim{c};
   if (c->stage_bytes < 3 * cols * sizeof(double)) {
     dev_free(c->d_stage);
     c->d_stage = nullptr;
@@ -595,7 +654,7 @@ int qpgpu_u0_h_u0(qpgpu_ctx* c, double* e_0, const double* u0, int n_st, int64_t
   cudaStream_t st = c->stream;
   const int grid = dot_grid(c);
   double* dpart = nullptr;
-  QP_CUDA(c, cudaMalloc((void**)&dpart, (size_t)grid * n_st * 2 * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, (void**)&dpart, (size_t)grid * n_st * 2 * sizeof(double)));
   std::vector<double> part((size_t)grid * n_st * 2);
   int* bad = nullptr;
   int hbad = 0;
@@ -612,7 +671,7 @@ int qpgpu_u0_h_u0(qpgpu_ctx* c, double* e_0, const double* u0, int n_st, int64_t
       rc = qpgpu_fail(c, QPGPU_ERR_CUDA, "copy of the dot products failed");
   }
   const cudaError_t e = cudaStreamSynchronize(st);
-  cudaFree(dpart);
+  qp_pool_free(c, dpart);
   if (!rc && e != cudaSuccess) rc = qpgpu_fail(c, QPGPU_ERR_CUDA, cudaGetErrorString(e));
   if (!rc && hbad) rc = qpgpu_fail(c, QPGPU_ERR_NUMERIC, "u_0 holds a NaN or an infinity");
   if (rc) return rc;
@@ -634,10 +693,11 @@ int qpgpu_h_s2_u0_work(qpgpu_ctx* c, double* v_t, double* s_t, const double* u_t
   if (!v_t || !s_t || !u_t || n_st < 1 || n_st > 8 || istart < 1 || iend > c->N || istep < 1 || ishift < 0)
     return qpgpu_fail(c, QPGPU_ERR_ARG, "bad h_s2_u0_work arguments");
   Lock l(c->mu);
+  PoolTrim trim{c};
   const int64_t N = c->N;
   const size_t cnt = (size_t)N * n_st;
   double* buf = nullptr;
-  QP_CUDA(c, cudaMalloc((void**)&buf, 3 * cnt * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, (void**)&buf, 3 * cnt * sizeof(double)));
   cudaStream_t st = c->stream;
   std::vector<double> hv(cnt), hs(cnt);
   rc = 0;
@@ -656,7 +716,7 @@ int qpgpu_h_s2_u0_work(qpgpu_ctx* c, double* v_t, double* s_t, const double* u_t
               cudaMemcpyAsync(hs.data(), buf + 2 * cnt, cnt * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess))
     rc = qpgpu_fail(c, QPGPU_ERR_CUDA, "copy of v_t/s_t failed");
   cudaError_t e = cudaStreamSynchronize(st);
-  cudaFree(buf);
+  qp_pool_free(c, buf);
   if (!rc && e != cudaSuccess) rc = qpgpu_fail(c, QPGPU_ERR_CUDA, cudaGetErrorString(e));
   if (!rc && hbad) rc = qpgpu_fail(c, QPGPU_ERR_NUMERIC, "u_t holds a NaN or an infinity");
   if (rc) return rc;
@@ -682,9 +742,10 @@ int qpgpu_diag(qpgpu_ctx* c, double* h_jj, double* s_jj) {
   int rc = check_ctx(c, true, true);
   if (rc) return rc;
   Lock l(c->mu);
+  PoolTrim trim{c};
   const int64_t N = c->N;
   double* buf = nullptr;
-  QP_CUDA(c, cudaMalloc((void**)&buf, 2 * N * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, (void**)&buf, 2 * N * sizeof(double)));
   cudaStream_t st = c->stream;
   qp_from_bilinear(c->d_hdiag, N, c->d_order, buf, 1, N, st);
   qp_from_bilinear(c->d_sdiag, N, c->d_order, buf + N, 1, N, st);
@@ -692,7 +753,7 @@ int qpgpu_diag(qpgpu_ctx* c, double* h_jj, double* s_jj) {
   if (h_jj && cudaMemcpyAsync(h_jj, buf, N * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -1;
   if (s_jj && cudaMemcpyAsync(s_jj, buf + N, N * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -1;
   cudaError_t e = cudaStreamSynchronize(st);
-  cudaFree(buf);
+  qp_pool_free(c, buf);
   if (rc || e != cudaSuccess) return qpgpu_fail(c, QPGPU_ERR_CUDA, "diag copy failed");
   return QPGPU_OK;
 }
@@ -703,6 +764,7 @@ int qpgpu_connected_pairs(qpgpu_ctx* c, int64_t* n_pairs, int32_t* I, int32_t* J
   if (rc) return rc;
   if (!n_pairs) return QPGPU_ERR_ARG;
   Lock l(c->mu);
+  PoolTrim trim{c};
   if (c->direct) return qpgpu_fail(c, QPGPU_ERR_STATE, "pairs are not stored (direct sigma)");
   *n_pairs = c->P;
   if (cap <= 0) return QPGPU_OK;
@@ -711,7 +773,7 @@ int qpgpu_connected_pairs(qpgpu_ctx* c, int64_t* n_pairs, int32_t* I, int32_t* J
   const int64_t P = c->P;
   char* buf = nullptr;
   const size_t bytes = P * (4 + 4 + 1 + 1 + 8 + 8) + 64;
-  QP_CUDA(c, cudaMalloc((void**)&buf, bytes));
+  QP_CUDA(c, qp_pool_alloc(c, (void**)&buf, bytes));
   int32_t* dI = (int32_t*)buf;
   int32_t* dJ = dI + P;
   double* dh = (double*)(((uintptr_t)(dJ + P) + 15) & ~(uintptr_t)15);
@@ -734,7 +796,7 @@ int qpgpu_connected_pairs(qpgpu_ctx* c, int64_t* n_pairs, int32_t* I, int32_t* J
       cudaMemcpyAsync(phase, dp, P, cudaMemcpyDeviceToHost, st) != cudaSuccess)
     rc = -1;
   cudaError_t e = cudaStreamSynchronize(st);
-  cudaFree(buf);
+  qp_pool_free(c, buf);
   if (rc || e != cudaSuccess) return qpgpu_fail(c, QPGPU_ERR_CUDA, "connected_pairs copy failed");
   return QPGPU_OK;
 }
@@ -745,6 +807,7 @@ int qpgpu_connected_pairs_rows(qpgpu_ctx* c, const int32_t* rows, int64_t n_rows
   if (rc) return rc;
   if (!n_pairs || n_rows < 0 || (n_rows > 0 && !rows)) return qpgpu_fail(c, QPGPU_ERR_ARG, "bad row list");
   Lock l(c->mu);
+  PoolTrim trim{c};
   if (c->direct) return qpgpu_fail(c, QPGPU_ERR_STATE, "pairs are not stored (direct sigma)");
   const int64_t N = c->N;
   for (int64_t i = 0; i < n_rows; ++i)
@@ -770,7 +833,7 @@ int qpgpu_connected_pairs_rows(qpgpu_ctx* c, const int32_t* rows, int64_t n_rows
     return qpgpu_fail(c, QPGPU_ERR_ARG, "connected_pairs_rows: cap below n_pairs or null output");
   char* buf = nullptr;
   const size_t bytes = P * (4 + 4 + 1 + 1 + 8 + 8) + sel.size() * (4 + 8) + 128;
-  QP_CUDA(c, cudaMalloc((void**)&buf, bytes));
+  QP_CUDA(c, qp_pool_alloc(c, (void**)&buf, bytes));
   double* dh = (double*)buf;
   int64_t* dbeg = (int64_t*)(dh + P);
   int32_t* dI = (int32_t*)(dbeg + sel.size());
@@ -802,7 +865,7 @@ int qpgpu_connected_pairs_rows(qpgpu_ctx* c, const int32_t* rows, int64_t n_rows
               cudaMemcpyAsync(phase, dp, P, cudaMemcpyDeviceToHost, st) != cudaSuccess))
     rc = -1;
   cudaError_t e = cudaStreamSynchronize(st);
-  cudaFree(buf);
+  qp_pool_free(c, buf);
   if (rc || e != cudaSuccess) return qpgpu_fail(c, QPGPU_ERR_CUDA, "connected_pairs_rows export failed");
   return QPGPU_OK;
 }

@@ -1002,22 +1002,22 @@ struct Dav {
   int* uexp = nullptr;  // [MAXM]
   int* bexp = nullptr;  // [2 MAXS + 1]: B exponents, then the status flag
   ~Dav() {
-    dev_free(U);
-    dev_free(W);
-    dev_free(S);
-    dev_free(R);
-    dev_free(u32);
-    dev_free(part);
-    dev_free(small);
+    qp_pool_free(c, U);
+    qp_pool_free(c, W);
+    qp_pool_free(c, S);
+    qp_pool_free(c, R);
+    qp_pool_free(c, u32);
+    qp_pool_free(c, part);
+    qp_pool_free(c, small);
     dev_free(cX);
     dev_free(cd);
     dev_free(cc);
-    dev_free(mlpX);
-    dev_free(mlpG);
-    dev_free(Uf);
-    dev_free(Bf);
-    dev_free(uexp);
-    dev_free(bexp);
+    qp_pool_free(c, mlpX);
+    qp_pool_free(c, mlpG);
+    qp_pool_free(c, Uf);
+    qp_pool_free(c, Bf);
+    qp_pool_free(c, uexp);
+    qp_pool_free(c, bexp);
   }
   double* blk(double* X, int b) const { return X + (int64_t)b * N * nsd; }
 };
@@ -1389,6 +1389,7 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
   const int max_sigma = prm->max_iter > 0 ? prm->max_iter : 1000;
 
   std::lock_guard<std::mutex> lk(c->mu);
+  PoolTrim trim{c};
   Dav d;
   d.c = c;
   d.st = c->stream;
@@ -1400,23 +1401,23 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
   d.tc = tcalg;
   d.rows_per_cta = (N + d.ncta - 1) / d.ncta;
   const size_t blkn = (size_t)N * nsd;
-  if (dev_alloc(&d.U, blkn * itermax) != cudaSuccess || dev_alloc(&d.W, blkn * itermax) != cudaSuccess ||
-      dev_alloc(&d.S, blkn * itermax) != cudaSuccess || dev_alloc(&d.R, blkn) != cudaSuccess ||
-      dev_alloc(&d.u32, (size_t)N * qp_pad_states(nsd)) != cudaSuccess || dev_alloc(&d.part, (size_t)d.ncta * MAXM * 2 * MAXS) != cudaSuccess ||
-      dev_alloc(&d.small, (size_t)SMALL_DOUBLES) != cudaSuccess) {
+  if (pool_alloc(c, &d.U, blkn * itermax) != cudaSuccess || pool_alloc(c, &d.W, blkn * itermax) != cudaSuccess ||
+      pool_alloc(c, &d.S, blkn * itermax) != cudaSuccess || pool_alloc(c, &d.R, blkn) != cudaSuccess ||
+      pool_alloc(c, &d.u32, (size_t)N * qp_pad_states(nsd)) != cudaSuccess || pool_alloc(c, &d.part, (size_t)d.ncta * MAXM * 2 * MAXS) != cudaSuccess ||
+      pool_alloc(c, &d.small, (size_t)SMALL_DOUBLES) != cudaSuccess) {
     cudaGetLastError();
     return qpgpu_fail(c, QPGPU_ERR_NOMEM, "Davidson work arrays do not fit on the device");
   }
   if (tcalg) {
-    if (qp_gram_oz_prepare() || dev_alloc(&d.uexp, MAXM) != cudaSuccess ||
-        dev_alloc(&d.bexp, 2 * MAXS + 1) != cudaSuccess) {
+    if (qp_gram_oz_prepare() || pool_alloc(c, &d.uexp, MAXM) != cudaSuccess ||
+        pool_alloc(c, &d.bexp, 2 * MAXS + 1) != cudaSuccess) {
       cudaGetLastError();
       return qpgpu_fail(c, QPGPU_ERR_NOMEM, "tensor-core Gram work arrays could not be set up");
     }
     QP_CUDA(c, cudaMemsetAsync(d.bexp, 0, (2 * MAXS + 1) * sizeof(int), d.st));
   }
   d.sUf = (int64_t)blkn;
-  if (ffalg && (dev_alloc(&d.Uf, blkn * itermax) != cudaSuccess || dev_alloc(&d.Bf, blkn * 2) != cudaSuccess)) {
+  if (ffalg && (pool_alloc(c, &d.Uf, blkn * itermax) != cudaSuccess || pool_alloc(c, &d.Bf, blkn * 2) != cudaSuccess)) {
     cudaGetLastError();
     return qpgpu_fail(c, QPGPU_ERR_NOMEM, "mixed-precision work arrays do not fit on the device");
   }
@@ -1432,8 +1433,8 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
   // extra mode: state k's learned correction uses the slot of Ritz vector nst + k
   const int mlp_extra = prm->preconditioner == 2;
   for (int k = 0; k < nst; ++k) mlp_on[k] = use_mlp && (!mlp_extra || nst + k < nsd);
-  if (use_mlp && (dev_alloc(&d.mlpX, (size_t)N * nst * QP_MLP_IN) != cudaSuccess ||
-                  dev_alloc(&d.mlpG, (size_t)N * nst) != cudaSuccess)) {
+  if (use_mlp && (pool_alloc(c, &d.mlpX, (size_t)N * nst * QP_MLP_IN) != cudaSuccess ||
+                  pool_alloc(c, &d.mlpG, (size_t)N * nst) != cudaSuccess)) {
     cudaGetLastError();
     return qpgpu_fail(c, QPGPU_ERR_NOMEM, "learned-step work arrays do not fit on the device");
   }
@@ -1459,7 +1460,7 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
   // guess vectors: u_in(dim_in, nsd) in psi_det order -> block 0, bilinear
   {
     double* hstage = nullptr;
-    QP_CUDA(c, cudaMalloc((void**)&hstage, blkn * sizeof(double)));
+    QP_CUDA(c, qp_pool_alloc(c, (void**)&hstage, blkn * sizeof(double)));
     QP_CUDA(c, cudaMemcpy2DAsync(hstage, N * sizeof(double), u_in, dim_in * sizeof(double), N * sizeof(double), nsd,
                                  cudaMemcpyHostToDevice, st));
     int* bad = nullptr;
@@ -1469,7 +1470,7 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
     qp_to_bilinear(hstage, N, c->d_order, d.U, nullptr, nsd, N, st, bad);
     QP_CUDA(c, cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
     QP_CUDA(c, cudaStreamSynchronize(st));
-    cudaFree(hstage);
+    qp_pool_free(c, hstage);
     if (hbad) {
       cudaEventDestroy(ev0);
       return qpgpu_fail(c, QPGPU_ERR_NUMERIC, "the guess vectors hold a NaN or an infinity");
@@ -1781,12 +1782,12 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
   // final vectors (block 0 after re-contraction) back to psi_det order
   {
     double* hstage = nullptr;
-    QP_CUDA(c, cudaMalloc((void**)&hstage, blkn * sizeof(double)));
+    QP_CUDA(c, qp_pool_alloc(c, (void**)&hstage, blkn * sizeof(double)));
     qp_from_bilinear(d.U, N, c->d_order, hstage, nsd, N, st);
     QP_CUDA(c, cudaMemcpy2DAsync(u_in, dim_in * sizeof(double), hstage, N * sizeof(double), N * sizeof(double), nsd,
                                  cudaMemcpyDeviceToHost, st));
     QP_CUDA(c, cudaStreamSynchronize(st));
-    cudaFree(hstage);
+    qp_pool_free(c, hstage);
   }
   for (int k = 0; k < nsd; ++k) {
     energies[k] = lambda[k];

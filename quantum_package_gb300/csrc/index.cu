@@ -31,12 +31,6 @@ inline unsigned grid_for(int64_t n, int tpb = TPB) {
   return (unsigned)g;
 }
 
-template <class T>
-struct Scoped {
-  T* p = nullptr;
-  ~Scoped() { dev_free(p); }
-};
-
 __global__ void k_iota(int* a, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     a[i] = (int)i;
@@ -225,16 +219,16 @@ __global__ void k_single_costs(const int* ptr, const int* idx, const int* loc, c
 template <class WordFn>
 int sort_multiword(qpgpu_ctx* c, int64_t n, int nwords, WordFn word_fn, int* perm_out) {
   cudaStream_t st = c->stream;
-  Scoped<u64> ka, kb;
-  Scoped<int> pa, pb;
-  Scoped<char> tmp;
-  QP_CUDA(c, dev_alloc(&ka.p, n));
-  QP_CUDA(c, dev_alloc(&kb.p, n));
-  QP_CUDA(c, dev_alloc(&pa.p, n));
-  QP_CUDA(c, dev_alloc(&pb.p, n));
+  Scoped<u64> ka(c), kb(c);
+  Scoped<int> pa(c), pb(c);
+  Scoped<char> tmp(c);
+  QP_CUDA(c, ka.alloc(n));
+  QP_CUDA(c, kb.alloc(n));
+  QP_CUDA(c, pa.alloc(n));
+  QP_CUDA(c, pb.alloc(n));
   size_t tbytes = 0;
   QP_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, tbytes, ka.p, kb.p, pa.p, pb.p, (int)n, 0, 64, st));
-  QP_CUDA(c, dev_alloc(&tmp.p, tbytes));
+  QP_CUDA(c, tmp.alloc(tbytes));
   k_iota<<<grid_for(n), TPB, 0, st>>>(pa.p, n);
   for (int w = 0; w < nwords; ++w) {
     word_fn(w, pa.p, ka.p);  // keys of the current permutation
@@ -249,10 +243,10 @@ int unique_spin(qpgpu_ctx* c, int spin, int* id_out, u64** uniq_out, int* nu_out
   const int64_t N = c->N;
   const int nint = c->nint;
   cudaStream_t st = c->stream;
-  Scoped<int> perm, flag, incl;
-  QP_CUDA(c, dev_alloc(&perm.p, N));
-  QP_CUDA(c, dev_alloc(&flag.p, N));
-  QP_CUDA(c, dev_alloc(&incl.p, N));
+  Scoped<int> perm(c), flag(c), incl(c);
+  QP_CUDA(c, perm.alloc(N));
+  QP_CUDA(c, flag.alloc(N));
+  QP_CUDA(c, incl.alloc(N));
   int rc = sort_multiword(c, N, nint, [&](int w, const int* p, u64* out) {
     k_gather_word<<<grid_for(N), TPB, 0, st>>>(c->d_dets, nint, spin, w, p, out, N);
   }, perm.p);
@@ -260,14 +254,14 @@ int unique_spin(qpgpu_ctx* c, int spin, int* id_out, u64** uniq_out, int* nu_out
   k_unique_flags<<<grid_for(N), TPB, 0, st>>>(c->d_dets, nint, spin, perm.p, flag.p, N);
   size_t tb = 0;
   QP_CUDA(c, cub::DeviceScan::InclusiveSum(nullptr, tb, flag.p, incl.p, (int)N, st));
-  Scoped<char> tmp;
-  QP_CUDA(c, dev_alloc(&tmp.p, tb));
+  Scoped<char> tmp(c);
+  QP_CUDA(c, tmp.alloc(tb));
   QP_CUDA(c, cub::DeviceScan::InclusiveSum(tmp.p, tb, flag.p, incl.p, (int)N, st));
   int nu = 0;
   QP_CUDA(c, cudaMemcpyAsync(&nu, incl.p + N - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
   u64* uniq = nullptr;
-  QP_CUDA(c, dev_alloc(&uniq, (size_t)nu * nint));
+  QP_CUDA(c, pool_alloc(c, &uniq, (size_t)nu * nint));
   k_unique_scatter<<<grid_for(N), TPB, 0, st>>>(c->d_dets, nint, spin, perm.p, incl.p, flag.p, id_out, uniq, N);
   *uniq_out = uniq;
   *nu_out = nu;
@@ -283,17 +277,17 @@ int singles_adjacency(qpgpu_ctx* c, const u64* uniq, int U, int ne, int** ptr_ou
   *idx_out = nullptr;
   *nnz = 0;
   int* ptr = nullptr;
-  QP_CUDA(c, dev_alloc(&ptr, (size_t)U + 1));
+  QP_CUDA(c, pool_alloc(c, &ptr, (size_t)U + 1));
   if (ne == 0 || m == 0) {
     QP_CUDA(c, cudaMemsetAsync(ptr, 0, sizeof(int) * ((size_t)U + 1), st));
     *ptr_out = ptr;
-    QP_CUDA(c, dev_alloc(idx_out, 1));
+    QP_CUDA(c, pool_alloc(c, idx_out, 1));
     return 0;
   }
-  Scoped<int> perm, flag, incl, rs, re;
-  QP_CUDA(c, dev_alloc(&perm.p, m));
-  QP_CUDA(c, dev_alloc(&flag.p, m));
-  QP_CUDA(c, dev_alloc(&incl.p, m));
+  Scoped<int> perm(c), flag(c), incl(c), rs(c), re(c);
+  QP_CUDA(c, perm.alloc(m));
+  QP_CUDA(c, flag.alloc(m));
+  QP_CUDA(c, incl.alloc(m));
   int rc = sort_multiword(c, m, nint, [&](int w, const int* p, u64* out) {
     k_deletion_word<<<grid_for(m), TPB, 0, st>>>(uniq, nint, ne, w, p, out, m);
   }, perm.p);
@@ -301,43 +295,43 @@ int singles_adjacency(qpgpu_ctx* c, const u64* uniq, int U, int ne, int** ptr_ou
   k_run_flags<<<grid_for(m), TPB, 0, st>>>(uniq, nint, ne, perm.p, flag.p, m);
   size_t tb = 0;
   QP_CUDA(c, cub::DeviceScan::InclusiveSum(nullptr, tb, flag.p, incl.p, (int)m, st));
-  Scoped<char> tmp;
-  QP_CUDA(c, dev_alloc(&tmp.p, tb));
+  Scoped<char> tmp(c);
+  QP_CUDA(c, tmp.alloc(tb));
   QP_CUDA(c, cub::DeviceScan::InclusiveSum(tmp.p, tb, flag.p, incl.p, (int)m, st));
   int nruns = 0;
   QP_CUDA(c, cudaMemcpyAsync(&nruns, incl.p + m - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
-  QP_CUDA(c, dev_alloc(&rs.p, nruns));
-  QP_CUDA(c, dev_alloc(&re.p, nruns));
+  QP_CUDA(c, rs.alloc(nruns));
+  QP_CUDA(c, re.alloc(nruns));
   k_run_bounds<<<grid_for(m), TPB, 0, st>>>(incl.p, rs.p, re.p, m);
-  Scoped<int64_t> cnt, off;
-  QP_CUDA(c, dev_alloc(&cnt.p, m + 1));
-  QP_CUDA(c, dev_alloc(&off.p, m + 1));
+  Scoped<int64_t> cnt(c), off(c);
+  QP_CUDA(c, cnt.alloc(m + 1));
+  QP_CUDA(c, off.alloc(m + 1));
   QP_CUDA(c, cudaMemsetAsync(cnt.p + m, 0, sizeof(int64_t), st));
   k_pair_counts<<<grid_for(m), TPB, 0, st>>>(incl.p, rs.p, re.p, cnt.p, m);
   size_t tb2 = 0;
   QP_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, tb2, cnt.p, off.p, (int)(m + 1), st));
-  Scoped<char> tmp2;
-  QP_CUDA(c, dev_alloc(&tmp2.p, tb2));
+  Scoped<char> tmp2(c);
+  QP_CUDA(c, tmp2.alloc(tb2));
   QP_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp2.p, tb2, cnt.p, off.p, (int)(m + 1), st));
   int64_t T = 0;
   QP_CUDA(c, cudaMemcpyAsync(&T, off.p + m, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
   if (T >= ((int64_t)1 << 31)) return qpgpu_fail(c, QPGPU_ERR_NOMEM, "singles adjacency too large");
   int* idx = nullptr;
-  QP_CUDA(c, dev_alloc(&idx, (size_t)(T > 0 ? T : 1)));
+  QP_CUDA(c, pool_alloc(c, &idx, (size_t)(T > 0 ? T : 1)));
   if (T > 0) {
-    Scoped<u64> k1, k2;
-    QP_CUDA(c, dev_alloc(&k1.p, T));
-    QP_CUDA(c, dev_alloc(&k2.p, T));
+    Scoped<u64> k1(c), k2(c);
+    QP_CUDA(c, k1.alloc(T));
+    QP_CUDA(c, k2.alloc(T));
     k_pair_emit<<<grid_for(m), TPB, 0, st>>>(perm.p, ne, incl.p, rs.p, re.p, off.p, k1.p, U, m);
     size_t tb3 = 0;
     QP_CUDA(c, cub::DeviceRadixSort::SortKeys(nullptr, tb3, k1.p, k2.p, (int)T, 0, 64, st));
-    Scoped<char> tmp3;
-    QP_CUDA(c, dev_alloc(&tmp3.p, tb3));
+    Scoped<char> tmp3(c);
+    QP_CUDA(c, tmp3.alloc(tb3));
     QP_CUDA(c, cub::DeviceRadixSort::SortKeys(tmp3.p, tb3, k1.p, k2.p, (int)T, 0, 64, st));
-    Scoped<int> src;
-    QP_CUDA(c, dev_alloc(&src.p, T));
+    Scoped<int> src(c);
+    QP_CUDA(c, src.alloc(T));
     k_split_pairs<<<grid_for(T), TPB, 0, st>>>(k2.p, U, src.p, idx, T);
     k_csr_ptr<<<grid_for(T + 1), TPB, 0, st>>>(src.p, ptr, T, U);
     QP_CUDA(c, cudaStreamSynchronize(st));
@@ -360,7 +354,7 @@ void qp_free_dets(qpgpu_ctx* c) {
                  (void**)&c->d_sb_ptr, (void**)&c->d_sb_idx, (void**)&c->d_cost_a, (void**)&c->d_cost_b,
                  (void**)&c->d_detfeat, (void**)&c->d_alpha_pos, (void**)&c->d_beta_tpos};
   for (auto p : ps) {
-    dev_free(*p);
+    qp_pool_free(c, *p);
     *p = nullptr;
   }
   c->have_dets = false;
@@ -383,9 +377,9 @@ __global__ void k_gather_strings(const u64* strings, const int* id, const int* p
 int qp_build_index(qpgpu_ctx* c) {
   const int64_t N = c->N;
   cudaStream_t st = c->stream;
-  Scoped<int> aid, bid;
-  QP_CUDA(c, dev_alloc(&aid.p, N));
-  QP_CUDA(c, dev_alloc(&bid.p, N));
+  Scoped<int> aid(c), bid(c);
+  QP_CUDA(c, aid.alloc(N));
+  QP_CUDA(c, bid.alloc(N));
   int rc = unique_spin(c, 0, aid.p, &c->d_alpha, &c->Ua);
   if (rc) return rc;
   rc = unique_spin(c, 1, bid.p, &c->d_beta, &c->Ub);
@@ -393,12 +387,12 @@ int qp_build_index(qpgpu_ctx* c) {
   qp_mark(c, "unique strings");
   const int Ua = c->Ua, Ub = c->Ub;
   // beta-major bilinear order: key = beta_id * Ua + alpha_id (spindeterminants.irp.f:417)
-  QP_CUDA(c, dev_alloc(&c->d_order, N));
-  QP_CUDA(c, dev_alloc(&c->d_rows, N));
-  QP_CUDA(c, dev_alloc(&c->d_cols, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_order, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_rows, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_cols, N));
   {
-    Scoped<u64> key;
-    QP_CUDA(c, dev_alloc(&key.p, N));
+    Scoped<u64> key(c);
+    QP_CUDA(c, key.alloc(N));
     k_make_key<<<grid_for(N), TPB, 0, st>>>(bid.p, aid.p, Ua, key.p, N);
     rc = sort_multiword(c, N, 1, [&](int, const int* p, u64* out) {
       k_gather_u64<<<grid_for(N), TPB, 0, st>>>(key.p, p, out, N);
@@ -406,30 +400,30 @@ int qp_build_index(qpgpu_ctx* c) {
     if (rc) return rc;
   }
   k_bilinear<<<grid_for(N), TPB, 0, st>>>(c->d_order, aid.p, bid.p, c->d_rows, c->d_cols, N);
-  QP_CUDA(c, dev_alloc(&c->d_col_loc, (size_t)Ub + 1));
+  QP_CUDA(c, pool_alloc(c, &c->d_col_loc, (size_t)Ub + 1));
   k_seg_starts<<<grid_for(N), TPB, 0, st>>>(c->d_cols, c->d_col_loc, N, Ub);
   // alpha-major (transposed) order over bilinear positions: key = alpha_id * Ub + beta_id
-  QP_CUDA(c, dev_alloc(&c->d_t_order, N));
-  QP_CUDA(c, dev_alloc(&c->d_t_cols, N));
-  QP_CUDA(c, dev_alloc(&c->d_row_loc, (size_t)Ua + 1));
+  QP_CUDA(c, pool_alloc(c, &c->d_t_order, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_t_cols, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_row_loc, (size_t)Ua + 1));
   {
-    Scoped<u64> key;
-    QP_CUDA(c, dev_alloc(&key.p, N));
+    Scoped<u64> key(c);
+    QP_CUDA(c, key.alloc(N));
     k_make_key<<<grid_for(N), TPB, 0, st>>>(c->d_rows, c->d_cols, Ub, key.p, N);
     rc = sort_multiword(c, N, 1, [&](int, const int* p, u64* out) {
       k_gather_u64<<<grid_for(N), TPB, 0, st>>>(key.p, p, out, N);
     }, c->d_t_order);
     if (rc) return rc;
-    Scoped<int> trows;
-    QP_CUDA(c, dev_alloc(&trows.p, N));
+    Scoped<int> trows(c);
+    QP_CUDA(c, trows.alloc(N));
     k_gather_int<<<grid_for(N), TPB, 0, st>>>(c->d_rows, c->d_t_order, trows.p, N);
     k_gather_int<<<grid_for(N), TPB, 0, st>>>(c->d_cols, c->d_t_order, c->d_t_cols, N);
     k_seg_starts<<<grid_for(N), TPB, 0, st>>>(trows.p, c->d_row_loc, N, Ua);
   }
   // spin strings in scan order: the pair kernels read the strings of a
   // column (row) as one contiguous span instead of index -> string gathers
-  QP_CUDA(c, dev_alloc(&c->d_alpha_pos, (size_t)N * c->nint));
-  QP_CUDA(c, dev_alloc(&c->d_beta_tpos, (size_t)N * c->nint));
+  QP_CUDA(c, pool_alloc(c, &c->d_alpha_pos, (size_t)N * c->nint));
+  QP_CUDA(c, pool_alloc(c, &c->d_beta_tpos, (size_t)N * c->nint));
   k_gather_strings<<<grid_for(N * c->nint), TPB, 0, st>>>(c->d_alpha, c->d_rows, nullptr, c->d_alpha_pos, N,
                                                           c->nint);
   k_gather_strings<<<grid_for(N * c->nint), TPB, 0, st>>>(c->d_beta, c->d_cols, c->d_t_order, c->d_beta_tpos, N,
@@ -445,8 +439,8 @@ int qp_build_index(qpgpu_ctx* c) {
   rc = qp_build_line_keys(c);
   if (rc) return rc;
   qp_mark(c, "deletion-key tables");
-  QP_CUDA(c, dev_alloc(&c->d_cost_a, (size_t)Ua));
-  QP_CUDA(c, dev_alloc(&c->d_cost_b, (size_t)Ub));
+  QP_CUDA(c, pool_alloc(c, &c->d_cost_a, (size_t)Ua));
+  QP_CUDA(c, pool_alloc(c, &c->d_cost_b, (size_t)Ub));
   k_single_costs<<<grid_for(Ua), TPB, 0, st>>>(c->d_sa_ptr, c->d_sa_idx, c->d_row_loc, c->d_rowkey,
                                                32 * (int64_t)(c->nb + 2), c->d_cost_a, Ua);
   k_single_costs<<<grid_for(Ub), TPB, 0, st>>>(c->d_sb_ptr, c->d_sb_idx, c->d_col_loc, c->d_colkey,

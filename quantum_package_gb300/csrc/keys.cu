@@ -40,12 +40,6 @@ inline unsigned grid_n(int64_t n) {
   return (unsigned)std::min<int64_t>(std::max<int64_t>(g, 1), (int64_t)1 << 20);
 }
 
-template <class T>
-struct Scoped {
-  T* p = nullptr;
-  ~Scoped() { dev_free(p); }
-};
-
 // flags of each line (n = loc[l+1] - loc[l] determinants): KEY_SINGLE when
 // n > t1, KEY_DOUBLE when n > t2; sums[0], sums[1]: positions of the flagged
 // lines
@@ -176,37 +170,38 @@ int build_table(qpgpu_ctx* c, int kind, unsigned char* lflags, int nlines, int64
   // member offsets would not fit 32 bits
   size_t fr = 0, total = 0;
   QP_CUDA(c, cudaMemGetInfo(&fr, &total));
+  fr += qp_pool_cached(c);
   const double need = 26.0 * (double)E + 12.0 * (double)N;
   if (E >= (int64_t)INT_MAX || need > 0.5 * (double)fr) {
     k_clear_flag<<<grid_n(nlines), TPB, 0, st>>>(lflags, nlines, bit);
     QP_CUDA(c, cudaGetLastError());
     return 0;
   }
-  Scoped<int> kpos;
-  QP_CUDA(c, dev_alloc(&kpos.p, (size_t)M));
+  Scoped<int> kpos(c);
+  QP_CUDA(c, kpos.alloc((size_t)M));
   {
-    Scoped<int> pf, off;
-    Scoped<char> tmp;
-    QP_CUDA(c, dev_alloc(&pf.p, (size_t)N));
-    QP_CUDA(c, dev_alloc(&off.p, (size_t)N));
+    Scoped<int> pf(c), off(c);
+    Scoped<char> tmp(c);
+    QP_CUDA(c, pf.alloc((size_t)N));
+    QP_CUDA(c, off.alloc((size_t)N));
     if (spin == 0)
       k_pos_flags<0><<<grid_n(N), TPB, 0, st>>>(c->d_cols, c->d_t_order, lflags, bit, pf.p, N);
     else
       k_pos_flags<1><<<grid_n(N), TPB, 0, st>>>(c->d_rows, c->d_t_order, lflags, bit, pf.p, N);
     size_t tb = 0;
     QP_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, tb, pf.p, off.p, (int)N, st));
-    QP_CUDA(c, dev_alloc(&tmp.p, tb));
+    QP_CUDA(c, tmp.alloc(tb));
     QP_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp.p, tb, pf.p, off.p, (int)N, st));
     k_pos_compact<<<grid_n(N), TPB, 0, st>>>(pf.p, off.p, kpos.p, N);
     QP_CUDA(c, cudaGetLastError());
     QP_CUDA(c, cudaStreamSynchronize(st));
   }
-  Scoped<u64> ka, kb;
-  Scoped<int> va, vb;
-  QP_CUDA(c, dev_alloc(&ka.p, (size_t)E));
-  QP_CUDA(c, dev_alloc(&kb.p, (size_t)E));
-  QP_CUDA(c, dev_alloc(&va.p, (size_t)E));
-  QP_CUDA(c, dev_alloc(&vb.p, (size_t)E));
+  Scoped<u64> ka(c), kb(c);
+  Scoped<int> va(c), vb(c);
+  QP_CUDA(c, ka.alloc((size_t)E));
+  QP_CUDA(c, kb.alloc((size_t)E));
+  QP_CUDA(c, va.alloc((size_t)E));
+  QP_CUDA(c, vb.alloc((size_t)E));
   if (spin == 0)
     k_key_emit<NINT, 0><<<grid_n(E), TPB, 0, st>>>(c->d_alpha_pos, c->d_cols, c->d_t_order, kpos.p, M, ne, dele,
                                                    kind, hmask, ka.p, va.p);
@@ -220,13 +215,13 @@ int build_table(qpgpu_ctx* c, int kind, unsigned char* lflags, int nlines, int64
   {
     size_t tb = 0;
     QP_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dv, (int)E, 0, bits, st));
-    Scoped<char> tmp;
-    QP_CUDA(c, dev_alloc(&tmp.p, tb));
+    Scoped<char> tmp(c);
+    QP_CUDA(c, tmp.alloc(tb));
     QP_CUDA(c, cub::DeviceRadixSort::SortPairs(tmp.p, tb, dk, dv, (int)E, 0, bits, st));
   }
   const int minlen = dele == 2 ? 2 : 1;
-  Scoped<unsigned long long> ng;
-  QP_CUDA(c, dev_alloc(&ng.p, 1));
+  Scoped<unsigned long long> ng(c);
+  QP_CUDA(c, ng.alloc(1));
   QP_CUDA(c, cudaMemsetAsync(ng.p, 0, sizeof(unsigned long long), st));
   k_key_groups<<<grid_n(E), TPB, 0, st>>>(dk.Current(), E, minlen, ng.p, nullptr, 0, 0);
   unsigned long long G = 0;
@@ -235,7 +230,7 @@ int build_table(qpgpu_ctx* c, int kind, unsigned char* lflags, int nlines, int64
   int64_t nslot = 16;
   while (nslot < 2 * (int64_t)G) nslot <<= 1;
   KeySlot* slot = nullptr;
-  QP_CUDA(c, dev_alloc(&slot, (size_t)nslot));
+  QP_CUDA(c, pool_alloc(c, &slot, (size_t)nslot));
   QP_CUDA(c, cudaMemsetAsync(slot, 0, sizeof(KeySlot) * (size_t)nslot, st));
   c->d_kslot[kind] = slot;
   c->kslots[kind] = nslot;
@@ -261,10 +256,10 @@ int build_line_keys_t(qpgpu_ctx* c) {
   const int64_t t1_row = c->key_min_single >= 0 ? c->key_min_single : 64 * (int64_t)(c->nb + 2);
   const int64_t t2 = c->key_min_double >= 0 ? c->key_min_double : 16384;
   const u64 hmask = c->key_hash_bits >= 64 ? ~0ull : ((1ull << std::max(1, c->key_hash_bits)) - 1ull);
-  QP_CUDA(c, dev_alloc(&c->d_colkey, (size_t)c->Ub));
-  QP_CUDA(c, dev_alloc(&c->d_rowkey, (size_t)c->Ua));
-  Scoped<unsigned long long> sums;
-  QP_CUDA(c, dev_alloc(&sums.p, 5));
+  QP_CUDA(c, pool_alloc(c, &c->d_colkey, (size_t)c->Ub));
+  QP_CUDA(c, pool_alloc(c, &c->d_rowkey, (size_t)c->Ua));
+  Scoped<unsigned long long> sums(c);
+  QP_CUDA(c, sums.alloc(5));
   QP_CUDA(c, cudaMemsetAsync(sums.p, 0, 5 * sizeof(unsigned long long), st));
   k_line_flags<<<grid_n(c->Ub), TPB, 0, st>>>(c->d_col_loc, c->Ub, t1_col, c->na >= 2 ? t2 : big, c->d_colkey,
                                                sums.p);
@@ -298,14 +293,14 @@ int qp_build_line_keys(qpgpu_ctx* c) {
 
 void qp_free_line_keys(qpgpu_ctx* c) {
   for (int k = 0; k < KT_N; ++k) {
-    dev_free(c->d_kslot[k]);
-    dev_free(c->d_kmem[k]);
+    qp_pool_free(c, c->d_kslot[k]);
+    qp_pool_free(c, c->d_kmem[k]);
     c->d_kslot[k] = nullptr;
     c->d_kmem[k] = nullptr;
     c->kslots[k] = c->kmem_n[k] = 0;
   }
-  dev_free(c->d_colkey);
-  dev_free(c->d_rowkey);
+  qp_pool_free(c, c->d_colkey);
+  qp_pool_free(c, c->d_rowkey);
   c->d_colkey = c->d_rowkey = nullptr;
   c->n_keyed_lines = 0;
 }

@@ -219,9 +219,9 @@ struct Lk {
 }  // namespace
 
 int qp_det_features(qpgpu_ctx* c) {
-  dev_free(c->d_detfeat);
+  qp_pool_free(c, c->d_detfeat);
   c->d_detfeat = nullptr;
-  QP_CUDA(c, cudaMalloc((void**)&c->d_detfeat, c->N * sizeof(float4)));
+  QP_CUDA(c, pool_alloc(c, &c->d_detfeat, (size_t)c->N * 4));
   if (c->nint == 1)
     k_det_features<1><<<gsz(c->N), 256, 0, c->stream>>>(c->tab, c->d_alpha, c->d_beta, c->d_rows, c->d_cols,
                                                         (float4*)c->d_detfeat, c->N);

@@ -42,12 +42,6 @@ inline unsigned nblocks(int64_t n, int tpb) {
   return (unsigned)(g < 1 ? 1 : g);
 }
 
-template <class T>
-struct Scoped {
-  T* p = nullptr;
-  ~Scoped() { dev_free(p); }
-};
-
 struct BuildArgs {
   DevTables t;
   int64_t N;
@@ -838,11 +832,11 @@ int sort_row_columns(qpgpu_ctx* c) {
   QP_CUDA(c, cudaMemcpyAsync(rp.data(), c->d_rowptr, (N + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
   const int64_t cap = std::min<int64_t>(P, (int64_t)1 << 30);
-  Scoped<int> tmp, offs;
-  Scoped<char> work;
+  Scoped<int> tmp(c), offs(c);
+  Scoped<char> work(c);
   size_t work_bytes = 0;
-  QP_CUDA(c, dev_alloc(&tmp.p, (size_t)cap));
-  QP_CUDA(c, dev_alloc(&offs.p, (size_t)N + 1));
+  QP_CUDA(c, tmp.alloc((size_t)cap));
+  QP_CUDA(c, offs.alloc((size_t)N + 1));
   for (int64_t r0 = 0; r0 < N;) {
     int64_t r1 = std::upper_bound(rp.begin() + r0 + 1, rp.end(), rp[r0] + cap) - rp.begin() - 1;
     if (r1 <= r0) r1 = r0 + 1;
@@ -854,9 +848,9 @@ int sort_row_columns(qpgpu_ctx* c) {
       QP_CUDA(c, cub::DeviceSegmentedSort::SortKeys(nullptr, tb, c->d_colidx + base, tmp.p, (int)n, (int)(r1 - r0),
                                                     offs.p, offs.p + 1, st));
       if (tb > work_bytes) {
-        dev_free(work.p);
+        qp_pool_free(c, work.p);
         work.p = nullptr;
-        QP_CUDA(c, dev_alloc(&work.p, tb));
+        QP_CUDA(c, work.alloc(tb));
         work_bytes = tb;
       }
       QP_CUDA(c, cub::DeviceSegmentedSort::SortKeys(work.p, tb, c->d_colidx + base, tmp.p, (int)n, (int)(r1 - r0),
@@ -875,11 +869,11 @@ int build_pairs_t(qpgpu_ctx* c) {
   const int64_t N = c->N;
   cudaStream_t st = c->stream;
   BuildArgs a = index_args(c);
-  Scoped<int> cA, cB, cC, cS;
-  QP_CUDA(c, dev_alloc(&cA.p, N));
-  QP_CUDA(c, dev_alloc(&cB.p, N));
-  QP_CUDA(c, dev_alloc(&cC.p, N));
-  QP_CUDA(c, dev_alloc(&cS.p, N));
+  Scoped<int> cA(c), cB(c), cC(c), cS(c);
+  QP_CUDA(c, cA.alloc(N));
+  QP_CUDA(c, cB.alloc(N));
+  QP_CUDA(c, cC.alloc(N));
+  QP_CUDA(c, cS.alloc(N));
   a.cntA = cA.p;
   a.cntB = cB.p;
   a.cntC = cC.p;
@@ -896,16 +890,16 @@ int build_pairs_t(qpgpu_ctx* c) {
   k_class_c<NINT, MODE_COUNT><<<gC, BLK, 0, st>>>(a);
   qp_mark(c, "count C (alpha x beta)");
   QP_CUDA(c, cudaGetLastError());
-  Scoped<int64_t> tot, stot;
-  QP_CUDA(c, dev_alloc(&tot.p, N + 1));
-  QP_CUDA(c, dev_alloc(&stot.p, N + 1));
+  Scoped<int64_t> tot(c), stot(c);
+  QP_CUDA(c, tot.alloc(N + 1));
+  QP_CUDA(c, stot.alloc(N + 1));
   k_row_totals<<<nblocks(N + 1, 256), 256, 0, st>>>(cA.p, cB.p, cC.p, cS.p, tot.p, stot.p, N);
-  QP_CUDA(c, dev_alloc(&c->d_rowptr, N + 1));
-  QP_CUDA(c, dev_alloc(&c->d_s2ptr, N + 1));
+  QP_CUDA(c, pool_alloc(c, &c->d_rowptr, N + 1));
+  QP_CUDA(c, pool_alloc(c, &c->d_s2ptr, N + 1));
   size_t tb = 0;
   QP_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, tb, tot.p, c->d_rowptr, (int)(N + 1), st));
-  Scoped<char> tmp;
-  QP_CUDA(c, dev_alloc(&tmp.p, tb));
+  Scoped<char> tmp(c);
+  QP_CUDA(c, tmp.alloc(tb));
   QP_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp.p, tb, tot.p, c->d_rowptr, (int)(N + 1), st));
   QP_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp.p, tb, stot.p, c->d_s2ptr, (int)(N + 1), st));
   QP_CUDA(c, cudaMemcpyAsync(&c->P, c->d_rowptr + N, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -919,6 +913,7 @@ int build_pairs_t(qpgpu_ctx* c) {
   if (c->sigma_mode == QPGPU_SIGMA_AUTO) {
     size_t fr = 0, total = 0;
     QP_CUDA(c, cudaMemGetInfo(&fr, &total));
+    fr += qp_pool_cached(c);
     const double need = 16.0 * (double)P + 8.0 * (double)PS + 28.0 * (double)N;
     direct = need + (double)total / 16.0 > (double)fr;
   }
@@ -933,9 +928,9 @@ int build_pairs_t(qpgpu_ctx* c) {
     c->h_rowptr.resize(N + 1);
     QP_CUDA(c, cudaMemcpyAsync(c->h_rowptr.data(), c->d_rowptr, (N + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
                                st));
-    QP_CUDA(c, dev_alloc(&c->d_hdiag, N));
-    QP_CUDA(c, dev_alloc(&c->d_sdiag, N));
-    QP_CUDA(c, dev_alloc(&c->d_hdiag32, N));
+    QP_CUDA(c, pool_alloc(c, &c->d_hdiag, N));
+    QP_CUDA(c, pool_alloc(c, &c->d_sdiag, N));
+    QP_CUDA(c, pool_alloc(c, &c->d_hdiag32, N));
     k_diag<NINT><<<nblocks(N, 256), 256, 0, st>>>(c->tab, c->d_alpha, c->d_beta, c->d_rows, c->d_cols, c->d_hdiag,
                                                    c->d_sdiag, c->d_hdiag32, N);
     qp_mark(c, "diagonal (direct sigma: no pairs stored)");
@@ -943,9 +938,9 @@ int build_pairs_t(qpgpu_ctx* c) {
     QP_CUDA(c, cudaStreamSynchronize(st));
     return 0;
   }
-  if (dev_alloc(&c->d_colidx, P) != cudaSuccess || dev_alloc(&c->d_val64, P) != cudaSuccess ||
-      dev_alloc(&c->d_val32, P) != cudaSuccess || dev_alloc(&c->d_s2col, PS) != cudaSuccess ||
-      dev_alloc(&c->d_s2val, PS) != cudaSuccess) {
+  if (pool_alloc(c, &c->d_colidx, P) != cudaSuccess || pool_alloc(c, &c->d_val64, P) != cudaSuccess ||
+      pool_alloc(c, &c->d_val32, P) != cudaSuccess || pool_alloc(c, &c->d_s2col, PS) != cudaSuccess ||
+      pool_alloc(c, &c->d_s2val, PS) != cudaSuccess) {
     cudaGetLastError();
     return qpgpu_fail(c, QPGPU_ERR_NOMEM,
                       "not enough device memory for " + std::to_string(P) + " connected pairs");
@@ -957,8 +952,8 @@ int build_pairs_t(qpgpu_ctx* c) {
   a.s2ptr = c->d_s2ptr;
   a.s2col = c->d_s2col;
   a.s2val = c->d_s2val;
-  Scoped<int> err;
-  QP_CUDA(c, dev_alloc(&err.p, 1));
+  Scoped<int> err(c);
+  QP_CUDA(c, err.alloc(1));
   QP_CUDA(c, cudaMemsetAsync(err.p, 0, sizeof(int), st));
   a.err = err.p;
   qp_mark(c, "scan + alloc");
@@ -987,9 +982,9 @@ int build_pairs_t(qpgpu_ctx* c) {
   QP_CUDA(c, cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
   if (herr) return qpgpu_fail(c, QPGPU_ERR_STATE, "pair fill disagrees with pair count (" + std::to_string(herr) + ")");
-  QP_CUDA(c, dev_alloc(&c->d_hdiag, N));
-  QP_CUDA(c, dev_alloc(&c->d_sdiag, N));
-  QP_CUDA(c, dev_alloc(&c->d_hdiag32, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_hdiag, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_sdiag, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_hdiag32, N));
   k_diag<NINT><<<nblocks(N, 256), 256, 0, st>>>(c->tab, c->d_alpha, c->d_beta, c->d_rows, c->d_cols, c->d_hdiag,
                                                  c->d_sdiag, c->d_hdiag32, N);
   qp_mark(c, "diagonal");
@@ -1205,6 +1200,7 @@ int qp_sigma_direct(qpgpu_ctx* c, double* v, double* s, const double* u, int nst
   if (!c->d_direct_cols) {  // column buffer: the whole set if it fits in half the free memory
     size_t fr = 0, total = 0;
     QP_CUDA(c, cudaMemGetInfo(&fr, &total));
+    fr += qp_pool_cached(c);
     int64_t maxrow = 0;
     for (int64_t k = 0; k < c->N; ++k) maxrow = std::max(maxrow, c->h_rowptr[k + 1] - c->h_rowptr[k]);
     int64_t cap = std::min<int64_t>(c->P, (int64_t)(fr / 2 / sizeof(int)));
@@ -1229,17 +1225,22 @@ int qp_sigma_direct(qpgpu_ctx* c, double* v, double* s, const double* u, int nst
 
 void qp_free_pairs(qpgpu_ctx* c) {
   void** ps[] = {(void**)&c->d_rowptr, (void**)&c->d_colidx, (void**)&c->d_val64, (void**)&c->d_val32,
-                 (void**)&c->d_val32lo,
                  (void**)&c->d_s2ptr, (void**)&c->d_s2col, (void**)&c->d_s2val, (void**)&c->d_hdiag,
                  (void**)&c->d_sdiag, (void**)&c->d_hdiag32};
   for (auto p : ps) {
-    dev_free(*p);
+    qp_pool_free(c, *p);
     *p = nullptr;
   }
   c->have_pairs = false;
   c->direct = false;
-  void** dp[] = {(void**)&c->d_cntA, (void**)&c->d_cntB, (void**)&c->d_direct_cols, (void**)&c->d_direct_err};
+  void** dp[] = {(void**)&c->d_cntA, (void**)&c->d_cntB};
   for (auto p : dp) {
+    qp_pool_free(c, *p);
+    *p = nullptr;
+  }
+  // grown by a sigma on the caller's stream: not from the pool
+  void** up[] = {(void**)&c->d_val32lo, (void**)&c->d_direct_cols, (void**)&c->d_direct_err};
+  for (auto p : up) {
     dev_free(*p);
     *p = nullptr;
   }

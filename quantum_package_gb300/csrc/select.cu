@@ -601,8 +601,9 @@ __global__ void k_sel_gather(const long long* idx, uint64_t take, const double* 
 }
 
 struct Dev {
+  qpgpu_ctx* c;
   void* p = nullptr;
-  ~Dev() { dev_free(p); }
+  ~Dev() { qp_pool_free(c, p); }
 };
 
 }  // namespace
@@ -619,6 +620,7 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   const int nint = c->nint, n = c->n_mo;
   const int n_list = (int)gens.size();
   cudaStream_t st = c->stream;
+  PoolTrim trim{c};
   // host copies of the listed generators (item list)
   std::vector<u64> gdet((size_t)n_list * 2 * nint);
   for (int l = 0; l < n_list; ++l)
@@ -662,32 +664,32 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
     return 0;
   }
   // device arrays
-  Dev d_items, d_gens, d_coef, d_e0, d_icnt, d_ioff, d_ilist, d_fcnt, d_foff, d_flist, d_fock, d_slot, d_part, d_cnt,
-      d_err, d_pt2;
+  Dev d_items{c}, d_gens{c}, d_coef{c}, d_e0{c}, d_icnt{c}, d_ioff{c}, d_ilist{c}, d_fcnt{c}, d_foff{c};
+  Dev d_flist{c}, d_fock{c}, d_slot{c}, d_part{c}, d_cnt{c}, d_err{c}, d_pt2{c};
   uint64_t hcap = 1;
   while (hcap < (uint64_t)(2 * N)) hcap <<= 1;
-  QP_CUDA(c, cudaMalloc(&d_items.p, items.size() * sizeof(SelItem)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_items.p, items.size() * sizeof(SelItem)));
   QP_CUDA(c, cudaMemcpyAsync(d_items.p, items.data(), items.size() * sizeof(SelItem), cudaMemcpyHostToDevice, st));
-  QP_CUDA(c, cudaMalloc(&d_gens.p, n_list * sizeof(int)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_gens.p, n_list * sizeof(int)));
   QP_CUDA(c, cudaMemcpyAsync(d_gens.p, gens.data(), n_list * sizeof(int), cudaMemcpyHostToDevice, st));
   // coefficients: column-major (N, n_st) on the host -> (N, n_st) row-major
   std::vector<double> crow((size_t)N * n_st);
   for (int s = 0; s < n_st; ++s)
     for (int64_t i = 0; i < N; ++i) crow[(size_t)i * n_st + s] = coef[(size_t)s * N + i];
-  QP_CUDA(c, cudaMalloc(&d_coef.p, crow.size() * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_coef.p, crow.size() * sizeof(double)));
   QP_CUDA(c, cudaMemcpyAsync(d_coef.p, crow.data(), crow.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-  QP_CUDA(c, cudaMalloc(&d_e0.p, n_st * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_e0.p, n_st * sizeof(double)));
   QP_CUDA(c, cudaMemcpyAsync(d_e0.p, e0, n_st * sizeof(double), cudaMemcpyHostToDevice, st));
-  QP_CUDA(c, cudaMalloc(&d_slot.p, hcap * sizeof(int)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_slot.p, hcap * sizeof(int)));
   QP_CUDA(c, cudaMemsetAsync(d_slot.p, 0xff, hcap * sizeof(int), st));
-  QP_CUDA(c, cudaMalloc(&d_fock.p, (size_t)n_list * 2 * (n + 2) * sizeof(double)));
-  QP_CUDA(c, cudaMalloc(&d_icnt.p, (n_list + 1) * sizeof(int64_t)));
-  QP_CUDA(c, cudaMalloc(&d_fcnt.p, (n_list + 1) * sizeof(int64_t)));
-  QP_CUDA(c, cudaMalloc(&d_cnt.p, 2 * sizeof(unsigned long long)));
-  QP_CUDA(c, cudaMalloc(&d_err.p, sizeof(int)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_fock.p, (size_t)n_list * 2 * (n + 2) * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_icnt.p, (n_list + 1) * sizeof(int64_t)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_fcnt.p, (n_list + 1) * sizeof(int64_t)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_cnt.p, 2 * sizeof(unsigned long long)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_err.p, sizeof(int)));
   QP_CUDA(c, cudaMemsetAsync(d_err.p, 0, sizeof(int), st));
-  QP_CUDA(c, cudaMalloc(&d_pt2.p, n_st * sizeof(double)));
-  QP_CUDA(c, cudaMalloc(&d_part.p, (size_t)n_items * n_st * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_pt2.p, n_st * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_part.p, (size_t)n_items * n_st * sizeof(double)));
   const u64* dets = c->d_dets;
   const int* dg = (const int*)d_gens.p;
   const int hb = (int)std::min<int64_t>((N + 255) / 256, (int64_t)c->n_sm * 8);
@@ -713,17 +715,17 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
     ioff[l + 1] = ioff[l] + icnt[l];
     foff[l + 1] = foff[l] + fcnt[l];
   }
-  QP_CUDA(c, cudaMalloc(&d_ioff.p, (n_list + 1) * sizeof(int64_t)));
-  QP_CUDA(c, cudaMalloc(&d_foff.p, (n_list + 1) * sizeof(int64_t)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_ioff.p, (n_list + 1) * sizeof(int64_t)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_foff.p, (n_list + 1) * sizeof(int64_t)));
   QP_CUDA(c, cudaMemcpyAsync(d_ioff.p, ioff.data(), (n_list + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
   QP_CUDA(c, cudaMemcpyAsync(d_foff.p, foff.data(), (n_list + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-  QP_CUDA(c, cudaMalloc(&d_ilist.p, std::max<int64_t>(1, ioff[n_list]) * sizeof(int)));
-  QP_CUDA(c, cudaMalloc(&d_flist.p, std::max<int64_t>(1, foff[n_list]) * sizeof(int)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_ilist.p, std::max<int64_t>(1, ioff[n_list]) * sizeof(int)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_flist.p, std::max<int64_t>(1, foff[n_list]) * sizeof(int)));
   // candidates (only when a buffer is asked for): at most one per entry
   uint64_t ub = 0;
   for (const SelItem& it : items) ub += (uint64_t)(it.e1 - it.e0);
   uint64_t cap = buf_size > 0 ? std::min<uint64_t>(ub, 1ull << 28) : 0;  // <= 10.7 GB of candidates
-  Dev d_cval, d_cdet;
+  Dev d_cval{c}, d_cdet{c};
   SelArgs A{};
   A.t = c->tab;
   A.dets = dets;
@@ -750,11 +752,11 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   const size_t smem = (size_t)std::max(max_ne * n_st, SBLK * n_st) * sizeof(double);
   unsigned long long hcnt[2] = {0, 0};
   for (int attempt = 0; attempt < 2; ++attempt) {
-    dev_free(d_cval.p);
-    dev_free(d_cdet.p);
+    qp_pool_free(c, d_cval.p);
+    qp_pool_free(c, d_cdet.p);
     d_cval.p = d_cdet.p = nullptr;
-    QP_CUDA(c, cudaMalloc(&d_cval.p, std::max<uint64_t>(1, cap) * sizeof(double)));
-    QP_CUDA(c, cudaMalloc(&d_cdet.p, std::max<uint64_t>(1, cap) * 2 * nint * sizeof(u64)));
+    QP_CUDA(c, qp_pool_alloc(c, &d_cval.p, std::max<uint64_t>(1, cap) * sizeof(double)));
+    QP_CUDA(c, qp_pool_alloc(c, &d_cdet.p, std::max<uint64_t>(1, cap) * 2 * nint * sizeof(u64)));
     A.cap = cap;
     A.cand_val = (double*)d_cval.p;
     A.cand_det = (u64*)d_cdet.p;
@@ -797,17 +799,17 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   if (nout > 0) {
     // sort by value on the device; the head (and any tie group crossing its
     // end) goes to the host, where equal values are put in determinant order
-    Dev kin, kout, vin, vout, tmp;
-    QP_CUDA(c, cudaMalloc(&kin.p, nc * 8));
-    QP_CUDA(c, cudaMalloc(&kout.p, nc * 8));
-    QP_CUDA(c, cudaMalloc(&vin.p, nc * 8));
-    QP_CUDA(c, cudaMalloc(&vout.p, nc * 8));
+    Dev kin{c}, kout{c}, vin{c}, vout{c}, tmp{c};
+    QP_CUDA(c, qp_pool_alloc(c, &kin.p, nc * 8));
+    QP_CUDA(c, qp_pool_alloc(c, &kout.p, nc * 8));
+    QP_CUDA(c, qp_pool_alloc(c, &vin.p, nc * 8));
+    QP_CUDA(c, qp_pool_alloc(c, &vout.p, nc * 8));
     k_sel_keys<<<(unsigned)std::min<uint64_t>((nc + 255) / 256, (uint64_t)c->n_sm * 8), 256, 0, st>>>(
         (const double*)d_cval.p, nc, (unsigned long long*)kin.p, (long long*)vin.p);
     size_t tb = 0;
     QP_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, tb, (unsigned long long*)kin.p, (unsigned long long*)kout.p,
                                                (long long*)vin.p, (long long*)vout.p, (int64_t)nc, 0, 64, st));
-    QP_CUDA(c, cudaMalloc(&tmp.p, tb));
+    QP_CUDA(c, qp_pool_alloc(c, &tmp.p, tb));
     QP_CUDA(c, cub::DeviceRadixSort::SortPairs(tmp.p, tb, (unsigned long long*)kin.p, (unsigned long long*)kout.p,
                                                (long long*)vin.p, (long long*)vout.p, (int64_t)nc, 0, 64, st));
     std::vector<unsigned long long> keys;
@@ -821,9 +823,9 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
     }
     std::vector<double> vals(take);
     std::vector<u64> dts(take * 2 * nint);
-    Dev gv, gd;
-    QP_CUDA(c, cudaMalloc(&gv.p, take * sizeof(double)));
-    QP_CUDA(c, cudaMalloc(&gd.p, take * 2 * nint * sizeof(u64)));
+    Dev gv{c}, gd{c};
+    QP_CUDA(c, qp_pool_alloc(c, &gv.p, take * sizeof(double)));
+    QP_CUDA(c, qp_pool_alloc(c, &gd.p, take * 2 * nint * sizeof(u64)));
     k_sel_gather<<<(unsigned)std::min<uint64_t>((take + 255) / 256, (uint64_t)c->n_sm * 8), 256, 0, st>>>(
         (const long long*)vout.p, take, (const double*)d_cval.p, (const u64*)d_cdet.p, 2 * nint, (double*)gv.p,
         (u64*)gd.p);

@@ -540,9 +540,9 @@ int tune_sigma32(qpgpu_ctx* c, SigmaItems* it, const SigArgs& a, int nst, cudaSt
 int qp_build_sigma_items(qpgpu_ctx* c, SigmaItems* it) {
   const int64_t N = c->N;
   cudaStream_t st = c->stream;
-  it->free_all();
-  QP_CUDA(c, dev_alloc(&it->row_nitems, N + 1));
-  QP_CUDA(c, dev_alloc(&it->row_item0, N + 1));
+  it->free_all(c);
+  QP_CUDA(c, pool_alloc(c, &it->row_nitems, N + 1));
+  QP_CUDA(c, pool_alloc(c, &it->row_item0, N + 1));
   k_row_nitems<<<gsz(N, 256), 256, 0, st>>>(c->d_rowptr, it->row_nitems, N);
   QP_CUDA(c, cudaMemsetAsync(it->row_nitems + N, 0, sizeof(int), st));
   std::vector<int> nit(N);
@@ -560,9 +560,9 @@ int qp_build_sigma_items(qpgpu_ctx* c, SigmaItems* it) {
   it->n_items = acc;
   it->n_multi = (int)multi.size();
   QP_CUDA(c, cudaMemcpyAsync(it->row_item0, item0.data(), (N + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-  QP_CUDA(c, dev_alloc(&it->item_row, acc));
-  QP_CUDA(c, dev_alloc(&it->item_sub, acc));
-  QP_CUDA(c, dev_alloc(&it->multi_rows, multi.size() + 1));
+  QP_CUDA(c, pool_alloc(c, &it->item_row, acc));
+  QP_CUDA(c, pool_alloc(c, &it->item_sub, acc));
+  QP_CUDA(c, pool_alloc(c, &it->multi_rows, multi.size() + 1));
   if (!multi.empty())
     QP_CUDA(c, cudaMemcpyAsync(it->multi_rows, multi.data(), multi.size() * sizeof(int), cudaMemcpyHostToDevice, st));
   k_fill_items<<<gsz(N, 256), 256, 0, st>>>(it->row_nitems, it->row_item0, it->item_row, it->item_sub, N);
