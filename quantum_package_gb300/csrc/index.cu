@@ -215,9 +215,19 @@ __global__ void k_single_costs(const int* ptr, const int* idx, const int* loc, c
   }
 }
 
-// LSD radix sort of multi-word keys produced by `word_fn(w, perm, out)`; perm is the result.
+// bits that hold the numbers below n
+inline int bits_below(u64 n) {
+  int b = 1;
+  while (b < 64 && (n - 1) >> b) ++b;
+  return b;
+}
+
+// LSD radix sort of multi-word keys produced by `word_fn(w, perm, out)`, whose
+// word w has no bit at or above bits[w] (a pass of the sort covers 8 bits, so
+// the 64-bit words of 40 or 80 orbitals would take up to twice the passes);
+// perm is the result.
 template <class WordFn>
-int sort_multiword(qpgpu_ctx* c, int64_t n, int nwords, WordFn word_fn, int* perm_out) {
+int sort_multiword(qpgpu_ctx* c, int64_t n, int nwords, const int* bits, WordFn word_fn, int* perm_out) {
   cudaStream_t st = c->stream;
   Scoped<u64> ka(c), kb(c);
   Scoped<int> pa(c), pb(c);
@@ -232,7 +242,7 @@ int sort_multiword(qpgpu_ctx* c, int64_t n, int nwords, WordFn word_fn, int* per
   k_iota<<<grid_for(n), TPB, 0, st>>>(pa.p, n);
   for (int w = 0; w < nwords; ++w) {
     word_fn(w, pa.p, ka.p);  // keys of the current permutation
-    QP_CUDA(c, cub::DeviceRadixSort::SortPairs(tmp.p, tbytes, ka.p, kb.p, pa.p, pb.p, (int)n, 0, 64, st));
+    QP_CUDA(c, cub::DeviceRadixSort::SortPairs(tmp.p, tbytes, ka.p, kb.p, pa.p, pb.p, (int)n, 0, bits[w], st));
     std::swap(pa.p, pb.p);
   }
   QP_CUDA(c, cudaMemcpyAsync(perm_out, pa.p, n * sizeof(int), cudaMemcpyDeviceToDevice, st));
@@ -247,7 +257,8 @@ int unique_spin(qpgpu_ctx* c, int spin, int* id_out, u64** uniq_out, int* nu_out
   QP_CUDA(c, perm.alloc(N));
   QP_CUDA(c, flag.alloc(N));
   QP_CUDA(c, incl.alloc(N));
-  int rc = sort_multiword(c, N, nint, [&](int w, const int* p, u64* out) {
+  const int bits[2] = {std::min(64, c->n_mo), std::max(1, c->n_mo - 64)};
+  int rc = sort_multiword(c, N, nint, bits, [&](int w, const int* p, u64* out) {
     k_gather_word<<<grid_for(N), TPB, 0, st>>>(c->d_dets, nint, spin, w, p, out, N);
   }, perm.p);
   if (rc) return rc;
@@ -288,7 +299,8 @@ int singles_adjacency(qpgpu_ctx* c, const u64* uniq, int U, int ne, int** ptr_ou
   QP_CUDA(c, perm.alloc(m));
   QP_CUDA(c, flag.alloc(m));
   QP_CUDA(c, incl.alloc(m));
-  int rc = sort_multiword(c, m, nint, [&](int w, const int* p, u64* out) {
+  const int bits[2] = {std::min(64, c->n_mo), std::max(1, c->n_mo - 64)};
+  int rc = sort_multiword(c, m, nint, bits, [&](int w, const int* p, u64* out) {
     k_deletion_word<<<grid_for(m), TPB, 0, st>>>(uniq, nint, ne, w, p, out, m);
   }, perm.p);
   if (rc) return rc;
@@ -326,10 +338,11 @@ int singles_adjacency(qpgpu_ctx* c, const u64* uniq, int U, int ne, int** ptr_ou
     QP_CUDA(c, k2.alloc(T));
     k_pair_emit<<<grid_for(m), TPB, 0, st>>>(perm.p, ne, incl.p, rs.p, re.p, off.p, k1.p, U, m);
     size_t tb3 = 0;
-    QP_CUDA(c, cub::DeviceRadixSort::SortKeys(nullptr, tb3, k1.p, k2.p, (int)T, 0, 64, st));
+    const int bits2 = bits_below((u64)U * (u64)U);
+    QP_CUDA(c, cub::DeviceRadixSort::SortKeys(nullptr, tb3, k1.p, k2.p, (int)T, 0, bits2, st));
     Scoped<char> tmp3(c);
     QP_CUDA(c, tmp3.alloc(tb3));
-    QP_CUDA(c, cub::DeviceRadixSort::SortKeys(tmp3.p, tb3, k1.p, k2.p, (int)T, 0, 64, st));
+    QP_CUDA(c, cub::DeviceRadixSort::SortKeys(tmp3.p, tb3, k1.p, k2.p, (int)T, 0, bits2, st));
     Scoped<int> src(c);
     QP_CUDA(c, src.alloc(T));
     k_split_pairs<<<grid_for(T), TPB, 0, st>>>(k2.p, U, src.p, idx, T);
@@ -394,7 +407,8 @@ int qp_build_index(qpgpu_ctx* c) {
     Scoped<u64> key(c);
     QP_CUDA(c, key.alloc(N));
     k_make_key<<<grid_for(N), TPB, 0, st>>>(bid.p, aid.p, Ua, key.p, N);
-    rc = sort_multiword(c, N, 1, [&](int, const int* p, u64* out) {
+    const int bits = bits_below((u64)Ua * (u64)Ub);
+    rc = sort_multiword(c, N, 1, &bits, [&](int, const int* p, u64* out) {
       k_gather_u64<<<grid_for(N), TPB, 0, st>>>(key.p, p, out, N);
     }, c->d_order);
     if (rc) return rc;
@@ -410,7 +424,8 @@ int qp_build_index(qpgpu_ctx* c) {
     Scoped<u64> key(c);
     QP_CUDA(c, key.alloc(N));
     k_make_key<<<grid_for(N), TPB, 0, st>>>(c->d_rows, c->d_cols, Ub, key.p, N);
-    rc = sort_multiword(c, N, 1, [&](int, const int* p, u64* out) {
+    const int bits = bits_below((u64)Ua * (u64)Ub);
+    rc = sort_multiword(c, N, 1, &bits, [&](int, const int* p, u64* out) {
       k_gather_u64<<<grid_for(N), TPB, 0, st>>>(key.p, p, out, N);
     }, c->d_t_order);
     if (rc) return rc;

@@ -209,7 +209,7 @@ int build_table(qpgpu_ctx* c, int kind, unsigned char* lflags, int nlines, int64
     k_key_emit<NINT, 1><<<grid_n(E), TPB, 0, st>>>(c->d_beta_tpos, c->d_rows, c->d_t_order, kpos.p, M, ne, dele,
                                                    kind, hmask, ka.p, va.p);
   QP_CUDA(c, cudaGetLastError());
-  const int bits = std::max(1, std::min(64, c->key_hash_bits));
+  const int bits = qp_key_bits(c);
   cub::DoubleBuffer<u64> dk(ka.p, kb.p);
   cub::DoubleBuffer<int> dv(va.p, vb.p);
   {
@@ -255,7 +255,7 @@ int build_line_keys_t(qpgpu_ctx* c) {
   const int64_t t1_col = c->key_min_single >= 0 ? c->key_min_single : 64 * (int64_t)(c->na + 2);
   const int64_t t1_row = c->key_min_single >= 0 ? c->key_min_single : 64 * (int64_t)(c->nb + 2);
   const int64_t t2 = c->key_min_double >= 0 ? c->key_min_double : 16384;
-  const u64 hmask = c->key_hash_bits >= 64 ? ~0ull : ((1ull << std::max(1, c->key_hash_bits)) - 1ull);
+  const u64 hmask = qp_key_mask(c);
   QP_CUDA(c, pool_alloc(c, &c->d_colkey, (size_t)c->Ub));
   QP_CUDA(c, pool_alloc(c, &c->d_rowkey, (size_t)c->Ua));
   Scoped<unsigned long long> sums(c);

@@ -28,10 +28,11 @@ inline unsigned gsz(int64_t n, int tpb = 256) {
 
 // static features of each determinant (bilinear order): excitation rank of the
 // alpha and beta strings relative to the reference, sum of h_pp over particles
-// minus holes (orbital-energy change); .w is set by k_row_coupling
+// minus holes (orbital-energy change); .w (the coupling strength) is set with
+// the stored elements (k_pair_values), and is 0 for the direct sigma
 template <int NINT>
 __global__ void k_det_features(DevTables t, const u64* alpha, const u64* beta, const int* rows, const int* cols,
-                               float4* out, int64_t N) {
+                               float4* out, int direct, int64_t N) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N; k += (int64_t)gridDim.x * blockDim.x) {
     const u64* a = alpha + (int64_t)rows[k] * NINT;
     const u64* b = beta + (int64_t)cols[k] * NINT;
@@ -53,22 +54,7 @@ __global__ void k_det_features(DevTables t, const u64* alpha, const u64* beta, c
         e += ((b[w] >> (p - 1 - 64 * w)) & 1ull) ? hp : -hp;
       }
     }
-    out[k] = make_float4(0.5f * ra, 0.5f * rb, (float)e, 0.f);
-  }
-}
-
-// coupling strength of each row: log10(sum_J H_IJ^2) / 4 (the scale of the
-// second-order shift of the diagonal denominator), one warp per row, into .w
-__global__ void k_row_coupling(const int64_t* rowptr, const double* val, float4* out, int64_t N) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t k = warp; k < N; k += nwarp) {
-    double s = 0.0;
-    for (int64_t e = rowptr[k] + lane; e < rowptr[k + 1]; e += 32) s = fma(val[e], val[e], s);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[k].w = (float)(log10(s + 1e-30) * 0.25);
+    out[k] = make_float4(0.5f * ra, 0.5f * rb, (float)e, direct ? 0.f : out[k].w);
   }
 }
 
@@ -219,18 +205,13 @@ struct Lk {
 }  // namespace
 
 int qp_det_features(qpgpu_ctx* c) {
-  qp_pool_free(c, c->d_detfeat);
-  c->d_detfeat = nullptr;
-  QP_CUDA(c, pool_alloc(c, &c->d_detfeat, (size_t)c->N * 4));
+  if (c->direct) QP_CUDA(c, pool_alloc(c, &c->d_detfeat, (size_t)c->N * 4));
   if (c->nint == 1)
     k_det_features<1><<<gsz(c->N), 256, 0, c->stream>>>(c->tab, c->d_alpha, c->d_beta, c->d_rows, c->d_cols,
-                                                        (float4*)c->d_detfeat, c->N);
+                                                        (float4*)c->d_detfeat, c->direct, c->N);
   else
     k_det_features<2><<<gsz(c->N), 256, 0, c->stream>>>(c->tab, c->d_alpha, c->d_beta, c->d_rows, c->d_cols,
-                                                        (float4*)c->d_detfeat, c->N);
-  // coupling feature from the stored elements (left at 0 with the direct sigma)
-  if (!c->direct)
-    k_row_coupling<<<gsz(c->N * 32), 256, 0, c->stream>>>(c->d_rowptr, c->d_val64, (float4*)c->d_detfeat, c->N);
+                                                        (float4*)c->d_detfeat, c->direct, c->N);
   QP_CUDA(c, cudaGetLastError());
   return 0;
 }

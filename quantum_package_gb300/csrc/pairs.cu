@@ -6,23 +6,24 @@
 //   class A  J in the same beta column, alpha strings 1 or 2 apart  (:277-332)
 //   class B  J in the same alpha row, beta strings 1 or 2 apart      (:336-415)
 //   class C  alpha single x beta single                              (:177-246)
-// with the diagonal kept apart (:418-441).  The fill writes row k's A hits,
-// then its B hits, then its C hits; the stored form then sorts each row's
-// columns ascending (the direct sigma keeps the fill order).
+// with the diagonal kept apart (:418-441).
 //
-// Two passes run the same deterministic traversal: the first counts hits per
-// row, the second writes them (column = bilinear position of J, FP64 and FP32
-// matrix elements).  A third mode (direct sigma, for determinant sets whose
-// pairs do not fit in device memory) runs the traversal at every sigma call
-// and accumulates h_IJ u_J for the row each thread (classes A, B) or warp
-// (class C) owns: class A writes v, class B adds to it, class C adds its sum
-// and the diagonal term and writes s, so no pair is stored and no atomic is
-// needed.  Same-spin classes scan a column (row) with one thread per
-// determinant; the column's strings are staged in shared memory and read by
-// every thread of the block as broadcasts.  Class C gives one warp per row and
-// compacts hits with __ballot_sync, scanning either the columns of the beta
-// singles of b (as the reference does) or the rows of the alpha singles of a,
-// whichever holds fewer determinants.
+// One warp owns a row: it scans the row's beta column (class A), alpha row
+// (class B) and the columns of the beta singles of b, or the rows of the alpha
+// singles of a, whichever hold fewer determinants (class C); lines with
+// deletion-key tables (keys.cu) are probed instead.  Hits are compacted with
+// __ballot_sync, so no atomics order them.
+//
+// Stored pairs.  The scans run once: each warp writes the hits of its rows
+// into chunks of a pool and counts them.  k_sort_rows then moves each row's
+// hits to their place in the CSR, ascending, and k_pair_values evaluates the
+// elements.  At 1e6 determinants the scans take 29 ms (68 ms as a count and a
+// fill pass).  Rows that found the pool full are scanned a second time and write
+// straight into the CSR; without a pool that is every row.
+//
+// Direct sigma (sets whose pairs do not fit in device memory).  The scans
+// count once at set-up and write one chunk of rows' columns at every sigma
+// call, row k's A hits, then its B hits, then its C hits, for k_pair_sigma.
 #include <algorithm>
 #include <climits>
 #include <vector>
@@ -35,7 +36,6 @@
 namespace {
 
 constexpr int BLK = 256;
-constexpr int TILE = 1024;
 
 inline unsigned nblocks(int64_t n, int tpb) {
   int64_t g = (n + tpb - 1) / tpb;
@@ -61,12 +61,19 @@ struct BuildArgs {
   const int* sb_idx;
   const int64_t* cost_a;
   const int64_t* cost_b;
-  // counts (count pass output, fill pass input)
-  int* cntA;
-  int* cntB;
-  int* cntC;
+  // hits of each row and class (A, B, C) and spin-flip pairs among the C hits
+  int* cnt[3];
   int* cntS;
-  // CSR (fill pass)
+  // MODE_POOL: pool of columns, handed out in chunks; pos[class][row] = first
+  // hit of the row's class in the pool (-1: the pool was full)
+  int* pool;
+  int64_t pool_cap;
+  int pool_chunk[3];
+  unsigned long long* pool_next;
+  int* pool_full;
+  int64_t* pos[3];
+  unsigned long long* next_row;  // MODE_POOL: rows handed out to warps (one counter per class)
+  // CSR (fill pass, sort, elements)
   const int64_t* rowptr;
   int* colidx;
   double* val64;
@@ -74,7 +81,10 @@ struct BuildArgs {
   const int64_t* s2ptr;
   int* s2col;
   float* s2val;
-  int* err;  // set when a fill pass would write past its row's segment
+  float4* feat;         // .w: coupling strength of the row (learned step), or null
+  const u64* det_pos;   // both strings at each bilinear position (2 NINT words)
+  const u64* det_tpos;  // the same at each alpha-major position (direct sigma)
+  int* err;  // set when a pass would write past its row's segment
   // direct sigma (k_pair_sigma): v, s = H u, S^2 u for the selected rows, u (N, nst)
   const double* u;
   const double* uT;  // u in alpha-major order: same-alpha partners are contiguous there
@@ -83,13 +93,12 @@ struct BuildArgs {
   const double* hdiag;
   const double* sdiag;
   int nst;
+  // a fill takes the rows row_first modulo row_step of [row_lo, row_hi)
   int row_lo, row_hi, row_first, row_step;
   // chunked direct sigma: the fill writes columns of rows [row_lo, row_hi) at
-  // rowptr[k] - col_base, class A blocks start at block blk_off, and same-alpha
-  // partners are written as alpha-major positions tagged with QP_TAG_T
+  // rowptr[k] - col_base, and same-alpha partners are written as alpha-major
+  // positions tagged with QP_TAG_T
   int64_t col_base;
-  int64_t blk_off;
-  int write_s2;
   int tag_t;
   // deletion-key tables of the heavy lines (keys.cu); colkey / rowkey null: none
   KeyView kv[KT_N];
@@ -100,146 +109,111 @@ struct BuildArgs {
 
 constexpr unsigned QP_TAG_T = 0x80000000u;  // column given as alpha-major position
 
-constexpr int MODE_COUNT = 0, MODE_FILL = 1;
+constexpr int MODE_COUNT = 0, MODE_FILL = 1, MODE_POOL = 2;
+enum { CLS_A = 0, CLS_B = 1, CLS_C = 2 };
 
 __device__ __forceinline__ bool dsel(const BuildArgs& a, int64_t k) {
   return k >= a.row_lo && k < a.row_hi && ((k - a.row_first) % a.row_step) == 0;
 }
 
-// ---- class A: same beta column, alpha singles / doubles -------------------
-template <int NINT, int MODE>
-__global__ void __launch_bounds__(BLK) k_class_a(BuildArgs a) {
-  constexpr bool FILL = MODE == MODE_FILL;
-  __shared__ u64 tile[TILE * NINT];
-  const int64_t r0 = ((int64_t)blockIdx.x + a.blk_off) * BLK;
-  if (r0 >= a.N) return;
-  const int64_t k = r0 + threadIdx.x;
-  const bool valid = k < a.N;
-  int cs = 0, ce = 0;
-  u64 my[2 * NINT];
-  int64_t out = 0;
-  bool keyed = false;  // the column has a 2-deletion table: k_same_keyed takes the row
-  if (valid) {
-    const int b = a.cols[k];
-    keyed = a.colkey && (a.colkey[b] & KEY_DOUBLE);
-    cs = a.col_loc[b];
-    ce = a.col_loc[b + 1];
-    const int ai = a.rows[k];
-#pragma unroll
-    for (int w = 0; w < NINT; ++w) {
-      my[w] = a.alpha[(int64_t)ai * NINT + w];
-      my[NINT + w] = a.beta[(int64_t)b * NINT + w];
+// Runs `row` on the rows of a scan of one class: MODE_COUNT all rows and
+// MODE_FILL the selected ones (with a pool, those that did not fit it) in the
+// order of the warps.  MODE_POOL takes them from a counter one at a time, the
+// next one while the current one runs: the rows of the lowest excitations
+// take up to 0.2 ms each and stand side by side, so that handing out four
+// (or 64 a block) left most SMs waiting for the last of them.
+template <int MODE, int CLS, class Row>
+__device__ __forceinline__ void for_rows(const BuildArgs& a, int lane, Row row) {
+  if (MODE == MODE_POOL) {
+    unsigned long long next = 0;
+    if (lane == 0) next = atomicAdd(a.next_row + CLS, 1ull);
+    while (true) {
+      const int64_t k = (int64_t)__shfl_sync(0xffffffffu, next, 0);
+      if (k >= a.N) return;
+      if (lane == 0) next = atomicAdd(a.next_row + CLS, 1ull);
+      row(k);
     }
-    if (FILL) out = a.rowptr[k] - a.col_base;
-  }
-  int cnt = 0;
-  const bool act = valid && !keyed && (MODE == MODE_COUNT || dsel(a, k));
-  // the tiles span the columns of the block's active rows
-  __shared__ int s_lo, s_hi;
-  if (threadIdx.x == 0) {
-    s_lo = INT_MAX;
-    s_hi = INT_MIN;
-  }
-  __syncthreads();
-  if (act) {
-    atomicMin(&s_lo, cs);
-    atomicMax(&s_hi, ce);
-  }
-  __syncthreads();
-  const int U0 = s_lo, U1 = s_hi;
-  for (int t0 = U0; t0 < U1; t0 += TILE) {
-    const int tn = min(TILE, U1 - t0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < tn * NINT; i += BLK) tile[i] = a.alpha_pos[(int64_t)t0 * NINT + i];
-    __syncthreads();
-    if (act) {
-      const int lo = max(cs, t0), hi = min(ce, t0 + tn);
-      for (int pos = lo; pos < hi; ++pos) {
-        const u64* c = &tile[(pos - t0) * NINT];
-        int d = 0;
-#pragma unroll
-        for (int w = 0; w < NINT; ++w) d += popc64(my[w] ^ c[w]);
-        if (d == 2 || d == 4) {
-          if (FILL) {  // elements: k_pair_values (stored) or k_pair_sigma (direct)
-            if (cnt < a.cntA[k])
-              a.colidx[out + cnt] = pos;
-            else
-              atomicOr(a.err, 1);
-          }
-          ++cnt;
-        }
-      }
+  } else {
+    const int64_t step = ((int64_t)gridDim.x * BLK) >> 5;
+    const int64_t end = MODE == MODE_FILL ? a.row_hi : a.N;
+    const int64_t first = (MODE == MODE_FILL ? a.row_lo : 0) + (int64_t)blockIdx.x * (BLK / 32) + (threadIdx.x >> 5);
+#pragma unroll 1
+    for (int64_t k = first; k < end; k += step) {
+      if (MODE == MODE_FILL && (!dsel(a, k) || (a.pool && a.pos[CLS][k] >= 0))) continue;
+      row(k);
     }
   }
-  if (MODE == MODE_COUNT && valid && !keyed) a.cntA[k] = cnt;
 }
 
-// ---- class B: same alpha row, beta singles / doubles ----------------------
-template <int NINT, int MODE>
-__global__ void __launch_bounds__(BLK) k_class_b(BuildArgs a) {
-  constexpr bool FILL = MODE == MODE_FILL;
-  __shared__ u64 tile[TILE * NINT];
-  const int64_t q0 = (int64_t)blockIdx.x * BLK;
-  if (q0 >= a.N) return;
-  const int64_t q = q0 + threadIdx.x;
-  const bool valid = q < a.N;
-  int rs = 0, re = 0;
-  int64_t k = 0, out = 0;
-  u64 my[2 * NINT];
-  bool keyed = false;  // the row has a 2-deletion table: k_same_keyed takes it
-  if (valid) {
-    k = a.t_order[q];
-    const int ai = a.rows[k], bi = a.cols[k];
-    keyed = a.rowkey && (a.rowkey[ai] & KEY_DOUBLE);
-    rs = a.row_loc[ai];
-    re = a.row_loc[ai + 1];
-#pragma unroll
-    for (int w = 0; w < NINT; ++w) {
-      my[w] = a.alpha[(int64_t)ai * NINT + w];
-      my[NINT + w] = a.beta[(int64_t)bi * NINT + w];
+// Writes the hits of one class of a row after the other.
+template <int MODE, int CLS>
+struct RowOut {
+  int64_t at = 0, room = 0;  // MODE_POOL: this warp's place in the pool and what is left of its chunk
+  int* dst = nullptr;
+  int cnt = 0, cap = 0;
+  __device__ __forceinline__ void begin(const BuildArgs& a, int64_t k) {
+    cnt = 0;
+    if (MODE == MODE_POOL) {
+      dst = a.pool + at;
+    } else if (MODE == MODE_FILL) {
+      const int before = CLS == CLS_A ? 0 : CLS == CLS_B ? a.cnt[CLS_A][k] : a.cnt[CLS_A][k] + a.cnt[CLS_B][k];
+      dst = a.colidx + (a.rowptr[k] - a.col_base + before);
+      cap = CLS == CLS_C ? (int)(a.rowptr[k + 1] - a.rowptr[k]) - before : a.cnt[CLS][k];
     }
-    if (FILL) out = a.rowptr[k] + a.cntA[k] - a.col_base;
   }
-  int cnt = 0;
-  const bool act = valid && !keyed && (MODE == MODE_COUNT || dsel(a, k));
-  __shared__ int s_lo, s_hi;
-  if (threadIdx.x == 0) {
-    s_lo = INT_MAX;
-    s_hi = INT_MIN;
+  // lanes with `hit` append col (every lane calls)
+  __device__ __forceinline__ void put(const BuildArgs& a, bool hit, int col, int lane) {
+    const unsigned bal = __ballot_sync(0xffffffffu, hit);
+    const int n = __popc(bal);
+    if (MODE == MODE_POOL && cnt + n > room) grow(a, cnt + n, lane);
+    if (MODE != MODE_COUNT && hit) {
+      const int o = cnt + __popc(bal & ((1u << lane) - 1u));
+      if (MODE == MODE_POOL) {
+        if (dst) dst[o] = col;
+      } else if (o < cap) {
+        dst[o] = col;
+      } else {
+        atomicOr(a.err, 1 << CLS);
+      }
+    }
+    cnt += n;
   }
-  __syncthreads();
-  if (act) {
-    atomicMin(&s_lo, rs);
-    atomicMax(&s_hi, re);
+  // a new chunk for a row that does not fit the rest of the current one: what
+  // the row has so far moves over
+  __device__ __forceinline__ void grow(const BuildArgs& a, int need, int lane) {
+    const int64_t size = max((int64_t)a.pool_chunk[CLS], 2 * (int64_t)need);
+    unsigned long long o = 0;
+    if (lane == 0) o = atomicAdd(a.pool_next, (unsigned long long)size);
+    o = __shfl_sync(0xffffffffu, o, 0);
+    if (dst == nullptr || (int64_t)o + size > a.pool_cap) {  // full: go on counting
+      if (lane == 0) *a.pool_full = 1;
+      dst = nullptr;
+      at = 0;
+      room = INT64_MAX;
+      return;
+    }
+    int* to = a.pool + o;
+    __syncwarp();
+    for (int i = lane; i < cnt; i += 32) to[i] = dst[i];
+    __syncwarp();
+    dst = to;
+    at = (int64_t)o;
+    room = size;
   }
-  __syncthreads();
-  const int V0 = s_lo, V1 = s_hi;
-  for (int t0 = V0; t0 < V1; t0 += TILE) {
-    const int tn = min(TILE, V1 - t0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < tn * NINT; i += BLK) tile[i] = a.beta_tpos[(int64_t)t0 * NINT + i];
-    __syncthreads();
-    if (act) {
-      const int lo = max(rs, t0), hi = min(re, t0 + tn);
-      for (int pos = lo; pos < hi; ++pos) {
-        const u64* c = &tile[(pos - t0) * NINT];
-        int d = 0;
-#pragma unroll
-        for (int w = 0; w < NINT; ++w) d += popc64(my[NINT + w] ^ c[w]);
-        if (d == 2 || d == 4) {
-          if (FILL) {  // elements: k_pair_values (stored) or k_pair_sigma (direct)
-            if (cnt < a.cntB[k])
-              a.colidx[out + cnt] = a.tag_t ? (int)(QP_TAG_T | (unsigned)pos) : a.t_order[pos];
-            else
-              atomicOr(a.err, 2);
-          }
-          ++cnt;
-        }
+  __device__ __forceinline__ void end(const BuildArgs& a, int64_t k, int lane) {
+    if (MODE == MODE_FILL) return;
+    if (lane == 0) a.cnt[CLS][k] = cnt;
+    if (MODE == MODE_POOL) {
+      if (lane == 0) a.pos[CLS][k] = dst ? at : -1;
+      if (dst) {
+        at += cnt;
+        room -= cnt;
+      } else {
+        room = 0;
       }
     }
   }
-  if (MODE == MODE_COUNT && valid && !keyed) a.cntB[k] = cnt;
-}
+};
 
 // spin flip test of an alpha-single x beta-single pair: the two excitations
 // swap the same two orbitals between the spins (get_s2, s2.irp.f:46-55)
@@ -261,14 +235,10 @@ __device__ __forceinline__ bool spin_flip(const u64* my, const u64* ca, const u6
 // each group are the alpha (beta) singles of the row in that column (row).
 template <int NINT, int MODE>
 __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
-  constexpr bool FILL = MODE == MODE_FILL;
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5;
-  const int64_t nwarp = ((int64_t)gridDim.x * BLK) >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  for (int64_t k = warp; k < a.N; k += nwarp) {
-    if (MODE != MODE_COUNT && !dsel(a, k)) continue;
+  RowOut<MODE, CLS_C> out;
+  for_rows<MODE, CLS_C>(a, lane, [&](int64_t k) {
     const int ai = a.rows[k], bi = a.cols[k];
     u64 my[2 * NINT];
 #pragma unroll
@@ -276,46 +246,13 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
       my[w] = a.alpha[(int64_t)ai * NINT + w];
       my[NINT + w] = a.beta[(int64_t)bi * NINT + w];
     }
-    int64_t out = 0, sout = 0;
-    if (FILL) {
-      out = a.rowptr[k] + a.cntA[k] + a.cntB[k] - a.col_base;
-      sout = a.s2ptr[k];
-    }
-    int cnt = 0, scnt = 0;
+    out.begin(a, k);
+    int scnt = 0;
     // 32 candidates, one per lane: hit = (ca, cb) is an alpha single x beta
-    // single of the row; col is what the fill writes, jpos the bilinear position
-    auto step = [&](bool hit, const u64* ca, const u64* cb, int col, int jpos) {
-      const unsigned bal = __ballot_sync(FULL, hit);
-      const bool flip = hit && spin_flip<NINT>(my, ca, cb);
-      const unsigned sbal = __ballot_sync(FULL, flip);
-      if (FILL && hit) {  // elements: k_pair_values; S^2 values of spin flips here
-        const int64_t o = out + cnt + __popc(bal & lt);
-        if (o < a.rowptr[k + 1] - a.col_base)
-          a.colidx[o] = col;
-        else
-          atomicOr(a.err, 4);
-        if (flip && a.write_s2) {
-          u64 J[2 * NINT];
-#pragma unroll
-          for (int w = 0; w < NINT; ++w) {
-            J[w] = ca[w];
-            J[NINT + w] = cb[w];
-          }
-          u64 E[2 * NINT];
-          det_parity<NINT>(my, E);
-          double s2;
-          h_double_ab<NINT>(a.t, my, J, E, &s2, nullptr, nullptr);
-          const int64_t so = sout + scnt + __popc(sbal & lt);
-          if (so < a.s2ptr[k + 1]) {
-            a.s2col[so] = jpos;
-            a.s2val[so] = (float)s2;
-          } else {
-            atomicOr(a.err, 8);
-          }
-        }
-      }
-      cnt += __popc(bal);
-      scnt += __popc(sbal);
+    // single of the row, written as col
+    auto step = [&](bool hit, const u64* ca, const u64* cb, int col) {
+      if (MODE != MODE_FILL) scnt += __popc(__ballot_sync(FULL, hit && spin_flip<NINT>(my, ca, cb)));
+      out.put(a, hit, col, lane);
     };
     // Lines of the row's singles, 32 at a time: the lanes read the bounds of
     // 32 lines at once, and the candidates of the scanned ones are packed
@@ -359,7 +296,7 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
         u64 ca[NINT], cb[NINT];
 #pragma unroll
         for (int w = 0; w < NINT; ++w) ca[w] = cb[w] = 0;
-        int col = 0, jpos = 0;
+        int col = 0;
         if (ci < total) {
           const int pos = sbeg + (ci - (sinc - slen));
           int d = 0;
@@ -373,7 +310,7 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
             if (hit) {
 #pragma unroll
               for (int w = 0; w < NINT; ++w) cb[w] = a.beta[(int64_t)sln * NINT + w];
-              col = jpos = pos;
+              col = pos;
             }
           } else {  // row sln (an alpha single): beta singles of the row
 #pragma unroll
@@ -385,12 +322,11 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
             if (hit) {
 #pragma unroll
               for (int w = 0; w < NINT; ++w) ca[w] = a.alpha[(int64_t)sln * NINT + w];
-              jpos = a.t_order[pos];
-              col = a.tag_t ? (int)(QP_TAG_T | (unsigned)pos) : jpos;
+              if (MODE != MODE_COUNT) col = a.tag_t ? (int)(QP_TAG_T | (unsigned)pos) : a.t_order[pos];
             }
           }
         }
-        step(hit, ca, cb, col, jpos);
+        step(hit, ca, cb, col);
       }
       unsigned kb = __ballot_sync(FULL, kl);
       while (kb) {
@@ -452,7 +388,7 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
               u64 ca[NINT], cb[NINT];
 #pragma unroll
               for (int w = 0; w < NINT; ++w) ca[w] = cb[w] = 0;
-              int col = 0, jpos = 0;
+              int col = 0;
               if (pos >= kbeg && pos < kend) {
                 int d = 0;
                 bool eq = true;
@@ -470,68 +406,73 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
                     ca[w] = by_cols ? y[w] : fixed[w];
                     cb[w] = by_cols ? fixed[w] : y[w];
                   }
-                  if (by_cols) {
-                    col = jpos = pos;
-                  } else {
-                    jpos = a.t_order[pos];
-                    col = a.tag_t ? (int)(QP_TAG_T | (unsigned)pos) : jpos;
-                  }
+                  if (by_cols)
+                    col = pos;
+                  else if (MODE != MODE_COUNT)
+                    col = a.tag_t ? (int)(QP_TAG_T | (unsigned)pos) : a.t_order[pos];
                 }
               }
-              step(hit, ca, cb, col, jpos);
+              step(hit, ca, cb, col);
             }
           }
         }
       }
     }
-    if (MODE == MODE_COUNT && lane == 0) {
-      a.cntC[k] = cnt;
-      a.cntS[k] = scnt;
-    }
-  }
+    out.end(a, k, lane);
+    if (MODE != MODE_FILL && lane == 0) a.cntS[k] = scnt;
+  });
 }
 
-// ---- same-spin pairs of the rows of keyed lines, one warp per row ----------
-// SPIN 0: rows of a beta column with a 2-deletion table (class A), SPIN 1:
-// rows of an alpha row with one (class B).  The lanes probe 32 of the row's
-// C(ne,2) keys at a time; then the members of the 32 groups are packed into
-// full warp steps (most groups hold a few strings).
+// ---- same-spin pairs, one warp per row -------------------------------------
+// SPIN 0: the row's beta column (class A), SPIN 1: its alpha row (class B).
+// A line without a 2-deletion table is scanned, 32 strings a step.  In a line
+// with one the lanes probe 32 of the row's C(ne,2) keys at a time; then the
+// members of the 32 groups are packed into full warp steps (most groups hold
+// a few strings).
 // A member y of the key K of x is a double when |x ^ y| = 4 and x & y = K,
 // and a single when |x ^ y| = 2 and K is x & y without its lowest electron:
 // each pair is accepted under exactly one key, whatever the hash collisions.
+// (A thread per row of a line staged in shared memory took 140 us for each
+// fill of a 5,000 determinant set, whose longest line gave 20 blocks work.)
 template <int NINT, int MODE, int SPIN>
-__global__ void __launch_bounds__(BLK) k_same_keyed(BuildArgs a) {
-  constexpr bool FILL = MODE == MODE_FILL;
+__global__ void __launch_bounds__(BLK, 5) k_same(BuildArgs a) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int kind = SPIN == 0 ? KT_COL2 : KT_ROW2;
   const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5;
-  const int64_t nwarp = ((int64_t)gridDim.x * BLK) >> 5;
-  const unsigned lt = (1u << lane) - 1u;
   const KeyView kv = a.kv[kind];
   const int ne = SPIN == 0 ? a.t.na : a.t.nb;
   const int nc = ne * (ne - 1) / 2;
   const unsigned char* lflag = SPIN == 0 ? a.colkey : a.rowkey;
   const u64* strs = SPIN == 0 ? a.alpha_pos : a.beta_tpos;
-  const int64_t lo = MODE == MODE_COUNT ? 0 : a.row_lo, hi = MODE == MODE_COUNT ? a.N : a.row_hi;
-  if (lflag == nullptr) return;
-  for (int64_t k = lo + warp; k < hi; k += nwarp) {
+  constexpr int CLS = SPIN == 0 ? CLS_A : CLS_B;
+  RowOut<MODE, CLS> out;
+  for_rows<MODE, CLS>(a, lane, [&](int64_t k) {
     const int line = SPIN == 0 ? a.cols[k] : a.rows[k];
-    if (!(lflag[line] & KEY_DOUBLE)) continue;
-    if (MODE != MODE_COUNT && !dsel(a, k)) continue;
     u64 x[NINT];
 #pragma unroll
     for (int w = 0; w < NINT; ++w)
       x[w] = SPIN == 0 ? a.alpha_pos[k * NINT + w] : a.beta[(int64_t)a.cols[k] * NINT + w];
     const int ls = SPIN == 0 ? a.col_loc[line] : a.row_loc[line];
     const int le = SPIN == 0 ? a.col_loc[line + 1] : a.row_loc[line + 1];
-    int64_t out = 0;
-    int cap = 0;
-    if (FILL) {
-      out = a.rowptr[k] + (SPIN == 0 ? 0 : a.cntA[k]) - a.col_base;
-      cap = SPIN == 0 ? a.cntA[k] : a.cntB[k];
+    out.begin(a, k);
+    auto column = [&](int p) {
+      return MODE == MODE_COUNT || SPIN == 0 ? p : (a.tag_t ? (int)(QP_TAG_T | (unsigned)p) : a.t_order[p]);
+    };
+    if (!(lflag && (lflag[line] & KEY_DOUBLE))) {
+      for (int p0 = ls; p0 < le; p0 += 32) {
+        const int p = p0 + lane;
+        bool hit = false;
+        if (p < le) {
+          int d = 0;
+#pragma unroll
+          for (int w = 0; w < NINT; ++w) d += popc64(x[w] ^ strs[(int64_t)p * NINT + w]);
+          hit = d == 2 || d == 4;
+        }
+        out.put(a, hit, hit ? column(p) : 0, lane);
+      }
+      out.end(a, k, lane);
+      return;
     }
-    int cnt = 0;
     for (int c0 = 0; c0 < nc; c0 += 32) {
       unsigned gs = 0, gl = 0;
       u64 K[NINT];
@@ -568,52 +509,283 @@ __global__ void __launch_bounds__(BLK) k_same_keyed(BuildArgs a) {
         u64 Kr[NINT];
 #pragma unroll
         for (int w = 0; w < NINT; ++w) Kr[w] = __shfl_sync(FULL, K[w], src);
-        {
-          const unsigned t = (unsigned)(mi - i0);
-          bool hit = false;
-          int p = 0;
-          if (mi < tot) {
-            p = kv.mem[s0 + t];
-            const bool dup = t > 0 && kv.mem[s0 + t - 1] == p;
-            if (!dup && p >= ls && p < le) {
-              u64 m[NINT];
-              int d = 0;
+        const unsigned t = (unsigned)(mi - i0);
+        bool hit = false;
+        int p = 0;
+        if (mi < tot) {
+          p = kv.mem[s0 + t];
+          const bool dup = t > 0 && kv.mem[s0 + t - 1] == p;
+          if (!dup && p >= ls && p < le) {
+            u64 m[NINT];
+            int d = 0;
 #pragma unroll
-              for (int w = 0; w < NINT; ++w) {
-                const u64 y = strs[(int64_t)p * NINT + w];
-                d += popc64(x[w] ^ y);
-                m[w] = x[w] & y;
-              }
-              if (d == 2) {  // canonical key of a single: drop the lowest common electron
-                bool done = false;
+            for (int w = 0; w < NINT; ++w) {
+              const u64 y = strs[(int64_t)p * NINT + w];
+              d += popc64(x[w] ^ y);
+              m[w] = x[w] & y;
+            }
+            if (d == 2) {  // canonical key of a single: drop the lowest common electron
+              bool done = false;
 #pragma unroll
-                for (int w = 0; w < NINT; ++w)
-                  if (!done && m[w]) {
-                    m[w] &= m[w] - 1;
-                    done = true;
-                  }
-              }
-              if (d == 2 || d == 4) {
-                bool eq = true;
+              for (int w = 0; w < NINT; ++w)
+                if (!done && m[w]) {
+                  m[w] &= m[w] - 1;
+                  done = true;
+                }
+            }
+            if (d == 2 || d == 4) {
+              bool eq = true;
 #pragma unroll
-                for (int w = 0; w < NINT; ++w) eq &= m[w] == Kr[w];
-                hit = eq;
-              }
+              for (int w = 0; w < NINT; ++w) eq &= m[w] == Kr[w];
+              hit = eq;
             }
           }
-          const unsigned bal = __ballot_sync(FULL, hit);
-          if (FILL && hit) {
-            const int o = cnt + __popc(bal & lt);
-            if (o < cap)
-              a.colidx[out + o] = SPIN == 0 ? p : (a.tag_t ? (int)(QP_TAG_T | (unsigned)p) : a.t_order[p]);
-            else
-              atomicOr(a.err, SPIN == 0 ? 1 : 2);
-          }
-          cnt += __popc(bal);
         }
+        out.put(a, hit, hit ? column(p) : 0, lane);
       }
     }
-    if (MODE == MODE_COUNT && lane == 0) (SPIN == 0 ? a.cntA : a.cntB)[k] = cnt;
+    out.end(a, k, lane);
+  });
+}
+
+// ---- each row's columns, ascending -----------------------------------------
+// Neighbouring lanes of the sigma gathers then read neighbouring coefficients,
+// whatever order the scans found the partners in.  Bitonic networks in
+// registers: element i of a row sits in register i % R of lane i / R, so of
+// the 55 steps of 1,024 elements 40 run inside a thread, 15 across lanes and
+// none needs shared memory; rows of 1,025 to 16,384 elements add exchanges between
+// up to 16 such warps through shared memory, longer ones go to a segmented
+// radix sort.  991M columns at 1e6 determinants: 10.2 ms (7.2 of them in the
+// rows of 2,049 to 4,096), against 43.2 ms for a segmented sort of every row.
+constexpr int SORT_WARP = 1024;          // elements of a warp
+constexpr int SORT_PAD = SORT_WARP + SORT_WARP / 32;
+
+// ascending merge of each thread's R registers (a bitonic run), steps J, J/2, ..., 1
+template <int R, int J = R / 2>
+__device__ __forceinline__ void merge_regs(unsigned (&v)[R]) {
+  if constexpr (J > 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if ((r & J) == 0) {
+        const unsigned lo = min(v[r], v[r | J]), hi = max(v[r], v[r | J]);
+        v[r] = lo;
+        v[r | J] = hi;
+      }
+    merge_regs<R, J / 2>(v);
+  }
+}
+// runs of K < R registers, their directions alternating (compile-time steps:
+// an array indexed by a loop variable would go to local memory)
+template <int R, int K, int J>
+__device__ __forceinline__ void short_runs(unsigned (&v)[R]) {
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if ((r & J) == 0) {
+      const unsigned lo = min(v[r], v[r | J]), hi = max(v[r], v[r | J]);
+      v[r] = (r & K) == 0 ? lo : hi;
+      v[r | J] = (r & K) == 0 ? hi : lo;
+    }
+  if constexpr (J > 1) short_runs<R, K, J / 2>(v);
+  else if constexpr (2 * K < R) short_runs<R, 2 * K, K>(v);
+}
+template <int R>
+__device__ __forceinline__ void flip(unsigned (&v)[R], unsigned m) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] ^= m;
+}
+// A bitonic run of `lanes` lanes, ascending: strides over lanes, then inside a
+// thread.  The loops stay loops: the network written out is 56 KB of
+// instructions, which the warps of an SM then fetch at different places.
+template <int R>
+__device__ __forceinline__ void merge_lanes(unsigned (&v)[R], int lane, int lanes) {
+#pragma unroll 1
+  for (int j = lanes / 2; j > 0; j >>= 1) {
+    const bool low = (lane & j) == 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const unsigned o = __shfl_xor_sync(0xffffffffu, v[r], j);
+      v[r] = low ? min(v[r], o) : max(v[r], o);
+    }
+  }
+  merge_regs<R>(v);
+}
+// The 32 R elements of a warp (element i in register i % R of lane i / R),
+// ascending when `up`.  A descending run is an ascending one of the
+// complements, so only the signs of the values change with the direction.
+template <int R>
+__device__ __forceinline__ void sort_warp(unsigned (&v)[R], int lane, bool up) {
+  if constexpr (R > 2) short_runs<R, 2, 1>(v);
+  unsigned m = 0;
+#pragma unroll 1
+  for (int lanes = 1; lanes <= 32; lanes <<= 1) {
+    const unsigned want = (lanes == 32 ? up : (lane & lanes) == 0) ? 0u : 0xffffffffu;
+    flip<R>(v, m ^ want);
+    m = want;
+    merge_lanes<R>(v, lane, lanes);
+  }
+  flip<R>(v, m);
+}
+// a bitonic sequence of 32 R elements, ascending when `up`
+template <int R>
+__device__ __forceinline__ void merge_warp(unsigned (&v)[R], int lane, bool up) {
+  const unsigned m = up ? 0u : 0xffffffffu;
+  flip<R>(v, m);
+  merge_lanes<R>(v, lane, 32);
+  flip<R>(v, m);
+}
+
+// hit i of row k: from the pool (classes one after the other) or its place in the CSR
+struct RowSrc {
+  const int* src[3];
+  int n0 = INT_MAX, n1 = INT_MAX;
+  __device__ __forceinline__ RowSrc(const BuildArgs& a, int64_t k) {
+    src[0] = src[1] = src[2] = a.colidx + a.rowptr[k];
+    if (a.pool) {
+      n0 = a.cnt[CLS_A][k];
+      n1 = n0 + a.cnt[CLS_B][k];
+      const int64_t p0 = a.pos[CLS_A][k], p1 = a.pos[CLS_B][k], p2 = a.pos[CLS_C][k];
+      if (p0 >= 0) src[0] = a.pool + p0;
+      if (p1 >= 0) src[1] = a.pool + p1 - n0;
+      if (p2 >= 0) src[2] = a.pool + p2 - n1;
+    }
+  }
+  __device__ __forceinline__ unsigned at(int i) const {
+    const int* p = i < n0 ? src[0] : i < n1 ? src[1] : src[2];
+    return (unsigned)p[i];
+  }
+};
+
+template <int R>
+__device__ __forceinline__ void sort_row_small(const RowSrc& row, int* out, int n, int lane, unsigned* sm) {
+  unsigned v[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = r * 32 + lane < n ? row.at(r * 32 + lane) : 0xffffffffu;
+  sort_warp<R>(v, lane, true);
+  if constexpr (R == 1) {
+    if (lane < n) out[lane] = (int)v[0];
+  } else {
+    // element lane R + r -> coalesced writes (one pad word in 32 keeps the banks apart)
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = lane * R + r;
+      sm[i + (i >> 5)] = v[r];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = r * 32 + lane;
+      if (i < n) out[i] = (int)sm[i + (i >> 5)];
+    }
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(BLK, 3) k_sort_rows(BuildArgs a) {
+  __shared__ unsigned sm[BLK / 32][SORT_PAD];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t warp = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5;
+  const int64_t nwarp = ((int64_t)gridDim.x * BLK) >> 5;
+  for (int64_t k = warp; k < a.N; k += nwarp) {
+    const int64_t e0 = a.rowptr[k], n64 = a.rowptr[k + 1] - e0;
+    if (n64 == 0 || n64 > SORT_WARP) continue;
+    const int n = (int)n64;
+    const RowSrc row(a, k);
+    int* out = a.colidx + e0;
+    if (n <= 32)
+      sort_row_small<1>(row, out, n, lane, sm[w]);
+    else if (n <= 128)
+      sort_row_small<4>(row, out, n, lane, sm[w]);
+    else if (n <= 256)
+      sort_row_small<8>(row, out, n, lane, sm[w]);
+    else if (n <= 512)
+      sort_row_small<16>(row, out, n, lane, sm[w]);
+    else
+      sort_row_small<32>(row, out, n, lane, sm[w]);
+  }
+}
+
+// rows of more than 512 W and at most 1024 W columns, a block of W warps each;
+// the rows (in any order) and their number come from k_long_rows
+template <int W>
+__global__ void __launch_bounds__(W * 32, W <= 8 ? 24 / W : 1) k_sort_rows_block(BuildArgs a, const int* list, const int* n_list) {
+  extern __shared__ unsigned smem[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int nl = *n_list;
+  for (int q = blockIdx.x; q < nl; q += gridDim.x) {
+    const int64_t k = list[q];
+    const int64_t e0 = a.rowptr[k];
+    const int n = (int)(a.rowptr[k + 1] - e0);
+    const RowSrc row(a, k);
+    unsigned v[32];
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+      const int i = w * SORT_WARP + r * 32 + lane;
+      v[r] = i < n ? row.at(i) : 0xffffffffu;
+    }
+    sort_warp<32>(v, lane, (w & 1) == 0);
+#pragma unroll 1
+    for (int kw = 2; kw <= W; kw <<= 1) {  // runs of kw warps
+      const bool up = (w & kw) == 0;
+#pragma unroll 1
+      for (int jw = kw / 2; jw > 0; jw >>= 1) {
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 32; ++r) smem[w * SORT_PAD + r * 32 + lane] = v[r];
+        __syncthreads();
+        const bool low = ((w & jw) == 0) == up;
+#pragma unroll
+        for (int r = 0; r < 32; ++r) {
+          const unsigned o = smem[(w ^ jw) * SORT_PAD + r * 32 + lane];
+          v[r] = low ? min(v[r], o) : max(v[r], o);
+        }
+      }
+      merge_warp<32>(v, lane, up);
+    }
+    __syncthreads();
+    unsigned* sw = smem + w * SORT_PAD;
+#pragma unroll
+    for (int r = 0; r < 32; ++r) sw[lane * 33 + r] = v[r];
+    __syncwarp();
+    int* out = a.colidx + e0;
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+      const int i = r * 32 + lane;
+      if (w * SORT_WARP + i < n) out[w * SORT_WARP + i] = (int)sw[i + (i >> 5)];
+    }
+    __syncthreads();
+  }
+}
+
+// rows longer than SORT_WARP, by the block that sorts them: list[b cap + ...],
+// b = 0..3 for 2, 4, 8, 16 warps, b = 4 for the segmented sort, whose rows'
+// lengths follow at list[5 cap + ...]
+constexpr int SORT_BINS = 5;
+__global__ void k_long_rows(const int64_t* rowptr, int64_t N, int64_t cap, int* list, int* n) {
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N; k += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t len = rowptr[k + 1] - rowptr[k];
+    if (len <= SORT_WARP) continue;
+    int b = 0;
+    while (b < SORT_BINS - 1 && len > (int64_t)SORT_WARP * (2 << b)) ++b;
+    const int o = atomicAdd(&n[b], 1);
+    if (o >= cap) continue;
+    list[b * cap + o] = (int)k;
+    if (b == SORT_BINS - 1) list[SORT_BINS * cap + o] = (int)len;
+  }
+}
+
+// the columns of listed rows, one block per row: into tmp at off[q], or back
+__global__ void k_gather_rows(BuildArgs a, const int* list, const int* off, int nl, int* tmp) {
+  for (int q = blockIdx.x; q < nl; q += gridDim.x) {
+    const RowSrc row(a, list[q]);
+    const int n = off[q + 1] - off[q];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) tmp[off[q] + i] = (int)row.at(i);
+  }
+}
+__global__ void k_scatter_rows(BuildArgs a, const int* list, const int* off, int nl, const int* tmp) {
+  for (int q = blockIdx.x; q < nl; q += gridDim.x) {
+    int* out = a.colidx + a.rowptr[list[q]];
+    const int n = off[q + 1] - off[q];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) out[i] = tmp[off[q] + i];
   }
 }
 
@@ -641,109 +813,155 @@ struct Deferred {
   }
 };
 
-// FP64 / FP32 elements of the stored pairs, after the fill pass has written
-// their columns: one warp per row, lanes over the row's pairs, so that the
-// dependent integral loads of 32 pairs are in flight at once (the fill's
-// scanning thread would evaluate its row's pairs one after the other).  The
-// columns are ascending, so the same-beta partners are one run (the row's own
-// beta column); same-alpha partners are told by their alpha id, and only the
-// string that differs is read.  Each class calls the same Slater routine with
-// the same arguments as the scans do, so the values are bit-identical.
-// Same-alpha pairs and single excitations (whose sums over the holes and
-// particles against the reference take several times a double's loads) are
-// deferred until 32 of a kind are there: with them inline almost every trip
-// paid for all branches.  991M pairs at 1e6 determinants: 35.4 -> 30.8 ms.
+// both strings of a determinant in one load (det_pos / det_tpos: 16 or 32 bytes a row)
 template <int NINT>
-__global__ void __launch_bounds__(BLK) k_pair_values(BuildArgs a) {
+__device__ __forceinline__ void load_det(const u64* det, int64_t p, u64 (&J)[2 * NINT]) {
+  if constexpr (NINT == 1) {
+    const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(det) + p);
+    J[0] = x.x;
+    J[1] = x.y;
+  } else {
+    asm("ld.global.nc.v4.u64 {%0,%1,%2,%3}, [%4];"
+        : "=l"(J[0]), "=l"(J[1]), "=l"(J[2]), "=l"(J[3])
+        : "l"(det + p * 4));
+  }
+}
+
+// FP64 / FP32 elements of the stored pairs, after their columns are in place:
+// one warp per row, lanes over the row's pairs, so that the integral loads of
+// 32 pairs are in flight at once.  A partner's two strings sit in one 32-byte
+// sector (det_pos): with the strings behind the beta id, a pair took four
+// requests and a chain of three dependent loads before its integral.  Each
+// class calls the same Slater routine with the same arguments as the scans
+// do, so the values are bit-identical.  Single excitations (whose sums over
+// the holes and particles against the reference take several times a double's
+// loads), and same-spin doubles where they are few in a trip, are deferred
+// until 32 of a kind are there (a row's own beta column is one run of its
+// ascending columns, whose trips take them at once).  The spin-flip pairs of the alpha x beta class are listed here, and
+// the row's sum of squared elements gives the coupling feature of the learned
+// step (log10(sum_J H_IJ^2) / 4), which took a pass of its own (4.2 ms).
+// 991M pairs at 1e6 determinants: 30.8 -> 22.9 ms; bound by the integer
+// instructions of the Slater routines (about 400 a pair, 45 % issue) with the
+// L2 latency of the integrals.
+template <int NINT>
+__global__ void __launch_bounds__(BLK, 4) k_pair_values(BuildArgs a) {
   __shared__ int s_q[BLK / 32][2][DEFER];
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const int64_t warp = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5;
   const int64_t nwarp = ((int64_t)gridDim.x * BLK) >> 5;
-  Deferred same_alpha{s_q[threadIdx.x >> 5][0], 0}, mono{s_q[threadIdx.x >> 5][1], 0};
+  Deferred same{s_q[threadIdx.x >> 5][0], 0}, mono{s_q[threadIdx.x >> 5][1], 0};
   for (int64_t k = warp; k < a.N; k += nwarp) {
     u64 my[2 * NINT], E[2 * NINT];
-    const int bi = a.cols[k], ai = a.rows[k];
-    const int cs = a.col_loc[bi], ce = a.col_loc[bi + 1];
-#pragma unroll
-    for (int w = 0; w < NINT; ++w) {
-      my[w] = a.alpha_pos[k * NINT + w];
-      my[NINT + w] = a.beta[(int64_t)bi * NINT + w];
-    }
+    load_det<NINT>(a.det_pos, k, my);
     det_parity<NINT>(my, E);
     const int64_t e0 = a.rowptr[k];
     const int n = (int)(a.rowptr[k + 1] - e0);
+    const int64_t s0 = a.s2ptr[k];
+    const int ns2 = (int)(a.s2ptr[k + 1] - s0);
+    int scnt = 0;
+    double sum2 = 0.0;
     auto put = [&](int x, double v) {
       a.val64[e0 + x] = v;
       a.val32[e0 + x] = (float)v;
+      sum2 = fma(v, v, sum2);
     };
     auto do_mono = [&](int x) {  // one string differs, by one electron
       if (x < 0) return;
-      const int j = a.colidx[e0 + x];
-      const bool beta = j < cs || j >= ce;
       u64 J[2 * NINT];
-      const int bj = beta ? a.cols[j] : bi;
+      load_det<NINT>(a.det_pos, a.colidx[e0 + x], J);
+      bool beta = true;
 #pragma unroll
-      for (int w = 0; w < NINT; ++w) {
-        J[w] = beta ? my[w] : a.alpha_pos[(int64_t)j * NINT + w];
-        J[NINT + w] = beta ? a.beta[(int64_t)bj * NINT + w] : my[NINT + w];
-      }
+      for (int w = 0; w < NINT; ++w) beta &= my[w] == J[w];
       put(x, h_mono_spin<NINT>(a.t, my, J, E, beta ? 2 : 1, nullptr, nullptr));
     };
-    auto do_same_alpha = [&](int x) -> bool {  // true: a single
-      if (x < 0) return false;
-      const int bj = a.cols[a.colidx[e0 + x]];
-      u64 J[NINT];
+    auto same_spin = [&](int x, const u64 (&J)[2 * NINT]) -> bool {  // true: a single
+      bool beta = true;
       int d = 0;
 #pragma unroll
+      for (int w = 0; w < NINT; ++w) beta &= my[w] == J[w];
+      u64 si[NINT], sj[NINT], Es[NINT];
+#pragma unroll
       for (int w = 0; w < NINT; ++w) {
-        J[w] = a.beta[(int64_t)bj * NINT + w];
-        d += popc64(my[NINT + w] ^ J[w]);
+        si[w] = beta ? my[NINT + w] : my[w];
+        sj[w] = beta ? J[NINT + w] : J[w];
+        Es[w] = beta ? E[NINT + w] : E[w];
+        d += popc64(si[w] ^ sj[w]);
       }
       if (d == 2) return true;
-      put(x, h_double_spin<NINT>(a.t, my + NINT, J, E + NINT, nullptr, nullptr));
+      put(x, h_double_spin<NINT>(a.t, si, sj, Es, nullptr, nullptr));
       return false;
     };
+    auto do_same = [&](int x) -> bool {
+      if (x < 0) return false;
+      u64 J[2 * NINT];
+      load_det<NINT>(a.det_pos, a.colidx[e0 + x], J);
+      return same_spin(x, J);
+    };
+    int j = lane < n ? a.colidx[e0 + lane] : -1;
     for (int x0 = 0; x0 < n; x0 += 32) {
       const int x = x0 + lane;
-      const bool in = x < n;
-      const int j = in ? a.colidx[e0 + x] : -1;
-      bool is_b = false, is_mono = false;
-      if (in && j >= cs && j < ce) {  // same beta column
-        u64 J[NINT];
-        int d = 0;
+      const int jn = x + 32 < n ? a.colidx[e0 + x + 32] : -1;  // the next trip's column
+      bool is_same = false, flip = false;
+      double s2 = 0.0;
+      u64 J[2 * NINT];
+      if (j >= 0) {
+        load_det<NINT>(a.det_pos, j, J);
+        bool samea = true, sameb = true;
 #pragma unroll
         for (int w = 0; w < NINT; ++w) {
-          J[w] = a.alpha_pos[(int64_t)j * NINT + w];
-          d += popc64(my[w] ^ J[w]);
+          samea &= J[w] == my[w];
+          sameb &= J[NINT + w] == my[NINT + w];
         }
-        is_mono = d == 2;
-        if (!is_mono) put(x, h_double_spin<NINT>(a.t, my, J, E, nullptr, nullptr));
-      } else if (in) {
-        is_b = a.rows[j] == ai;  // same alpha row
-        if (!is_b) {             // alpha single x beta single
-          const int bj = a.cols[j];
-          u64 J[2 * NINT];
-#pragma unroll
-          for (int w = 0; w < NINT; ++w) {
-            J[w] = a.alpha_pos[(int64_t)j * NINT + w];
-            J[NINT + w] = a.beta[(int64_t)bj * NINT + w];
+        is_same = samea || sameb;
+        if (!is_same) put(x, h_double_ab<NINT>(a.t, my, J, E, &s2, nullptr, nullptr));
+      }
+      if (ns2 > 0) {
+        flip = s2 != 0.0;
+        const unsigned fb = __ballot_sync(0xffffffffu, flip);
+        if (flip) {
+          const int o = scnt + __popc(fb & lt);
+          if (o < ns2) {
+            a.s2col[s0 + o] = j;
+            a.s2val[s0 + o] = (float)s2;
           }
-          double s2;
-          put(x, h_double_ab<NINT>(a.t, my, J, E, &s2, nullptr, nullptr));
         }
+        scnt += __popc(fb);
       }
-      if (mono.push(is_mono, x, lt)) do_mono(mono.pop(lane));
-      if (same_alpha.push(is_b, x, lt)) {
-        const int y = same_alpha.pop(lane);
-        if (mono.push(do_same_alpha(y), y, lt)) do_mono(mono.pop(lane));
+      if (__popc(__ballot_sync(0xffffffffu, is_same)) >= 12) {
+        if (mono.push(is_same && same_spin(x, J), x, lt)) do_mono(mono.pop(lane));
+      } else if (same.push(is_same, x, lt)) {
+        const int y = same.pop(lane);
+        if (mono.push(do_same(y), y, lt)) do_mono(mono.pop(lane));
       }
+      j = jn;
     }
     {
-      const int y = same_alpha.pop(lane);
-      if (mono.push(do_same_alpha(y), y, lt)) do_mono(mono.pop(lane));
+      const int y = same.pop(lane);
+      if (mono.push(do_same(y), y, lt)) do_mono(mono.pop(lane));
     }
     do_mono(mono.pop(lane));
+    if (scnt != ns2 && lane == 0) atomicOr(a.err, 8);
+    if (a.feat) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
+      if (lane == 0) a.feat[k].w = (float)(log10(sum2 + 1e-30) * 0.25);
+    }
+  }
+}
+
+// out[p] = strings of the determinant at bilinear position p (perm null) or at
+// alpha-major position p (perm = t_order)
+template <int NINT>
+__global__ void k_det_pos(const u64* alpha, const u64* beta, const int* rows, const int* cols, const int* perm,
+                          u64* out, int64_t N) {
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = perm ? perm[p] : p;
+#pragma unroll
+    for (int w = 0; w < NINT; ++w) {
+      out[p * 2 * NINT + w] = alpha[(int64_t)rows[k] * NINT + w];
+      out[p * 2 * NINT + NINT + w] = beta[(int64_t)cols[k] * NINT + w];
+    }
   }
 }
 
@@ -800,8 +1018,6 @@ BuildArgs index_args(const qpgpu_ctx* c) {
   a.row_first = 0;
   a.row_step = 1;
   a.col_base = 0;
-  a.blk_off = 0;
-  a.write_s2 = 1;
   a.tag_t = 0;
   for (int t = 0; t < KT_N; ++t) {
     a.kv[t].slot = c->d_kslot[t];
@@ -810,58 +1026,95 @@ BuildArgs index_args(const qpgpu_ctx* c) {
   }
   a.colkey = c->d_colkey;
   a.rowkey = c->d_rowkey;
-  a.hmask = c->key_hash_bits >= 64 ? ~0ull : ((1ull << std::max(1, c->key_hash_bits)) - 1ull);
+  a.hmask = qp_key_mask(c);
   return a;
 }
 
-__global__ void k_rel_offsets(const int64_t* rowptr, int64_t base, int* out, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = (int)(rowptr[i] - base);
+template <int W>
+int sort_block_bin(qpgpu_ctx* c, const BuildArgs& a, const int* list, const int* n_list, int n) {
+  if (n == 0) return 0;
+  const int smem = W * SORT_PAD * (int)sizeof(unsigned);
+  if (smem > 48 * 1024)
+    QP_CUDA(c, cudaFuncSetAttribute(k_sort_rows_block<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k_sort_rows_block<W><<<(unsigned)std::min(n, c->n_sm * 64), W * 32, smem, c->stream>>>(a, list, n_list);
+  return 0;
 }
 
-// Each row's columns in ascending order (stored pairs, before the elements
-// are evaluated): neighbouring lanes of the sigma gathers then read
-// neighbouring coefficients, whatever order the scans and the deletion-key
-// probes found the partners in.  Segmented sorts over batches of rows of at
-// most 2^30 pairs.
-int sort_row_columns(qpgpu_ctx* c) {
-  const int64_t N = c->N, P = c->P;
+// every row's columns to their place in the CSR, ascending (from the pool, or
+// in place when a.pool is null)
+int sort_row_columns(qpgpu_ctx* c, const BuildArgs& a) {
+  const int64_t N = c->N;
   cudaStream_t st = c->stream;
-  if (P == 0) return 0;
-  std::vector<int64_t> rp(N + 1);
-  QP_CUDA(c, cudaMemcpyAsync(rp.data(), c->d_rowptr, (N + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  if (c->P == 0) return 0;
+  k_sort_rows<<<nblocks(N * 32, BLK), BLK, 0, st>>>(a);
+  // at most P / 1025 rows are longer than a warp's share
+  const int64_t cap = std::min<int64_t>(N, c->P / (SORT_WARP + 1));
+  if (cap == 0) return 0;
+  Scoped<int> list(c), num(c);
+  QP_CUDA(c, list.alloc((size_t)(SORT_BINS + 1) * cap));
+  QP_CUDA(c, num.alloc(SORT_BINS));
+  QP_CUDA(c, cudaMemsetAsync(num.p, 0, SORT_BINS * sizeof(int), st));
+  k_long_rows<<<std::min(nblocks(N, 256), (unsigned)c->n_sm * 8), 256, 0, st>>>(c->d_rowptr, N, cap, list.p, num.p);
+  int hn[SORT_BINS];
+  QP_CUDA(c, cudaMemcpyAsync(hn, num.p, sizeof(hn), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
-  const int64_t cap = std::min<int64_t>(P, (int64_t)1 << 30);
-  Scoped<int> tmp(c), offs(c);
-  Scoped<char> work(c);
-  size_t work_bytes = 0;
-  QP_CUDA(c, tmp.alloc((size_t)cap));
-  QP_CUDA(c, offs.alloc((size_t)N + 1));
-  for (int64_t r0 = 0; r0 < N;) {
-    int64_t r1 = std::upper_bound(rp.begin() + r0 + 1, rp.end(), rp[r0] + cap) - rp.begin() - 1;
-    if (r1 <= r0) r1 = r0 + 1;
-    const int64_t base = rp[r0], n = rp[r1] - base;
-    if (n > cap) return qpgpu_fail(c, QPGPU_ERR_NOMEM, "a row holds more than 2^30 pairs");
-    if (n > 0) {
-      k_rel_offsets<<<nblocks(r1 - r0 + 1, 256), 256, 0, st>>>(c->d_rowptr + r0, base, offs.p, r1 - r0 + 1);
-      size_t tb = 0;
-      QP_CUDA(c, cub::DeviceSegmentedSort::SortKeys(nullptr, tb, c->d_colidx + base, tmp.p, (int)n, (int)(r1 - r0),
-                                                    offs.p, offs.p + 1, st));
-      if (tb > work_bytes) {
-        qp_pool_free(c, work.p);
-        work.p = nullptr;
-        QP_CUDA(c, work.alloc(tb));
-        work_bytes = tb;
-      }
-      QP_CUDA(c, cub::DeviceSegmentedSort::SortKeys(work.p, tb, c->d_colidx + base, tmp.p, (int)n, (int)(r1 - r0),
-                                                    offs.p, offs.p + 1, st));
-      QP_CUDA(c, cudaMemcpyAsync(c->d_colidx + base, tmp.p, (size_t)n * sizeof(int), cudaMemcpyDeviceToDevice, st));
-    }
-    r0 = r1;
-  }
+  int rc = sort_block_bin<2>(c, a, list.p, num.p, hn[0]);
+  if (!rc) rc = sort_block_bin<4>(c, a, list.p + cap, num.p + 1, hn[1]);
+  if (!rc) rc = sort_block_bin<8>(c, a, list.p + 2 * cap, num.p + 2, hn[2]);
+  if (!rc) rc = sort_block_bin<16>(c, a, list.p + 3 * cap, num.p + 3, hn[3]);
+  if (rc) return rc;
   QP_CUDA(c, cudaGetLastError());
+  if (hn[4] == 0) return 0;
+  // the few rows beyond a block: gathered into one buffer, at most 2^28
+  // columns (or one row) at a time, sorted as segments and written back
+  const int* lrow = list.p + 4 * cap;
+  std::vector<int> len(hn[4]);
+  QP_CUDA(c, cudaMemcpyAsync(len.data(), lrow + cap, len.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
+  for (size_t q0 = 0; q0 < len.size();) {
+    std::vector<int> off{0};
+    size_t q1 = q0;
+    int64_t sum = 0;
+    while (q1 < len.size() && (q1 == q0 || sum + len[q1] <= ((int64_t)1 << 28))) {
+      sum += len[q1++];
+      if (sum >= ((int64_t)1 << 31) - 1) return qpgpu_fail(c, QPGPU_ERR_NOMEM, "a row holds more than 2^31 pairs");
+      off.push_back((int)sum);
+    }
+    const int nl = (int)(q1 - q0);
+    Scoped<int> doff(c), t0(c), t1(c);
+    Scoped<char> work(c);
+    QP_CUDA(c, doff.alloc(off.size()));
+    QP_CUDA(c, t0.alloc((size_t)sum));
+    QP_CUDA(c, t1.alloc((size_t)sum));
+    QP_CUDA(c, cudaMemcpyAsync(doff.p, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+    k_gather_rows<<<(unsigned)std::min(nl, 65535), 512, 0, st>>>(a, lrow + q0, doff.p, nl, t0.p);
+    size_t tb = 0;
+    QP_CUDA(c, cub::DeviceSegmentedSort::SortKeys(nullptr, tb, t0.p, t1.p, (int)sum, nl, doff.p, doff.p + 1, st));
+    QP_CUDA(c, work.alloc(tb));
+    QP_CUDA(c, cub::DeviceSegmentedSort::SortKeys(work.p, tb, t0.p, t1.p, (int)sum, nl, doff.p, doff.p + 1, st));
+    k_scatter_rows<<<(unsigned)std::min(nl, 65535), 512, 0, st>>>(a, lrow + q0, doff.p, nl, t1.p);
+    QP_CUDA(c, cudaGetLastError());
+    QP_CUDA(c, cudaStreamSynchronize(st));  // off is read by the copy
+    q0 = q1;
+  }
   return 0;
+}
+
+// the scans of all three classes; a pool pass runs as many blocks as are
+// resident (six per SM of the same-spin scans, three of the alpha x beta
+// one, by their registers)
+template <int NINT, int MODE>
+void launch_scans(qpgpu_ctx* c, const BuildArgs& a) {
+  cudaStream_t st = c->stream;
+  const unsigned g = nblocks(c->N * 32, BLK);
+  const unsigned gs = MODE == MODE_POOL ? std::min(g, (unsigned)c->n_sm * 6) : g;
+  const unsigned gc = MODE == MODE_POOL ? std::min(g, (unsigned)c->n_sm * 3) : g;
+  k_same<NINT, MODE, 0><<<gs, BLK, 0, st>>>(a);
+  qp_mark(c, "scan A (same beta)");
+  k_same<NINT, MODE, 1><<<gs, BLK, 0, st>>>(a);
+  qp_mark(c, "scan B (same alpha)");
+  k_class_c<NINT, MODE><<<gc, BLK, 0, st>>>(a);
+  qp_mark(c, "scan C (alpha x beta)");
 }
 
 template <int NINT>
@@ -869,26 +1122,58 @@ int build_pairs_t(qpgpu_ctx* c) {
   const int64_t N = c->N;
   cudaStream_t st = c->stream;
   BuildArgs a = index_args(c);
-  Scoped<int> cA(c), cB(c), cC(c), cS(c);
+  Scoped<int> cA(c), cB(c), cC(c), cS(c), pool(c);
+  Scoped<int64_t> pos(c);
+  Scoped<unsigned long long> ctr(c);
   QP_CUDA(c, cA.alloc(N));
   QP_CUDA(c, cB.alloc(N));
   QP_CUDA(c, cC.alloc(N));
   QP_CUDA(c, cS.alloc(N));
-  a.cntA = cA.p;
-  a.cntB = cB.p;
-  a.cntC = cC.p;
+  QP_CUDA(c, ctr.alloc(8));  // next row of each class; next free entry of the pool; its full flag
+  QP_CUDA(c, cudaMemsetAsync(ctr.p, 0, 8 * sizeof(unsigned long long), st));
+  a.cnt[CLS_A] = cA.p;
+  a.cnt[CLS_B] = cB.p;
+  a.cnt[CLS_C] = cC.p;
   a.cntS = cS.p;
-  const unsigned gAB = nblocks(N, BLK);
-  const unsigned gC = nblocks(N * 32, BLK);
+  a.next_row = ctr.p;
+  a.pool_next = ctr.p + 3;
+  a.pool_full = (int*)(ctr.p + 4);
   qp_mark(c, "pair setup");
-  k_class_a<NINT, MODE_COUNT><<<gAB, BLK, 0, st>>>(a);
-  k_same_keyed<NINT, MODE_COUNT, 0><<<gC, BLK, 0, st>>>(a);
-  qp_mark(c, "count A (same beta)");
-  k_class_b<NINT, MODE_COUNT><<<gAB, BLK, 0, st>>>(a);
-  k_same_keyed<NINT, MODE_COUNT, 1><<<gC, BLK, 0, st>>>(a);
-  qp_mark(c, "count B (same alpha)");
-  k_class_c<NINT, MODE_COUNT><<<gC, BLK, 0, st>>>(a);
-  qp_mark(c, "count C (alpha x beta)");
+  size_t fr = 0, total = 0;
+  QP_CUDA(c, cudaMemGetInfo(&fr, &total));
+  fr += qp_pool_cached(c);
+  if (c->sigma_mode != QPGPU_SIGMA_DIRECT) {
+    // room for as many pairs a row as the context's last set had (1,200 when
+    // it had none; the bench system has 991 at 1e6 determinants), 0.3 of that
+    // for what rows leave behind when they outgrow a chunk, and for the
+    // unfinished chunks of the warps; a pool that is too
+    // small costs its rows a second scan, one that would not fit beside the
+    // stored pairs is left out
+    const double per_row = c->pairs_per_row > 0 ? c->pairs_per_row : 1200.0;
+    const double est = per_row * (double)N;
+    // chunks: an eighth of a warp's share of about 0.3 / 0.3 / 0.6 of the pairs
+    const int64_t all = nblocks(N * 32, BLK);
+    const int64_t ws = std::min<int64_t>(all, c->n_sm * 6) * (BLK / 32), wc = std::min<int64_t>(all, c->n_sm * 3) * (BLK / 32);
+    auto chunk_of = [&](double share, int64_t warps) {
+      return (int)std::min(65536.0, std::max(256.0, share * est / (8.0 * (double)warps)));
+    };
+    a.pool_chunk[CLS_A] = a.pool_chunk[CLS_B] = chunk_of(0.3, ws);
+    a.pool_chunk[CLS_C] = chunk_of(0.6, wc);
+    const double slack = 2.0 * (double)ws * a.pool_chunk[CLS_A] + (double)wc * a.pool_chunk[CLS_C];
+    const double cap = std::min(1.3 * est + slack, 3.0 * (double)N * (double)N);
+    const bool room = 16.0 * est + 4.0 * cap + 28.0 * (double)N + (double)total / 16.0 < (double)fr;
+    if (room && pool.alloc((size_t)cap + 1) == cudaSuccess && pos.alloc(3 * (size_t)N) == cudaSuccess) {
+      a.pool = pool.p;
+      a.pool_cap = (int64_t)cap;
+      for (int q = 0; q < 3; ++q) a.pos[q] = pos.p + q * N;
+    } else {
+      cudaGetLastError();
+    }
+  }
+  if (a.pool)
+    launch_scans<NINT, MODE_POOL>(c, a);
+  else
+    launch_scans<NINT, MODE_COUNT>(c, a);
   QP_CUDA(c, cudaGetLastError());
   Scoped<int64_t> tot(c), stot(c);
   QP_CUDA(c, tot.alloc(N + 1));
@@ -902,22 +1187,31 @@ int build_pairs_t(qpgpu_ctx* c) {
   QP_CUDA(c, tmp.alloc(tb));
   QP_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp.p, tb, tot.p, c->d_rowptr, (int)(N + 1), st));
   QP_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp.p, tb, stot.p, c->d_s2ptr, (int)(N + 1), st));
+  int full = 0;
   QP_CUDA(c, cudaMemcpyAsync(&c->P, c->d_rowptr + N, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaMemcpyAsync(&c->P_s2, c->d_s2ptr + N, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  QP_CUDA(c, cudaMemcpyAsync(&full, a.pool_full, sizeof(int), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
   const int64_t P = c->P, PS = c->P_s2;
+  c->pairs_per_row = (double)P / (double)N;
   // stored pairs (16 B each, S^2 pairs 8 B) or the direct sigma: forced by
   // qpgpu_set_sigma_mode, else direct when the stored pairs would leave less
   // than 1/16 of the device memory free
   bool direct = c->sigma_mode == QPGPU_SIGMA_DIRECT;
   if (c->sigma_mode == QPGPU_SIGMA_AUTO) {
-    size_t fr = 0, total = 0;
-    QP_CUDA(c, cudaMemGetInfo(&fr, &total));
-    fr += qp_pool_cached(c);
     const double need = 16.0 * (double)P + 8.0 * (double)PS + 28.0 * (double)N;
     direct = need + (double)total / 16.0 > (double)fr;
   }
   c->direct = direct;
+  QP_CUDA(c, pool_alloc(c, &c->d_hdiag, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_sdiag, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_hdiag32, N));
+  k_diag<NINT><<<nblocks(N, 256), 256, 0, st>>>(c->tab, c->d_alpha, c->d_beta, c->d_rows, c->d_cols, c->d_hdiag,
+                                                 c->d_sdiag, c->d_hdiag32, N);
+  qp_mark(c, "row starts, diagonal");
+  Scoped<u64> det(c);
+  QP_CUDA(c, det.alloc(2 * NINT * (size_t)N));
+  k_det_pos<NINT><<<nblocks(N, 256), 256, 0, st>>>(c->d_alpha, c->d_beta, c->d_rows, c->d_cols, nullptr, det.p, N);
   if (direct) {
     // the direct sigma regenerates the columns chunk by chunk: keep the
     // per-row counts of the same-spin classes and the row starts on the host
@@ -925,22 +1219,21 @@ int build_pairs_t(qpgpu_ctx* c) {
     cA.p = nullptr;
     c->d_cntB = cB.p;
     cB.p = nullptr;
+    c->d_det_pos = det.p;
+    det.p = nullptr;
+    QP_CUDA(c, pool_alloc(c, &c->d_det_tpos, 2 * NINT * (size_t)N));
+    k_det_pos<NINT><<<nblocks(N, 256), 256, 0, st>>>(c->d_alpha, c->d_beta, c->d_rows, c->d_cols, c->d_t_order,
+                                                      c->d_det_tpos, N);
     c->h_rowptr.resize(N + 1);
     QP_CUDA(c, cudaMemcpyAsync(c->h_rowptr.data(), c->d_rowptr, (N + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
                                st));
-    QP_CUDA(c, pool_alloc(c, &c->d_hdiag, N));
-    QP_CUDA(c, pool_alloc(c, &c->d_sdiag, N));
-    QP_CUDA(c, pool_alloc(c, &c->d_hdiag32, N));
-    k_diag<NINT><<<nblocks(N, 256), 256, 0, st>>>(c->tab, c->d_alpha, c->d_beta, c->d_rows, c->d_cols, c->d_hdiag,
-                                                   c->d_sdiag, c->d_hdiag32, N);
-    qp_mark(c, "diagonal (direct sigma: no pairs stored)");
     QP_CUDA(c, cudaGetLastError());
     QP_CUDA(c, cudaStreamSynchronize(st));
     return 0;
   }
   if (pool_alloc(c, &c->d_colidx, P) != cudaSuccess || pool_alloc(c, &c->d_val64, P) != cudaSuccess ||
       pool_alloc(c, &c->d_val32, P) != cudaSuccess || pool_alloc(c, &c->d_s2col, PS) != cudaSuccess ||
-      pool_alloc(c, &c->d_s2val, PS) != cudaSuccess) {
+      pool_alloc(c, &c->d_s2val, PS) != cudaSuccess || pool_alloc(c, &c->d_detfeat, (size_t)N * 4) != cudaSuccess) {
     cudaGetLastError();
     return qpgpu_fail(c, QPGPU_ERR_NOMEM,
                       "not enough device memory for " + std::to_string(P) + " connected pairs");
@@ -952,44 +1245,31 @@ int build_pairs_t(qpgpu_ctx* c) {
   a.s2ptr = c->d_s2ptr;
   a.s2col = c->d_s2col;
   a.s2val = c->d_s2val;
+  a.det_pos = det.p;
+  a.feat = (float4*)c->d_detfeat;
   Scoped<int> err(c);
   QP_CUDA(c, err.alloc(1));
   QP_CUDA(c, cudaMemsetAsync(err.p, 0, sizeof(int), st));
   a.err = err.p;
-  qp_mark(c, "scan + alloc");
-  k_class_a<NINT, MODE_FILL><<<gAB, BLK, 0, st>>>(a);
-  k_same_keyed<NINT, MODE_FILL, 0><<<gC, BLK, 0, st>>>(a);
-  qp_mark(c, "fill A");
-  k_class_b<NINT, MODE_FILL><<<gAB, BLK, 0, st>>>(a);
-  k_same_keyed<NINT, MODE_FILL, 1><<<gC, BLK, 0, st>>>(a);
-  qp_mark(c, "fill B");
-  k_class_c<NINT, MODE_FILL><<<gC, BLK, 0, st>>>(a);
-  qp_mark(c, "fill C");
-  {
+  if (!a.pool || full) {
+    launch_scans<NINT, MODE_FILL>(c, a);
     int herr = 0;
     QP_CUDA(c, cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     QP_CUDA(c, cudaStreamSynchronize(st));
     if (herr)
       return qpgpu_fail(c, QPGPU_ERR_STATE, "pair fill disagrees with pair count (" + std::to_string(herr) + ")");
-    const int rc = sort_row_columns(c);
-    if (rc) return rc;
   }
+  const int rc = sort_row_columns(c, a);
+  if (rc) return rc;
   qp_mark(c, "row columns sorted");
-  k_pair_values<NINT><<<gC, BLK, 0, st>>>(a);
+  pool.reset();
+  k_pair_values<NINT><<<nblocks(N * 32, BLK), BLK, 0, st>>>(a);
   qp_mark(c, "pair elements");
   QP_CUDA(c, cudaGetLastError());
   int herr = 0;
   QP_CUDA(c, cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
   if (herr) return qpgpu_fail(c, QPGPU_ERR_STATE, "pair fill disagrees with pair count (" + std::to_string(herr) + ")");
-  QP_CUDA(c, pool_alloc(c, &c->d_hdiag, N));
-  QP_CUDA(c, pool_alloc(c, &c->d_sdiag, N));
-  QP_CUDA(c, pool_alloc(c, &c->d_hdiag32, N));
-  k_diag<NINT><<<nblocks(N, 256), 256, 0, st>>>(c->tab, c->d_alpha, c->d_beta, c->d_rows, c->d_cols, c->d_hdiag,
-                                                 c->d_sdiag, c->d_hdiag32, N);
-  qp_mark(c, "diagonal");
-  QP_CUDA(c, cudaGetLastError());
-  QP_CUDA(c, cudaStreamSynchronize(st));
   return 0;
 }
 
@@ -1041,7 +1321,7 @@ __global__ void __launch_bounds__(BLK, 3) k_pair_sigma(BuildArgs a, const int* _
     };
     const int64_t e0 = a.rowptr[k];
     const int* prow = pc + (e0 - a.col_base);
-    const int n = (int)(a.rowptr[k + 1] - e0), nA = a.cntA[k], nB = nA + a.cntB[k];
+    const int n = (int)(a.rowptr[k + 1] - e0), nA = a.cnt[CLS_A][k], nB = nA + a.cnt[CLS_B][k];
     auto do_mono = [&](int x) {
       if (x < 0) return;
       const bool beta = x >= nA;
@@ -1083,14 +1363,8 @@ __global__ void __launch_bounds__(BLK, 3) k_pair_sigma(BuildArgs a, const int* _
       const unsigned cj = (unsigned)prow[x];
       const bool via_t = (cj & QP_TAG_T) != 0;
       const int q = (int)(cj & ~QP_TAG_T);
-      const int j = via_t ? a.t_order[q] : q;
-      const int bj = a.cols[j];
       u64 J[2 * NINT];
-#pragma unroll
-      for (int w = 0; w < NINT; ++w) {
-        J[w] = a.alpha_pos[(int64_t)j * NINT + w];
-        J[NINT + w] = a.beta[(int64_t)bj * NINT + w];
-      }
+      load_det<NINT>(via_t ? a.det_tpos : a.det_pos, q, J);
       double s2;
       const double v = h_double_ab<NINT>(a.t, my, J, E, &s2, nullptr, nullptr);
       const double* uj = (via_t ? a.uT : a.u) + (int64_t)q * nst;
@@ -1136,18 +1410,17 @@ int sigma_direct_t(qpgpu_ctx* c, double* v, double* s, const double* u, const do
   a.nst = nst;
   a.rowptr = c->d_rowptr;
   a.s2ptr = c->d_s2ptr;
-  a.cntA = c->d_cntA;
-  a.cntB = c->d_cntB;
+  a.cnt[CLS_A] = c->d_cntA;
+  a.cnt[CLS_B] = c->d_cntB;
+  a.det_pos = c->d_det_pos;
+  a.det_tpos = c->d_det_tpos;
   a.colidx = c->d_direct_cols;
   a.err = c->d_direct_err;
-  a.write_s2 = 0;
   a.tag_t = 1;
   a.row_first = row_first;
   a.row_step = row_step;
   const int64_t N = c->N;
   const std::vector<int64_t>& rp = c->h_rowptr;
-  const unsigned gAB = nblocks(N, BLK);
-  const unsigned gC = nblocks(N * 32, BLK);
   int64_t clo = 0;
   while (clo < N) {
     // largest chi with rp[chi] - rp[clo] <= capacity (at least one row)
@@ -1159,18 +1432,14 @@ int sigma_direct_t(qpgpu_ctx* c, double* v, double* s, const double* u, const do
       a.row_lo = (int)lo;
       a.row_hi = (int)hi;
       a.col_base = rp[lo];
-      a.blk_off = lo / BLK;
-      const unsigned gA = (unsigned)((hi - 1) / BLK - lo / BLK + 1);
       const unsigned gK = nblocks((hi - lo) * 32, BLK);
       const bool marks = st == c->stream;  // QPGPU_PROFILE=1: phase times on the context stream
       if (marks) qp_mark(c, "direct: chunk start");
-      k_class_a<NINT, MODE_FILL><<<gA, BLK, 0, st>>>(a);
-      k_same_keyed<NINT, MODE_FILL, 0><<<gK, BLK, 0, st>>>(a);
+      k_same<NINT, MODE_FILL, 0><<<gK, BLK, 0, st>>>(a);
       if (marks) qp_mark(c, "direct: scan A");
-      k_class_b<NINT, MODE_FILL><<<gAB, BLK, 0, st>>>(a);
-      k_same_keyed<NINT, MODE_FILL, 1><<<gK, BLK, 0, st>>>(a);
+      k_same<NINT, MODE_FILL, 1><<<gK, BLK, 0, st>>>(a);
       if (marks) qp_mark(c, "direct: scan B");
-      k_class_c<NINT, MODE_FILL><<<gC, BLK, 0, st>>>(a);
+      k_class_c<NINT, MODE_FILL><<<gK, BLK, 0, st>>>(a);
       if (marks) qp_mark(c, "direct: scan C");
       launch_pair_sigma<NINT>(a, c->d_direct_cols, gK, st);
       if (marks) qp_mark(c, "direct: elements");
@@ -1233,7 +1502,7 @@ void qp_free_pairs(qpgpu_ctx* c) {
   }
   c->have_pairs = false;
   c->direct = false;
-  void** dp[] = {(void**)&c->d_cntA, (void**)&c->d_cntB};
+  void** dp[] = {(void**)&c->d_cntA, (void**)&c->d_cntB, (void**)&c->d_det_pos, (void**)&c->d_det_tpos};
   for (auto p : dp) {
     qp_pool_free(c, *p);
     *p = nullptr;

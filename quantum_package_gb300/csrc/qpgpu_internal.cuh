@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -404,27 +405,28 @@ __device__ __forceinline__ bool key_find(const KeyView& kv, u64 h, unsigned& sta
   }
   return false;
 }
-// orbital index (word * 64 + bit) of the j-th electron (0-based) of s
+// orbital index (word * 64 + bit) of the j-th electron (0-based) of s; the
+// word is selected by value (an early return per word becomes a run-time word
+// index, which puts s in local memory)
 template <int NINT>
 __device__ __forceinline__ int nth_electron(const u64* s, int j) {
-#pragma unroll
-  for (int w = 0; w < NINT; ++w) {
-    const int c = __popcll(s[w]);
-    if (j < c) {
-      u64 v = s[w];
-      for (int t = 0; t < j; ++t) v &= v - 1;
-      return w * 64 + __ffsll((long long)v) - 1;
-    }
-    j -= c;
+  u64 v = s[0];
+  int base = 0;
+  if constexpr (NINT == 2) {
+    const int c = __popcll(s[0]);
+    const bool hi = j >= c;
+    v = s[0] ^ ((s[0] ^ s[NINT - 1]) & (0ull - (u64)hi));
+    base = hi ? 64 : 0;
+    j -= hi ? c : 0;
   }
-  return -1;
+  for (int t = 0; t < j; ++t) v &= v - 1;
+  return base + __ffsll((long long)v) - 1;
 }
 // clear orbital b (word * 64 + bit) of s, with constant word indices (s stays in registers)
 template <int NINT>
 __device__ __forceinline__ void clear_orbital(u64* s, int b) {
 #pragma unroll
-  for (int w = 0; w < NINT; ++w)
-    if (w == (b >> 6)) s[w] &= ~(1ull << (b & 63));
+  for (int w = 0; w < NINT; ++w) s[w] &= ~(w == (b >> 6) ? 1ull << (b & 63) : 0ull);
 }
 // pair (i, j), i < j, of the c-th 2-electron combination of ne electrons
 __device__ __forceinline__ void pair_of_combo(int c, int ne, int& i, int& j) {
@@ -586,10 +588,13 @@ struct qpgpu_ctx {
   size_t direct_ut_n = 0;
   int* d_cntA = nullptr;              // direct sigma: same-beta / same-alpha pairs per row
   int* d_cntB = nullptr;
+  u64* d_det_pos = nullptr;           // direct sigma: both strings at each bilinear / alpha-major position
+  u64* d_det_tpos = nullptr;
   std::vector<int64_t> h_rowptr;      // direct sigma: row starts (host)
   int* d_direct_cols = nullptr;       // direct sigma: columns of one chunk of rows
   int64_t direct_cols_cap = 0;
   int* d_direct_err = nullptr;
+  double pairs_per_row = 0.0;         // of the last set (sizes the next set-up's pool of hits)
   int64_t P = 0;
   int64_t* d_rowptr = nullptr;  // N+1
   int* d_colidx = nullptr;      // P
@@ -683,6 +688,23 @@ struct Scoped {
 int qp_build_index(qpgpu_ctx* c);      // index.cu
 int qp_build_line_keys(qpgpu_ctx* c);  // keys.cu (inside qp_build_index)
 void qp_free_line_keys(qpgpu_ctx* c);  // keys.cu
+// bits kept of a key hash: the caller's (qpgpu_set_line_keys), at most 12 more
+// than the number of keys of the largest possible table has, so that the radix
+// sorts of the tables stop there.  A cut hash can only make two of some 2^12
+// keys' neighbours share a group, whose members are verified one by one.
+inline int qp_key_bits(const qpgpu_ctx* c) {
+  double keys = (double)c->N * 0.5 * (double)c->na * (double)(c->na + 1);
+  int b = 13;
+  while (keys > 1.0 && b < 64) {
+    keys *= 0.5;
+    ++b;
+  }
+  return std::max(1, std::min(c->key_hash_bits, b));
+}
+inline u64 qp_key_mask(const qpgpu_ctx* c) {
+  const int b = qp_key_bits(c);
+  return b >= 64 ? ~0ull : (1ull << b) - 1ull;
+}
 int qp_build_pairs(qpgpu_ctx* c);      // pairs.cu
 void qp_free_dets(qpgpu_ctx* c);       // index.cu
 void qp_free_pairs(qpgpu_ctx* c);      // pairs.cu
