@@ -72,6 +72,11 @@ struct BuildArgs {
   unsigned long long* pool_next;
   int* pool_full;
   int64_t* pos[3];
+  // MODE_POOL: spin-flip pairs (row, place in the row, column, +-1), in any order
+  int4* s2rec;
+  int64_t s2rec_cap;
+  unsigned long long* s2rec_next;
+  int write_s2;  // MODE_FILL: write the spin-flip pairs at s2ptr
   unsigned long long* next_row;  // MODE_POOL: rows handed out to warps (one counter per class)
   // CSR (fill pass, sort, elements)
   const int64_t* rowptr;
@@ -248,10 +253,42 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
     }
     out.begin(a, k);
     int scnt = 0;
+    // the spin-flip pairs of a step, in the order of the scan, with <I|S^2|J>
+    auto put_flip = [&](bool flip, unsigned fb, const u64* ca, const u64* cb, int col) {
+      unsigned long long at = 0;
+      if (MODE == MODE_POOL) {
+        if (lane == 0) at = atomicAdd(a.s2rec_next, (unsigned long long)__popc(fb));
+        at = __shfl_sync(FULL, at, 0);
+      }
+      if (!flip) return;
+      u64 J[2 * NINT], E[2 * NINT];
+#pragma unroll
+      for (int w = 0; w < NINT; ++w) {
+        J[w] = ca[w];
+        J[NINT + w] = cb[w];
+      }
+      det_parity<NINT>(my, E);
+      double s2;
+      h_double_ab<NINT>(a.t, my, J, E, &s2, nullptr, nullptr);
+      const int rank = __popc(fb & ((1u << lane) - 1u));
+      if (MODE == MODE_POOL) {
+        if ((int64_t)at + rank < a.s2rec_cap) a.s2rec[at + rank] = make_int4((int)k, scnt + rank, col, (int)s2);
+      } else if (a.s2ptr[k] + scnt + rank < a.s2ptr[k + 1]) {
+        a.s2col[a.s2ptr[k] + scnt + rank] = col;
+        a.s2val[a.s2ptr[k] + scnt + rank] = (float)s2;
+      } else {
+        atomicOr(a.err, 8);
+      }
+    };
     // 32 candidates, one per lane: hit = (ca, cb) is an alpha single x beta
     // single of the row, written as col
     auto step = [&](bool hit, const u64* ca, const u64* cb, int col) {
-      if (MODE != MODE_FILL) scnt += __popc(__ballot_sync(FULL, hit && spin_flip<NINT>(my, ca, cb)));
+      if (MODE != MODE_FILL || a.write_s2) {
+        const bool flip = hit && spin_flip<NINT>(my, ca, cb);
+        const unsigned fb = __ballot_sync(FULL, flip);
+        if (MODE != MODE_COUNT && fb) put_flip(flip, fb, ca, cb, col);
+        scnt += __popc(fb);
+      }
       out.put(a, hit, col, lane);
     };
     // Lines of the row's singles, 32 at a time: the lanes read the bounds of
@@ -837,8 +874,7 @@ __device__ __forceinline__ void load_det(const u64* det, int64_t p, u64 (&J)[2 *
 // the holes and particles against the reference take several times a double's
 // loads), and same-spin doubles where they are few in a trip, are deferred
 // until 32 of a kind are there (a row's own beta column is one run of its
-// ascending columns, whose trips take them at once).  The spin-flip pairs of the alpha x beta class are listed here, and
-// the row's sum of squared elements gives the coupling feature of the learned
+// ascending columns, whose trips take them at once).  The row's sum of squared elements gives the coupling feature of the learned
 // step (log10(sum_J H_IJ^2) / 4), which took a pass of its own (4.2 ms).
 // 991M pairs at 1e6 determinants: 30.8 -> 22.9 ms; bound by the integer
 // instructions of the Slater routines (about 400 a pair, 45 % issue) with the
@@ -857,9 +893,6 @@ __global__ void __launch_bounds__(BLK, 4) k_pair_values(BuildArgs a) {
     det_parity<NINT>(my, E);
     const int64_t e0 = a.rowptr[k];
     const int n = (int)(a.rowptr[k + 1] - e0);
-    const int64_t s0 = a.s2ptr[k];
-    const int ns2 = (int)(a.s2ptr[k + 1] - s0);
-    int scnt = 0;
     double sum2 = 0.0;
     auto put = [&](int x, double v) {
       a.val64[e0 + x] = v;
@@ -902,8 +935,7 @@ __global__ void __launch_bounds__(BLK, 4) k_pair_values(BuildArgs a) {
     for (int x0 = 0; x0 < n; x0 += 32) {
       const int x = x0 + lane;
       const int jn = x + 32 < n ? a.colidx[e0 + x + 32] : -1;  // the next trip's column
-      bool is_same = false, flip = false;
-      double s2 = 0.0;
+      bool is_same = false;
       u64 J[2 * NINT];
       if (j >= 0) {
         load_det<NINT>(a.det_pos, j, J);
@@ -914,19 +946,8 @@ __global__ void __launch_bounds__(BLK, 4) k_pair_values(BuildArgs a) {
           sameb &= J[NINT + w] == my[NINT + w];
         }
         is_same = samea || sameb;
+        double s2;
         if (!is_same) put(x, h_double_ab<NINT>(a.t, my, J, E, &s2, nullptr, nullptr));
-      }
-      if (ns2 > 0) {
-        flip = s2 != 0.0;
-        const unsigned fb = __ballot_sync(0xffffffffu, flip);
-        if (flip) {
-          const int o = scnt + __popc(fb & lt);
-          if (o < ns2) {
-            a.s2col[s0 + o] = j;
-            a.s2val[s0 + o] = (float)s2;
-          }
-        }
-        scnt += __popc(fb);
       }
       if (__popc(__ballot_sync(0xffffffffu, is_same)) >= 12) {
         if (mono.push(is_same && same_spin(x, J), x, lt)) do_mono(mono.pop(lane));
@@ -941,7 +962,6 @@ __global__ void __launch_bounds__(BLK, 4) k_pair_values(BuildArgs a) {
       if (mono.push(do_same(y), y, lt)) do_mono(mono.pop(lane));
     }
     do_mono(mono.pop(lane));
-    if (scnt != ns2 && lane == 0) atomicOr(a.err, 8);
     if (a.feat) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
@@ -962,6 +982,15 @@ __global__ void k_det_pos(const u64* alpha, const u64* beta, const int* rows, co
       out[p * 2 * NINT + w] = alpha[(int64_t)rows[k] * NINT + w];
       out[p * 2 * NINT + NINT + w] = beta[(int64_t)cols[k] * NINT + w];
     }
+  }
+}
+
+// the recorded spin-flip pairs to their places
+__global__ void k_s2_scatter(const int4* rec, int64_t n, const int64_t* s2ptr, int* s2col, float* s2val) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int4 r = rec[i];
+    s2col[s2ptr[r.x] + r.y] = r.z;
+    s2val[s2ptr[r.x] + r.y] = (float)r.w;
   }
 }
 
@@ -1123,13 +1152,15 @@ int build_pairs_t(qpgpu_ctx* c) {
   cudaStream_t st = c->stream;
   BuildArgs a = index_args(c);
   Scoped<int> cA(c), cB(c), cC(c), cS(c), pool(c);
+  Scoped<int4> s2rec(c);
   Scoped<int64_t> pos(c);
   Scoped<unsigned long long> ctr(c);
   QP_CUDA(c, cA.alloc(N));
   QP_CUDA(c, cB.alloc(N));
   QP_CUDA(c, cC.alloc(N));
   QP_CUDA(c, cS.alloc(N));
-  QP_CUDA(c, ctr.alloc(8));  // next row of each class; next free entry of the pool; its full flag
+  // next row of each class; next free entry of the pool; its full flag; next spin-flip record
+  QP_CUDA(c, ctr.alloc(8));
   QP_CUDA(c, cudaMemsetAsync(ctr.p, 0, 8 * sizeof(unsigned long long), st));
   a.cnt[CLS_A] = cA.p;
   a.cnt[CLS_B] = cB.p;
@@ -1138,6 +1169,7 @@ int build_pairs_t(qpgpu_ctx* c) {
   a.next_row = ctr.p;
   a.pool_next = ctr.p + 3;
   a.pool_full = (int*)(ctr.p + 4);
+  a.s2rec_next = ctr.p + 5;
   qp_mark(c, "pair setup");
   size_t fr = 0, total = 0;
   QP_CUDA(c, cudaMemGetInfo(&fr, &total));
@@ -1162,7 +1194,10 @@ int build_pairs_t(qpgpu_ctx* c) {
     const double slack = 2.0 * (double)ws * a.pool_chunk[CLS_A] + (double)wc * a.pool_chunk[CLS_C];
     const double cap = std::min(1.3 * est + slack, 3.0 * (double)N * (double)N);
     const bool room = 16.0 * est + 4.0 * cap + 28.0 * (double)N + (double)total / 16.0 < (double)fr;
-    if (room && pool.alloc((size_t)cap + 1) == cudaSuccess && pos.alloc(3 * (size_t)N) == cudaSuccess) {
+    a.s2rec_cap = 4 * N + (1 << 16);
+    if (room && pool.alloc((size_t)cap + 1) == cudaSuccess && pos.alloc(3 * (size_t)N) == cudaSuccess &&
+        s2rec.alloc((size_t)a.s2rec_cap) == cudaSuccess) {
+      a.s2rec = s2rec.p;
       a.pool = pool.p;
       a.pool_cap = (int64_t)cap;
       for (int q = 0; q < 3; ++q) a.pos[q] = pos.p + q * N;
@@ -1194,6 +1229,12 @@ int build_pairs_t(qpgpu_ctx* c) {
   QP_CUDA(c, cudaStreamSynchronize(st));
   const int64_t P = c->P, PS = c->P_s2;
   c->pairs_per_row = (double)P / (double)N;
+  if (a.pool && PS > a.s2rec_cap) {  // not all spin-flip pairs recorded: class C again, for every row
+    QP_CUDA(c, cudaMemsetAsync(a.pos[CLS_C], 0xff, (size_t)N * sizeof(int64_t), st));
+    full = 1;
+    a.write_s2 = 1;
+  }
+  if (!a.pool) a.write_s2 = 1;
   // stored pairs (16 B each, S^2 pairs 8 B) or the direct sigma: forced by
   // qpgpu_set_sigma_mode, else direct when the stored pairs would leave less
   // than 1/16 of the device memory free
@@ -1259,6 +1300,8 @@ int build_pairs_t(qpgpu_ctx* c) {
     if (herr)
       return qpgpu_fail(c, QPGPU_ERR_STATE, "pair fill disagrees with pair count (" + std::to_string(herr) + ")");
   }
+  if (!a.write_s2 && PS > 0)
+    k_s2_scatter<<<nblocks(PS, 256), 256, 0, st>>>(a.s2rec, PS, c->d_s2ptr, c->d_s2col, c->d_s2val);
   const int rc = sort_row_columns(c, a);
   if (rc) return rc;
   qp_mark(c, "row columns sorted");
