@@ -33,7 +33,8 @@ namespace {
 constexpr int BBLK = 256;
 constexpr int BMAXS = 8;    // N_st_diag
 constexpr int BMAXM = 64;   // N_st_diag * itermax
-constexpr int BROWS = 2048; // rows per algebra CTA
+constexpr int BROWS = 2048; // rows of a Gram partial
+constexpr int BSTEP = 256;  // rows of a CTA of the step
 
 inline unsigned gsz(int64_t n, int tpb = BBLK) {
   int64_t g = (n + tpb - 1) / tpb;
@@ -73,7 +74,8 @@ struct BProb {
   float* u32;
   double* pv;
   double* ps;
-  int ncta;  // algebra CTAs of this problem
+  int ncta;   // Gram partials of this problem
+  int nstep;  // CTAs of its step
 };
 
 // ---- persistent sigma over the whole batch ---------------------------------
@@ -241,42 +243,43 @@ __device__ __forceinline__ double* barr(const BProb& P, int sel) {
 }
 
 // partial Gram G[i][j] = sum_r A_i[r] B_j[r]: A = blocks a0..a0+nbA-1 of array
-// asel, B = block bb of array bsel; rows [c*BROWS, ...) of CTA c; one partial
-// per (problem, CTA).  As the single-problem k_gram: a lane owns one row at a
-// time and CI = 32 / NSD columns of A for all NSD columns of B (every FP64 FMA
-// useful), warps hold column groups (or split the rows when there are fewer
-// groups), gridDim.z passes cover the rest, and the sums are combined in a
-// fixed order (reduce-scatter over lanes, shared memory over warps).
+// asel, B = block bb of array bsel, over the BROWS rows of partial c.  As the
+// single-problem k_gram: a lane owns one row at a time and CI = 32 / NSD
+// columns of A for all NSD columns of B (every FP64 FMA useful); groups of
+// eight column groups (or fewer, the rows then split over the rest of the
+// eight slots) make a slice.  A block is one warp: slot blockIdx.z % 8 of
+// slice blockIdx.z / 8 writes its own share of the partial, and k_breduce adds
+// the row groups' shares in order before the partials, which gives the sums of
+// eight warps sharing a block.  As such blocks the 73 partials of a
+// 16-problem batch kept half of the SMs' FP64 pipes without work.
 template <int NSD>
-__global__ void __launch_bounds__(BBLK) k_bgram(const BProb* __restrict__ probs, int asel, int a0, int nbA, int bsel,
-                                                int bb, double* partial, int pstride,
-                                                const int* skip /* per problem, stride sstride */, int sstride,
-                                                int ncta_max) {
+__global__ void __launch_bounds__(32) k_bgram(const BProb* __restrict__ probs, int asel, int a0, int nbA, int bsel,
+                                              int bb, double* partial, int pstride,
+                                              const int* skip /* per problem, stride sstride */, int sstride,
+                                              int ncta_max) {
   constexpr int CI = 32 / NSD;
-  constexpr int NW = BBLK / 32;
-  __shared__ double red[NW][32];
+  constexpr int NW = 8;
   const BProb& P = probs[blockIdx.y];
   const int c = blockIdx.x;
   if (!P.active || c >= P.ncta) return;
   const int m = nbA * NSD;
   const int ncg = (m + CI - 1) / CI;
-  const int cg0 = blockIdx.z * NW;
-  if (cg0 >= ncg) return;
-  double* out = partial + ((int64_t)blockIdx.y * ncta_max + c) * pstride;
+  const int w = blockIdx.z % NW, cg0 = (blockIdx.z / NW) * NW, lane = threadIdx.x;
+  const int ncg_here = min(NW, ncg - cg0);
+  const int rg = NW / ncg_here;
+  const int cgl = w % ncg_here, rgi = w / ncg_here;
+  if (rgi >= rg) return;
+  const int cg = cg0 + cgl;
+  const int nq = min(CI, m - cg * CI);
+  double* out = partial + (((int64_t)blockIdx.y * ncta_max + c) * NW + rgi) * pstride;
+  const int oq = lane / NSD, oj = lane % NSD, oi = cg * CI + oq;  // the entry this lane ends with
   if (skip && skip[(int64_t)blockIdx.y * sstride]) {
-    for (int p = cg0 * CI * NSD + threadIdx.x; p < min(m, (cg0 + NW) * CI) * NSD; p += BBLK) out[p] = 0.0;
+    if (oq < CI && oi < m) out[(int64_t)oi * NSD + oj] = 0.0;
     return;
   }
   const int64_t N = P.N;
   const double* A = barr(P, asel) + (int64_t)a0 * N * NSD;
   const double* B = barr(P, bsel) + (int64_t)bb * N * NSD;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ncg_here = min(NW, ncg - cg0);
-  const int rg = NW / ncg_here;
-  const int cgl = w % ncg_here, rgi = w / ncg_here;
-  const bool act = rgi < rg;
-  const int cg = cg0 + cgl;
-  const int nq = min(CI, m - cg * CI);
   const double* ap[CI];
 #pragma unroll
   for (int q = 0; q < CI; ++q) {
@@ -287,40 +290,45 @@ __global__ void __launch_bounds__(BBLK) k_bgram(const BProb* __restrict__ probs,
 #pragma unroll
   for (int k = 0; k < 32; ++k) acc[k] = 0.0;
   const int64_t r0 = (int64_t)c * BROWS, r1 = min(r0 + BROWS, N);
-  if (act) {
-    for (int64_t r = r0 + (int64_t)rgi * 32 + lane; r < r1; r += (int64_t)rg * 32) {
-      double a[CI], b[NSD];
+  for (int64_t r = r0 + (int64_t)rgi * 32 + lane; r < r1; r += (int64_t)rg * 32) {
+    double a[CI], b[NSD];
 #pragma unroll
-      for (int q = 0; q < CI; ++q) a[q] = (q < nq) ? ap[q][r * NSD] : 0.0;
-      load_row<NSD>(B, r, b);
+    for (int q = 0; q < CI; ++q) a[q] = (q < nq) ? ap[q][r * NSD] : 0.0;
+    load_row<NSD>(B, r, b);
 #pragma unroll
-      for (int q = 0; q < CI; ++q)
-        if (q < nq)
+    for (int q = 0; q < CI; ++q)
+      if (q < nq)
 #pragma unroll
-          for (int j = 0; j < NSD; ++j) acc[q * NSD + j] = fma(a[q], b[j], acc[q * NSD + j]);
-    }
+        for (int j = 0; j < NSD; ++j) acc[q * NSD + j] = fma(a[q], b[j], acc[q * NSD + j]);
   }
   const double v = reduce_scatter64<32>(acc, lane);  // lane L: entry (L / NSD, L % NSD)
-  if (act) red[w][lane] = v;
-  __syncthreads();
-  if (w < ncg_here) {
-    double t = 0.0;
-    for (int g = 0; g < rg; ++g) t += red[g * ncg_here + w][lane];
-    const int q = lane / NSD, j = lane % NSD, i = cg * CI + q;
-    if (q < CI && i < m) out[(int64_t)i * NSD + j] = t;
-  }
+  if (oq < CI && oi < m) out[(int64_t)oi * NSD + oj] = v;
 }
 
-// out[problem][p] = sum over its CTAs of the partials (warp per element)
-__global__ void k_breduce(const BProb* __restrict__ probs, const double* partial, int pstride, int ncta_max, int npe,
-                          double* out, int ostride) {
+// row groups of column group cg of m columns (k_bgram's split of its slice)
+__device__ __forceinline__ int bgram_row_groups(int m, int nsd, int i) {
+  const int ci = 32 / nsd, ncg = (m + ci - 1) / ci;
+  const int cg0 = (i / ci) / 8 * 8;
+  return 8 / min(8, ncg - cg0);
+}
+
+// out[problem][p] = sum over its partials (warp per element): the shares of
+// the row groups of a partial first, then the partials
+__global__ void k_breduce(const BProb* __restrict__ probs, const double* partial, int pstride, int ncta_max, int m,
+                          int nsd, double* out, int ostride) {
   const BProb& P = probs[blockIdx.y];
   if (!P.active) return;
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-  const double* part = partial + (int64_t)blockIdx.y * ncta_max * pstride;
-  for (int p = blockIdx.x * wpb + (threadIdx.x >> 5); p < npe; p += gridDim.x * wpb) {
+  const double* part = partial + (int64_t)blockIdx.y * ncta_max * 8 * pstride;
+  for (int p = blockIdx.x * wpb + (threadIdx.x >> 5); p < m * nsd; p += gridDim.x * wpb) {
+    const int rg = bgram_row_groups(m, nsd, p / nsd);
     double s = 0.0;
-    for (int c = lane; c < P.ncta; c += 32) s += part[(int64_t)c * pstride + p];
+    for (int c = lane; c < P.ncta; c += 32) {
+      const double* pc = part + (int64_t)c * 8 * pstride + p;
+      double t = 0.0;
+      for (int g = 0; g < rg; ++g) t += pc[(int64_t)g * pstride];
+      s += t;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) out[(int64_t)blockIdx.y * ostride + p] = s;
@@ -446,39 +454,34 @@ struct BStepPar {
   double lambda[BMAXS], s2[BMAXS];
 };
 __global__ void __launch_bounds__(BBLK) k_bstep(const BProb* __restrict__ probs, const BStepPar* par, int nsd, int blk,
-                                                double sz2sz, double* partial, int ncta_max) {
+                                                double sz2sz, double* partial, int nstep_max) {
   const BProb& P = probs[blockIdx.y];
-  if (!P.active || (int)blockIdx.x >= P.ncta) return;
-  __shared__ double red[BMAXS][BBLK / 32];
-  const BStepPar pp = par[blockIdx.y];
+  if (!P.active || (int)blockIdx.x >= P.nstep) return;
+  // a thread owns elements of one state, as in k_step
+  __shared__ double red[BBLK];
+  const BStepPar& pp = par[blockIdx.y];
   const int64_t N = P.N, off = (int64_t)blk * N * nsd;
-  double acc[BMAXS];
-#pragma unroll
-  for (int k = 0; k < BMAXS; ++k) acc[k] = 0.0;
-  const int64_t r0 = (int64_t)blockIdx.x * BROWS, r1 = min(r0 + BROWS, N);
-  for (int64_t r = r0 + threadIdx.x; r < r1; r += BBLK) {
-    const double h = P.hdiag[r];
-    for (int k = 0; k < nsd; ++k) {
-      const int64_t x = off + r * nsd + k;
-      const double u = P.U[x];
-      const double v = (pp.lambda[k] * u - P.W[x]) * (1.0 + pp.s2[k] * u - P.S[x] - sz2sz) / fmax(h - pp.lambda[k], 1e-2);
-      P.U[x] = v;
-      if (k < P.nst) acc[k] = fma(v, v, acc[k]);
+  const int nthr = BBLK / nsd * nsd, k = threadIdx.x % nsd;
+  const double lambda = pp.lambda[k], s2 = pp.s2[k];
+  double acc = 0.0;
+  const int64_t x0 = (int64_t)blockIdx.x * BSTEP * nsd, x1 = min(x0 + (int64_t)BSTEP * nsd, N * nsd);
+  if ((int)threadIdx.x < nthr)
+    for (int64_t x = x0 + threadIdx.x; x < x1; x += nthr) {
+      const double h = P.hdiag[x / nsd];
+      const double u = P.U[off + x];
+      const double v = (lambda * u - P.W[off + x]) * (1.0 + s2 * u - P.S[off + x] - sz2sz) / fmax(h - lambda, 1e-2);
+      P.U[off + x] = v;
+      acc = fma(v, v, acc);
     }
-  }
+  red[threadIdx.x] = acc;
+  __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < BMAXS; ++k) {
-    double s = acc[k];
+  if (w < nsd) {  // BBLK / 32 = BMAXS warps
+    double s = 0.0;
+    for (int t = w + nsd * lane; t < nthr; t += nsd * 32) s += red[t];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) red[k][w] = s;
-  }
-  __syncthreads();
-  if (threadIdx.x < BMAXS) {
-    double s = 0.0;
-    for (int i = 0; i < BBLK / 32; ++i) s += red[threadIdx.x][i];
-    partial[((int64_t)blockIdx.y * ncta_max + blockIdx.x) * BMAXS + threadIdx.x] = s;
+    if (lane == 0) partial[((int64_t)blockIdx.y * nstep_max + blockIdx.x) * BMAXS + w] = s;
   }
 }
 
@@ -567,8 +570,8 @@ void bsigma(qpgpu_batch* B, int nsd, int prec, int blk, int warps, int bps) {
 
 struct BDav {
   qpgpu_batch* B;
-  int nsd, itermax, ncta_max;
-  double* part = nullptr;   // [np][ncta_max][512]
+  int nsd, itermax, ncta_max, nstep_max;
+  double* part = nullptr;   // Gram partials [np][ncta_max][8][512], or step norms [np][nstep_max][BMAXS]
   double* small = nullptr;  // [np][SMALL]
   BStepPar* step = nullptr;
   int* mper = nullptr;      // [np] basis size of each problem's last Ritz step
@@ -580,12 +583,12 @@ void bgram(BDav& D, int asel, int a0, int nbA, int bsel, int bb, int out_off, co
   const int m = nbA * D.nsd;
   const int ci = 32 / D.nsd;
   const int ncg = (m + ci - 1) / ci;
-  const dim3 grid(D.ncta_max, B->np, (ncg + BBLK / 32 - 1) / (BBLK / 32));
+  const dim3 grid(D.ncta_max, B->np, (ncg + 7) / 8 * 8);
   const int ss = SMALL * 2;
   switch (D.nsd) {
 #define QP_BG(NS)                                                                                          \
   case NS:                                                                                                 \
-    k_bgram<NS><<<grid, BBLK, 0, B->st>>>(B->d, asel, a0, nbA, bsel, bb, D.part, 512, skip, ss, D.ncta_max); \
+    k_bgram<NS><<<grid, 32, 0, B->st>>>(B->d, asel, a0, nbA, bsel, bb, D.part, 512, skip, ss, D.ncta_max); \
     break;
     QP_BG(1)
     QP_BG(2)
@@ -597,7 +600,7 @@ void bgram(BDav& D, int asel, int a0, int nbA, int bsel, int bb, int out_off, co
     QP_BG(8)
 #undef QP_BG
   }
-  k_breduce<<<dim3(gsz((int64_t)m * D.nsd * 32), B->np), BBLK, 0, B->st>>>(B->d, D.part, 512, D.ncta_max, m * D.nsd,
+  k_breduce<<<dim3(gsz((int64_t)m * D.nsd * 32), B->np), BBLK, 0, B->st>>>(B->d, D.part, 512, D.ncta_max, m, D.nsd,
                                                                            D.small + out_off, SMALL);
 }
 
@@ -642,7 +645,7 @@ void segment_b(BDav& D, int b, double sz2sz, int64_t maxN) {
   const int nsd = D.nsd;
   BLin L{{AU, AW, AS}, {AU, AW, AS}, {b + 1, b + 1, b + 1}, 3};
   blin(D, L, 0, (b + 1) * nsd, nullptr, O_Y, 0, nullptr, 0, maxN);
-  k_bstep<<<dim3(D.ncta_max, B->np), BBLK, 0, B->st>>>(B->d, D.step, nsd, b + 1, sz2sz, D.part, D.ncta_max);
+  k_bstep<<<dim3(D.nstep_max, B->np), BBLK, 0, B->st>>>(B->d, D.step, nsd, b + 1, sz2sz, D.part, D.nstep_max);
 }
 
 // capture `fn` on the batch stream once and replay it afterwards
@@ -681,7 +684,6 @@ int qpgpu_batch_create(qpgpu_ctx* const* ctxs, int n, qpgpu_batch** out) {
     delete B;
     return QPGPU_ERR_CUDA;
   }
-  // the fixed-order group reduction of k_bgram uses up to 64 KB of shared memory
   B->h.resize(n);
   int64_t base = 0;
   for (int i = 0; i < n; ++i) {
@@ -708,6 +710,7 @@ int qpgpu_batch_create(qpgpu_ctx* const* ctxs, int n, qpgpu_batch** out) {
     p.n_multi = c->items.n_multi;
     p.item_base = base;
     p.ncta = (int)((c->N + BROWS - 1) / BROWS);
+    p.nstep = (int)((c->N + BSTEP - 1) / BSTEP);
     base += p.n_items;
   }
   B->total_items = base;
@@ -760,8 +763,11 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
   D.B = B;
   D.nsd = nsd;
   D.itermax = itermax;
-  D.ncta_max = 1;
-  for (auto& p : B->h) D.ncta_max = std::max(D.ncta_max, p.ncta);
+  D.ncta_max = D.nstep_max = 1;
+  for (auto& p : B->h) {
+    D.ncta_max = std::max(D.ncta_max, p.ncta);
+    D.nstep_max = std::max(D.nstep_max, p.nstep);
+  }
   // Davidson storage of the problems: pieces of one allocation (256-byte
   // aligned), sized in a first pass and handed out in a second
   if (B->slab_nsd != nsd || B->slab_itermax != itermax) {
@@ -787,7 +793,7 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
       P.nst = n_states[p];
       P.active = 1;
     }
-    take(D.part, (size_t)np * D.ncta_max * 512 * 8);
+    take(D.part, (size_t)np * std::max(D.ncta_max * 8 * 512, D.nstep_max * BMAXS) * 8);
     take(D.small, (size_t)np * SMALL * 8);
     take(D.step, (size_t)np * sizeof(BStepPar));
     take(D.mper, (size_t)np * sizeof(int));
@@ -857,7 +863,7 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
       return bfail(B, QPGPU_ERR_ARG, "all problems of a batch must have the same S_z");
   const int mmax = itermax * nsd;
   std::vector<std::vector<double>> H(np, std::vector<double>((size_t)mmax * mmax)), S2m = H;
-  std::vector<double> hostsmall((size_t)np * 1024), ystage((size_t)np * 512, 0.0), parts((size_t)np * D.ncta_max * BMAXS);
+  std::vector<double> hostsmall((size_t)np * 1024), ystage((size_t)np * 512, 0.0), parts((size_t)np * D.nstep_max * BMAXS);
   std::vector<BStepPar> sp(np);
   std::vector<std::vector<double>> lam(np, std::vector<double>(mmax)), s2v = lam;
   std::vector<int> mper(np, 0), copyf(np, 0), conv(np, 0), iters(np, 0);
@@ -900,14 +906,14 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
             ss[(size_t)i * shift2 + j] = s[(size_t)i * mmax + j];
           }
         qp_eigh(hs, shift2, w, y);
-        for (int k = 0; k < shift2; ++k) {
+        for (int k = 0; k < shift2; ++k) lam[p][k] = w[k];
+        for (int k = 0; k < (prm->s2_eig ? shift2 : nsd); ++k) {  // the filter looks at all of them
           double acc = 0.0;
           for (int i = 0; i < shift2; ++i) {
             double t = 0.0;
             for (int j = 0; j < shift2; ++j) t += ss[(size_t)i * shift2 + j] * y[(size_t)j * shift2 + k];
             acc += y[(size_t)i * shift2 + k] * t;
           }
-          lam[p][k] = w[k];
           s2v[p][k] = acc + sz2sz[p];
         }
         if (prm->s2_eig) {
@@ -949,7 +955,7 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
         double mx = 0.0;
         for (int k = 0; k < B->h[p].nst; ++k) {
           double r = 0.0;
-          for (int q = 0; q < B->h[p].ncta; ++q) r += parts[((size_t)p * D.ncta_max + q) * BMAXS + k];
+          for (int q = 0; q < B->h[p].nstep; ++q) r += parts[((size_t)p * D.nstep_max + q) * BMAXS + k];
           res[(size_t)p * BMAXS + k] = r;
           mx = std::max(mx, r);
         }

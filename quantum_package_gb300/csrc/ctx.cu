@@ -316,6 +316,7 @@ int qpgpu_destroy(qpgpu_ctx* c) {
     dev_free(c->d_direct_ut);
     dev_free(c->d_flag);
     dev_free(c->d_tc_scratch);
+    if (c->h_pin) cudaFreeHost(c->h_pin);
     cudaStreamSynchronize(c->stream);
     cudaMemPoolDestroy(c->pool);
     cudaStreamDestroy(c->stream);

@@ -467,10 +467,10 @@ template <int NSD>
 __global__ void __launch_bounds__(DBLK) k_lincomb(LinComb L, int nb, int64_t N, const double* C, const int* skip) {
   if (skip && *skip) return;
   __shared__ __align__(16) double Cs[MAXM * MAXS];
-  for (int i = threadIdx.x; i < nb * NSD * NSD; i += DBLK) Cs[i] = C[i];
+  for (int i = threadIdx.x; i < nb * NSD * NSD; i += blockDim.x) Cs[i] = C[i];
   __syncthreads();
   const int64_t sA = N * NSD;
-  for (int64_t r = blockIdx.x * (int64_t)DBLK + threadIdx.x; r < N; r += (int64_t)gridDim.x * DBLK) {
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < N; r += (int64_t)gridDim.x * blockDim.x) {
     for (int t = 0; t < L.n; ++t) {
       const double* a = L.A[t] + r * NSD;
       double acc[NSD], x[NSD], xn[NSD];
@@ -511,14 +511,14 @@ template <int NSD>
 __global__ void __launch_bounds__(DBLK) k_lincomb_ff(LinComb L, int nb, int64_t N, const double* C, const int* skip) {
   if (skip && *skip) return;
   __shared__ float2 Cs[MAXM * MAXS];
-  for (int i = threadIdx.x; i < nb * NSD * NSD; i += DBLK) {
+  for (int i = threadIdx.x; i < nb * NSD * NSD; i += blockDim.x) {
     float h, l;
     qpsig::split_ff(C[i], h, l);
     Cs[i] = make_float2(h, l);
   }
   __syncthreads();
   const int64_t sA = N * NSD;
-  for (int64_t r = blockIdx.x * (int64_t)DBLK + threadIdx.x; r < N; r += (int64_t)gridDim.x * DBLK) {
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < N; r += (int64_t)gridDim.x * blockDim.x) {
     for (int t = 0; t < L.n; ++t) {
       const double* a = L.A[t] + r * NSD;
       float ah[NSD], al[NSD];
@@ -579,10 +579,10 @@ __device__ __forceinline__ double f64_from(float f) {
 template <int NSD>
 __global__ void __launch_bounds__(DBLK) k_lincomb32(LinComb L, int nb, int64_t N, const double* C) {
   __shared__ float Cs[MAXM * MAXS];
-  for (int i = threadIdx.x; i < nb * NSD * NSD; i += DBLK) Cs[i] = f32_trunc(C[i]);
+  for (int i = threadIdx.x; i < nb * NSD * NSD; i += blockDim.x) Cs[i] = f32_trunc(C[i]);
   __syncthreads();
   const int64_t sA = N * NSD;
-  for (int64_t r = blockIdx.x * (int64_t)DBLK + threadIdx.x; r < N; r += (int64_t)gridDim.x * DBLK) {
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < N; r += (int64_t)gridDim.x * blockDim.x) {
     for (int t = 0; t < L.n; ++t) {
       const double* a = L.A[t] + r * NSD;
       float acc[NSD];
@@ -672,14 +672,21 @@ __global__ void k_chol_inv(const double* G, int nsd, double* Rinv) {
 // *skip2 = 0 asks for a second pass (mode 1), which always fuses.  Mode 1
 // returns at once when *skip2 is set.  A vanishing Cholesky pivot (a
 // dependent column) gives a zero column, as in k_chol_inv.
-__global__ void k_cgs_coef(const double* X, int m, int nsd, double* K, int* skip2, int mode) {
+//
+// One block; X is staged in shared memory first (a thread that walks it in
+// global memory waits for L2 at every term: 5.9 us at m = 20, nsd = 4).
+__global__ void __launch_bounds__(128) k_cgs_coef(const double* X, int m, int nsd, double* K, int* skip2, int mode) {
   if (mode == 1 && *skip2) return;
+  __shared__ double Xs[(MAXM + MAXS) * MAXS];
   __shared__ double G[MAXS][MAXS], R[MAXS][MAXS], Ri[MAXS][MAXS];
   __shared__ int need;
+  for (int idx = threadIdx.x; idx < (m + nsd) * nsd; idx += blockDim.x) Xs[idx] = X[idx];
+  __syncthreads();
   for (int idx = threadIdx.x; idx < nsd * nsd; idx += blockDim.x) {
     const int i = idx / nsd, j = idx % nsd;
-    double g = X[(m + i) * nsd + j];
-    for (int k = 0; k < m; ++k) g -= X[k * nsd + i] * X[k * nsd + j];
+    double g = Xs[(m + i) * nsd + j];
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) g -= Xs[k * nsd + i] * Xs[k * nsd + j];
     G[i][j] = g;
   }
   __syncthreads();
@@ -687,7 +694,7 @@ __global__ void k_cgs_coef(const double* X, int m, int nsd, double* K, int* skip
     int nd = 0;
     if (mode == 0)
       for (int j = 0; j < nsd; ++j)
-        if (!(G[j][j] > 0.25 * X[(m + j) * nsd + j])) nd = 1;
+        if (!(G[j][j] > 0.25 * Xs[(m + j) * nsd + j])) nd = 1;
     need = nd;
     if (mode == 0) *skip2 = nd ? 0 : 1;
   }
@@ -701,9 +708,9 @@ __global__ void k_cgs_coef(const double* X, int m, int nsd, double* K, int* skip
     if (i < m) {
       if (fuse) {
         v = 0.0;
-        for (int k = 0; k <= j; ++k) v -= X[i * nsd + k] * Ri[k][j];
+        for (int k = 0; k <= j; ++k) v -= Xs[i * nsd + k] * Ri[k][j];
       } else {
-        v = -X[i * nsd + j];
+        v = -Xs[i * nsd + j];
       }
     } else {
       v = fuse ? Ri[i - m][j] : (i - m == j ? 1.0 : 0.0);
@@ -719,39 +726,48 @@ struct StepParams {
   int nsd, nst;
 };
 
-// Davidson step (diagonalization_hs2.irp.f:386-391), in place on the Ritz
-// block, and per-CTA partial sums of its squared norms (:395)
-__global__ void __launch_bounds__(DBLK) k_step(double* Un, const double* Wn, const double* Sn, const double* hjj,
-                                               int64_t N, StepParams p, double* partial) {
-  __shared__ double red[MAXS][DBLK / 32];
-  double acc[MAXS];
-#pragma unroll
-  for (int k = 0; k < MAXS; ++k) acc[k] = 0.0;
-  for (int64_t r = blockIdx.x * (int64_t)DBLK + threadIdx.x; r < N; r += (int64_t)gridDim.x * DBLK) {
-    const double h = hjj[r];
-    for (int k = 0; k < p.nsd; ++k) {
-      const int64_t x = r * p.nsd + k;
-      const double u = Un[x];
-      const double v = (p.lambda[k] * u - Wn[x]) * (1.0 + p.s2[k] * u - Sn[x] - p.sz2sz) /
-                       fmax(h - p.lambda[k], 1e-2);
-      Un[x] = v;
-      if (k < p.nst) acc[k] = fma(v, v, acc[k]);
-    }
-  }
+// per-block sums of acc over the threads of each state (state = thread index
+// modulo nsd): shared memory, then one warp per state in a fixed order
+__device__ __forceinline__ void block_state_sums(double acc, int nsd, int nthr, double* red, double* partial) {
+  red[threadIdx.x] = acc;
+  __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < MAXS; ++k) {
-    double s = acc[k];
+  if (w < nsd) {  // DBLK / 32 = MAXS warps
+    double s = 0.0;
+    for (int t = w + nsd * lane; t < nthr; t += nsd * 32) s += red[t];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) red[k][w] = s;
+    if (lane == 0) partial[(int64_t)blockIdx.x * MAXS + w] = s;
   }
-  __syncthreads();
-  if (threadIdx.x < MAXS) {
-    double s = 0.0;
-    for (int i = 0; i < DBLK / 32; ++i) s += red[threadIdx.x][i];
-    partial[(int64_t)blockIdx.x * MAXS + threadIdx.x] = s;
-  }
+}
+
+// Davidson step (diagonalization_hs2.irp.f:386-391), in place on the Ritz
+// block, and per-CTA partial sums of its squared norms (:395).  A thread owns
+// elements of one state (the first nsd floor(256 / nsd) threads of a block
+// work), as the FP64 division of a row's states one after the other left a
+// 1e4 set on 40 SMs with a 12.7 us chain each.
+__global__ void __launch_bounds__(DBLK) k_step(double* Un, const double* Wn, const double* Sn, const double* hjj,
+                                               int64_t N, StepParams p, double* partial) {
+  __shared__ double red[DBLK];
+  const int nthr = DBLK / p.nsd * p.nsd;
+  const int k = threadIdx.x % p.nsd;
+  double lambda = 0.0, s2 = 0.0;
+#pragma unroll
+  for (int q = 0; q < MAXS; ++q)
+    if (q == k) {
+      lambda = p.lambda[q];
+      s2 = p.s2[q];
+    }
+  double acc = 0.0;
+  if ((int)threadIdx.x < nthr)
+    for (int64_t x = blockIdx.x * (int64_t)nthr + threadIdx.x; x < N * p.nsd; x += (int64_t)gridDim.x * nthr) {
+      const double h = hjj[x / p.nsd];
+      const double u = Un[x];
+      const double v = (lambda * u - Wn[x]) * (1.0 + s2 * u - Sn[x] - p.sz2sz) / fmax(h - lambda, 1e-2);
+      Un[x] = v;
+      acc = fma(v, v, acc);
+    }
+  block_state_sums(acc, p.nsd, nthr, red, partial);
 }
 
 // The Davidson step of k_step for the mixed-precision loop: the residual
@@ -762,43 +778,31 @@ __global__ void __launch_bounds__(DBLK) k_step(double* Un, const double* Wn, con
 // convergence measure, both needed to a few digits.
 __global__ void __launch_bounds__(DBLK) k_step_mixed(double* Un, const double* Wn, const double* Sn, const double* hjj,
                                                      int64_t N, StepParams p, double* partial) {
-  __shared__ double red[MAXS][DBLK / 32];
-  float acc[MAXS];
+  __shared__ double red[DBLK];
+  const int nthr = DBLK / p.nsd * p.nsd;
+  const int k = threadIdx.x % p.nsd;
+  double lambda = 0.0;
+  float s2f = 0.f;
 #pragma unroll
-  for (int k = 0; k < MAXS; ++k) acc[k] = 0.f;
+  for (int q = 0; q < MAXS; ++q)
+    if (q == k) {
+      lambda = p.lambda[q];
+      s2f = (float)p.s2[q];
+    }
   const float sz2sz = (float)p.sz2sz;
-  float s2f[MAXS];
-#pragma unroll
-  for (int k = 0; k < MAXS; ++k) s2f[k] = (float)p.s2[k];
-  for (int64_t r = blockIdx.x * (int64_t)DBLK + threadIdx.x; r < N; r += (int64_t)gridDim.x * DBLK) {
-    const double h = hjj[r];
-#pragma unroll
-    for (int k = 0; k < MAXS; ++k) {
-      if (k >= p.nsd) break;
-      const int64_t x = r * p.nsd + k;
+  float acc = 0.f;
+  if ((int)threadIdx.x < nthr)
+    for (int64_t x = blockIdx.x * (int64_t)nthr + threadIdx.x; x < N * p.nsd; x += (int64_t)gridDim.x * nthr) {
+      const double h = hjj[x / p.nsd];
       const double u = Un[x];
-      const float num = f32_trunc(fma(p.lambda[k], u, -Wn[x]));
-      const float fac = 1.0f + s2f[k] * f32_trunc(u) - f32_trunc(Sn[x]) - sz2sz;
-      const float den = fmaxf(f32_trunc(h - p.lambda[k]), 1e-2f);
+      const float num = f32_trunc(fma(lambda, u, -Wn[x]));
+      const float fac = 1.0f + s2f * f32_trunc(u) - f32_trunc(Sn[x]) - sz2sz;
+      const float den = fmaxf(f32_trunc(h - lambda), 1e-2f);
       const float v = __fdiv_rn(num * fac, den);
       Un[x] = f64_from(v);
-      if (k < p.nst) acc[k] = fmaf(v, v, acc[k]);
+      acc = fmaf(v, v, acc);
     }
-  }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < MAXS; ++k) {
-    double s = (double)acc[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) red[k][w] = s;
-  }
-  __syncthreads();
-  if (threadIdx.x < MAXS) {
-    double s = 0.0;
-    for (int i = 0; i < DBLK / 32; ++i) s += red[threadIdx.x][i];
-    partial[(int64_t)blockIdx.x * MAXS + threadIdx.x] = s;
-  }
+  block_state_sums((double)acc, p.nsd, nthr, red, partial);
 }
 
 // Features of the target states for the learned step (qp_features), one row
@@ -1031,6 +1035,17 @@ constexpr int OFF_RINV = OFF_G + MAXS * MAXS;
 constexpr int OFF_FLAG = OFF_RINV + MAXS * MAXS;
 constexpr int SMALL_DOUBLES = OFF_FLAG + 8;
 
+// launch shape of the linear combinations (a thread per row): blocks of 64
+// rows as long as 256 would leave SMs without one (the FP64 pipe of an SM is
+// their bound, so 40 blocks of a 1e4 set use 40 of 152 of them)
+struct RowShape {
+  unsigned grid, block;
+};
+inline RowShape row_shape(const Dav& d) {
+  const unsigned bs = d.N <= (int64_t)DBLK * 2 * d.c->n_sm ? 64 : DBLK;
+  return {std::min<unsigned>(gsz(d.N, (int)bs), d.c->n_sm * 8 * (DBLK / bs)), bs};
+}
+
 // out (m x nbc) = A^T [B0 (B1)] with A = m columns of consecutive blocks
 int gram(Dav& d, const double* A, int m, const double* B0, const double* B1, double* out, const int* skip = nullptr) {
   const int nbc = d.nsd * (B1 ? 2 : 1);
@@ -1165,11 +1180,11 @@ void lincomb(Dav& d, int m, const double* C, const double* A0, double* O0, const
     L.n = 3;
   }
   const int nb = m / d.nsd;
-  const unsigned grid = std::min<unsigned>(gsz(d.N), d.c->n_sm * 8);
+  const RowShape sh = row_shape(d);
   switch (d.nsd) {
 #define QP_LC_CASE(NS) \
   case NS:             \
-    k_lincomb<NS><<<grid, DBLK, 0, d.st>>>(L, nb, d.N, C, skip); \
+    k_lincomb<NS><<<sh.grid, sh.block, 0, d.st>>>(L, nb, d.N, C, skip); \
     break;
     QP_LC_CASE(1)
     QP_LC_CASE(2)
@@ -1202,11 +1217,11 @@ void lincomb_ff(Dav& d, int m, const double* C, const double* A0, double* O0, co
     L.n = 3;
   }
   const int nb = m / d.nsd;
-  const unsigned grid = std::min<unsigned>(gsz(d.N), d.c->n_sm * 8);
+  const RowShape sh = row_shape(d);
   switch (d.nsd) {
 #define QP_LCF_CASE(NS) \
   case NS:              \
-    k_lincomb_ff<NS><<<grid, DBLK, 0, d.st>>>(L, nb, d.N, C, skip); \
+    k_lincomb_ff<NS><<<sh.grid, sh.block, 0, d.st>>>(L, nb, d.N, C, skip); \
     break;
     QP_LCF_CASE(1)
     QP_LCF_CASE(2)
@@ -1232,11 +1247,11 @@ void lincomb32(Dav& d, int m, const double* C, const double* A0, double* O0, con
   L.out[2] = O2;
   L.n = 3;
   const int nb = m / d.nsd;
-  const unsigned grid = std::min<unsigned>(gsz(d.N), d.c->n_sm * 8);
+  const RowShape sh = row_shape(d);
   switch (d.nsd) {
 #define QP_LC32_CASE(NS) \
   case NS:               \
-    k_lincomb32<NS><<<grid, DBLK, 0, d.st>>>(L, nb, d.N, C); \
+    k_lincomb32<NS><<<sh.grid, sh.block, 0, d.st>>>(L, nb, d.N, C); \
     break;
     QP_LC32_CASE(1)
     QP_LC32_CASE(2)
@@ -1481,16 +1496,41 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
   const double sz2sz = Sz * (Sz - 1.0), expected_s2 = Sz * (Sz + 1.0);
   const int mmax = itermax * nsd;
   std::vector<double> h((size_t)mmax * mmax, 0.0), s_((size_t)mmax * mmax, 0.0);
-  std::vector<double> hcol((size_t)mmax * nsd), scol((size_t)mmax * nsd), hscol((size_t)mmax * 2 * nsd);
-  std::vector<double> lambda(mmax), s2(mmax), y, wv, res(MAXS, 0.0), partial((size_t)d.ncta * MAXS);
+  std::vector<double> hcol((size_t)mmax * nsd), scol((size_t)mmax * nsd);
+  std::vector<double> lambda(mmax), s2(mmax), y, wv, res(MAXS, 0.0);
+  // pinned staging of the small copies: Gram columns, y, norms, status
+  const size_t n_pin = (size_t)MAXM * 2 * MAXS + (size_t)MAXM * MAXS + (size_t)d.ncta * MAXS + 2;
+  if (c->h_pin_doubles < n_pin) {
+    if (c->h_pin) cudaFreeHost(c->h_pin);
+    c->h_pin = nullptr;
+    c->h_pin_doubles = 0;
+    QP_CUDA(c, cudaMallocHost((void**)&c->h_pin, n_pin * sizeof(double)));
+    c->h_pin_doubles = n_pin;
+  }
+  double* const hscol = c->h_pin;
+  double* const ycoef = hscol + MAXM * 2 * MAXS;
+  double* const partial = ycoef + MAXM * MAXS;
+  int* const tc_status = (int*)(partial + (size_t)d.ncta * MAXS);
+  *tc_status = 0;
+  struct Event {
+    cudaEvent_t e = nullptr;
+    ~Event() {
+      if (e) cudaEventDestroy(e);
+    }
+  } norms_ready;
+  QP_CUDA(c, cudaEventCreateWithFlags(&norms_ready.e, cudaEventDisableTiming));
+  bool ortho_done = false;  // the next block was orthonormalised ahead
   int n_sigma = 0, shift2 = 0, trace_n = 0;
   bool converged = false, failed = false;
-  auto record = [&](int prec) {
+  auto record_time = [&] {
     if (!trace || trace_n >= trace->cap) return;
     cudaEvent_t e;
     cudaEventCreate(&e);
     cudaEventRecord(e, st);
     evs.push_back(e);
+  };
+  auto record = [&](int prec) {
+    if (!trace || trace_n >= trace->cap) return;
     if (trace->sigma_precision) trace->sigma_precision[trace_n] = prec;
     for (int k = 0; k < nst; ++k) {
       if (trace->energies) trace->energies[(size_t)trace_n * nst + k] = lambda[k];
@@ -1507,7 +1547,8 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
       const int b = iter - 1;
       const int shift = nsd * b;
       shift2 = nsd * iter;
-      orthonormalise(d, b, ffalg);
+      if (!ortho_done) orthonormalise(d, b, ffalg);
+      ortho_done = false;
       prof.mark(DavProf::ORTHO);
       // sigma on block b
       const int prec = (mixed && iter > 1) ? QPGPU_FP32 : restart_prec;
@@ -1530,7 +1571,7 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
       } else {
         gram(d, d.U, shift2, d.blk(d.W, b), d.blk(d.S, b), d.small + OFF_X);
       }
-      QP_CUDA(c, cudaMemcpyAsync(hscol.data(), d.small + OFF_X, (size_t)shift2 * 2 * nsd * sizeof(double),
+      QP_CUDA(c, cudaMemcpyAsync(hscol, d.small + OFF_X, (size_t)shift2 * 2 * nsd * sizeof(double),
                                  cudaMemcpyDeviceToHost, st));
       QP_CUDA(c, cudaStreamSynchronize(st));
       for (int i = 0; i < shift2; ++i)
@@ -1555,8 +1596,9 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
         }
       qp_eigh(hs, shift2, wv, y);
       for (int k = 0; k < shift2; ++k) lambda[k] = wv[k];
-      // S^2 of the Ritz vectors (:289-301): s2_k = y_k^T s y_k + S_z(S_z-1)
-      for (int k = 0; k < shift2; ++k) {
+      // S^2 of the Ritz vectors (:289-301): s2_k = y_k^T s y_k + S_z(S_z-1),
+      // of all of them only when the filter looks at them
+      for (int k = 0; k < (prm->s2_eig ? shift2 : nsd); ++k) {
         double acc = 0.0;
         for (int i = 0; i < shift2; ++i) {
           double t = 0.0;
@@ -1610,12 +1652,11 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
         }
       }
       // Ritz vectors into block b+1 (:376-381); coefficients y(0:shift2, 0:nsd)
-      std::vector<double> ycoef((size_t)shift2 * nsd);
       for (int i = 0; i < shift2; ++i)
         for (int j = 0; j < nsd; ++j) ycoef[(size_t)i * nsd + j] = y[(size_t)i * shift2 + j];
       double* ydev = d.small + OFF_Y;
       prof.mark(DavProf::HOST);
-      QP_CUDA(c, cudaMemcpyAsync(ydev, ycoef.data(), ycoef.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+      QP_CUDA(c, cudaMemcpyAsync(ydev, ycoef, (size_t)shift2 * nsd * sizeof(double), cudaMemcpyHostToDevice, st));
       if ((ffalg || tcalg) && prec == QPGPU_FP32)  // W, S from the FP32 sigma: FP32 Ritz vectors feed the step
         lincomb32(d, shift2, ydev, d.U, d.blk(d.U, iter), d.W, d.blk(d.W, iter), d.S, d.blk(d.S, iter));
       else if (ffalg)  // restart iteration: float-float
@@ -1656,12 +1697,19 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
       else
         k_step<<<d.ncta, DBLK, 0, st>>>(d.blk(d.U, iter), d.blk(d.W, iter), d.blk(d.S, iter), hjj, N, sp, d.part);
       QP_CUDA(c, cudaGetLastError());
-      QP_CUDA(c, cudaMemcpyAsync(partial.data(), d.part, partial.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-      int tc_status = 0;
+      QP_CUDA(c, cudaMemcpyAsync(partial, d.part, (size_t)d.ncta * MAXS * sizeof(double), cudaMemcpyDeviceToHost, st));
       if (tcalg)
-        QP_CUDA(c, cudaMemcpyAsync(&tc_status, d.bexp + 2 * MAXS, sizeof(int), cudaMemcpyDeviceToHost, st));
-      QP_CUDA(c, cudaStreamSynchronize(st));
-      if (tc_status) {
+        QP_CUDA(c, cudaMemcpyAsync(tc_status, d.bexp + 2 * MAXS, sizeof(int), cudaMemcpyDeviceToHost, st));
+      record_time();
+      QP_CUDA(c, cudaEventRecord(norms_ready.e, st));
+      // the next block is orthonormalised while the norms travel; when they
+      // end the cycle or the run its block is not read
+      if (iter < itermax - 1 && n_sigma < max_sigma) {
+        orthonormalise(d, iter, ffalg);
+        ortho_done = true;
+      }
+      QP_CUDA(c, cudaEventSynchronize(norms_ready.e));
+      if (*tc_status) {
         cudaEventDestroy(ev0);
         return qpgpu_fail(c, QPGPU_ERR_TIMEOUT, "Davidson: a bounded tensor-core wait of the Gram blocks ran out");
       }
@@ -1704,11 +1752,8 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
       if (n_sigma >= max_sigma) break;
     }
     // re-contract (:419-420): U(:,0..shift2) y(:,0..nsd) -> block 0
-    std::vector<double> ycoef((size_t)shift2 * nsd);
-    for (int i = 0; i < shift2; ++i)
-      for (int j = 0; j < nsd; ++j) ycoef[(size_t)i * nsd + j] = y[(size_t)i * shift2 + j];
-    double* ydev = d.small + OFF_Y;
-    QP_CUDA(c, cudaMemcpyAsync(ydev, ycoef.data(), ycoef.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+    ortho_done = false;
+    double* ydev = d.small + OFF_Y;  // still the coefficients of the last Ritz vectors
     if (ffalg)
       lincomb_ff(d, shift2, ydev, d.U, d.R);
     else if (tcalg)

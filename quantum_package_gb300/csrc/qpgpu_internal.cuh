@@ -619,6 +619,8 @@ struct qpgpu_ctx {
   bool profile = false;
   std::vector<std::pair<std::string, cudaEvent_t>> marks;
 
+  double* h_pin = nullptr;  // pinned staging of the Davidson's small copies
+  size_t h_pin_doubles = 0;
   int* d_flag = nullptr;  // NaN / Inf flag of the host-array entry points
   void* d_tc_scratch = nullptr;  // qpgpu_gram_tc: per-CTA partials, exponents, status
   size_t tc_scratch_bytes = 0;
