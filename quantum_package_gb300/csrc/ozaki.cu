@@ -11,8 +11,8 @@
 // fixed-point integer F = round(|x| 2^(56 - E_c)) and written in balanced
 // base 128, F = sum_p d_p 2^(49 - 7p) with d_1..d_7 in [-64, 63] and d_0 in
 // [0, 128], every digit times the sign of x: integers exact in BF16.  The
-// digits are those of F + 64 (1 + 2^7 + ... + 2^49) less 64 each, so they
-// come out of independent shifts and masks, with no carry chain.
+// digits below the first are those of F + 64 (1 + 2^7 + ... + 2^42) less 64
+// each, so they come out of independent shifts and masks, with no carry chain.
 // Balanced digits make both the rounding and the dropped low-order products
 // zero-mean, so they do not pile up in sums of squares (Gram diagonals).
 //
@@ -30,16 +30,16 @@
 //
 // Pipeline (one CTA per SM over a contiguous block of rows, chunks of 32
 // rows), one role per warp:
-//  * warp 13 streams the raw FP64 rows of each chunk into a ring of raw
+//  * the last warp streams the raw FP64 rows of each chunk into a ring of raw
 //    stages (cp.async.bulk per operand block, completing on rawfull[r]; a
 //    block whose rows are strided or unaligned is copied by the warp's lanes);
-//  * warps 0-7 cut the chunk into digit planes (stores of 2, 4 or 8 rows of
+//  * warps 0-11 cut the chunk into digit planes (stores of 2, 4 or 8 rows of
 //    one column), free the raw stage (rawempty[r]) and fill digit stage s
 //    (full[s]);
-//  * warp 12 issues the chunk's 16 MMAs once full[s] completes and commits
+//  * one warp issues the chunk's 16 MMAs once full[s] completes and commits
 //    them to empty[s] and, at the end of a window, to accf[b]; the windows
 //    rotate over four tensor-memory accumulator buffers b;
-//  * warps 8-11, whose lane quarters cover the 128 accumulator rows, add a
+//  * four warps, whose lane quarters cover the 128 accumulator rows, add a
 //    finished window to their int64 sums and arrive on acce[b], so that the
 //    integer work never holds up the splitting.
 // A plane p of A meets B planes 0..7-p only (levels p..7), so its MMA has
@@ -54,11 +54,12 @@
 
 namespace {
 
-constexpr int OZ_SPLIT = 256;                // splitting threads (warps 0-7)
-constexpr int OZ_FLUSH_WARP = 8;             // warps 8-11 flush the accumulators
-constexpr int OZ_MMA_WARP = 12;              // issues the MMAs, owns the tensor memory
-constexpr int OZ_LOAD_WARP = 13;             // streams the raw rows
-constexpr int OZ_THREADS = 14 * 32;
+constexpr int OZ_SPLIT = 384;                // splitting threads (warps 0-11)
+constexpr int OZ_FLUSH_WARP = OZ_SPLIT / 32;       // the next 4 warps flush the accumulators (a multiple of 4)
+constexpr int OZ_MMA_WARP = OZ_FLUSH_WARP + 4;     // issues the MMAs, owns the tensor memory
+constexpr int OZ_LOAD_WARP = OZ_MMA_WARP + 1;      // streams the raw rows
+constexpr int OZ_THREADS = (OZ_LOAD_WARP + 1) * 32;
+static_assert(OZ_FLUSH_WARP % 4 == 0, "flush warp w reads the accumulator lanes of quarter w % 4");
 constexpr int OZ_M = 128;                    // MMA M: columns of A (padded)
 constexpr int OZ_N = 16;                     // columns of B (padded)
 constexpr int OZ_KC = 32;                    // rows per chunk (MMA K = 2 x 16)
@@ -125,43 +126,56 @@ __device__ __forceinline__ uint32_t oz_idesc(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(OZ_M >> 4) << 24);
 }
 
-// 64 in every base-128 digit position of a 56-bit integer
-constexpr unsigned long long OZ_H = 64ull * ((1ull << 49) | (1ull << 42) | (1ull << 35) | (1ull << 28) |
-                                             (1ull << 21) | (1ull << 14) | (1ull << 7) | 1ull);
+// 64 in every base-128 digit position of a 56-bit integer but the first
+constexpr unsigned long long OZ_H = 64ull * ((1ull << 42) | (1ull << 35) | (1ull << 28) | (1ull << 21) |
+                                             (1ull << 14) | (1ull << 7) | 1ull);
 
-// the 8 balanced digits of x against the column's biased max exponent eb
-// (|x| < 2^(eb - 1022)), as FP32 values (exact small integers, so their top
-// 16 bits are their BF16 bits).  F = round(|x| 2^(56 - E)), E = eb - 1022,
-// is the 53-bit significand M = m53 2^3 rounded-shifted right by eb - ex
-// (<= 2^56).  With G = F + OZ_H, the plain base-128 digits g_p of G less 64
-// are a balanced expansion of F: F = sum_p (g_p - 64) 2^(49 - 7p), d_0 in
-// [0, 128] and d_1..d_7 in [-64, 63].  No digit waits on another: each is a
-// shift, a mask with the 2^23 exponent bits, and one exact FMA that removes
-// 2^23 + 64 and applies the sign of x.
-__device__ __forceinline__ void oz_digits(double x, int eb, float (&d)[OZ_DIG]) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const uint32_t bh = (uint32_t)(b >> 32);
+// 2 (F + OZ_H) + (0 or 1) of x against the biased max exponent eb
+// (|x| < 2^(eb - 1022)): F = round(|x| 2^(56 - E)), E = eb - 1022, is the
+// 53-bit significand times 2^3 shifted right by eb - ex and rounded (half
+// up).  Shifted one bit less, the rounding is the carry of an added 1, and it
+// and the digit offsets are one addition; the digits then sit one bit higher.
+__device__ __forceinline__ unsigned long long oz_fixed(uint32_t bh, uint32_t bl, int eb) {
   const int ex = (int)((bh >> 20) & 0x7FF);
-  const int k = max(eb - ex, 0);
-  unsigned long long F = 0;
-  if (ex != 0 && k < 57) {
-    const unsigned long long M = ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 3;
-    F = k == 0 ? M : (M + (1ull << (k - 1))) >> k;
-  }
-  const unsigned long long G = F + OZ_H;
-  const uint32_t gl = (uint32_t)G, gh = (uint32_t)(G >> 32);
-  const uint32_t sbit = bh & 0x80000000u;
-  const float sg = __uint_as_float(sbit | 0x3F800000u);   // +-1
-  const float sc = __uint_as_float(sbit | 0x4B000040u);   // +-(2^23 + 64)
-  const uint32_t g[OZ_DIG] = {gh >> 17, gh >> 10, gh >> 3, __funnelshift_r(gl, gh, 28), gl >> 21, gl >> 14, gl >> 7, gl};
-#pragma unroll
-  for (int p = 0; p < OZ_DIG; ++p)
-    d[p] = __fmaf_rn(sg, __uint_as_float(0x4B000000u | (g[p] & (p == 0 ? 0xFFu : 0x7Fu))), -sc);
+  int k = min(max(eb - ex, 0), 63);
+  if (ex == 0) k = 63;  // zeros and subnormals: F = 0
+  const uint32_t mh = __funnelshift_l(bl, (bh & 0xFFFFFu) | 0x100000u, 4), ml = bl << 4;
+  return ((((unsigned long long)mh << 32) | ml) >> k) + (2 * OZ_H + 1);
 }
 
-// BF16 bits of two exact small-integer FP32 values, packed (lo, hi)
-__device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
-  return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+// the 8 balanced digits of two values against the biased max exponents e0,
+// e1, as BF16 pairs (x0 in the low half).  With G = F + OZ_H, the plain
+// base-128 digits g_p of G give F = sum_p d_p 2^(49 - 7p) with d_0 = g_0 in
+// [0, 128] and d_p = g_p - 64 in [-64, 63].  A digit n in the low bits of
+// 0x4300 is the BF16 value 128 + n (128 gives 256), so a plane of both values
+// is a mask and the exponent bits in one instruction and one packed FMA that
+// takes off 128 (+ 64) and applies the signs, all exact; a pair of digits
+// shares one 16-bit window of each value.  About 29 integer instructions a
+// value, against about 40 with a digit at a time through FP32.
+__device__ __forceinline__ uint32_t bf16_fma2(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+__device__ __forceinline__ void oz_digits2(double x0, double x1, int e0, int e1, uint32_t (&d)[OZ_DIG]) {
+  const uint32_t h0 = (uint32_t)__double2hiint(x0), l0 = (uint32_t)__double2loint(x0);
+  const uint32_t h1 = (uint32_t)__double2hiint(x1), l1 = (uint32_t)__double2loint(x1);
+  const unsigned long long g0 = oz_fixed(h0, l0, e0), g1 = oz_fixed(h1, l1, e1);
+  const uint32_t a0 = (uint32_t)g0, b0 = (uint32_t)(g0 >> 32), a1 = (uint32_t)g1, b1 = (uint32_t)(g1 >> 32);
+  // 16-bit windows of both values: digit pairs (6, 7), (4, 5), (2, 3), (0, 1)
+  const uint32_t w3 = __byte_perm(a0 >> 1, a1 >> 1, 0x5410), w2 = __byte_perm(a0 >> 15, a1 >> 15, 0x5410);
+  const uint32_t w1 = __byte_perm(__funnelshift_r(a0, b0, 29), __funnelshift_r(a1, b1, 29), 0x5410);
+  const uint32_t w0 = __byte_perm(b0 >> 11, b1 >> 11, 0x5410);
+  const uint32_t sg = __byte_perm(h0, h1, 0x7632) & 0x80008000u;
+  const uint32_t one = sg | 0x3F803F80u, c128 = sg ^ 0xC300C300u, c192 = sg ^ 0xC340C340u;  // +-1, -+128, -+192
+  d[0] = bf16_fma2(((w0 >> 7) & 0x00FF00FFu) + 0x43004300u, one, c128);
+  d[1] = bf16_fma2((w0 & 0x007F007Fu) | 0x43004300u, one, c192);
+  d[2] = bf16_fma2(((w1 >> 7) & 0x007F007Fu) | 0x43004300u, one, c192);
+  d[3] = bf16_fma2((w1 & 0x007F007Fu) | 0x43004300u, one, c192);
+  d[4] = bf16_fma2(((w2 >> 7) & 0x007F007Fu) | 0x43004300u, one, c192);
+  d[5] = bf16_fma2((w2 & 0x007F007Fu) | 0x43004300u, one, c192);
+  d[6] = bf16_fma2(((w3 >> 7) & 0x007F007Fu) | 0x43004300u, one, c192);
+  d[7] = bf16_fma2((w3 & 0x007F007Fu) | 0x43004300u, one, c192);
 }
 
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
@@ -229,11 +243,10 @@ __device__ __forceinline__ void oz_split(const double* rsrc, uint8_t* sa, uint8_
     uint32_t pk[OZ_DIG][RPT / 2];
 #pragma unroll
     for (int k = 0; k < RPT; k += 2) {
-      float d0[OZ_DIG], d1[OZ_DIG];
-      oz_digits(k0 + k < nrow ? xs[k * wcol] : 0.0, eb, d0);
-      oz_digits(k0 + k + 1 < nrow ? xs[(k + 1) * wcol] : 0.0, eb, d1);
+      uint32_t d[OZ_DIG];
+      oz_digits2(k0 + k < nrow ? xs[k * wcol] : 0.0, k0 + k + 1 < nrow ? xs[(k + 1) * wcol] : 0.0, eb, eb, d);
 #pragma unroll
-      for (int p = 0; p < OZ_DIG; ++p) pk[p][k >> 1] = bf16x2(d0[p], d1[p]);
+      for (int p = 0; p < OZ_DIG; ++p) pk[p][k >> 1] = d[p];
     }
     uint8_t* dst = (isA ? sa : sb) + kmaj(cc, k0);
     const int tile = isA ? OZ_A_TILE : OZ_B_TILE;
@@ -512,23 +525,43 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
 // The contraction runs over i, so each row r of A gets its own exponent
 // (the largest over its m values) and C one per column j; the digits and
 // levels are those of k_gram_oz, and a level of one entry sums at most
-// m <= 128 products, below 2^23.  One CTA per SM walks tiles of 128 rows:
-// the tile's rows are loaded into shared memory, its row exponents formed,
-// then each K step of 16 columns is cut into the 8 A digit planes (two
-// stages, so that the split of step c + 1 overlaps the MMAs of step c) and
-// one thread issues its 8 MMAs (M = 128 rows, N = (8 - p) 16, K = 16) into
-// the tile's accumulator; when the tile's MMAs are done, warps 0-3 read the
-// 8 levels of their rows and write O in FP64.  The digit planes of C are
-// built once per CTA.  Waits are bounded as in k_gram_oz.
-constexpr int LC_THREADS = 512;             // 16 warps: 4 threads per row of a tile
-constexpr int LC_RQ = LC_THREADS / 128;      // threads per row
+// m <= 128 products, below 2^23.
+//
+// One CTA per SM walks tiles of 128 rows, one role per warp:
+//  * the load warp streams the tile's blocks into shared memory (one
+//    cp.async.bulk per block, completing on rawf) and refills a block with
+//    the next tile's rows as soon as the K step that read it last is cut
+//    (cons[c]);
+//  * warps 0-15 form the row exponents and cut each K step of 16 columns into
+//    the 8 A digit planes of stage s (full[s]); a warp owns 8 rows, its lanes
+//    4 columns each, so that a row's exponent is two shuffles and the two
+//    16-byte loads of a lane, the second half first in the upper columns,
+//    touch every bank once;
+//  * the MMA warp issues the step's 8 MMAs (M = 128 rows, N = (8 - p) 16,
+//    K = 16) into one of two tensor-memory accumulators and commits them to
+//    empty[s] and, at the end of a tile, to accf[b];
+//  * four warps read a finished accumulator, add its levels as integers and
+//    write the tile's rows of O in FP64 (acce[b]).
+// The digit planes of C are built once per CTA.  Waits are bounded as in
+// k_gram_oz.  1e6 rows x 80 -> 8 columns: 798 us when all warps cut, issued
+// and flushed in turn behind block barriers (30k cycles a tile).
+constexpr int LC_SPLIT_WARPS = 16;
+constexpr int LC_FLUSH_WARP = LC_SPLIT_WARPS;    // a multiple of 4: warp w reads lane quarter w % 4
+constexpr int LC_MMA_WARP = LC_FLUSH_WARP + 4;
+constexpr int LC_LOAD_WARP = LC_MMA_WARP + 1;
+constexpr int LC_THREADS = (LC_LOAD_WARP + 1) * 32;
 constexpr int LC_TM = 128;                       // rows per tile (MMA M)
 constexpr int LC_KS = 16;                        // K step (columns of A)
 constexpr int LC_APLANE = LC_TM * LC_KS * 2;     // 4 KB: one A digit plane of one K step
 constexpr int LC_ASTAGE = OZ_DIG * LC_APLANE;    // 32 KB
 constexpr int LC_BCHUNK = OZ_DIG * OZ_N * LC_KS * 2;  // 4 KB: the 8 C planes of one K step
 constexpr int LC_MAXM = 128;
-constexpr int LC_TMEM_COLS = OZ_LEVELS * OZ_N;   // 128
+constexpr int LC_MAXKS = LC_MAXM / LC_KS;
+constexpr int LC_ACC_COLS = OZ_LEVELS * OZ_N;    // 128 tensor-memory columns per accumulator
+constexpr int LC_TMEM_COLS = 2 * LC_ACC_COLS;
+// barrier slots
+constexpr int LC_B_FULL = 0, LC_B_EMPTY = 2, LC_B_ACCF = 4, LC_B_ACCE = 6, LC_B_RAWF = 8, LC_B_CONS = 9,
+              LC_NBARS = LC_B_CONS + LC_MAXKS;
 
 struct LcArgs {
   const double* A;
@@ -538,7 +571,7 @@ struct LcArgs {
   double* O;
   int64_t ldO;
   int64_t N, rows_per_cta;
-  int row_stride;  // doubles per staged row in shared memory
+  int lane_copies;  // some block of some tile is not whole 16-byte lines
   const int* skip;
   int* status;
 };
@@ -553,10 +586,18 @@ __device__ __forceinline__ uint64_t sdesc16(uint32_t addr) {
          ((uint64_t)1 << 46);
 }
 
-__device__ __forceinline__ int biased_exp(double x) {
-  return (int)(((unsigned long long)__double_as_longlong(x) >> 52) & 0x7FF);
+__device__ __forceinline__ int biased_exp(double x) { return (int)(((unsigned)__double2hiint(x) >> 20) & 0x7FF); }
+
+// 8 columns of one level (exact integers below 2^23) of this warp's 32 lanes
+__device__ __forceinline__ void lc_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr));
 }
 
+// VEC: nsd a multiple of 4, so that the four columns of a lane are two 16-byte
+// loads of one staged block
+template <bool VEC>
 __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
   if (g.skip && *g.skip) return;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -565,48 +606,53 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
   uint8_t* bdig = sbase + 2 * LC_ASTAGE;                  // nks x 8 C planes
   const int m = g.m, nsd = g.nsd, nb = m / nsd;
   const int nks = (m + LC_KS - 1) / LC_KS;
-  const int rs = g.row_stride;                            // doubles per staged row (nsd, or nsd + 1: odd)
-  double* raw = (double*)(bdig + (size_t)nks * LC_BCHUNK);  // [block][128 rows][rs]
-  int* eb = (int*)(raw + (size_t)nb * LC_TM * rs);        // [128] row exponents
-  int* ej = eb + LC_TM;                                    // [16] column exponents of C
-  // [LC_RQ][128] partial row exponents: in digit stage 1, idle at the start
-  // of a tile (the previous tile's MMAs are done, its flush used stage 0)
-  int* eh = (int*)(adig + LC_ASTAGE);
-  uint64_t* bars = (uint64_t*)(((uintptr_t)(ej + OZ_N) + 7) & ~(uintptr_t)7);  // stage[2], tile
-  uint32_t* tmem_slot = (uint32_t*)(bars + 3);
+  double* raw = (double*)(bdig + (size_t)nks * LC_BCHUNK);  // [block][128 rows][nsd]
+  int* eb = (int*)(raw + (size_t)m * LC_TM);              // [2][128] row exponents of two tiles
+  int* ej = eb + 2 * LC_TM;                               // [16] column exponents of C
+  uint64_t* bars = (uint64_t*)(((uintptr_t)(ej + OZ_N) + 7) & ~(uintptr_t)7);
+  uint32_t* tmem_slot = (uint32_t*)(bars + LC_NBARS);
   int* sflag = (int*)(tmem_slot + 1);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t bar0 = smem_u32(bars);
+  auto BAR = [&](int slot) { return bar0 + 8u * (uint32_t)slot; };
 
-  if (warp == 0) {
+  if (warp == LC_MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(LC_TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    for (int b = 0; b < 3; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8u * b));
+    for (int b = 0; b < LC_NBARS; ++b) {
+      const bool split = b < LC_B_EMPTY || b >= LC_B_CONS;  // full, cons: one arrival per splitting warp
+      const int count = split ? LC_SPLIT_WARPS
+                        : (b == LC_B_ACCE || b == LC_B_ACCE + 1) ? 4
+                        : (b == LC_B_RAWF && g.lane_copies) ? 33
+                                                            : 1;
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(BAR(b)), "r"(count));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;");
     *sflag = 0;
   }
   // C: column exponents, then its digit planes (rows j of plane q at q 16 + j)
   for (int x = tid; x < nks * LC_BCHUNK / 16; x += LC_THREADS) reinterpret_cast<uint4*>(bdig)[x] = make_uint4(0, 0, 0, 0);
-  if (tid < OZ_N) {
+  if (warp < OZ_N) {
     int e = 0;
-    if (tid < nsd)
-      for (int i = 0; i < m; ++i) e = max(e, biased_exp(g.C[(int64_t)i * nsd + tid]));
-    ej[tid] = e;
+    if (warp < nsd)
+      for (int i = lane; i < m; i += 32) e = max(e, biased_exp(g.C[(int64_t)i * nsd + warp]));
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) ej[warp] = e;
   }
   __syncthreads();
   for (int x = tid; x < m * nsd; x += LC_THREADS) {
     const int i = x / nsd, j = x - i * nsd;
-    float d[OZ_DIG];
-    oz_digits(g.C[x], ej[j], d);
+    uint32_t d[OZ_DIG];
+    oz_digits2(g.C[x], 0.0, ej[j], ej[j], d);
     uint8_t* base = bdig + (size_t)(i / LC_KS) * LC_BCHUNK;
     const int k = i % LC_KS;
 #pragma unroll
-    for (int q = 0; q < OZ_DIG; ++q)
-      *reinterpret_cast<uint16_t*>(base + kmaj16(q * OZ_N + j, k)) = (uint16_t)(__float_as_uint(d[q]) >> 16);
+    for (int q = 0; q < OZ_DIG; ++q) *reinterpret_cast<uint16_t*>(base + kmaj16(q * OZ_N + j, k)) = (uint16_t)d[q];
   }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the C planes are read by the MMAs
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
@@ -615,161 +661,271 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
   const int64_t r0 = (int64_t)blockIdx.x * g.rows_per_cta;
   const int64_t r1 = min(r0 + g.rows_per_cta, g.N);
   const int ntile = r1 > r0 ? (int)((r1 - r0 + LC_TM - 1) / LC_TM) : 0;
-  int gstep = 0;            // K steps issued so far (stage = gstep & 1)
-  bool ok = true;
-  uint32_t last_bar = 0, last_par = 0;
-  // tile tt's rows into the padded staging rows with asynchronous 8-byte
-  // copies: thread (row r, quarter h) copies blocks h, h + 4, ... of its row
-  auto issue_rows = [&](int tt) {
-    const int64_t Rt = r0 + (int64_t)tt * LC_TM;
-    const int nrt = (int)min((int64_t)LC_TM, r1 - Rt);
-    const int r = tid & (LC_TM - 1), h = tid >> 7;
-    if (r < nrt)
-      for (int b = h; b < nb; b += LC_RQ) {
-        const double* src = g.A + (int64_t)b * g.sA + (Rt + r) * nsd;
-        const uint32_t dst = smem_u32(raw + ((size_t)b * LC_TM + r) * rs);
-        for (int c = 0; c < nsd; ++c)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * c), "l"(src + c) : "memory");
-      }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  if (ntile > 0) issue_rows(0);
-  for (int t = 0; t < ntile && ok; ++t) {
-    const int64_t R = r0 + (int64_t)t * LC_TM;
-    const int nr = (int)min((int64_t)LC_TM, r1 - R);
-    // this tile's rows have landed: their largest exponents
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    {
-      const int r = tid & (LC_TM - 1), h = tid >> 7;
-      int e = 0;
-      if (r < nr)
-        for (int b = h; b < nb; b += LC_RQ) {
-          const double* row = raw + ((size_t)b * LC_TM + r) * rs;
-          for (int c = 0; c < nsd; ++c) e = max(e, biased_exp(row[c]));
+
+  if (warp < LC_SPLIT_WARPS) {
+    // ---- splitting warps: lane (row rl, columns 4 q .. 4 q + 3 of a step) --
+    const int q = lane & 3, r = warp * 8 + (lane >> 2);
+    const int swap = q >> 1;
+    bool ok = true;
+    int gstep = 0;
+    // columns i .. i + 3 of row r (0 beyond m)
+    auto load4 = [&](int i, double (&x)[4]) {
+      if constexpr (VEC) {
+        if (i < m) {
+          const int b = i / nsd;
+          const double2* p = reinterpret_cast<const double2*>(raw + (size_t)b * LC_TM * nsd + r * nsd + (i - b * nsd));
+          const double2 u = p[swap], w = p[1 - swap];
+          x[0] = swap ? w.x : u.x;
+          x[1] = swap ? w.y : u.y;
+          x[2] = swap ? u.x : w.x;
+          x[3] = swap ? u.y : w.y;
+        } else {
+          x[0] = x[1] = x[2] = x[3] = 0.0;
         }
-      eh[h * LC_TM + r] = e;
-    }
-    __syncthreads();
-    if (tid < LC_TM) eb[tid] = max(max(eh[tid], eh[LC_TM + tid]), max(eh[2 * LC_TM + tid], eh[3 * LC_TM + tid]));
-    __syncthreads();
-    for (int c = 0; c < nks; ++c, ++gstep) {
-      const int s = gstep & 1;
-      // the MMAs of step gstep - 2 are done with stage s
-      if (gstep >= 2 && !mbar_wait(bar0 + 8u * s, (uint32_t)((gstep >> 1) - 1) & 1u, sflag)) ok = false;
-      if (!__syncthreads_and(ok)) {
+      } else {
+        int b = i / nsd, s = i - b * nsd;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          x[k] = 0.0;
+          if (i + k < m) x[k] = raw[(size_t)b * LC_TM * nsd + r * nsd + s];
+          if (++s == nsd) {
+            s = 0;
+            ++b;
+          }
+        }
+      }
+    };
+    for (int t = 0; t < ntile && ok; ++t) {
+      ok = mbar_wait(BAR(LC_B_RAWF), (uint32_t)t & 1u, sflag);
+      if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         break;
       }
-      uint8_t* sa = adig + s * LC_ASTAGE;
-      {
-        // thread: row r, 4 consecutive K of the step (half a 16-byte core row per plane)
-        const int r = tid & (LC_TM - 1), k0 = (tid >> 7) * 4;
-        const int er = eb[r];
-        // column i of A is (block bi, column si) of the staged rows
-        const int ibeg = c * LC_KS + k0;
-        int bi = ibeg / nsd, si = ibeg - bi * nsd;
-        double xv[4];
+      // the row's largest exponent
+      int e = 0;
+      for (int i = 4 * q; i < m; i += LC_KS) {
+        double x[4];
+        load4(i, x);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          xv[k] = (r < nr && ibeg + k < m) ? raw[((size_t)bi * LC_TM + r) * rs + si] : 0.0;
-          if (++si == nsd) {
-            si = 0;
-            ++bi;
-          }
-        }
-        uint32_t pk[OZ_DIG][2];
-#pragma unroll
-        for (int k = 0; k < 4; k += 2) {
-          float d0[OZ_DIG], d1[OZ_DIG];
-          oz_digits(xv[k], er, d0);
-          oz_digits(xv[k + 1], er, d1);
-#pragma unroll
-          for (int p = 0; p < OZ_DIG; ++p) pk[p][k >> 1] = bf16x2(d0[p], d1[p]);
-        }
-#pragma unroll
-        for (int p = 0; p < OZ_DIG; ++p)
-          *reinterpret_cast<uint2*>(sa + p * LC_APLANE + kmaj16(r, k0)) = make_uint2(pk[p][0], pk[p][1]);
+        for (int k = 0; k < 4; ++k) e = max(e, __double2hiint(x[k]) & 0x7fffffff);
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncthreads();
-      if (tid == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t a0 = smem_u32(sa), b0 = smem_u32(bdig + (size_t)c * LC_BCHUNK);
-#pragma unroll
-        for (int p = 0; p < OZ_DIG; ++p) {
-          const uint32_t acc = (c == 0 && p == 0) ? 0u : 1u;
-          asm volatile(
-              "{\n .reg .pred pa;\n setp.ne.b32 pa, %4, 0;\n"
-              " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, pa;\n}" ::"r"(tmem + (uint32_t)(p * OZ_N)),
-              "l"(sdesc16(a0 + p * LC_APLANE)), "l"(sdesc16(b0)), "r"(oz_idesc((OZ_LEVELS - p) * OZ_N)), "r"(acc));
+      e >>= 20;
+      e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
+      e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
+      // tile t - 2 has been written: its exponents may go
+      if (t >= 2) ok = mbar_wait(BAR(LC_B_ACCE + (t & 1)), (uint32_t)((t >> 1) - 1) & 1u, sflag);
+      if (!__all_sync(0xffffffffu, ok)) {
+        ok = false;
+        break;
+      }
+      if (q == 0) eb[(t & 1) * LC_TM + r] = e;
+      for (int c = 0; c < nks; ++c, ++gstep) {
+        const int s = gstep & 1;
+        double x[4];
+        load4(c * LC_KS + 4 * q, x);
+        uint32_t d0[OZ_DIG], d1[OZ_DIG];
+        oz_digits2(x[0], x[1], e, e, d0);
+        oz_digits2(x[2], x[3], e, e, d1);
+        // the MMAs of step gstep - 2 are done with stage s
+        if (gstep >= 2) ok = mbar_wait(BAR(LC_B_EMPTY + s), (uint32_t)((gstep >> 1) - 1) & 1u, sflag);
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
         }
-        mma_commit(bar0 + 8u * s);
-        last_bar = bar0 + 8u * s;
-        last_par = (uint32_t)(gstep >> 1) & 1u;
+        uint8_t* dst = adig + s * LC_ASTAGE + kmaj16(r, 4 * q);
+#pragma unroll
+        for (int p = 0; p < OZ_DIG; ++p) *reinterpret_cast<uint2*>(dst + p * LC_APLANE) = make_uint2(d0[p], d1[p]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(BAR(LC_B_FULL + s));
+          mbar_arrive(BAR(LC_B_CONS + c));
+        }
       }
     }
-    if (!ok) break;
-    // every split of this tile is done, so the staging rows are free: the
-    // next tile's copies fly during this tile's MMA tail and flush
-    if (t + 1 < ntile) issue_rows(t + 1);
-    // the tile's MMAs are done: warps 0-3 write its rows
-    if (tid == 0) mma_commit(bar0 + 16u);
-    if (!mbar_wait(bar0 + 16u, (uint32_t)t & 1u, sflag)) ok = false;
-    if (!__syncthreads_and(ok)) {
-      ok = false;
-      break;
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    {
-      // warps w and w + 4 share lane quarter w % 4 (rows 32 (w % 4) ..):
-      // warp w sums levels 0-3, warp w + 4 levels 4-7; both halves meet in
-      // shared memory (the digit stages are free now)
-      long long acc[OZ_N];
-#pragma unroll
-      for (int j = 0; j < OZ_N; ++j) acc[j] = 0;
-      const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-      if (warp < 4) {
-#pragma unroll
-        for (int L = 0; L < OZ_LEVELS / 2; ++L) oz_flush1(ta + L * OZ_N, 7 * (3 - L), acc);
-      } else if (warp < 8) {
-#pragma unroll
-        for (int L = OZ_LEVELS / 2; L < OZ_LEVELS; ++L) oz_flush1(ta + L * OZ_N, 7 * (7 - L), acc);
+    if (!ok && lane == 0) atomicExch(sflag, 1);
+  } else if (warp < LC_MMA_WARP) {
+    // ---- flush warps: lane quarter q = warp % 4 holds rows 32 q .. 32 q + 31
+    const int r = (warp & 3) * 32 + lane;
+    const uint32_t lrow = (uint32_t)((warp & 3) * 32) << 16;
+    const bool o16 = (((uintptr_t)g.O & 15) == 0) && (g.ldO & 1) == 0 && (nsd & 1) == 0;
+    for (int t = 0; t < ntile; ++t) {
+      const int buf = t & 1;
+      const bool ok = mbar_wait(BAR(LC_B_ACCF + buf), (uint32_t)(t >> 1) & 1u, sflag);
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) atomicExch(sflag, 1);
+        break;
       }
-      long long* lo_s = reinterpret_cast<long long*>(adig);  // [128 rows][17]: odd stride, no bank conflicts
-      const int r = tid & (LC_TM - 1);
-      if (warp >= 4 && warp < 8)
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t ta = tmem + lrow + (uint32_t)(buf * LC_ACC_COLS);
+      const int64_t row = r0 + (int64_t)t * LC_TM + r;
+      const int er = eb[buf * LC_TM + r];
+      for (int j0 = 0; j0 < nsd; j0 += 8) {
+        long long hi[8], lo[8];
 #pragma unroll
-        for (int j = 0; j < OZ_N; ++j) lo_s[r * (OZ_N + 1) + j] = acc[j];
-      __syncthreads();
-      if (warp < 4 && r < nr) {
-        double* o = g.O + (R + r) * g.ldO;
+        for (int j = 0; j < 8; ++j) hi[j] = lo[j] = 0;
 #pragma unroll
-        for (int j = 0; j < OZ_N; ++j)
-          if (j < nsd) {
-            const int e = (eb[r] - 1022) + (ej[j] - 1022);
-            const double h = (double)acc[j], l = (double)lo_s[r * (OZ_N + 1) + j];
-            double v;
-            if (e - 63 >= -1022 && e - 35 <= 1023)  // both scales are normal powers of two: exact products
-              v = h * __longlong_as_double((long long)(e - 35 + 1023) << 52) +
-                  l * __longlong_as_double((long long)(e - 63 + 1023) << 52);
+        for (int L = 0; L < OZ_LEVELS; L += 2) {
+          uint32_t v0[8], v1[8];
+          lc_ld8(ta + L * OZ_N + j0, v0);
+          lc_ld8(ta + (L + 1) * OZ_N + j0, v1);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const long long i0 = (long long)__float2int_rn(__uint_as_float(v0[j]));
+            const long long i1 = (long long)__float2int_rn(__uint_as_float(v1[j]));
+            if (L < OZ_LEVELS / 2)
+              hi[j] += (i0 << (7 * (3 - L))) + (i1 << (7 * (2 - L < 0 ? 0 : 2 - L)));
             else
-              v = ldexp(h, e - 35) + ldexp(l, e - 63);
-            o[j] = v;
+              lo[j] += (i0 << (7 * (7 - L))) + (i1 << (7 * (6 - L < 0 ? 0 : 6 - L)));
           }
+        }
+        if (j0 + 8 >= nsd) {  // everything of this accumulator and tile is read
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(BAR(LC_B_ACCE + buf));
+        }
+        if (row < r1) {
+          double* o = g.O + row * g.ldO + j0;
+          double v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (j0 + j < nsd) {
+              const int ex = (er - 1022) + (ej[j0 + j] - 1022);
+              const double h = (double)hi[j], l = (double)lo[j];
+              if (ex - 63 >= -1022 && ex - 35 <= 1023)  // both scales are normal powers of two: exact products
+                v[j] = h * __longlong_as_double((long long)(ex - 35 + 1023) << 52) +
+                       l * __longlong_as_double((long long)(ex - 63 + 1023) << 52);
+              else
+                v[j] = ldexp(h, ex - 35) + ldexp(l, ex - 63);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) {
+            if (o16) {
+              if (j0 + j < nsd) *reinterpret_cast<double2*>(o + j) = make_double2(v[j], v[j + 1]);
+            } else {
+              if (j0 + j < nsd) o[j] = v[j];
+              if (j0 + j + 1 < nsd) o[j + 1] = v[j + 1];
+            }
+          }
+        }
       }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
+  } else if (warp == LC_MMA_WARP) {
+    // ---- MMA warp: lane 0 issues, the warp stays converged ----------------
+    uint32_t last_bar = 0, last_par = 0;  // the latest commit: its completion covers every MMA
+    int gstep = 0;
+    bool ok = true;
+    for (int t = 0; t < ntile && ok; ++t)
+      for (int c = 0; c < nks && ok; ++c, ++gstep) {
+        const int s = gstep & 1, buf = t & 1;
+        if (lane == 0) {
+          // accumulator written out (tile t - 2), digit stage s full
+          if (c == 0 && t >= 2) ok = mbar_wait(BAR(LC_B_ACCE + buf), (uint32_t)((t >> 1) - 1) & 1u, sflag);
+          if (ok) ok = mbar_wait(BAR(LC_B_FULL + s), (uint32_t)(gstep >> 1) & 1u, sflag);
+          if (ok) {
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const uint32_t a0 = smem_u32(adig + s * LC_ASTAGE), b0 = smem_u32(bdig + (size_t)c * LC_BCHUNK);
+#pragma unroll
+            for (int p = 0; p < OZ_DIG; ++p) {
+              const uint32_t acc = (c == 0 && p == 0) ? 0u : 1u;
+              asm volatile(
+                  "{\n .reg .pred pa;\n setp.ne.b32 pa, %4, 0;\n"
+                  " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, pa;\n}" ::"r"(
+                      tmem + (uint32_t)(buf * LC_ACC_COLS + p * OZ_N)),
+                  "l"(sdesc16(a0 + p * LC_APLANE)), "l"(sdesc16(b0)), "r"(oz_idesc((OZ_LEVELS - p) * OZ_N)), "r"(acc));
+            }
+            mma_commit(BAR(LC_B_EMPTY + s));
+            last_bar = BAR(LC_B_EMPTY + s);
+            last_par = (uint32_t)(gstep >> 1) & 1u;
+            if (c == nks - 1) mma_commit(BAR(LC_B_ACCF + buf));
+          } else {
+            atomicExch(sflag, 1);
+          }
+        }
+        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+      }
+    // before the tensor memory is freed, every MMA issued must have completed
+    if (lane == 0 && last_bar != 0 && !mbar_drain(last_bar, last_par)) atomicExch(sflag, 1);
+    __syncwarp();
+  } else {
+    // ---- load warp: blocks of tile t in order, each as one bulk copy, or by
+    // the lanes when it is not whole 16-byte lines (g.lane_copies: some are not)
+    auto span = [&](int t, int b, const double*& src) -> uint32_t {
+      const int64_t R = r0 + (int64_t)t * LC_TM;
+      src = g.A + (int64_t)b * g.sA + R * nsd;
+      return (uint32_t)(min((int64_t)LC_TM, r1 - R) * nsd * 8);
+    };
+    auto whole = [](const double* src, uint32_t bytes) { return ((((uintptr_t)src) | bytes) & 15) == 0; };
+    auto expect = [&](int t) {
+      if (lane == 0) {
+        uint32_t total = 0;
+        for (int b = 0; b < nb; ++b) {
+          const double* src;
+          const uint32_t bytes = span(t, b, src);
+          if (whole(src, bytes)) total += bytes;
+        }
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(BAR(LC_B_RAWF)), "r"(total)
+                     : "memory");
+      }
+      __syncwarp();
+    };
+    auto copy = [&](int t, int b) {
+      const double* src;
+      const uint32_t bytes = span(t, b, src);
+      const uint32_t dst = smem_u32(raw + (size_t)b * LC_TM * nsd);
+      if (whole(src, bytes)) {
+        if (lane == 0)
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                           dst),
+                       "l"(src), "r"(bytes), "r"(BAR(LC_B_RAWF))
+                       : "memory");
+      } else {
+        for (uint32_t x = lane; x < bytes / 8; x += 32)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * x), "l"(src + x) : "memory");
+      }
+    };
+    auto finish = [&] {  // the lanes' share of the tile arrives once their copies have landed
+      if (g.lane_copies)
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(BAR(LC_B_RAWF)) : "memory");
+    };
+    int issued = 0;  // tiles whose copies are all on their way
+    if (ntile > 0) {
+      expect(0);
+      for (int b = 0; b < nb; ++b) copy(0, b);
+      finish();
+      issued = 1;
+    }
+    for (int t = 0; t + 1 < ntile; ++t) {
+      int b = 0;
+      bool ok = true;
+      for (int c = 0; c < nks && ok; ++c) {
+        ok = mbar_wait(BAR(LC_B_CONS + c), (uint32_t)t & 1u, sflag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        if (c == 0) expect(t + 1);
+        for (; b < nb && (b + 1) * nsd <= (c + 1) * LC_KS; ++b) copy(t + 1, b);
+      }
+      if (!ok) {
+        if (lane == 0) atomicExch(sflag, 1);
+        break;
+      }
+      for (; b < nb; ++b) copy(t + 1, b);
+      finish();
+      issued = t + 2;
+    }
+    // the copies still in flight land before the CTA may exit
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (lane == 0 && issued > 0 && !mbar_drain(BAR(LC_B_RAWF), (uint32_t)(issued - 1) & 1u)) atomicExch(sflag, 1);
+    __syncwarp();
   }
-  // no copy or MMA may be in flight when the CTA exits / frees its tensor memory
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (tid == 0 && last_bar != 0 && !mbar_drain(last_bar, last_par)) atomicExch(sflag, 1);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  if (tid == 0 && (!ok || *(volatile int*)sflag)) atomicExch(g.status, 1);
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(LC_TMEM_COLS));
+  if (tid == 0 && *(volatile int*)sflag) atomicExch(g.status, 1);
+  if (warp == LC_MMA_WARP)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(LC_TMEM_COLS));
 }
 
 // biased max exponent of each column (nsd <= 256 columns per block, rows ld
@@ -891,7 +1047,10 @@ static int lincomb_oz_prepare() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
   if (done[dev]) return 0;
-  if (cudaFuncSetAttribute(k_lincomb_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM_MAX) != cudaSuccess)
+  if (cudaFuncSetAttribute(k_lincomb_oz<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM_MAX) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_lincomb_oz<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM_MAX) !=
+          cudaSuccess)
     return -1;
   done[dev] = 1;
   return 0;
@@ -906,15 +1065,8 @@ int qp_lincomb_oz(const double* A, int64_t sA, int m, int nsd, const double* C, 
   if (lincomb_oz_prepare()) return -1;
   const int nks = (m + LC_KS - 1) / LC_KS;
   const int nb = m / nsd;
-  // staged rows of an odd number of doubles (no shared-memory bank
-  // conflicts between consecutive rows) when they fit, else unpadded
-  auto need = [&](int rsd) {
-    return 1024 + 2 * (size_t)LC_ASTAGE + (size_t)nks * LC_BCHUNK + (size_t)nb * LC_TM * rsd * 8 +
-           (LC_TM + OZ_N) * 4 + 64;
-  };
-  int rsd = (nsd & 1) ? nsd : nsd + 1;
-  if (need(rsd) > (size_t)OZ_SMEM_MAX) rsd = nsd;
-  const size_t smem = need(rsd);
+  const size_t smem = 1024 + 2 * (size_t)LC_ASTAGE + (size_t)nks * LC_BCHUNK + (size_t)m * LC_TM * 8 +
+                      (2 * LC_TM + OZ_N) * 4 + (LC_NBARS + 2) * 8;
   if (smem > (size_t)OZ_SMEM_MAX) return -1;
   LcArgs g;
   g.A = A;
@@ -928,10 +1080,14 @@ int qp_lincomb_oz(const double* A, int64_t sA, int m, int nsd, const double* C, 
   int64_t rpc = (N + ncta - 1) / ncta;
   rpc = (rpc + LC_TM - 1) / LC_TM * LC_TM;
   g.rows_per_cta = rpc;
-  g.row_stride = rsd;
+  // blocks start on 16-byte lines, and the last tile's rows fill them
+  g.lane_copies = ((uintptr_t)A & 15) != 0 || (nb > 1 && (sA & 1) != 0) || ((N % LC_TM) * nsd & 1) != 0;
   g.skip = skip;
   g.status = status;
-  k_lincomb_oz<<<ncta, LC_THREADS, smem, st>>>(g);
+  if ((nsd & 3) == 0)
+    k_lincomb_oz<true><<<ncta, LC_THREADS, smem, st>>>(g);
+  else
+    k_lincomb_oz<false><<<ncta, LC_THREADS, smem, st>>>(g);
   return 0;
 }
 
