@@ -528,10 +528,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
 // m <= 128 products, below 2^23.
 //
 // One CTA per SM walks tiles of 128 rows, one role per warp:
-//  * the load warp streams the tile's blocks into shared memory (one
-//    cp.async.bulk per block, completing on rawf) and refills a block with
-//    the next tile's rows as soon as the K step that read it last is cut
-//    (cons[c]);
+//  * the load warp streams the tiles' blocks through a ring of block slots in
+//    shared memory (one cp.async.bulk per block, completing on the tile's
+//    rawf[t % 2]); a slot is refilled once the K step that read it last is
+//    cut, which the MMA warp publishes as it waits for the steps in order, so
+//    up to a whole tile is on its way while a tile is cut;
 //  * warps 0-15 form the row exponents and cut each K step of 16 columns into
 //    the 8 A digit planes of stage s (full[s]); a warp owns 8 rows, its lanes
 //    4 columns each, so that a row's exponent is two shuffles and the two
@@ -556,12 +557,11 @@ constexpr int LC_APLANE = LC_TM * LC_KS * 2;     // 4 KB: one A digit plane of o
 constexpr int LC_ASTAGE = OZ_DIG * LC_APLANE;    // 32 KB
 constexpr int LC_BCHUNK = OZ_DIG * OZ_N * LC_KS * 2;  // 4 KB: the 8 C planes of one K step
 constexpr int LC_MAXM = 128;
-constexpr int LC_MAXKS = LC_MAXM / LC_KS;
 constexpr int LC_ACC_COLS = OZ_LEVELS * OZ_N;    // 128 tensor-memory columns per accumulator
 constexpr int LC_TMEM_COLS = 2 * LC_ACC_COLS;
 // barrier slots
-constexpr int LC_B_FULL = 0, LC_B_EMPTY = 2, LC_B_ACCF = 4, LC_B_ACCE = 6, LC_B_RAWF = 8, LC_B_CONS = 9,
-              LC_NBARS = LC_B_CONS + LC_MAXKS;
+constexpr int LC_B_FULL = 0, LC_B_EMPTY = 2, LC_B_ACCF = 4, LC_B_ACCE = 6, LC_B_RAWF = 8,
+              LC_NBARS = 10;
 
 struct LcArgs {
   const double* A;
@@ -572,6 +572,7 @@ struct LcArgs {
   int64_t ldO;
   int64_t N, rows_per_cta;
   int lane_copies;  // some block of some tile is not whole 16-byte lines
+  int nslots;       // block slots of the ring: nb .. 2 nb
   const int* skip;
   int* status;
 };
@@ -606,12 +607,14 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
   uint8_t* bdig = sbase + 2 * LC_ASTAGE;                  // nks x 8 C planes
   const int m = g.m, nsd = g.nsd, nb = m / nsd;
   const int nks = (m + LC_KS - 1) / LC_KS;
-  double* raw = (double*)(bdig + (size_t)nks * LC_BCHUNK);  // [block][128 rows][nsd]
-  int* eb = (int*)(raw + (size_t)m * LC_TM);              // [2][128] row exponents of two tiles
+  double* raw = (double*)(bdig + (size_t)nks * LC_BCHUNK);  // [slot][128 rows][nsd]
+  const int nslots = g.nslots;
+  int* eb = (int*)(raw + (size_t)nslots * nsd * LC_TM);   // [2][128] row exponents of two tiles
   int* ej = eb + 2 * LC_TM;                               // [16] column exponents of C
   uint64_t* bars = (uint64_t*)(((uintptr_t)(ej + OZ_N) + 7) & ~(uintptr_t)7);
   uint32_t* tmem_slot = (uint32_t*)(bars + LC_NBARS);
   int* sflag = (int*)(tmem_slot + 1);
+  volatile int* sdone = sflag + 1;                        // K steps cut by all splitting warps
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t bar0 = smem_u32(bars);
   auto BAR = [&](int slot) { return bar0 + 8u * (uint32_t)slot; };
@@ -623,15 +626,15 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
   }
   if (tid == 0) {
     for (int b = 0; b < LC_NBARS; ++b) {
-      const bool split = b < LC_B_EMPTY || b >= LC_B_CONS;  // full, cons: one arrival per splitting warp
-      const int count = split ? LC_SPLIT_WARPS
+      const int count = b < LC_B_EMPTY ? LC_SPLIT_WARPS
                         : (b == LC_B_ACCE || b == LC_B_ACCE + 1) ? 4
-                        : (b == LC_B_RAWF && g.lane_copies) ? 33
+                        : (b >= LC_B_RAWF && g.lane_copies) ? 33
                                                             : 1;
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(BAR(b)), "r"(count));
     }
     asm volatile("fence.mbarrier_init.release.cluster;");
     *sflag = 0;
+    *sdone = 0;
   }
   // C: column exponents, then its digit planes (rows j of plane q at q 16 + j)
   for (int x = tid; x < nks * LC_BCHUNK / 16; x += LC_THREADS) reinterpret_cast<uint4*>(bdig)[x] = make_uint4(0, 0, 0, 0);
@@ -667,13 +670,17 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
     const int q = lane & 3, r = warp * 8 + (lane >> 2);
     const int swap = q >> 1;
     bool ok = true;
-    int gstep = 0;
+    int gstep = 0, slot0 = 0;  // slot of the tile's first block
+    auto block = [&](int b) {
+      const int x = slot0 + b;
+      return raw + (size_t)(x < nslots ? x : x - nslots) * LC_TM * nsd;
+    };
     // columns i .. i + 3 of row r (0 beyond m)
     auto load4 = [&](int i, double (&x)[4]) {
       if constexpr (VEC) {
         if (i < m) {
           const int b = i / nsd;
-          const double2* p = reinterpret_cast<const double2*>(raw + (size_t)b * LC_TM * nsd + r * nsd + (i - b * nsd));
+          const double2* p = reinterpret_cast<const double2*>(block(b) + r * nsd + (i - b * nsd));
           const double2 u = p[swap], w = p[1 - swap];
           x[0] = swap ? w.x : u.x;
           x[1] = swap ? w.y : u.y;
@@ -687,7 +694,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           x[k] = 0.0;
-          if (i + k < m) x[k] = raw[(size_t)b * LC_TM * nsd + r * nsd + s];
+          if (i + k < m) x[k] = block(b)[r * nsd + s];
           if (++s == nsd) {
             s = 0;
             ++b;
@@ -696,7 +703,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
       }
     };
     for (int t = 0; t < ntile && ok; ++t) {
-      ok = mbar_wait(BAR(LC_B_RAWF), (uint32_t)t & 1u, sflag);
+      if (t > 0) slot0 = (slot0 + nb) % nslots;
+      ok = mbar_wait(BAR(LC_B_RAWF + (t & 1)), (uint32_t)(t >> 1) & 1u, sflag);
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         break;
@@ -737,10 +745,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
         for (int p = 0; p < OZ_DIG; ++p) *reinterpret_cast<uint2*>(dst + p * LC_APLANE) = make_uint2(d0[p], d1[p]);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(BAR(LC_B_FULL + s));
-          mbar_arrive(BAR(LC_B_CONS + c));
-        }
+        if (lane == 0) mbar_arrive(BAR(LC_B_FULL + s));
       }
     }
     if (!ok && lane == 0) atomicExch(sflag, 1);
@@ -825,6 +830,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
           if (c == 0 && t >= 2) ok = mbar_wait(BAR(LC_B_ACCE + buf), (uint32_t)((t >> 1) - 1) & 1u, sflag);
           if (ok) ok = mbar_wait(BAR(LC_B_FULL + s), (uint32_t)(gstep >> 1) & 1u, sflag);
           if (ok) {
+            *sdone = gstep + 1;
             asm volatile("tcgen05.fence::after_thread_sync;");
             const uint32_t a0 = smem_u32(adig + s * LC_ASTAGE), b0 = smem_u32(bdig + (size_t)c * LC_BCHUNK);
 #pragma unroll
@@ -866,58 +872,68 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
           const uint32_t bytes = span(t, b, src);
           if (whole(src, bytes)) total += bytes;
         }
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(BAR(LC_B_RAWF)), "r"(total)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(BAR(LC_B_RAWF + (t & 1))),
+                     "r"(total)
                      : "memory");
       }
       __syncwarp();
     };
-    auto copy = [&](int t, int b) {
+    auto copy = [&](int t, int b, int slot) {
       const double* src;
       const uint32_t bytes = span(t, b, src);
-      const uint32_t dst = smem_u32(raw + (size_t)b * LC_TM * nsd);
+      const uint32_t dst = smem_u32(raw + (size_t)slot * LC_TM * nsd);
       if (whole(src, bytes)) {
         if (lane == 0)
           asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                            dst),
-                       "l"(src), "r"(bytes), "r"(BAR(LC_B_RAWF))
+                       "l"(src), "r"(bytes), "r"(BAR(LC_B_RAWF + (t & 1)))
                        : "memory");
       } else {
         for (uint32_t x = lane; x < bytes / 8; x += 32)
           asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * x), "l"(src + x) : "memory");
       }
     };
-    auto finish = [&] {  // the lanes' share of the tile arrives once their copies have landed
+    auto finish = [&](int t) {  // the lanes' share of the tile arrives once their copies have landed
       if (g.lane_copies)
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(BAR(LC_B_RAWF)) : "memory");
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(BAR(LC_B_RAWF + (t & 1))) : "memory");
     };
-    int issued = 0;  // tiles whose copies are all on their way
-    if (ntile > 0) {
-      expect(0);
-      for (int b = 0; b < nb; ++b) copy(0, b);
-      finish();
-      issued = 1;
-    }
-    for (int t = 0; t + 1 < ntile; ++t) {
-      int b = 0;
-      bool ok = true;
-      for (int c = 0; c < nks && ok; ++c) {
-        ok = mbar_wait(BAR(LC_B_CONS + c), (uint32_t)t & 1u, sflag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        if (c == 0) expect(t + 1);
-        for (; b < nb && (b + 1) * nsd <= (c + 1) * LC_KS; ++b) copy(t + 1, b);
+    // bounded wait for K step `step` of the whole run to be cut
+    auto cut = [&](int step) {
+      bool ok = false;
+      for (long long it = 0; it < OZ_WAIT_LIMIT && !ok; ++it) {
+        ok = *sdone > step;
+        if (!ok && (it & 255) == 255 && *(volatile const int*)sflag) break;
+      }
+      __threadfence_block();
+      return __all_sync(0xffffffffu, ok) != 0;
+    };
+    int issued = 0, slot = 0;  // tiles whose copies are all on their way; next slot
+    bool ok = true;
+    for (int t = 0; t < ntile && ok; ++t) {
+      for (int b = 0; b < nb && ok; ++b) {
+        // the slot's last block: nslots blocks back, free after its last K step
+        const int old = t * nb + b - nslots;
+        if (old >= 0) {
+          const int ot = old / nb, ob = old - ot * nb;
+          ok = cut(ot * nks + ((ob + 1) * nsd - 1) / LC_KS);
+          if (!ok) break;
+        }
+        if (b == 0) expect(t);
+        copy(t, b, slot);
+        if (++slot == nslots) slot = 0;
       }
       if (!ok) {
         if (lane == 0) atomicExch(sflag, 1);
         break;
       }
-      for (; b < nb; ++b) copy(t + 1, b);
-      finish();
-      issued = t + 2;
+      finish(t);
+      issued = t + 1;
     }
     // the copies still in flight land before the CTA may exit
     asm volatile("cp.async.wait_all;" ::: "memory");
-    if (lane == 0 && issued > 0 && !mbar_drain(BAR(LC_B_RAWF), (uint32_t)(issued - 1) & 1u)) atomicExch(sflag, 1);
+    if (lane == 0)
+      for (int t = max(0, issued - 2); t < issued; ++t)
+        if (!mbar_drain(BAR(LC_B_RAWF + (t & 1)), (uint32_t)(t >> 1) & 1u)) atomicExch(sflag, 1);
     __syncwarp();
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -1065,9 +1081,12 @@ int qp_lincomb_oz(const double* A, int64_t sA, int m, int nsd, const double* C, 
   if (lincomb_oz_prepare()) return -1;
   const int nks = (m + LC_KS - 1) / LC_KS;
   const int nb = m / nsd;
-  const size_t smem = 1024 + 2 * (size_t)LC_ASTAGE + (size_t)nks * LC_BCHUNK + (size_t)m * LC_TM * 8 +
-                      (2 * LC_TM + OZ_N) * 4 + (LC_NBARS + 2) * 8;
-  if (smem > (size_t)OZ_SMEM_MAX) return -1;
+  const size_t fixed = 1024 + 2 * (size_t)LC_ASTAGE + (size_t)nks * LC_BCHUNK + (2 * LC_TM + OZ_N) * 4 +
+                       (LC_NBARS + 3) * 8;
+  const size_t slot_bytes = (size_t)LC_TM * nsd * 8;
+  const int nslots = std::min<int>(2 * nb, (int)((OZ_SMEM_MAX - fixed) / slot_bytes));
+  if (nslots < nb) return -1;
+  const size_t smem = fixed + nslots * slot_bytes;
   LcArgs g;
   g.A = A;
   g.sA = sA;
@@ -1080,6 +1099,7 @@ int qp_lincomb_oz(const double* A, int64_t sA, int m, int nsd, const double* C, 
   int64_t rpc = (N + ncta - 1) / ncta;
   rpc = (rpc + LC_TM - 1) / LC_TM * LC_TM;
   g.rows_per_cta = rpc;
+  g.nslots = nslots;
   // blocks start on 16-byte lines, and the last tile's rows fill them
   g.lane_copies = ((uintptr_t)A & 15) != 0 || (nb > 1 && (sA & 1) != 0) || ((N % LC_TM) * nsd & 1) != 0;
   g.skip = skip;
