@@ -67,11 +67,8 @@ constexpr int OZ_DIG = 8;                    // digit planes per operand
 constexpr int OZ_LEVELS = 8;                 // levels p + q = 0..7 kept
 constexpr int OZ_WINDOW = 4;                 // chunks per accumulator window (128 rows)
 constexpr int OZ_NBUF = 4;                   // accumulator buffers
-constexpr int OZ_A_TILE = OZ_M * OZ_KC * 2;  // bytes of one A digit plane
-constexpr int OZ_B_TILE = OZ_N * OZ_KC * 2;
-// a digit stage: the 8 A planes, then the 8 B planes, so that B planes
-// 0..n-1 form one K-major operand of 16 n rows
-constexpr int OZ_STAGE = OZ_DIG * OZ_A_TILE + OZ_DIG * OZ_B_TILE;
+constexpr int OZ_B_TILE = OZ_N * OZ_KC * 2;  // bytes of one B digit plane
+constexpr int OZ_MAXST = 3;                  // digit stages at most
 constexpr int OZ_TAB = 6144;  // alignment, exponents, block tables, barriers
 constexpr int OZ_SMEM_MAX = 232448;
 constexpr int OZ_MAXRAW = 8;  // raw stages at most
@@ -82,7 +79,7 @@ constexpr int OZ_TMEM_COLS = OZ_NBUF * OZ_ACC_COLS;  // 512: the whole tensor me
 constexpr long long OZ_WAIT_LIMIT = 1LL << 25;
 
 // barrier slots
-constexpr int OZ_B_FULL = 0, OZ_B_EMPTY = 2, OZ_B_ACCF = 4, OZ_B_ACCE = OZ_B_ACCF + OZ_NBUF,
+constexpr int OZ_B_FULL = 0, OZ_B_EMPTY = OZ_MAXST, OZ_B_ACCF = 2 * OZ_MAXST, OZ_B_ACCE = OZ_B_ACCF + OZ_NBUF,
               OZ_B_RAWF = OZ_B_ACCE + OZ_NBUF, OZ_B_RAWE = OZ_B_RAWF + OZ_MAXRAW, OZ_NBARS = OZ_B_RAWE + OZ_MAXRAW;
 
 struct OzArgs {
@@ -98,6 +95,11 @@ struct OzArgs {
   double* partial;  // [cta][m][nbc]
   const int* skip;
   int* status;
+  // digit stages: the 8 A planes (a_tile bytes each, the columns of A rounded
+  // up to 8), then the 8 B planes, so that B planes 0..n-1 form one K-major
+  // operand of 16 n rows.  An MMA reads 128 rows from each A plane: those past
+  // its own are other digits, and their accumulator rows are never read.
+  int nst, a_tile, stage;
   int nraw;        // raw stages in the ring
   int raw_stride;  // doubles per raw stage
   int rpt;         // rows per splitting task: 2, 4 or 8
@@ -162,20 +164,20 @@ __device__ __forceinline__ void oz_digits2(double x0, double x1, int e0, int e1,
   const uint32_t h1 = (uint32_t)__double2hiint(x1), l1 = (uint32_t)__double2loint(x1);
   const unsigned long long g0 = oz_fixed(h0, l0, e0), g1 = oz_fixed(h1, l1, e1);
   const uint32_t a0 = (uint32_t)g0, b0 = (uint32_t)(g0 >> 32), a1 = (uint32_t)g1, b1 = (uint32_t)(g1 >> 32);
-  // 16-bit windows of both values: digit pairs (6, 7), (4, 5), (2, 3), (0, 1)
-  const uint32_t w3 = __byte_perm(a0 >> 1, a1 >> 1, 0x5410), w2 = __byte_perm(a0 >> 15, a1 >> 15, 0x5410);
+  // 16-bit windows of both values: digit pairs (6, 7) one bit up, (4, 5), (2, 3), (0, 1)
+  const uint32_t w3 = __byte_perm(a0, a1, 0x5410), w2 = __byte_perm(a0 >> 15, a1 >> 15, 0x5410);
   const uint32_t w1 = __byte_perm(__funnelshift_r(a0, b0, 29), __funnelshift_r(a1, b1, 29), 0x5410);
   const uint32_t w0 = __byte_perm(b0 >> 11, b1 >> 11, 0x5410);
   const uint32_t sg = __byte_perm(h0, h1, 0x7632) & 0x80008000u;
   const uint32_t one = sg | 0x3F803F80u, c128 = sg ^ 0xC300C300u, c192 = sg ^ 0xC340C340u;  // +-1, -+128, -+192
-  d[0] = bf16_fma2(((w0 >> 7) & 0x00FF00FFu) + 0x43004300u, one, c128);
+  d[0] = bf16_fma2(((w0 >> 7) & 0x00FF00FFu) | 0x43004300u, one, c128);
   d[1] = bf16_fma2((w0 & 0x007F007Fu) | 0x43004300u, one, c192);
   d[2] = bf16_fma2(((w1 >> 7) & 0x007F007Fu) | 0x43004300u, one, c192);
   d[3] = bf16_fma2((w1 & 0x007F007Fu) | 0x43004300u, one, c192);
   d[4] = bf16_fma2(((w2 >> 7) & 0x007F007Fu) | 0x43004300u, one, c192);
   d[5] = bf16_fma2((w2 & 0x007F007Fu) | 0x43004300u, one, c192);
-  d[6] = bf16_fma2(((w3 >> 7) & 0x007F007Fu) | 0x43004300u, one, c192);
-  d[7] = bf16_fma2((w3 & 0x007F007Fu) | 0x43004300u, one, c192);
+  d[6] = bf16_fma2(((w3 >> 8) & 0x007F007Fu) | 0x43004300u, one, c192);
+  d[7] = bf16_fma2(((w3 >> 1) & 0x007F007Fu) | 0x43004300u, one, c192);
 }
 
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
@@ -213,6 +215,17 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// i 2^k exactly, |i| < 2^51, -1022 <= k <= 960: i is added to the low bits of
+// 1.5 2^52, and one FMA scales it and takes the offset off.  (The 64-bit
+// conversion instructions run on the FP64 pipe, two lanes a clock, several
+// times each.)
+__device__ __forceinline__ double scaled_int(long long i, int k) {
+  const double x = __longlong_as_double(i + 0x4338000000000000ll);
+  const double s = __longlong_as_double((long long)(k + 1023) << 52);
+  const double off = __longlong_as_double(((long long)(k + 1023 + 52) << 52) | 0x8008000000000000ll);  // -1.5 2^(52 + k)
+  return __fma_rn(x, s, off);
+}
+
 // level L of accumulator buffer `buf` (this warp's 32 lanes, 16 columns),
 // exact integers below 2^23, shifted by sh into acc
 __device__ __forceinline__ void oz_flush1(uint32_t taddr, int sh, long long (&acc)[OZ_N]) {
@@ -229,9 +242,32 @@ __device__ __forceinline__ void oz_flush1(uint32_t taddr, int sh, long long (&ac
 
 // digit planes of one chunk: task (column, group of RPT rows) writes RPT
 // rows of one column into each of the 8 planes of stage (sa, sb)
+// RPT rows of one column (rows wcol doubles apart, nr of them real) into each
+// of the 8 planes, `tile` bytes apart
+template <int RPT>
+__device__ __forceinline__ void oz_split_task(const double* xs, int wcol, int nr, int eb, uint8_t* dst, int tile) {
+  uint32_t pk[OZ_DIG][RPT / 2];
+#pragma unroll
+  for (int k = 0; k < RPT; k += 2) {
+    uint32_t d[OZ_DIG];
+    oz_digits2(k < nr ? xs[k * wcol] : 0.0, k + 1 < nr ? xs[(k + 1) * wcol] : 0.0, eb, eb, d);
+#pragma unroll
+    for (int p = 0; p < OZ_DIG; ++p) pk[p][k >> 1] = d[p];
+  }
+#pragma unroll
+  for (int p = 0; p < OZ_DIG; ++p) {
+    if constexpr (RPT == 8)
+      *reinterpret_cast<uint4*>(dst + p * tile) = make_uint4(pk[p][0], pk[p][1], pk[p][2], pk[p][3]);
+    else if constexpr (RPT == 4)
+      *reinterpret_cast<uint2*>(dst + p * tile) = make_uint2(pk[p][0], pk[p][1]);
+    else
+      *reinterpret_cast<uint32_t*>(dst + p * tile) = pk[p][0];
+  }
+}
+
 template <int RPT>
 __device__ __forceinline__ void oz_split(const double* rsrc, uint8_t* sa, uint8_t* sb, int m, int rw, int nrow,
-                                         const int* coff, const int* cw, const int* sE, int tid) {
+                                         const int* coff, const int* cw, const int* sE, int tid, int a_tile) {
   const int ntask = rw * (OZ_KC / RPT);
   for (int t = tid; t < ntask; t += OZ_SPLIT) {
     const int grp = t / rw, col = t - grp * rw;
@@ -239,26 +275,8 @@ __device__ __forceinline__ void oz_split(const double* rsrc, uint8_t* sa, uint8_
     const int cc = isA ? col : col - m;
     const int eb = sE[isA ? cc : OZ_M + cc];
     const int wcol = cw[col], k0 = RPT * grp;
-    const double* xs = rsrc + coff[col] + k0 * wcol;
-    uint32_t pk[OZ_DIG][RPT / 2];
-#pragma unroll
-    for (int k = 0; k < RPT; k += 2) {
-      uint32_t d[OZ_DIG];
-      oz_digits2(k0 + k < nrow ? xs[k * wcol] : 0.0, k0 + k + 1 < nrow ? xs[(k + 1) * wcol] : 0.0, eb, eb, d);
-#pragma unroll
-      for (int p = 0; p < OZ_DIG; ++p) pk[p][k >> 1] = d[p];
-    }
-    uint8_t* dst = (isA ? sa : sb) + kmaj(cc, k0);
-    const int tile = isA ? OZ_A_TILE : OZ_B_TILE;
-#pragma unroll
-    for (int p = 0; p < OZ_DIG; ++p) {
-      if constexpr (RPT == 8)
-        *reinterpret_cast<uint4*>(dst + p * tile) = make_uint4(pk[p][0], pk[p][1], pk[p][2], pk[p][3]);
-      else if constexpr (RPT == 4)
-        *reinterpret_cast<uint2*>(dst + p * tile) = make_uint2(pk[p][0], pk[p][1]);
-      else
-        *reinterpret_cast<uint32_t*>(dst + p * tile) = pk[p][0];
-    }
+    oz_split_task<RPT>(rsrc + coff[col] + k0 * wcol, wcol, nrow - k0, eb, (isA ? sa : sb) + kmaj(cc, k0),
+                       isA ? a_tile : OZ_B_TILE);
   }
 }
 
@@ -267,8 +285,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sbase = (uint8_t*)(((uintptr_t)smem + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles = sbase;                                 // digit stage s: A planes, then B planes
-  double* raw = (double*)(sbase + 2 * OZ_STAGE);          // nraw stages, operand blocks of [OZ_KC][width]
-  const double** bsrc = (const double**)(sbase + 2 * OZ_STAGE + (size_t)g.nraw * g.raw_stride * 8);  // block bases
+  const int nst = g.nst;
+  double* raw = (double*)(sbase + nst * g.stage);         // nraw stages, operand blocks of [OZ_KC][width]
+  const double** bsrc = (const double**)(raw + (size_t)g.nraw * g.raw_stride);  // block bases
   int* bw = (int*)(bsrc + OZ_MAXBLK);                     // [OZ_MAXBLK] block widths
   int* bld = bw + OZ_MAXBLK;                              // [OZ_MAXBLK] row strides
   int* boff = bld + OZ_MAXBLK;                            // [OZ_MAXBLK] raw-stage offsets (doubles)
@@ -284,7 +303,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
   const uint32_t bar0 = smem_u32(bars);
   auto BAR = [&](int slot, int i) { return bar0 + 8u * (uint32_t)(slot + i); };
 
-  for (int i = tid; i < 2 * OZ_STAGE / 16; i += OZ_THREADS) reinterpret_cast<uint4*>(tiles)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = tid; i < nst * g.stage / 16; i += OZ_THREADS) reinterpret_cast<uint4*>(tiles)[i] = make_uint4(0, 0, 0, 0);
   for (int i = tid; i < OZ_M; i += OZ_THREADS) sE[i] = i < m ? g.eA[i] : 0;
   for (int j = tid; j < OZ_N; j += OZ_THREADS) sE[OZ_M + j] = j < nbc ? g.eB[j] : 0;
   if (warp == OZ_MMA_WARP) {
@@ -293,7 +312,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < OZ_MAXST; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(BAR(OZ_B_FULL, s)), "r"(OZ_SPLIT / 32));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(BAR(OZ_B_EMPTY, s)));
     }
@@ -346,40 +365,62 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
   const int nchunks = r1 > r0 ? (int)((r1 - r0 + OZ_KC - 1) / OZ_KC) : 0;
   const int nwin = (nchunks + OZ_WINDOW - 1) / OZ_WINDOW;
   const int nraw = g.nraw;
-  long long hi[OZ_N], lo[OZ_N];  // fixed-point sums of this thread's A column (flush warps)
-#pragma unroll
-  for (int j = 0; j < OZ_N; ++j) hi[j] = lo[j] = 0;
 
   if (warp < OZ_SPLIT / 32) {
     // ---- splitting warps -------------------------------------------------
+    // up to 96 columns in tasks of 8 rows: a thread has the same task in every chunk
+    const int ntask = rw * (OZ_KC / 8);
+    const bool one = g.rpt == 8 && ntask <= OZ_SPLIT;
+    int t_src = 0, t_w = 0, t_k0 = 0, t_e = 0, t_dst = 0, t_tile = 0;
+    if (one && tid < ntask) {
+      const int grp = tid / rw, col = tid - grp * rw;
+      const bool isA = col < m;
+      const int cc = isA ? col : col - m;
+      t_k0 = 8 * grp;
+      t_w = cw[col];
+      t_src = coff[col] + t_k0 * t_w;
+      t_e = sE[isA ? cc : OZ_M + cc];
+      t_dst = (isA ? 0 : OZ_DIG * g.a_tile) + kmaj(cc, t_k0);
+      t_tile = isA ? g.a_tile : OZ_B_TILE;
+    }
+    // digit stage s and raw stage rs of the chunk, and the parities of their uses
+    int s = 0, rs = 0;
+    uint32_t sp = 0, rp = 0;
     for (int c = 0; c < nchunks; ++c) {
-      const int s = c & 1, rs = c % nraw;
-      // chunk c's raw rows have landed; the MMAs of chunk c - 2 are done with digit stage s
-      bool ok = mbar_wait(BAR(OZ_B_RAWF, rs), (uint32_t)(c / nraw) & 1u, sflag);
-      if (ok && c >= 2) ok = mbar_wait(BAR(OZ_B_EMPTY, s), (uint32_t)((c >> 1) - 1) & 1u, sflag);
+      // chunk c's raw rows have landed; the MMAs of chunk c - nst are done with digit stage s
+      bool ok = mbar_wait(BAR(OZ_B_RAWF, rs), rp, sflag);
+      if (ok && c >= nst) ok = mbar_wait(BAR(OZ_B_EMPTY, s), sp ^ 1u, sflag);
       if (!__all_sync(0xffffffffu, ok)) {
         if (lane == 0) atomicExch(sflag, 1);
         break;
       }
-      uint8_t* sa = tiles + s * OZ_STAGE;
-      uint8_t* sb = sa + OZ_DIG * OZ_A_TILE;
+      uint8_t* sa = tiles + s * g.stage;
+      uint8_t* sb = sa + OZ_DIG * g.a_tile;
       const double* rsrc = raw + (size_t)rs * g.raw_stride;
       const int nrow = (int)min((int64_t)OZ_KC, r1 - (r0 + (int64_t)c * OZ_KC));
-      if (g.rpt == 8)
-        oz_split<8>(rsrc, sa, sb, m, rw, nrow, coff, cw, sE, tid);
+      if (one) {
+        if (tid < ntask) oz_split_task<8>(rsrc + t_src, t_w, nrow - t_k0, t_e, sa + t_dst, t_tile);
+      } else if (g.rpt == 8)
+        oz_split<8>(rsrc, sa, sb, m, rw, nrow, coff, cw, sE, tid, g.a_tile);
       else if (g.rpt == 4)
-        oz_split<4>(rsrc, sa, sb, m, rw, nrow, coff, cw, sE, tid);
+        oz_split<4>(rsrc, sa, sb, m, rw, nrow, coff, cw, sE, tid, g.a_tile);
       else
-        oz_split<2>(rsrc, sa, sb, m, rw, nrow, coff, cw, sE, tid);
+        oz_split<2>(rsrc, sa, sb, m, rw, nrow, coff, cw, sE, tid, g.a_tile);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(BAR(OZ_B_RAWE, rs));
         mbar_arrive(BAR(OZ_B_FULL, s));
       }
+      if (++s == nst) s = 0, sp ^= 1u;
+      if (++rs == nraw) rs = 0, rp ^= 1u;
     }
   } else if (warp < OZ_MMA_WARP) {
     // ---- flush warps: lane quarter q = warp % 4 holds rows 32 q .. 32 q + 31
+    // (the sums live in this branch alone: the splitting warps need the registers)
+    long long hi[OZ_N], lo[OZ_N];  // fixed-point sums of this thread's A column
+#pragma unroll
+    for (int j = 0; j < OZ_N; ++j) hi[j] = lo[j] = 0;
     const uint32_t lrow = (uint32_t)((warp & 3) * 32) << 16;
     for (int w = 0; w < nwin; ++w) {
       const int buf = w % OZ_NBUF;
@@ -398,22 +439,34 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
       __syncwarp();
       if (lane == 0) mbar_arrive(BAR(OZ_B_ACCE, buf));
     }
+    const bool ok = *(volatile int*)sflag == 0;  // an error sets *status, whatever is written here
+    const int i = (warp & 3) * 32 + lane;
+    if (i < m)
+#pragma unroll
+      for (int j = 0; j < OZ_N; ++j)
+        if (j < nbc) {
+          const int e = (sE[i] - 1022) + (sE[OZ_M + j] - 1022);
+          const double v = ldexp((double)hi[j], e - 35) + ldexp((double)lo[j], e - 63);
+          g.partial[((int64_t)blockIdx.x * m + i) * nbc + j] = ok ? v : 0.0;
+        }
   } else if (warp == OZ_MMA_WARP) {
     // ---- MMA warp: lane 0 issues, the warp stays converged ----------------
     uint32_t last_bar = 0, last_par = 0;  // the latest commit: its completion covers every MMA
+    int s = 0;
+    uint32_t sp = 0;
     for (int c = 0; c < nchunks; ++c) {
-      const int s = c & 1, w = c / OZ_WINDOW, buf = w % OZ_NBUF;
+      const int w = c / OZ_WINDOW, buf = w % OZ_NBUF;
       bool ok = true;
       if (lane == 0) {
         // accumulator buffer flushed (window w - 4), digit stage s full
         if (c % OZ_WINDOW == 0 && w >= OZ_NBUF)
           ok = mbar_wait(BAR(OZ_B_ACCE, buf), (uint32_t)(w / OZ_NBUF - 1) & 1u, sflag);
-        if (ok) ok = mbar_wait(BAR(OZ_B_FULL, s), (uint32_t)(c >> 1) & 1u, sflag);
+        if (ok) ok = mbar_wait(BAR(OZ_B_FULL, s), sp, sflag);
         if (ok) {
           asm volatile("tcgen05.fence::after_thread_sync;");
           const bool first = (c % OZ_WINDOW) == 0;
-          const uint32_t a0 = smem_u32(tiles + s * OZ_STAGE);
-          const uint32_t b0 = a0 + OZ_DIG * OZ_A_TILE;  // B planes 0..7
+          const uint32_t a0 = smem_u32(tiles + s * g.stage);
+          const uint32_t b0 = a0 + OZ_DIG * g.a_tile;  // B planes 0..7
 #pragma unroll
           for (int p = 0; p < OZ_DIG; ++p)
 #pragma unroll
@@ -425,18 +478,19 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
                   "{\n .reg .pred pa;\n setp.ne.b32 pa, %4, 0;\n"
                   " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, pa;\n}" ::"r"(
                       tmem + (uint32_t)(buf * OZ_ACC_COLS + p * OZ_N)),
-                  "l"(sdesc(a0 + p * OZ_A_TILE + kt * 256)), "l"(sdesc(b0 + kt * 256)),
+                  "l"(sdesc(a0 + p * g.a_tile + kt * 256)), "l"(sdesc(b0 + kt * 256)),
                   "r"(oz_idesc((OZ_LEVELS - p) * OZ_N)), "r"(acc));
             }
           mma_commit(BAR(OZ_B_EMPTY, s));
           last_bar = BAR(OZ_B_EMPTY, s);
-          last_par = (uint32_t)(c >> 1) & 1u;
+          last_par = sp;
           if (c % OZ_WINDOW == OZ_WINDOW - 1 || c == nchunks - 1) mma_commit(BAR(OZ_B_ACCF, buf));
         } else {
           atomicExch(sflag, 1);
         }
       }
       if (!__shfl_sync(0xffffffffu, (int)ok, 0)) break;
+      if (++s == nst) s = 0, sp ^= 1u;
     }
     // before the tensor memory is freed, every MMA issued must have completed
     if (lane == 0 && last_bar != 0 && !mbar_drain(last_bar, last_par)) atomicExch(sflag, 1);
@@ -500,17 +554,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
   asm volatile("tcgen05.fence::after_thread_sync;");
   const bool ok = *(volatile int*)sflag == 0;
   if (!ok && tid == 0) atomicExch(g.status, 1);
-  if (warp >= OZ_FLUSH_WARP && warp < OZ_MMA_WARP) {
-    const int i = (warp & 3) * 32 + lane;
-    if (i < m)
-#pragma unroll
-      for (int j = 0; j < OZ_N; ++j)
-        if (j < nbc) {
-          const int e = (sE[i] - 1022) + (sE[OZ_M + j] - 1022);
-          const double v = ldexp((double)hi[j], e - 35) + ldexp((double)lo[j], e - 63);
-          g.partial[((int64_t)blockIdx.x * m + i) * nbc + j] = ok ? v : 0.0;
-        }
-  }
   if (warp == OZ_MMA_WARP)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(OZ_TMEM_COLS));
 }
@@ -544,8 +587,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
 //  * four warps read a finished accumulator, add its levels as integers and
 //    write the tile's rows of O in FP64 (acce[b]).
 // The digit planes of C are built once per CTA.  Waits are bounded as in
-// k_gram_oz.  1e6 rows x 80 -> 8 columns: 798 us when all warps cut, issued
-// and flushed in turn behind block barriers (30k cycles a tile).
+// k_gram_oz.  1e6 rows x 80 -> 8 columns: 350 us, against 798 us when all
+// warps cut, issued and flushed in turn behind block barriers.  What is left
+// (14k cycles a tile): the digit stores and operand reads of shared memory
+// (about 1k cycles a K step), the integer instructions of the cut (50 us of
+// the time), the exponent pass and the wait for a tile's last blocks (50 us
+// each).
 constexpr int LC_SPLIT_WARPS = 16;
 constexpr int LC_FLUSH_WARP = LC_SPLIT_WARPS;    // a multiple of 4: warp w reads lane quarter w % 4
 constexpr int LC_MMA_WARP = LC_FLUSH_WARP + 4;
@@ -560,8 +607,9 @@ constexpr int LC_MAXM = 128;
 constexpr int LC_ACC_COLS = OZ_LEVELS * OZ_N;    // 128 tensor-memory columns per accumulator
 constexpr int LC_TMEM_COLS = 2 * LC_ACC_COLS;
 // barrier slots
-constexpr int LC_B_FULL = 0, LC_B_EMPTY = 2, LC_B_ACCF = 4, LC_B_ACCE = 6, LC_B_RAWF = 8,
-              LC_NBARS = 10;
+constexpr int LC_MAXST = 3;                      // digit stages: 3 where shared memory allows, else 2
+constexpr int LC_B_FULL = 0, LC_B_EMPTY = LC_B_FULL + LC_MAXST, LC_B_ACCF = LC_B_EMPTY + LC_MAXST,
+              LC_B_ACCE = LC_B_ACCF + 2, LC_B_RAWF = LC_B_ACCE + 2, LC_NBARS = LC_B_RAWF + 2;
 
 struct LcArgs {
   const double* A;
@@ -573,6 +621,7 @@ struct LcArgs {
   int64_t N, rows_per_cta;
   int lane_copies;  // some block of some tile is not whole 16-byte lines
   int nslots;       // block slots of the ring: nb .. 2 nb
+  int nst;          // digit stages
   const int* skip;
   int* status;
 };
@@ -603,8 +652,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
   if (g.skip && *g.skip) return;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sbase = (uint8_t*)(((uintptr_t)smem + 1023) & ~(uintptr_t)1023);
-  uint8_t* adig = sbase;                                  // 2 stages of 8 A planes
-  uint8_t* bdig = sbase + 2 * LC_ASTAGE;                  // nks x 8 C planes
+  uint8_t* adig = sbase;                                  // nst stages of 8 A planes
+  const int nst = g.nst;
+  uint8_t* bdig = sbase + nst * LC_ASTAGE;                // nks x 8 C planes
   const int m = g.m, nsd = g.nsd, nb = m / nsd;
   const int nks = (m + LC_KS - 1) / LC_KS;
   double* raw = (double*)(bdig + (size_t)nks * LC_BCHUNK);  // [slot][128 rows][nsd]
@@ -670,17 +720,21 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
     const int q = lane & 3, r = warp * 8 + (lane >> 2);
     const int swap = q >> 1;
     bool ok = true;
-    int gstep = 0, slot0 = 0;  // slot of the tile's first block
+    int s = 0, round = 0;  // digit stage of the next K step, uses of it so far
+    int slot0 = 0;         // slot of the tile's first block
     auto block = [&](int b) {
       const int x = slot0 + b;
       return raw + (size_t)(x < nslots ? x : x - nslots) * LC_TM * nsd;
     };
-    // columns i .. i + 3 of row r (0 beyond m)
-    auto load4 = [&](int i, double (&x)[4]) {
+    // walks the columns 4 q, 4 q + 16, ... of row r: load() gives the next four (0 beyond m)
+    struct Walk {
+      int i, b, s;
+    };
+    const int b0 = 4 * q / nsd, s0 = 4 * q - b0 * nsd;
+    auto load = [&](Walk& at, double (&x)[4]) {
       if constexpr (VEC) {
-        if (i < m) {
-          const int b = i / nsd;
-          const double2* p = reinterpret_cast<const double2*>(block(b) + r * nsd + (i - b * nsd));
+        if (at.i < m) {
+          const double2* p = reinterpret_cast<const double2*>(block(at.b) + r * nsd + at.s);
           const double2 u = p[swap], w = p[1 - swap];
           x[0] = swap ? w.x : u.x;
           x[1] = swap ? w.y : u.y;
@@ -690,16 +744,22 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
           x[0] = x[1] = x[2] = x[3] = 0.0;
         }
       } else {
-        int b = i / nsd, s = i - b * nsd;
+        int b = at.b, s = at.s;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           x[k] = 0.0;
-          if (i + k < m) x[k] = block(b)[r * nsd + s];
+          if (at.i + k < m) x[k] = block(b)[r * nsd + s];
           if (++s == nsd) {
             s = 0;
             ++b;
           }
         }
+      }
+      at.i += LC_KS;
+      at.s += LC_KS;
+      while (at.s >= nsd) {
+        at.s -= nsd;
+        ++at.b;
       }
     };
     for (int t = 0; t < ntile && ok; ++t) {
@@ -711,12 +771,15 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
       }
       // the row's largest exponent
       int e = 0;
-      for (int i = 4 * q; i < m; i += LC_KS) {
+      Walk at{4 * q, b0, s0};
+#pragma unroll 2
+      for (int c = 0; c < nks; ++c) {
         double x[4];
-        load4(i, x);
+        load(at, x);
 #pragma unroll
         for (int k = 0; k < 4; ++k) e = max(e, __double2hiint(x[k]) & 0x7fffffff);
       }
+      at = Walk{4 * q, b0, s0};
       e >>= 20;
       e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
       e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
@@ -727,15 +790,14 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
         break;
       }
       if (q == 0) eb[(t & 1) * LC_TM + r] = e;
-      for (int c = 0; c < nks; ++c, ++gstep) {
-        const int s = gstep & 1;
+      for (int c = 0; c < nks; ++c) {
         double x[4];
-        load4(c * LC_KS + 4 * q, x);
+        load(at, x);
         uint32_t d0[OZ_DIG], d1[OZ_DIG];
         oz_digits2(x[0], x[1], e, e, d0);
         oz_digits2(x[2], x[3], e, e, d1);
-        // the MMAs of step gstep - 2 are done with stage s
-        if (gstep >= 2) ok = mbar_wait(BAR(LC_B_EMPTY + s), (uint32_t)((gstep >> 1) - 1) & 1u, sflag);
+        // the MMAs of nst steps ago are done with stage s
+        if (round > 0) ok = mbar_wait(BAR(LC_B_EMPTY + s), (uint32_t)(round - 1) & 1u, sflag);
         if (!__all_sync(0xffffffffu, ok)) {
           ok = false;
           break;
@@ -746,6 +808,10 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR(LC_B_FULL + s));
+        if (++s == nst) {
+          s = 0;
+          ++round;
+        }
       }
     }
     if (!ok && lane == 0) atomicExch(sflag, 1);
@@ -797,12 +863,10 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
           for (int j = 0; j < 8; ++j) {
             if (j0 + j < nsd) {
               const int ex = (er - 1022) + (ej[j0 + j] - 1022);
-              const double h = (double)hi[j], l = (double)lo[j];
-              if (ex - 63 >= -1022 && ex - 35 <= 1023)  // both scales are normal powers of two: exact products
-                v[j] = h * __longlong_as_double((long long)(ex - 35 + 1023) << 52) +
-                       l * __longlong_as_double((long long)(ex - 63 + 1023) << 52);
+              if (ex - 63 >= -1022 && ex - 35 <= 960)  // both parts exact, one rounding
+                v[j] = scaled_int(hi[j], ex - 35) + scaled_int(lo[j], ex - 63);
               else
-                v[j] = ldexp(h, ex - 35) + ldexp(l, ex - 63);
+                v[j] = ldexp((double)hi[j], ex - 35) + ldexp((double)lo[j], ex - 63);
             }
           }
 #pragma unroll
@@ -820,15 +884,15 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
   } else if (warp == LC_MMA_WARP) {
     // ---- MMA warp: lane 0 issues, the warp stays converged ----------------
     uint32_t last_bar = 0, last_par = 0;  // the latest commit: its completion covers every MMA
-    int gstep = 0;
+    int gstep = 0, s = 0, round = 0;
     bool ok = true;
     for (int t = 0; t < ntile && ok; ++t)
       for (int c = 0; c < nks && ok; ++c, ++gstep) {
-        const int s = gstep & 1, buf = t & 1;
+        const int buf = t & 1;
         if (lane == 0) {
           // accumulator written out (tile t - 2), digit stage s full
           if (c == 0 && t >= 2) ok = mbar_wait(BAR(LC_B_ACCE + buf), (uint32_t)((t >> 1) - 1) & 1u, sflag);
-          if (ok) ok = mbar_wait(BAR(LC_B_FULL + s), (uint32_t)(gstep >> 1) & 1u, sflag);
+          if (ok) ok = mbar_wait(BAR(LC_B_FULL + s), (uint32_t)round & 1u, sflag);
           if (ok) {
             *sdone = gstep + 1;
             asm volatile("tcgen05.fence::after_thread_sync;");
@@ -844,11 +908,15 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
             }
             mma_commit(BAR(LC_B_EMPTY + s));
             last_bar = BAR(LC_B_EMPTY + s);
-            last_par = (uint32_t)(gstep >> 1) & 1u;
+            last_par = (uint32_t)round & 1u;
             if (c == nks - 1) mma_commit(BAR(LC_B_ACCF + buf));
           } else {
             atomicExch(sflag, 1);
           }
+        }
+        if (++s == nst) {
+          s = 0;
+          ++round;
         }
         ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
       }
@@ -976,11 +1044,24 @@ __global__ void __launch_bounds__(256) k_col_maxexp(const double* X, int nblk, i
 }
 
 // out[p] = sum over CTAs c = 0, 1, ... of partial[c][p], in that order
-__global__ void k_oz_reduce(const double* partial, int ncta, int np, double* out, const int* skip) {
+// The CTAs' partial sums of one entry per thread, added in the CTAs' order.
+// Bound by the latency of the loads, so OZ_RED_AHEAD of them are in flight
+// at a time and the entries are spread over one warp per block.
+constexpr int OZ_RED_AHEAD = 16;
+__global__ void k_oz_reduce(const double* __restrict__ partial, int ncta, int np, double* __restrict__ out,
+                            const int* skip) {
   if (skip && *skip) return;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int c = 0; c < ncta; ++c) s += partial[(int64_t)c * np + p];
+    int c = 0;
+    for (; c + OZ_RED_AHEAD <= ncta; c += OZ_RED_AHEAD) {
+      double v[OZ_RED_AHEAD];
+#pragma unroll
+      for (int i = 0; i < OZ_RED_AHEAD; ++i) v[i] = partial[(int64_t)(c + i) * np + p];
+#pragma unroll
+      for (int i = 0; i < OZ_RED_AHEAD; ++i) s += v[i];
+    }
+    for (; c < ncta; ++c) s += partial[(int64_t)c * np + p];
     out[p] = s;
   }
 }
@@ -988,7 +1069,7 @@ __global__ void k_oz_reduce(const double* partial, int ncta, int np, double* out
 }  // namespace
 
 void qp_oz_reduce(const double* partial, int ncta, int np, double* out, const int* skip, cudaStream_t st) {
-  k_oz_reduce<<<(np + 127) / 128, 128, 0, st>>>(partial, ncta, np, out, skip);
+  k_oz_reduce<<<(np + 31) / 32, 32, 0, st>>>(partial, ncta, np, out, skip);
 }
 
 // Opt-in shared memory of k_gram_oz on the current device (once per device).
@@ -1039,8 +1120,14 @@ void qp_gram_oz(const double* A, int64_t sA, int m, int nsdA, int ldA, const dou
   // many as fit beside the digit stages, up to OZ_MAXRAW
   const int rw = m + nbc;
   g.raw_stride = (OZ_KC * rw + 31) / 32 * 32;
-  g.nraw = std::max(1, std::min(OZ_MAXRAW, (OZ_SMEM_MAX - 2 * OZ_STAGE - OZ_TAB) / (g.raw_stride * 8)));
-  const int smem = 2 * OZ_STAGE + g.nraw * g.raw_stride * 8 + OZ_TAB;
+  // digit stages of the columns in use; the MMAs of the last stage read up to
+  // 128 rows of its last A plane, inside its B planes and the raw stages
+  g.a_tile = (m + 7) / 8 * 8 * OZ_KC * 2;
+  g.stage = OZ_DIG * (g.a_tile + OZ_B_TILE);
+  auto rawfit = [&](int nst) { return (OZ_SMEM_MAX - nst * g.stage - OZ_TAB) / (g.raw_stride * 8); };
+  g.nst = rawfit(3) >= 2 ? 3 : 2;
+  g.nraw = std::max(1, std::min(OZ_MAXRAW, rawfit(g.nst)));
+  const int smem = g.nst * g.stage + g.nraw * g.raw_stride * 8 + OZ_TAB;
   // rows per splitting task: the fewest rows per thread on the longest
   // thread's path (more, narrower stores only where that gains)
   int best = 1 << 30;
@@ -1081,12 +1168,15 @@ int qp_lincomb_oz(const double* A, int64_t sA, int m, int nsd, const double* C, 
   if (lincomb_oz_prepare()) return -1;
   const int nks = (m + LC_KS - 1) / LC_KS;
   const int nb = m / nsd;
-  const size_t fixed = 1024 + 2 * (size_t)LC_ASTAGE + (size_t)nks * LC_BCHUNK + (2 * LC_TM + OZ_N) * 4 +
-                       (LC_NBARS + 3) * 8;
+  // three digit stages where a quarter of a tile can still be loaded ahead
   const size_t slot_bytes = (size_t)LC_TM * nsd * 8;
-  const int nslots = std::min<int>(2 * nb, (int)((OZ_SMEM_MAX - fixed) / slot_bytes));
+  auto fixed = [&](int nst) {
+    return 1024 + (size_t)nst * LC_ASTAGE + (size_t)nks * LC_BCHUNK + (2 * LC_TM + OZ_N) * 4 + (LC_NBARS + 3) * 8;
+  };
+  const int nst = fixed(3) + (nb + (nb + 3) / 4) * slot_bytes <= (size_t)OZ_SMEM_MAX ? 3 : 2;
+  const int nslots = std::min<int>(2 * nb, (int)((OZ_SMEM_MAX - fixed(nst)) / slot_bytes));
   if (nslots < nb) return -1;
-  const size_t smem = fixed + nslots * slot_bytes;
+  const size_t smem = fixed(nst) + nslots * slot_bytes;
   LcArgs g;
   g.A = A;
   g.sA = sA;
@@ -1100,6 +1190,7 @@ int qp_lincomb_oz(const double* A, int64_t sA, int m, int nsd, const double* C, 
   rpc = (rpc + LC_TM - 1) / LC_TM * LC_TM;
   g.rows_per_cta = rpc;
   g.nslots = nslots;
+  g.nst = nst;
   // blocks start on 16-byte lines, and the last tile's rows fill them
   g.lane_copies = ((uintptr_t)A & 15) != 0 || (nb > 1 && (sA & 1) != 0) || ((N % LC_TM) * nsd & 1) != 0;
   g.skip = skip;
