@@ -83,16 +83,14 @@ template <int NST>
 __device__ __forceinline__ void bstore(const BProb& P, int64_t it, int k, int lane, double hv, double sv, bool has_s2,
                                        const double* u, double* v, double* s) {
   constexpr int SH = 5 - Pow2<NST>::lg;
-  const int st = lane >> SH;
-  const bool owner = (lane & ((1 << SH) - 1)) == 0 && st < NST;
-  if (!owner) return;
+  const int st = lane >> SH, sub = lane & ((1 << SH) - 1);
+  if (sub > 1 || st >= NST) return;
+  const double sum = sub == 0 ? hv : has_s2 ? sv : 0.0;
   if (P.row_nitems[k] == 1) {
-    const double uk = u[(int64_t)k * NST + st];
-    v[(int64_t)k * NST + st] = hv + P.hdiag[k] * uk;
-    s[(int64_t)k * NST + st] = (has_s2 ? sv : 0.0) + P.sdiag[k] * uk;
+    const double d = sub == 0 ? P.hdiag[k] : P.sdiag[k];
+    (sub == 0 ? v : s)[(int64_t)k * NST + st] = fma(d, u[(int64_t)k * NST + st], sum);
   } else {
-    P.pv[it * NST + st] = hv;
-    P.ps[it * NST + st] = has_s2 ? sv : 0.0;
+    (sub == 0 ? P.pv : P.ps)[it * NST + st] = sum;
   }
 }
 
@@ -167,41 +165,14 @@ __global__ void k_bsigma(const BProb* __restrict__ probs, int np, int64_t total,
       double acc[NP];
 #pragma unroll
       for (int st = 0; st < NP; ++st) acc[st] = 0.0;
-      constexpr int U2 = 2;
-      for (int64_t e0 = beg + lane; e0 < end; e0 += 32 * U2) {
-        int col[U2];
-        double hv[U2];
-#pragma unroll
-        for (int q = 0; q < U2; ++q) {
-          const int64_t e = e0 + 32 * q;
-          col[q] = e < end ? __ldg(&P.colidx[e]) : k;
-          hv[q] = e < end ? __ldg(&P.val64[e]) : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < U2; ++q) {
-          double x[NST];
-          load_row<NST>(u, col[q], x);
-#pragma unroll
-          for (int st = 0; st < NST; ++st) acc[st] = fma(hv[q], x[st], acc[st]);
-        }
-      }
+      sum_pairs64<NST, NP, 2>(u, P.colidx, P.val64, beg, end, k, lane, acc);
       hsum = reduce_scatter64<NP>(acc, lane);
     }
     double ssum = 0.0;
     const int64_t sb = P.s2ptr[k], se = P.s2ptr[k + 1];
     const bool has_s2 = (j == 0) && (se > sb);
     if (has_s2) {
-      double sacc[NP];
-#pragma unroll
-      for (int st = 0; st < NP; ++st) sacc[st] = 0.0;
-      for (int64_t e = sb + lane; e < se; e += 32) {
-        const double sv = (double)__ldg(&P.s2val[e]);
-        double x[NST];
-        load_row<NST>(u, __ldg(&P.s2col[e]), x);
-#pragma unroll
-        for (int st = 0; st < NST; ++st) sacc[st] = fma(sv, x[st], sacc[st]);
-      }
-      ssum = reduce_scatter64<NP>(sacc, lane);
+      ssum = s2_row_sum<NST, NP>(u, P.s2col, P.s2val, sb, se, lane);
     }
     bstore<NST>(P, it, k, lane, hsum, ssum, has_s2, u, v, s);
   }
@@ -821,7 +792,7 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
   for (int p = 0; p < np; ++p) {
     BProb& P = B->h[p];
     QB_CUDA(B, cudaMemcpy2DAsync(P.R, P.N * 8, u_in[p], dim_in[p] * 8, P.N * 8, nsd, cudaMemcpyHostToDevice, st));
-    qp_to_bilinear(P.R, P.N, B->ctx[p]->d_order, P.U, nullptr, nsd, P.N, st);
+    qp_to_bilinear(P.R, P.N, B->ctx[p]->d_pos, P.U, nullptr, nsd, P.N, st);
   }
   QB_CUDA(B, cudaStreamSynchronize(st));
   // autotune the persistent sigma's launch shape once per batch
@@ -996,7 +967,7 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
   int n_conv = 0;
   for (int p = 0; p < np; ++p) {
     BProb& P = B->h[p];
-    qp_from_bilinear(P.U, P.N, B->ctx[p]->d_order, P.R, nsd, P.N, st);
+    qp_from_bilinear(P.U, P.N, B->ctx[p]->d_pos, P.R, nsd, P.N, st);
     QB_CUDA(B, cudaMemcpy2DAsync(u_in[p], dim_in[p] * 8, P.R, P.N * 8, P.N * 8, nsd, cudaMemcpyDeviceToHost, st));
     for (int k = 0; k < nsd; ++k) {
       energies[(size_t)p * nsd + k] = lam[p][k];

@@ -242,6 +242,18 @@ int qp_numeric_flag(qpgpu_ctx* c, cudaStream_t st, int** flag) {
   return 0;
 }
 
+int qp_pin(qpgpu_ctx* c, size_t n, double** p) {
+  if (c->h_pin_doubles < n) {
+    if (c->h_pin) cudaFreeHost(c->h_pin);
+    c->h_pin = nullptr;
+    c->h_pin_doubles = 0;
+    QP_CUDA(c, cudaMallocHost((void**)&c->h_pin, n * sizeof(double)));
+    c->h_pin_doubles = n;
+  }
+  *p = c->h_pin;
+  return 0;
+}
+
 namespace {
 
 struct Lock {
@@ -528,13 +540,12 @@ int h_s2_u0_dev(qpgpu_ctx* c, double* v0, double* s0, const double* u0, int n_st
   float* ut32 = (float*)(stt + (size_t)N * nb);
   for (int s0i = 0; s0i < n_st; s0i += 8) {
     const int m = (n_st - s0i) < 8 ? (n_st - s0i) : 8;
-    qp_to_bilinear(u0 + (int64_t)s0i * ld, ld, c->d_order, ut, precision == QPGPU_FP32 ? ut32 : nullptr, m, N, st,
+    qp_to_bilinear(u0 + (int64_t)s0i * ld, ld, c->d_pos, ut, precision == QPGPU_FP32 ? ut32 : nullptr, m, N, st,
                    bad);
     rc = qp_sigma_launch(c, &c->items, vt, stt, ut, ut32, m, precision, st, 0, (int)N, 0, 1);
     if (!rc && dressed) rc = qp_dress(c, vt, stt, ut, m, st);
     if (rc) return rc;
-    qp_from_bilinear(vt, ld, c->d_order, v0 + (int64_t)s0i * ld, m, N, st);
-    qp_from_bilinear(stt, ld, c->d_order, s0 + (int64_t)s0i * ld, m, N, st);
+    qp_from_bilinear(vt, ld, c->d_pos, v0 + (int64_t)s0i * ld, m, N, st, stt, s0 + (int64_t)s0i * ld);
   }
   QP_CUDA(c, cudaGetLastError());
   return QPGPU_OK;
@@ -554,6 +565,37 @@ int qpgpu_h_s2_u0_device(qpgpu_ctx* c, double* v0, double* s0, const double* u0,
 }
 
 namespace {
+// Small blocks of host arrays: the kernels read u_0 from pinned memory and
+// write v_0, s_0 and the NaN flag there, so that a call is three kernels and
+// one wait.  (As copies from and to the caller's pageable arrays, a memset
+// and a copy of the flag, a call on 1,000 determinants took 62 us, now
+// 31.)  Past the limit the host's own copies out of pinned memory cost more:
+// 5,000 x 1 78 -> 52 us, 5,000 x 4 107 -> 88, 20,000 x 2 128 -> 131, 30,000 x 4
+// 213 -> 331.
+constexpr size_t H_S2_PIN_DOUBLES = 3 << 13;
+int h_s2_u0_pinned(qpgpu_ctx* c, double* v0, double* s0, const double* u0, int n_st, int64_t ld, bool dressed) {
+  const int64_t N = c->N;
+  const size_t cols = (size_t)N * n_st;
+  double* pu = nullptr;
+  int rc = qp_pin(c, 3 * cols + 1, &pu);
+  if (rc) return rc;
+  double *pv = pu + cols, *ps = pv + cols;
+  volatile int* const bad = (volatile int*)(ps + cols);
+  *bad = 0;
+  if (dressed && !c->dress.on) return qpgpu_fail(c, QPGPU_ERR_STATE, "no dressing set");
+  for (int k = 0; k < n_st; ++k) std::memcpy(pu + (size_t)k * N, u0 + (int64_t)k * ld, N * sizeof(double));
+  rc = h_s2_u0_dev(c, pv, ps, pu, n_st, N, QPGPU_FP64, c->stream, (int*)bad, dressed);
+  const cudaError_t e = cudaStreamSynchronize(c->stream);
+  if (rc) return rc;
+  if (e != cudaSuccess) return qpgpu_fail(c, QPGPU_ERR_CUDA, cudaGetErrorString(e));
+  for (int k = 0; k < n_st; ++k) {
+    std::memcpy(v0 + (int64_t)k * ld, pv + (size_t)k * N, N * sizeof(double));
+    std::memcpy(s0 + (int64_t)k * ld, ps + (size_t)k * N, N * sizeof(double));
+  }
+  if (*bad) return qpgpu_fail(c, QPGPU_ERR_NUMERIC, "u_0 holds a NaN or an infinity");
+  return 0;
+}
+
 int h_s2_u0_host(qpgpu_ctx* c, double* v0, double* s0, const double* u0, int n_st, int64_t ld, bool dressed) {
   int rc = check_ctx(c, true, true);
   if (rc) return rc;
@@ -561,6 +603,7 @@ int h_s2_u0_host(qpgpu_ctx* c, double* v0, double* s0, const double* u0, int n_s
   const int64_t N = c->N;
   const size_t cols = (size_t)N * n_st;
   Lock l(c->mu);
+  if (cols <= H_S2_PIN_DOUBLES) return h_s2_u0_pinned(c, v0, s0, u0, n_st, ld, dressed);
   if (c->stage_bytes < 3 * cols * sizeof(double)) {
     dev_free(c->d_stage);
     c->d_stage = nullptr;
@@ -748,8 +791,7 @@ int qpgpu_diag(qpgpu_ctx* c, double* h_jj, double* s_jj) {
   double* buf = nullptr;
   QP_CUDA(c, qp_pool_alloc(c, (void**)&buf, 2 * N * sizeof(double)));
   cudaStream_t st = c->stream;
-  qp_from_bilinear(c->d_hdiag, N, c->d_order, buf, 1, N, st);
-  qp_from_bilinear(c->d_sdiag, N, c->d_order, buf + N, 1, N, st);
+  qp_from_bilinear(c->d_hdiag, N, c->d_pos, buf, 1, N, st, c->d_sdiag, buf + N);
   rc = 0;
   if (h_jj && cudaMemcpyAsync(h_jj, buf, N * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -1;
   if (s_jj && cudaMemcpyAsync(s_jj, buf + N, N * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -1;

@@ -1482,7 +1482,7 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
     int hbad = 0;
     const int rcf = qp_numeric_flag(c, st, &bad);
     if (rcf) return rcf;
-    qp_to_bilinear(hstage, N, c->d_order, d.U, nullptr, nsd, N, st, bad);
+    qp_to_bilinear(hstage, N, c->d_pos, d.U, nullptr, nsd, N, st, bad);
     QP_CUDA(c, cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
     QP_CUDA(c, cudaStreamSynchronize(st));
     qp_pool_free(c, hstage);
@@ -1500,14 +1500,9 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
   std::vector<double> lambda(mmax), s2(mmax), y, wv, res(MAXS, 0.0);
   // pinned staging of the small copies: Gram columns, y, norms, status
   const size_t n_pin = (size_t)MAXM * 2 * MAXS + (size_t)MAXM * MAXS + (size_t)d.ncta * MAXS + 2;
-  if (c->h_pin_doubles < n_pin) {
-    if (c->h_pin) cudaFreeHost(c->h_pin);
-    c->h_pin = nullptr;
-    c->h_pin_doubles = 0;
-    QP_CUDA(c, cudaMallocHost((void**)&c->h_pin, n_pin * sizeof(double)));
-    c->h_pin_doubles = n_pin;
-  }
-  double* const hscol = c->h_pin;
+  double* hscol = nullptr;
+  const int rc_pin = qp_pin(c, n_pin, &hscol);
+  if (rc_pin) return rc_pin;
   double* const ycoef = hscol + MAXM * 2 * MAXS;
   double* const partial = ycoef + MAXM * MAXS;
   int* const tc_status = (int*)(partial + (size_t)d.ncta * MAXS);
@@ -1828,7 +1823,7 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
   {
     double* hstage = nullptr;
     QP_CUDA(c, qp_pool_alloc(c, (void**)&hstage, blkn * sizeof(double)));
-    qp_from_bilinear(d.U, N, c->d_order, hstage, nsd, N, st);
+    qp_from_bilinear(d.U, N, c->d_pos, hstage, nsd, N, st);
     QP_CUDA(c, cudaMemcpy2DAsync(u_in, dim_in * sizeof(double), hstage, N * sizeof(double), N * sizeof(double), nsd,
                                  cudaMemcpyDeviceToHost, st));
     QP_CUDA(c, cudaStreamSynchronize(st));

@@ -76,11 +76,13 @@ __global__ void k_make_key(const int* hi, const int* lo, int64_t mul, u64* key, 
 }
 
 // bilinear (beta-major): rows/cols at position p from the sorted permutation
-__global__ void k_bilinear(const int* order, const int* aid, const int* bid, int* rows, int* cols, int64_t n) {
+__global__ void k_bilinear(const int* order, const int* aid, const int* bid, int* rows, int* cols, int* pos,
+                           int64_t n) {
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
     int k = order[p];
     rows[p] = aid[k];
     cols[p] = bid[k];
+    pos[k] = (int)p;
   }
 }
 
@@ -362,7 +364,7 @@ int singles_adjacency(qpgpu_ctx* c, const u64* uniq, int U, int ne, int** ptr_ou
 void qp_free_dets(qpgpu_ctx* c) {
   qp_free_line_keys(c);
   void** ps[] = {(void**)&c->d_dets, (void**)&c->d_alpha, (void**)&c->d_beta, (void**)&c->d_rows,
-                 (void**)&c->d_cols, (void**)&c->d_order, (void**)&c->d_col_loc, (void**)&c->d_t_order,
+                 (void**)&c->d_cols, (void**)&c->d_order, (void**)&c->d_pos, (void**)&c->d_col_loc, (void**)&c->d_t_order,
                  (void**)&c->d_t_cols, (void**)&c->d_row_loc, (void**)&c->d_sa_ptr, (void**)&c->d_sa_idx,
                  (void**)&c->d_sb_ptr, (void**)&c->d_sb_idx, (void**)&c->d_cost_a, (void**)&c->d_cost_b,
                  (void**)&c->d_detfeat, (void**)&c->d_alpha_pos, (void**)&c->d_beta_tpos};
@@ -401,6 +403,7 @@ int qp_build_index(qpgpu_ctx* c) {
   const int Ua = c->Ua, Ub = c->Ub;
   // beta-major bilinear order: key = beta_id * Ua + alpha_id (spindeterminants.irp.f:417)
   QP_CUDA(c, pool_alloc(c, &c->d_order, N));
+  QP_CUDA(c, pool_alloc(c, &c->d_pos, N));
   QP_CUDA(c, pool_alloc(c, &c->d_rows, N));
   QP_CUDA(c, pool_alloc(c, &c->d_cols, N));
   {
@@ -413,7 +416,7 @@ int qp_build_index(qpgpu_ctx* c) {
     }, c->d_order);
     if (rc) return rc;
   }
-  k_bilinear<<<grid_for(N), TPB, 0, st>>>(c->d_order, aid.p, bid.p, c->d_rows, c->d_cols, N);
+  k_bilinear<<<grid_for(N), TPB, 0, st>>>(c->d_order, aid.p, bid.p, c->d_rows, c->d_cols, c->d_pos, N);
   QP_CUDA(c, pool_alloc(c, &c->d_col_loc, (size_t)Ub + 1));
   k_seg_starts<<<grid_for(N), TPB, 0, st>>>(c->d_cols, c->d_col_loc, N, Ub);
   // alpha-major (transposed) order over bilinear positions: key = alpha_id * Ub + beta_id

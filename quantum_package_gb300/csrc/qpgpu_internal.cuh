@@ -553,6 +553,7 @@ struct qpgpu_ctx {
   int* d_rows = nullptr;       // bilinear (beta-major) position -> alpha id (0-based)
   int* d_cols = nullptr;       // -> beta id
   int* d_order = nullptr;      // bilinear position -> original index
+  int* d_pos = nullptr;        // original index -> bilinear position
   int* d_col_loc = nullptr;    // (U_b+1) first bilinear position of each beta column
   int* d_t_order = nullptr;    // alpha-major position -> bilinear position
   int* d_t_cols = nullptr;     // alpha-major position -> beta id
@@ -619,7 +620,7 @@ struct qpgpu_ctx {
   bool profile = false;
   std::vector<std::pair<std::string, cudaEvent_t>> marks;
 
-  double* h_pin = nullptr;  // pinned staging of the Davidson's small copies
+  double* h_pin = nullptr;  // pinned staging of small copies (qp_pin)
   size_t h_pin_doubles = 0;
   int* d_flag = nullptr;  // NaN / Inf flag of the host-array entry points
   void* d_tc_scratch = nullptr;  // qpgpu_gram_tc: per-CTA partials, exponents, status
@@ -724,15 +725,21 @@ int qp_sigma_ff(qpgpu_ctx* c, SigmaItems* it, double* v, double* s, const double
                 int row_lo, int row_hi, int row_first, int row_step);
 // FP32 row length that keeps a row of n_st coefficients in one 32-byte sector
 inline int qp_pad_states(int nst) { return nst <= 1 ? 1 : nst <= 2 ? 2 : nst <= 4 ? 4 : 8; }
-// bad (optional, device int): set to 1 when an input coefficient is not finite
-void qp_to_bilinear(const double* u0, int64_t ld, const int* order, double* ut, float* ut32, int nst, int64_t N,
+// Determinant order (columns ld apart) -> bilinear rows and back; pos is the
+// bilinear position of each determinant.  bad (optional, readable by the
+// device): set to 1 when an input coefficient is not finite.  ut (of an even
+// n_st) and ut32 (of 4 or 8 states) are 16-byte aligned.
+void qp_to_bilinear(const double* u0, int64_t ld, const int* pos, double* ut, float* ut32, int nst, int64_t N,
                     cudaStream_t st, int* bad = nullptr);
 void qp_flag_nonfinite(const double* x, int64_t n, int* bad, cudaStream_t st);
 // device flag of the context for the NaN / Inf checks of host-array entry
 // points (allocated on first use), cleared on stream st
 int qp_numeric_flag(qpgpu_ctx* c, cudaStream_t st, int** flag);
-void qp_from_bilinear(const double* vt, int64_t ld, const int* order, double* v0, int nst, int64_t N,
-                      cudaStream_t st);
+// (optionally a second array, with the same leading dimension, in one launch)
+void qp_from_bilinear(const double* vt, int64_t ld, const int* pos, double* v0, int nst, int64_t N,
+                      cudaStream_t st, const double* wt = nullptr, double* w0 = nullptr);
+// at least n doubles of the context's pinned staging in *p
+int qp_pin(qpgpu_ctx* c, size_t n, double** p);
 void qp_to_float(const double* x, float* y, int64_t N, int nst, int ld, cudaStream_t st);
 
 // records a named event on the context stream when profiling is on

@@ -55,31 +55,42 @@ __device__ __forceinline__ bool row_selected(const SigArgs& a, int k) {
 
 using namespace qpsig;
 
-// write the reduced state sums (lane L holds state L >> shift) and the diagonal
+// write the reduced state sums (lane L holds state L >> shift) and the
+// diagonal: of each state's lanes the first does v, the second s, in one FP64
+// instruction
 template <int NST>
 __device__ __forceinline__ void store_row(const SigArgs& a, int64_t it, int k, int lane, double hv, double sv,
                                           bool has_s2) {
   constexpr int SH = 5 - Pow2<NST>::lg;
-  const int st = lane >> SH;
-  const bool owner = (lane & ((1 << SH) - 1)) == 0 && st < NST;
-  if (!owner) return;
+  const int st = lane >> SH, sub = lane & ((1 << SH) - 1);
+  if (sub > 1 || st >= NST) return;
+  const double sum = sub == 0 ? hv : has_s2 ? sv : 0.0;
   if (a.row_nitems[k] == 1) {
-    const double uk = a.u[(int64_t)k * NST + st];
-    a.v[(int64_t)k * NST + st] = hv + a.hdiag[k] * uk;
-    a.s[(int64_t)k * NST + st] = (has_s2 ? sv : 0.0) + a.sdiag[k] * uk;
+    const double d = __ldg(sub == 0 ? &a.hdiag[k] : &a.sdiag[k]);
+    (sub == 0 ? a.v : a.s)[(int64_t)k * NST + st] = fma(d, a.u[(int64_t)k * NST + st], sum);
   } else {
-    a.pv[it * NST + st] = hv;
-    a.ps[it * NST + st] = has_s2 ? sv : 0.0;
+    (sub == 0 ? a.pv : a.ps)[it * NST + st] = sum;
   }
 }
 
 
 
-constexpr int UNR = 2;    // FP64 sigma: pairs per lane per loop trip (FP64-pipe bound)
+constexpr int UNR = 4;    // FP64 sigma: pairs per lane per loop trip
 constexpr int UNR32 = 4;  // FP32 sigma: more independent loads in flight (latency bound)
 
+// FP64 sigma.  From 3 states on it is bound by the FP64 pipe: an instruction of
+// a warp takes 64 cycles of its scheduler's pipe, against one for the integer
+// work beside it, so what is not a product is kept off the pipe (empty groups
+// of the last trip, conversions of the +-1 of S^2, zeros added in its
+// reduction, a second instruction for the diagonal).  With fewer states the
+// gathers' latency bounds it, hence four pairs in flight per lane and
+// registers for 5 or 6 blocks of an SM.  1e6 determinants x 4 states: 7.42 ->
+// 7.27 ms; 2e5 x 1, 2, 3, 4, 8: 287, 390, 512, 626, 1161 -> 244, 359, 489,
+// 608, 1142 us.  (256-bit gathers, rows of 3 and 5-7 states padded for them,
+// changed that by -1 to +3 percent; six pairs in flight or 8 blocks gain
+// nothing but at 2 states.)
 template <int NST>
-__global__ void __launch_bounds__(SBLK) k_sigma64(SigArgs a) {
+__global__ void __launch_bounds__(SBLK, NST == 1 ? 6 : 5) k_sigma64(SigArgs a) {
   constexpr int NP = Pow2<NST>::v;
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * SBLK + threadIdx.x) >> 5;
@@ -94,39 +105,13 @@ __global__ void __launch_bounds__(SBLK) k_sigma64(SigArgs a) {
     double acc[NP];
 #pragma unroll
     for (int st = 0; st < NP; ++st) acc[st] = 0.0;
-    for (int64_t e0 = beg + lane; e0 < end; e0 += 32 * UNR) {
-      int col[UNR];
-      double hv[UNR];
-#pragma unroll
-      for (int q = 0; q < UNR; ++q) {
-        const int64_t e = e0 + 32 * q;
-        col[q] = e < end ? __ldg(&a.colidx[e]) : k;
-        hv[q] = e < end ? __ldg(&a.val64[e]) : 0.0;
-      }
-#pragma unroll
-      for (int q = 0; q < UNR; ++q) {
-        double x[NST];
-        load_row<NST>(a.u, col[q], x);
-#pragma unroll
-        for (int st = 0; st < NST; ++st) acc[st] = fma(hv[q], x[st], acc[st]);
-      }
-    }
+    sum_pairs64<NST, NP, UNR>(a.u, a.colidx, a.val64, beg, end, k, lane, acc);
     const double hsum = reduce_scatter64<NP>(acc, lane);
     double ssum = 0.0;
     const int64_t sb = a.s2ptr[k], se = a.s2ptr[k + 1];
     const bool has_s2 = (j == 0) && (se > sb);
     if (has_s2) {
-      double sacc[NP];
-#pragma unroll
-      for (int st = 0; st < NP; ++st) sacc[st] = 0.0;
-      for (int64_t e = sb + lane; e < se; e += 32) {
-        const double sv = (double)__ldg(&a.s2val[e]);
-        double x[NST];
-        load_row<NST>(a.u, __ldg(&a.s2col[e]), x);
-#pragma unroll
-        for (int st = 0; st < NST; ++st) sacc[st] = fma(sv, x[st], sacc[st]);
-      }
-      ssum = reduce_scatter64<NP>(sacc, lane);
+      ssum = s2_row_sum<NST, NP>(a.u, a.s2col, a.s2val, sb, se, lane);
     }
     store_row<NST>(a, it, k, lane, hsum, ssum, has_s2);
   }
@@ -265,8 +250,8 @@ __global__ void k_sigma_combine(SigArgs a, const int* multi_rows, const int* row
       as += a.ps[(int64_t)(i0 + i) * nst + st];
     }
     const double uk = a.u[(int64_t)k * nst + st];
-    a.v[(int64_t)k * nst + st] = av + a.hdiag[k] * uk;
-    a.s[(int64_t)k * nst + st] = as + a.sdiag[k] * uk;
+    a.v[(int64_t)k * nst + st] = fma(a.hdiag[k], uk, av);
+    a.s[(int64_t)k * nst + st] = fma(a.sdiag[k], uk, as);
   }
 }
 
@@ -293,31 +278,71 @@ __global__ void k_fill_items(const int* nit, const int* item0, const int* split0
   }
 }
 
-// bad (optional): set to 1 when an input coefficient is NaN or infinite
-template <class T>
-__global__ void k_to_bilinear(const T* u0, int64_t ld, const int* order, double* ut, float* ut32, int nst,
-                              int64_t N, int* bad) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < N * nst; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = t / nst;
-    const int st = (int)(t % nst);
-    const double x = (double)u0[(int64_t)st * ld + order[p]];
-    if (bad && !isfinite(x)) *bad = 1;
-    if (ut) ut[t] = x;
-    if (ut32) ut32[t] = (float)x;
+// A thread per determinant d: the columns are read and written in order, and
+// the row of d at its position is one or two 32-byte sectors of the L2 (with a
+// thread per value in bilinear order each column access moved a sector for 8
+// bytes: 30 and 2 x 42 us at 1e6 x 4, now 15 and 28 us).
+// bad (optional): set to 1 when an input coefficient is NaN or infinite.
+template <int NST>
+__global__ void k_to_bilinear(const double* u0, int64_t ld, const int* pos, double* ut, float* ut32, int64_t N,
+                              int* bad) {
+  for (int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; d < N; d += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = pos[d];
+    double x[NST];
+#pragma unroll
+    for (int st = 0; st < NST; ++st) x[st] = u0[(int64_t)st * ld + d];
+    if (bad) {
+      bool fin = true;
+#pragma unroll
+      for (int st = 0; st < NST; ++st) fin = fin && isfinite(x[st]);
+      if (!fin) *bad = 1;
+    }
+    double* const r = ut + p * NST;
+    if constexpr (NST % 2 == 0) {
+#pragma unroll
+      for (int st = 0; st < NST; st += 2) *reinterpret_cast<double2*>(r + st) = make_double2(x[st], x[st + 1]);
+    } else {
+#pragma unroll
+      for (int st = 0; st < NST; ++st) r[st] = x[st];
+    }
+    if (!ut32) continue;
+    float* const r32 = ut32 + p * NST;
+    if constexpr (NST % 4 == 0) {
+#pragma unroll
+      for (int st = 0; st < NST; st += 4)
+        *reinterpret_cast<float4*>(r32 + st) =
+            make_float4((float)x[st], (float)x[st + 1], (float)x[st + 2], (float)x[st + 3]);
+    } else {
+#pragma unroll
+      for (int st = 0; st < NST; ++st) r32[st] = (float)x[st];
+    }
+  }
+}
+
+template <int NST>
+__global__ void k_from_bilinear(const double* vt, const double* wt, int64_t ld, const int* pos, double* v0,
+                                double* w0, int64_t N) {
+  for (int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; d < N; d += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = pos[d];
+    double x[NST], y[NST];
+#pragma unroll
+    for (int st = 0; st < NST; ++st) x[st] = vt[p * NST + st];
+    if (wt) {
+#pragma unroll
+      for (int st = 0; st < NST; ++st) y[st] = wt[p * NST + st];
+    }
+#pragma unroll
+    for (int st = 0; st < NST; ++st) v0[(int64_t)st * ld + d] = x[st];
+    if (wt) {
+#pragma unroll
+      for (int st = 0; st < NST; ++st) w0[(int64_t)st * ld + d] = y[st];
+    }
   }
 }
 
 __global__ void k_nonfinite(const double* x, int64_t n, int* bad) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     if (!isfinite(x[i])) *bad = 1;
-}
-
-__global__ void k_from_bilinear(const double* vt, int64_t ld, const int* order, double* v0, int nst, int64_t N) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < N * nst; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = t / nst;
-    const int st = (int)(t % nst);
-    v0[(int64_t)st * ld + order[p]] = vt[t];
-  }
 }
 
 // y (N rows of ld floats) <- x (N rows of nst doubles)
@@ -512,14 +537,25 @@ void launch_any(const SigArgs& a, int nst, int precision, unsigned grid, cudaStr
 
 // Times every FP32 launch shape on this determinant set (two launches each,
 // the second timed with events on the caller's stream) and keeps the fastest
-// for n_st.  Runs once per determinant set and n_st, on the first FP32 call;
-// the outputs it writes are those of the call itself.
-int tune_sigma32(qpgpu_ctx* c, SigmaItems* it, const SigArgs& a, int nst, cudaStream_t st, int slot) {
+// for n_st.  Runs once per determinant set and n_st, on the first FP32 call,
+// whose own launch follows.  A stretch of an eighth of the work items is
+// enough to tell the shapes apart (of all of them where they are few): over
+// all the items the choice cost 8 sigmas, 9.3 of the 11.3 ms of a first call
+// at 5e5 determinants x 8 states.
+int tune_sigma32(qpgpu_ctx* c, SigmaItems* it, const SigArgs& all, int nst, cudaStream_t st, int slot) {
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
     cudaGetLastError();
     return qpgpu_fail(c, QPGPU_ERR_CUDA, "cudaEventCreate failed while tuning the FP32 sigma");
   }
+  SigArgs a = all;
+  const int64_t n = std::min<int64_t>(all.n_items, std::max<int64_t>(all.n_items / 8, 1 << 16));
+  const int64_t first = (all.n_items - n) / 2;
+  a.n_items = n;
+  a.item_row += first;
+  a.item_sub += first;
+  a.pv += first * nst;
+  a.ps += first * nst;
   int best = 0;
   float best_ms = 1e30f;
   for (int v = 0; v < kNSig32Shapes; ++v) {
@@ -649,18 +685,34 @@ int qp_sigma_launch(qpgpu_ctx* c, SigmaItems* it, double* v, double* s, const do
   return 0;
 }
 
-void qp_to_bilinear(const double* u0, int64_t ld, const int* order, double* ut, float* ut32, int nst, int64_t N,
+#define QP_PER_NST(nst, CALL)  \
+  switch (nst) {               \
+    case 1: CALL(1); break;    \
+    case 2: CALL(2); break;    \
+    case 3: CALL(3); break;    \
+    case 4: CALL(4); break;    \
+    case 5: CALL(5); break;    \
+    case 6: CALL(6); break;    \
+    case 7: CALL(7); break;    \
+    case 8: CALL(8); break;    \
+  }
+
+void qp_to_bilinear(const double* u0, int64_t ld, const int* pos, double* ut, float* ut32, int nst, int64_t N,
                     cudaStream_t st, int* bad) {
-  k_to_bilinear<double><<<gsz(N * nst, 256), 256, 0, st>>>(u0, ld, order, ut, ut32, nst, N, bad);
+#define QP_TO(NS) k_to_bilinear<NS><<<gsz(N, 128), 128, 0, st>>>(u0, ld, pos, ut, ut32, N, bad)
+  QP_PER_NST(nst, QP_TO)
+#undef QP_TO
 }
 
 void qp_flag_nonfinite(const double* x, int64_t n, int* bad, cudaStream_t st) {
   k_nonfinite<<<gsz(n, 256), 256, 0, st>>>(x, n, bad);
 }
 
-void qp_from_bilinear(const double* vt, int64_t ld, const int* order, double* v0, int nst, int64_t N,
-                      cudaStream_t st) {
-  k_from_bilinear<<<gsz(N * nst, 256), 256, 0, st>>>(vt, ld, order, v0, nst, N);
+void qp_from_bilinear(const double* vt, int64_t ld, const int* pos, double* v0, int nst, int64_t N,
+                      cudaStream_t st, const double* wt, double* w0) {
+#define QP_FROM(NS) k_from_bilinear<NS><<<gsz(N, 128), 128, 0, st>>>(vt, wt, ld, pos, v0, w0, N)
+  QP_PER_NST(nst, QP_FROM)
+#undef QP_FROM
 }
 
 int qp_sigma_ff(qpgpu_ctx* c, SigmaItems* it, double* v, double* s, const double* u, int nst, cudaStream_t st,

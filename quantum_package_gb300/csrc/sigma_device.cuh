@@ -32,6 +32,33 @@ __device__ __forceinline__ double reduce_scatter64(double (&acc)[NSTP], int lane
   return x;
 }
 
+// The same for values that only lanes 0..n-1 hold, +0 in the others (n >= 1,
+// the same in all lanes).  In a round that joins lanes off >= n apart one side
+// of each addition is that +0, so the bits are merged instead: an FP64
+// addition takes the warp 64 cycles of its scheduler's FP64 pipe.
+template <int NSTP>
+__device__ __forceinline__ double reduce_scatter64_few(double (&acc)[NSTP], int lane, int n) {
+  int off = 16;
+#pragma unroll
+  for (int m = NSTP; m > 1; m >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < m / 2; ++i) {
+      const double send = up ? acc[i] : acc[i + m / 2];
+      const double keep = up ? acc[i + m / 2] : acc[i];
+      const double got = __shfl_xor_sync(0xffffffffu, send, off);
+      acc[i] = off >= n ? __longlong_as_double(__double_as_longlong(keep) | __double_as_longlong(got)) : keep + got;
+    }
+  }
+  double x = acc[0];
+#pragma unroll
+  for (; off > 0; off >>= 1) {
+    const double got = __shfl_xor_sync(0xffffffffu, x, off);
+    x = off >= n ? __longlong_as_double(__double_as_longlong(x) | __double_as_longlong(got)) : x + got;
+  }
+  return x;
+}
+
 // Float-float (hi + lo) form of a double, built with integer and FP32
 // instructions only: hi keeps the top 24 bits of the significand
 // (truncated), lo the next 23 (the last 6 bits, below 2^-46 |x|, are
@@ -186,5 +213,70 @@ __device__ __forceinline__ void load_row_ld(const float* u, int64_t col, float (
   }
 }
 
+
+// acc[st] += sum over the pairs [beg, end) of a row chunk, UNR x 32 pairs a
+// trip; groups of 32 past the end are left out, lanes past it multiply the
+// row's own coefficients by 0.
+template <int NST, int NP, int UNR>
+__device__ __forceinline__ void sum_pairs64(const double* u, const int* colidx, const double* val, int64_t beg,
+                                            int64_t end, int k, int lane, double (&acc)[NP]) {
+  int64_t b = beg;
+  for (; b + 32 * (UNR - 1) < end; b += 32 * UNR) {
+    int col[UNR];
+    double hv[UNR];
+#pragma unroll
+    for (int q = 0; q < UNR; ++q) {
+      const int64_t e = b + 32 * q + lane;
+      const bool in = q < UNR - 1 || e < end;
+      col[q] = in ? __ldg(&colidx[e]) : k;
+      hv[q] = in ? __ldg(&val[e]) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < UNR; ++q) {
+      double x[NST];
+      load_row<NST>(u, col[q], x);
+#pragma unroll
+      for (int st = 0; st < NST; ++st) acc[st] = fma(hv[q], x[st], acc[st]);
+    }
+  }
+  for (; b < end; b += 32) {
+    const int64_t e = b + lane;
+    const bool in = e < end;
+    const int col = in ? __ldg(&colidx[e]) : k;
+    const double hv = in ? __ldg(&val[e]) : 0.0;
+    double x[NST];
+    load_row<NST>(u, col, x);
+#pragma unroll
+    for (int st = 0; st < NST; ++st) acc[st] = fma(hv, x[st], acc[st]);
+  }
+}
+
+// Sum over the spin-flip list [sb, se) (not empty) of a row: the elements are
+// +-1, so a term is the coefficient with its sign changed by an integer
+// instruction and the lane's first term is no addition at all.  Most rows have
+// a handful of partners, and then (reduce_scatter64_few) a few additions
+// are all that the FP64 pipe sees.
+template <int NST, int NP>
+__device__ __forceinline__ double s2_row_sum(const double* u, const int* s2col, const float* s2val, int64_t sb,
+                                             int64_t se, int lane) {
+  double acc[NP];
+#pragma unroll
+  for (int st = 0; st < NP; ++st) acc[st] = 0.0;
+  for (int64_t e0 = sb; e0 < se; e0 += 32) {
+    const int64_t e = e0 + lane;
+    double x[NST];
+#pragma unroll
+    for (int st = 0; st < NST; ++st) x[st] = 0.0;
+    if (e < se) {
+      const long long flip = (long long)(__float_as_uint(__ldg(&s2val[e])) & 0x80000000u) << 32;
+      load_row<NST>(u, __ldg(&s2col[e]), x);
+#pragma unroll
+      for (int st = 0; st < NST; ++st) x[st] = __longlong_as_double(__double_as_longlong(x[st]) ^ flip);
+    }
+#pragma unroll
+    for (int st = 0; st < NST; ++st) acc[st] = e0 == sb ? x[st] : acc[st] + x[st];
+  }
+  return reduce_scatter64_few<NP>(acc, lane, (int)(se - sb < 32 ? se - sb : 32));
+}
 
 }  // namespace qpsig
