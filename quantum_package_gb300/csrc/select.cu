@@ -37,9 +37,13 @@
 // kept transposed: one bit per selector for each virtual orbital and each k.
 // An entry finds its connected selectors with a few AND / OR per 32 selectors
 // and visits those alone.  Testing every selector against every entry
-// instead bound the kernel by integer issue: the call over 8 generators,
-// 2,000 selectors and 10.1M entries (14a+14b in 80 MOs) took 18.8 ms and
-// takes 12.5 ms this way.
+// instead bound the kernel by integer issue: over 8 generators, 2,000
+// selectors and 10.1M entries (14a+14b in 80 MOs) it ran 18.4 ms.  It takes
+// 3.8 ms with these masks, the work split evenly over the CTAs, three of them
+// resident on an SM and the FP64 instructions of the energies that depend on
+// one particle only shared by an item's entries; what is left is the latency
+// of the elements' integrals (1.7 ms), the staging of the selectors and the
+// lanes that wait for the entry with the most of them.
 //
 // Banned determinants.  a is dropped when it is in the wave function
 // (device hash set of psi_det) or within a double excitation of an earlier
@@ -71,6 +75,9 @@ constexpr int SEL_DTILE = 256;     // selectors staged per pass (one word of 32 
 constexpr int SEL_DWORDS = SEL_DTILE / 32;
 static_assert(SEL_DWORDS == SBLK / 32 && SBLK <= SEL_DTILE, "each warp transposes one word of staged selectors");
 constexpr int SEL_MAXST = 8;       // states
+constexpr int SEL_MQ = 128;        // single-excitation elements a warp evaluates ahead
+constexpr int SEL_MG = 4;          // entries per lane they are collected from
+static_assert(SEL_DTILE <= 256 && SEL_MG <= 8, "codes of 3 + 5 + 8 bits");
 constexpr int SEL_MAXFG = 2048;    // earlier generators kept per item in shared memory (else read from the global list)
 
 enum { IT_SINGLE = 0, IT_SAME = 1, IT_AB = 2 };
@@ -82,6 +89,7 @@ struct SelItem {
   int spin;      // single / same-spin double: 0 alpha, 1 beta
   int h1, h2;    // holes (1-based); alpha-beta: h1 alpha, h2 beta
   int e0, e1;    // entry range
+  int part;      // its place in pt2_part (generators in order)
 };
 
 struct SelArgs {
@@ -99,7 +107,7 @@ struct SelArgs {
   const double* fock;        // per listed generator: build_fock_tmp, [gl][2][n_mo + 2]
   const int* hslot;          // hash set of psi_det: det index or -1
   uint64_t hmask;
-  double* pt2_part;          // [item][n_st]
+  double* pt2_part;          // [part][n_st]
   unsigned long long* n_ext;
   unsigned long long* n_cand;
   uint64_t cap;
@@ -303,24 +311,21 @@ __device__ __forceinline__ void tri_decode(int e, int& i1, int& i2) {
   i1 = e - j * (j - 1) / 2;
 }
 
+// bit c of lane r -> bit r of lane c
+__device__ __forceinline__ unsigned transpose32(unsigned x, int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned lo = o == 16 ? 0x0000ffffu : o == 8 ? 0x00ff00ffu : o == 4 ? 0x0f0f0f0fu : o == 2 ? 0x33333333u
+                                                                                                   : 0x55555555u;
+    const unsigned y = __shfl_xor_sync(0xffffffffu, x, o);
+    x = lane & o ? (x & ~lo) | ((y >> o) & lo) : (x & lo) | ((y & lo) << o);
+  }
+  return x;
+}
+
+// the generator without the item's holes
 template <int NINT>
-__global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
-  extern __shared__ double tile[];  // [entry - e0][n_st]
-  __shared__ u64 sdet[SEL_DTILE][2 * NINT];
-  __shared__ int sidx[SEL_DTILE];
-  __shared__ unsigned char sk[SEL_DTILE];
-  __shared__ unsigned shas[SEL_DWORDS][2][QPGPU_MAX_MO];  // staged selectors that hold a virtual orbital of g
-  __shared__ unsigned skm[SEL_DWORDS][3];                 // staged selectors with k = 0, 1, 2
-  __shared__ int vir[2][QPGPU_MAX_MO];
-  __shared__ int nvir[2];
-  __shared__ int fgen[SEL_MAXFG];
-  __shared__ int nfg;
-  __shared__ int wsum[SBLK / 32];
-  const SelItem it = A.items[blockIdx.x];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nst = A.n_st, n = A.t.n;
-  const u64* gd = A.dets + (int64_t)it.g * 2 * NINT;
-  u64 mask[2 * NINT];
+__device__ __forceinline__ void item_mask(const SelItem& it, const u64* gd, u64* mask) {
 #pragma unroll
   for (int w = 0; w < 2 * NINT; ++w) mask[w] = gd[w];
   if (it.kind == IT_SINGLE) {
@@ -332,6 +337,64 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
     set_orb<NINT>(mask, 0, it.h1, false);
     set_orb<NINT>(mask, 1, it.h2, false);
   }
+}
+
+// Work of an item, in matrix elements: with k electrons of the mask missing, a
+// selector is connected to every entry (k = 0; singles also k = 1), to those
+// that hold one of its three electrons outside the mask (k = 1) or to a few
+// (k = 2).  An entry's energy counts as ENTRY_COST elements.  One warp per
+// item.
+constexpr double ENTRY_COST = 2.5, LIST_COST = 1.5;
+template <int NINT>
+__global__ void __launch_bounds__(SBLK) k_sel_weigh(SelArgs A, int64_t n_items, float* weight) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t i = (blockIdx.x * (int64_t)SBLK + threadIdx.x) >> 5; i < n_items; i += ((int64_t)gridDim.x * SBLK) >> 5) {
+    const SelItem it = A.items[i];
+    u64 mask[2 * NINT];
+    item_mask<NINT>(it, A.dets + (int64_t)it.g * 2 * NINT, mask);
+    int n0 = 0, n1 = 0, n2 = 0;
+    const int64_t i1 = A.ilist_off[it.gl + 1];
+    for (int64_t q = A.ilist_off[it.gl] + lane; q < i1; q += 32) {
+      const u64* D = A.dets + (int64_t)A.ilist[q] * 2 * NINT;
+      int k = 0;
+#pragma unroll
+      for (int w = 0; w < 2 * NINT; ++w) k += popc64(mask[w] & ~__ldg(&D[w]));
+      n0 += k == 0;
+      n1 += k == 1;
+      n2 += k == 2;
+    }
+    n0 = __reduce_add_sync(0xffffffffu, n0);
+    n1 = __reduce_add_sync(0xffffffffu, n1);
+    n2 = __reduce_add_sync(0xffffffffu, n2);
+    if (lane == 0) {
+      const float ne = (float)(it.e1 - it.e0);
+      const float near = it.kind == IT_SINGLE ? ne : fminf(ne, 3.0f * (float)A.t.n);
+      weight[i] = ne * ((float)n0 + (float)ENTRY_COST) + (float)n1 * near + 4.0f * (float)n2;
+    }
+  }
+}
+
+template <int NINT>
+__global__ void __launch_bounds__(SBLK, 3) k_sel_items(SelArgs A) {
+  extern __shared__ double tile[];  // [entry - e0][n_st]
+  __shared__ u64 sdet[SEL_DTILE][2 * NINT];
+  __shared__ int sidx[SEL_DTILE];
+  __shared__ unsigned char sk[SEL_DTILE];
+  __shared__ unsigned shas[SEL_DWORDS][2][QPGPU_MAX_MO];  // staged selectors that hold an orbital
+  __shared__ unsigned skm[SEL_DWORDS][3];                 // staged selectors with k = 0, 1, 2
+  __shared__ int vir[2][QPGPU_MAX_MO];
+  __shared__ int nvir[2];
+  __shared__ int fgen[SEL_MAXFG];
+  __shared__ int nfg;
+  __shared__ int wsum[SBLK / 32];
+  __shared__ double mono_h[SBLK / 32][SEL_MQ];
+  __shared__ unsigned short mono_c[SBLK / 32][SEL_MQ];
+  const SelItem it = A.items[blockIdx.x];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nst = A.n_st, n = A.t.n;
+  const u64* gd = A.dets + (int64_t)it.g * 2 * NINT;
+  u64 mask[2 * NINT];
+  item_mask<NINT>(it, gd, mask);
   if (tid < 2) {
     int c = 0;
     for (int o = 1; o <= n; ++o)
@@ -362,7 +425,7 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
   const int sp1 = it.kind == IT_AB ? 0 : it.spin;  // spin of particle 1
   const int sp2 = it.kind == IT_AB ? 1 : it.spin;  // spin of particle 2
   const bool two = it.kind != IT_SINGLE;
-  // positions of an entry's particles in vir[sp1], vir[sp2]
+  // an entry's particles: their positions in vir[sp1], vir[sp2] and the orbitals
   auto entry = [&](int e, int& v1, int& v2) {
     if (it.kind == IT_SINGLE) {
       v1 = e;
@@ -374,6 +437,12 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
       v1 = e / nb;
       v2 = e - v1 * nb;
     }
+  };
+  auto particles = [&](int e, int& p1, int& p2) {
+    int v1, v2;
+    entry(e, v1, v2);
+    p1 = vir[sp1][v1];
+    p2 = two ? vir[sp2][v2] : 0;
   };
   const int64_t i0 = A.ilist_off[it.gl], i1 = A.ilist_off[it.gl + 1];
   int64_t base = i0;
@@ -419,22 +488,16 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
     __syncthreads();
     const int nw = (ns + 31) >> 5;
     // transposed tile: warp w turns selectors 32 w .. 32 w + 31 into one word
-    // per virtual orbital and one per k
+    // per orbital and one per k
     if (warp < nw) {
       const int j = warp * 32 + lane;
       const bool live = j < ns;
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        u64 x[NINT];
-#pragma unroll
-        for (int w = 0; w < NINT; ++w) x[w] = live ? sdet[j][s * NINT + w] : 0ull;
-        for (int v = 0; v < nvir[s]; ++v) {
-          const int o = vir[s][v] - 1;
-          u64 xw = x[0];
-          if (NINT == 2 && o >= 64) xw = x[NINT - 1];
-          const unsigned bal = __ballot_sync(0xffffffffu, (xw >> (o & 63)) & 1ull);
-          if (lane == 0) shas[warp][s][v] = bal;
-        }
+      for (int c = 0; c < 2 * 2 * NINT; ++c) {  // 32 orbitals each
+        const int sp = c / (2 * NINT), part = c % (2 * NINT);
+        if (part * 32 >= n) continue;
+        const u64 x = live ? sdet[j][sp * NINT + part / 2] : 0ull;
+        shas[warp][sp][part * 32 + lane] = transpose32((unsigned)(part & 1 ? x >> 32 : x), lane);
       }
       const int k = live ? sk[j] : 3;
 #pragma unroll
@@ -446,54 +509,152 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
     __syncthreads();
     // every thread: its entries against their connected selectors, in order.
     // deg = k + [p1 not in D] + [p2 not in D] is 1 or 2 for 32 selectors at a
-    // time (deg 0: a = D, in the wave function)
-    for (int e = tid; e < ne; e += SBLK) {
-      int v1, v2;
-      entry(it.e0 + e, v1, v2);
-      u64 a[2 * NINT];
+    // time (deg 0: a = D, in the wave function).  The few single excitations
+    // (deg 1) are sums over all electrons, whose dozens of FP64 instructions
+    // cost a warp the same for one lane as for 32: the warp collects those of
+    // its next SEL_MG x 32 entries first and evaluates them side by side.
+    auto words = [&](int w, int p1, int p2, unsigned& deg1, unsigned& deg12) {
+      const unsigned h1 = shas[w][sp1][p1 - 1], h2 = two ? shas[w][sp2][p2 - 1] : 0xffffffffu;
+      const unsigned k0 = skm[w][0], k1 = skm[w][1];
+      deg1 = (k0 & (h1 ^ h2)) | (k1 & h1 & h2);
+      deg12 = (k0 & ~(h1 & h2)) | (k1 & (h1 | h2)) | (skm[w][2] & h1 & h2);
+    };
+    auto external = [&](int p1, int p2, u64* a, u64* E) {
 #pragma unroll
       for (int w = 0; w < 2 * NINT; ++w) a[w] = mask[w];
-      set_orb<NINT>(a, sp1, vir[sp1][v1], true);
-      if (two) set_orb<NINT>(a, sp2, vir[sp2][v2], true);
-      u64 E[2 * NINT];
+      set_orb<NINT>(a, sp1, p1, true);
+      if (two) set_orb<NINT>(a, sp2, p2, true);
       det_parity<NINT>(a, E);
-      double* m = tile + (size_t)e * nst;
-      double m0 = m[0];
-      int w = -1;
-      unsigned bits = 0;
-      while (true) {
-        while (bits == 0 && ++w < nw) {
-          const unsigned h1 = shas[w][sp1][v1], h2 = two ? shas[w][sp2][v2] : 0xffffffffu;
-          bits = (skm[w][0] & ~(h1 & h2)) | (skm[w][1] & (h1 | h2)) | (skm[w][2] & h1 & h2);
+    };
+    for (int eb = warp * 32; eb < ne; eb += SEL_MG * SBLK) {
+      int n1 = 0;
+      for (int q = 0; q < SEL_MG; ++q) {
+        const int e = eb + q * SBLK + lane;
+        if (e >= ne) break;
+        int p1, p2;
+        particles(it.e0 + e, p1, p2);
+        for (int w = 0; w < nw; ++w) {
+          unsigned deg1, deg12;
+          words(w, p1, p2, deg1, deg12);
+          n1 += __popc(deg1);
         }
-        if (bits == 0) break;
-        const int j = w * 32 + __ffs(bits) - 1;
-        bits &= bits - 1;
-        u64 Dw[2 * NINT];
-#pragma unroll
-        for (int x = 0; x < 2 * NINT; ++x) Dw[x] = sdet[j][x];
-        const double h = ihj<NINT>(A.t, a, Dw, E);
-        const double* cD = A.coef + (int64_t)sidx[j] * nst;
-        m0 = fma(__ldg(&cD[0]), h, m0);
-        for (int s = 1; s < nst; ++s) m[s] = fma(__ldg(&cD[s]), h, m[s]);
       }
-      m[0] = m0;
+      int upto = n1;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += x;
+      }
+      const int n1_warp = min(__shfl_sync(0xffffffffu, upto, 31), SEL_MQ);
+      int at = upto - n1;
+      if (n1_warp > 0) {
+        int put = at;
+        for (int q = 0; n1 > 0 && q < SEL_MG; ++q) {
+          const int e = eb + q * SBLK + lane;
+          if (e >= ne) break;
+          int p1, p2;
+          particles(it.e0 + e, p1, p2);
+          for (int w = 0; w < nw; ++w) {
+            unsigned deg1, deg12;
+            words(w, p1, p2, deg1, deg12);
+            for (; deg1; deg1 &= deg1 - 1, ++put)
+              if (put < SEL_MQ)
+                mono_c[warp][put] = (unsigned short)((q << 13) | (lane << 8) | (w * 32 + __ffs(deg1) - 1));
+          }
+        }
+        __syncwarp();
+        for (int i = lane; i < n1_warp; i += 32) {
+          const int code = mono_c[warp][i];
+          int p1, p2;
+          particles(it.e0 + eb + (code >> 13) * SBLK + ((code >> 8) & 31), p1, p2);
+          u64 a[2 * NINT], E[2 * NINT], Dw[2 * NINT];
+          external(p1, p2, a, E);
+#pragma unroll
+          for (int x = 0; x < 2 * NINT; ++x) Dw[x] = sdet[code & 255][x];
+          bool beta = true;
+#pragma unroll
+          for (int x = 0; x < NINT; ++x) beta = beta && a[x] == Dw[x];
+          mono_h[warp][i] = h_mono_spin<NINT>(A.t, a, Dw, E, beta ? 2 : 1, nullptr, nullptr);
+        }
+        __syncwarp();
+      }
+      for (int q = 0; q < SEL_MG; ++q) {
+        const int e = eb + q * SBLK + lane;
+        if (e >= ne) break;
+        int p1, p2;
+        particles(it.e0 + e, p1, p2);
+        u64 a[2 * NINT], E[2 * NINT];
+        external(p1, p2, a, E);
+        double* m = tile + (size_t)e * nst;
+        double m0 = m[0];
+        int w = -1;
+        unsigned bits = 0, deg1 = 0;
+        while (true) {
+          while (bits == 0 && ++w < nw) words(w, p1, p2, deg1, bits);
+          if (bits == 0) break;
+          const unsigned b = bits & (0u - bits);
+          const int j = w * 32 + __ffs(bits) - 1;
+          bits ^= b;
+          const bool single = deg1 & b;
+          at += single;
+          double h;
+          if (single && at <= SEL_MQ) {
+            h = mono_h[warp][at - 1];
+          } else {
+            u64 Dw[2 * NINT];
+#pragma unroll
+            for (int x = 0; x < 2 * NINT; ++x) Dw[x] = sdet[j][x];
+            h = ihj<NINT>(A.t, a, Dw, E);
+          }
+          const double* cD = A.coef + (int64_t)sidx[j] * nst;
+          m0 = fma(__ldg(&cD[0]), h, m0);
+          for (int s = 1; s < nst; ++s) m[s] = fma(__ldg(&cD[s]), h, m[s]);
+        }
+        m[0] = m0;
+      }
+      __syncwarp();
     }
+    __syncthreads();
+  }
+  // diag_H_mat_elem_fock (slater_rules.irp.f:1800-1866), holes and particles
+  // ascending within a spin as decode_exc lists them: what depends on one
+  // particle only is summed once per item, in the same order
+  const int st = n + 2;
+  const double* F = A.fock + (int64_t)it.gl * 2 * st;
+  const double eg = F[n + 1];
+  double* const hp1 = mono_h[0];
+  double* const hp2 = mono_h[1];
+  double* const hq2 = mono_h[2];
+  static_assert(SEL_MQ >= QPGPU_MAX_MO, "the particles' shares take the place of the queue");
+  const double* pp = it.kind == IT_AB ? A.t.jj : A.t.ja;  // between the two spins of the item
+  {
+    const double* F1 = F + sp1 * st;
+    const double* F2 = F + sp2 * st;
+    const int h1 = it.h1, h2 = it.h2;  // same spin: h1 < h2, p1 < p2
+    for (int v = tid; v < nvir[sp1]; v += SBLK) {
+      const int p1 = vir[sp1][v];
+      double x = eg - F1[h1] + (F1[p1] - tab2(A.t.ja, n, h1, p1));
+      if (two) x = x - (F2[h2] - tab2(pp, n, h1, h2) + tab2(pp, n, p1, h2));
+      hp1[v] = x;
+    }
+    if (two)
+      for (int v = tid; v < nvir[sp2]; v += SBLK) {
+        const int p2 = vir[sp2][v];
+        hp2[v] = F2[p2] - tab2(pp, n, h1, p2);
+        hq2[v] = tab2(A.t.ja, n, h2, p2);
+      }
     __syncthreads();
   }
   // energies of this thread's entries
   double pt[SEL_MAXST];
 #pragma unroll
   for (int s = 0; s < SEL_MAXST; ++s) pt[s] = 0.0;
-  const int st = n + 2;
-  const double* F = A.fock + (int64_t)it.gl * 2 * st;
-  const double eg = F[n + 1];
   unsigned long long next = 0;
   for (int e = tid; e < ne; e += SBLK) {
     const double* m = tile + (size_t)e * nst;
-    double sabs = 0.0;
-    for (int s = 0; s < nst; ++s) sabs += fabs(m[s]);
-    if (sabs == 0.0) continue;
+    unsigned long long any = 0;
+    for (int s = 0; s < nst; ++s) any |= (unsigned long long)__double_as_longlong(m[s]) << 1;
+    if (any == 0) continue;
     int v1, v2;
     entry(it.e0 + e, v1, v2);
     const int p1 = vir[sp1][v1], p2 = two ? vir[sp2][v2] : 0;
@@ -511,26 +672,8 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
     }
     if (banned) continue;
     ++next;
-    // diag_H_mat_elem_fock (slater_rules.irp.f:1800-1866); holes and
-    // particles ascending within a spin, as decode_exc lists them
-    double haa;
-    const double* Fa = F;
-    const double* Fb = F + st;
-    if (it.kind == IT_SINGLE) {
-      const double* Fs = it.spin ? Fb : Fa;
-      haa = eg - Fs[it.h1] + (Fs[p1] - tab2(A.t.ja, n, it.h1, p1));
-    } else if (it.kind == IT_SAME) {
-      const double* Fs = it.spin ? Fb : Fa;
-      const int h1 = it.h1, h2 = it.h2;  // h1 < h2, p1 < p2
-      haa = eg - Fs[h1] + (Fs[p1] - tab2(A.t.ja, n, h1, p1)) -
-            (Fs[h2] - tab2(A.t.ja, n, h1, h2) + tab2(A.t.ja, n, p1, h2)) +
-            (Fs[p2] - tab2(A.t.ja, n, h1, p2) + tab2(A.t.ja, n, p1, p2) - tab2(A.t.ja, n, h2, p2));
-    } else {
-      const int h1 = it.h1, h2 = it.h2;
-      haa = eg - Fa[h1] + (Fa[p1] - tab2(A.t.ja, n, h1, p1)) -
-            (Fb[h2] - tab2(A.t.jj, n, h1, h2) + tab2(A.t.jj, n, p1, h2)) +
-            (Fb[p2] - tab2(A.t.jj, n, h1, p2) + tab2(A.t.jj, n, p1, p2) - tab2(A.t.ja, n, h2, p2));
-    }
+    double haa = hp1[v1];
+    if (two) haa += (hp2[v2] + tab2(pp, n, p1, p2)) - hq2[v2];
     double mine = 0.0;
     for (int s = 0; s < nst; ++s) {
       const double delta = A.e0[s] - haa;
@@ -561,17 +704,17 @@ __global__ void __launch_bounds__(SBLK) k_sel_items(SelArgs A) {
   if (tid < nst) {
     double acc = 0.0;
     for (int x = 0; x < SBLK; ++x) acc += tile[x * nst + tid];
-    A.pt2_part[(int64_t)blockIdx.x * nst + tid] = acc;
+    A.pt2_part[(int64_t)it.part * nst + tid] = acc;
   }
 }
 
-// pt2[s] = sum over items: one CTA per state, strided partial sums combined in
+// pt2[s] = sum over units: one CTA per state, strided partial sums combined in
 // thread order (one thread walking 3,248 items waited 193 us on its loads)
-__global__ void __launch_bounds__(SBLK) k_sel_pt2(const double* part, int64_t n_items, int nst, double* pt2) {
+__global__ void __launch_bounds__(SBLK) k_sel_pt2(const double* part, int64_t n_units, int nst, double* pt2) {
   __shared__ double red[SBLK];
   const int s = blockIdx.x;
   double acc = 0.0;
-  for (int64_t i = threadIdx.x; i < n_items; i += SBLK) acc += part[i * nst + s];
+  for (int64_t i = threadIdx.x; i < n_units; i += SBLK) acc += part[i * nst + s];
   red[threadIdx.x] = acc;
   __syncthreads();
   for (int o = SBLK / 2; o > 0; o >>= 1) {
@@ -629,7 +772,6 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   QP_CUDA(c, cudaStreamSynchronize(st));
   const int tile_entries = SEL_TILE / n_st;
   std::vector<SelItem> items;
-  std::vector<int64_t> item_first(n_list + 1);
   auto push = [&](SelItem it, int ne) {
     for (int a = 0; a < ne; a += tile_entries) {
       it.e0 = a;
@@ -638,7 +780,6 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
     }
   };
   for (int l = 0; l < n_list; ++l) {
-    item_first[l] = (int64_t)items.size();
     const int g = gens[l];
     std::vector<int> occ[2];
     for (int s = 0; s < 2; ++s)
@@ -646,15 +787,14 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
         if ((gdet[(size_t)l * 2 * nint + s * nint + ((o - 1) >> 6)] >> ((o - 1) & 63)) & 1ull) occ[s].push_back(o);
     const int nv[2] = {n - (int)occ[0].size(), n - (int)occ[1].size()};
     for (int s = 0; s < 2; ++s)
-      for (int h : occ[s]) push(SelItem{g, l, IT_SINGLE, s, h, 0, 0, 0}, nv[s]);
+      for (int h : occ[s]) push(SelItem{g, l, IT_SINGLE, s, h, 0, 0, 0, 0}, nv[s]);
     for (int s = 0; s < 2; ++s)
       for (size_t x = 0; x < occ[s].size(); ++x)
         for (size_t y = x + 1; y < occ[s].size(); ++y)
-          push(SelItem{g, l, IT_SAME, s, occ[s][x], occ[s][y], 0, 0}, nv[s] * (nv[s] - 1) / 2);
+          push(SelItem{g, l, IT_SAME, s, occ[s][x], occ[s][y], 0, 0, 0}, nv[s] * (nv[s] - 1) / 2);
     for (int ha : occ[0])
-      for (int hb : occ[1]) push(SelItem{g, l, IT_AB, 0, ha, hb, 0, 0}, nv[0] * nv[1]);
+      for (int hb : occ[1]) push(SelItem{g, l, IT_AB, 0, ha, hb, 0, 0, 0}, nv[0] * nv[1]);
   }
-  item_first[n_list] = (int64_t)items.size();
   const int64_t n_items = (int64_t)items.size();
   for (int s = 0; s < n_st; ++s) pt2[s] = 0.0;
   if (n_ext) *n_ext = 0;
@@ -665,11 +805,12 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   }
   // device arrays
   Dev d_items{c}, d_gens{c}, d_coef{c}, d_e0{c}, d_icnt{c}, d_ioff{c}, d_ilist{c}, d_fcnt{c}, d_foff{c};
-  Dev d_flist{c}, d_fock{c}, d_slot{c}, d_part{c}, d_cnt{c}, d_err{c}, d_pt2{c};
+  Dev d_flist{c}, d_fock{c}, d_slot{c}, d_part{c}, d_cnt{c}, d_err{c}, d_pt2{c}, d_wgt{c}, d_units{c};
   uint64_t hcap = 1;
   while (hcap < (uint64_t)(2 * N)) hcap <<= 1;
   QP_CUDA(c, qp_pool_alloc(c, &d_items.p, items.size() * sizeof(SelItem)));
   QP_CUDA(c, cudaMemcpyAsync(d_items.p, items.data(), items.size() * sizeof(SelItem), cudaMemcpyHostToDevice, st));
+  QP_CUDA(c, qp_pool_alloc(c, &d_wgt.p, items.size() * sizeof(float)));
   QP_CUDA(c, qp_pool_alloc(c, &d_gens.p, n_list * sizeof(int)));
   QP_CUDA(c, cudaMemcpyAsync(d_gens.p, gens.data(), n_list * sizeof(int), cudaMemcpyHostToDevice, st));
   // coefficients: column-major (N, n_st) on the host -> (N, n_st) row-major
@@ -689,7 +830,6 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   QP_CUDA(c, qp_pool_alloc(c, &d_err.p, sizeof(int)));
   QP_CUDA(c, cudaMemsetAsync(d_err.p, 0, sizeof(int), st));
   QP_CUDA(c, qp_pool_alloc(c, &d_pt2.p, n_st * sizeof(double)));
-  QP_CUDA(c, qp_pool_alloc(c, &d_part.p, (size_t)n_items * n_st * sizeof(double)));
   const u64* dets = c->d_dets;
   const int* dg = (const int*)d_gens.p;
   const int hb = (int)std::min<int64_t>((N + 255) / 256, (int64_t)c->n_sm * 8);
@@ -733,7 +873,7 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   A.e0 = (const double*)d_e0.p;
   A.n_st = n_st;
   A.N = N;
-  A.items = (const SelItem*)d_items.p;
+  A.items = (const SelItem*)d_items.p;  // the items are weighed, then split into units
   A.ilist_off = (const int64_t*)d_ioff.p;
   A.ilist = (const int*)d_ilist.p;
   A.flist_off = (const int64_t*)d_foff.p;
@@ -741,14 +881,68 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   A.fock = (const double*)d_fock.p;
   A.hslot = (const int*)d_slot.p;
   A.hmask = hcap - 1;
-  A.pt2_part = (double*)d_part.p;
   A.n_ext = (unsigned long long*)d_cnt.p;
   A.n_cand = (unsigned long long*)d_cnt.p + 1;
   A.err = (int*)d_err.p;
-  // dynamic shared memory: the largest item's numerator tile (at least the
+#define QP_SEL_WEIGH(NI)                                                                                           \
+  k_sel_lists<NI><<<n_list, SBLK, 0, st>>>(dets, dg, n_list, n_sel, 0, 1, nullptr, (const int64_t*)d_ioff.p,       \
+                                           (int*)d_ilist.p);                                                       \
+  k_sel_lists<NI><<<n_list, SBLK, 0, st>>>(dets, dg, n_list, n_sel, 1, 1, nullptr, (const int64_t*)d_foff.p,       \
+                                           (int*)d_flist.p);                                                       \
+  k_sel_weigh<NI><<<(unsigned)((n_items + 7) / 8), SBLK, 0, st>>>(A, n_items, (float*)d_wgt.p);
+  if (nint == 1) {
+    QP_SEL_WEIGH(1)
+  } else {
+    QP_SEL_WEIGH(2)
+  }
+#undef QP_SEL_WEIGH
+  QP_CUDA(c, cudaGetLastError());
+  std::vector<float> wgt(items.size());
+  QP_CUDA(c, cudaMemcpyAsync(wgt.data(), d_wgt.p, items.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
+  QP_CUDA(c, cudaStreamSynchronize(st));
+  // Units: an item whose work is above the share of a CTA is split by entries
+  // (in multiples of SPLIT_ENTRIES), and the heaviest units start first.  The
+  // work differs by up to a hundred times between items: the call of the
+  // header's example ran 8.0 ms with one CTA per item in their order, the last
+  // percent of them alone in the second half of that, and 6.1 ms this way.  A
+  // share is at least several times what the staging of a CTA costs; 3, 4, 6
+  // and 12 shares per resident CTA took 4.4, 3.8, 3.9 and 4.3 ms.
+  constexpr int SPLIT_ENTRIES = SBLK / 2, SHARES = 4;
+  double work = 0.0;
+  for (float w : wgt) work += w;
+  const double staging = LIST_COST * (double)ioff[n_list] / n_list;
+  const double share = std::max(work / ((double)c->n_sm * 3 * SHARES), 4.0 * staging);
+  std::vector<SelItem> units;
+  std::vector<float> uw;
+  std::vector<int64_t> unit_first(n_list + 1, 0);
+  for (size_t i = 0; i < items.size(); ++i) {
+    SelItem it = items[i];
+    const int ne = it.e1 - it.e0, blocks = (ne + SPLIT_ENTRIES - 1) / SPLIT_ENTRIES;
+    const int parts = (int)std::min<double>(std::ceil(wgt[i] / share), blocks);
+    const int step = parts <= 1 ? ne : (blocks + parts - 1) / parts * SPLIT_ENTRIES;
+    for (int a = 0; a < ne; a += step) {
+      it.e0 = items[i].e0 + a;
+      it.e1 = std::min(items[i].e1, it.e0 + step);
+      it.part = (int)units.size();
+      units.push_back(it);
+      uw.push_back(wgt[i] * (float)(it.e1 - it.e0) / (float)ne);
+    }
+    unit_first[it.gl + 1] = (int64_t)units.size();
+  }
+  for (int l = 0; l < n_list; ++l) unit_first[l + 1] = std::max(unit_first[l + 1], unit_first[l]);
+  const int64_t n_units = (int64_t)units.size();
+  std::sort(units.begin(), units.end(), [&](const SelItem& x, const SelItem& y) {
+    return uw[x.part] != uw[y.part] ? uw[x.part] > uw[y.part] : x.part < y.part;
+  });
+  QP_CUDA(c, qp_pool_alloc(c, &d_units.p, n_units * sizeof(SelItem)));
+  QP_CUDA(c, cudaMemcpyAsync(d_units.p, units.data(), n_units * sizeof(SelItem), cudaMemcpyHostToDevice, st));
+  QP_CUDA(c, qp_pool_alloc(c, &d_part.p, (size_t)n_units * n_st * sizeof(double)));
+  A.items = (const SelItem*)d_units.p;
+  A.pt2_part = (double*)d_part.p;
+  // dynamic shared memory: the largest unit's numerator tile (at least the
   // SBLK x n_st doubles of the final reduction), so that several CTAs fit an SM
   int max_ne = 0;
-  for (const SelItem& it : items) max_ne = std::max(max_ne, it.e1 - it.e0);
+  for (const SelItem& it : units) max_ne = std::max(max_ne, it.e1 - it.e0);
   const size_t smem = (size_t)std::max(max_ne * n_st, SBLK * n_st) * sizeof(double);
   unsigned long long hcnt[2] = {0, 0};
   for (int attempt = 0; attempt < 2; ++attempt) {
@@ -762,12 +956,8 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
     A.cand_det = (u64*)d_cdet.p;
     QP_CUDA(c, cudaMemsetAsync(d_cnt.p, 0, 2 * sizeof(unsigned long long), st));
 #define QP_SEL_RUN(NI)                                                                                             \
-  k_sel_lists<NI><<<n_list, SBLK, 0, st>>>(dets, dg, n_list, n_sel, 0, 1, nullptr, (const int64_t*)d_ioff.p,       \
-                                           (int*)d_ilist.p);                                                       \
-  k_sel_lists<NI><<<n_list, SBLK, 0, st>>>(dets, dg, n_list, n_sel, 1, 1, nullptr, (const int64_t*)d_foff.p,       \
-                                           (int*)d_flist.p);                                                       \
   QP_CUDA(c, cudaFuncSetAttribute(k_sel_items<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));       \
-  k_sel_items<NI><<<(unsigned)n_items, SBLK, smem, st>>>(A);
+  k_sel_items<NI><<<(unsigned)n_units, SBLK, smem, st>>>(A);
     if (nint == 1) {
       QP_SEL_RUN(1)
     } else {
@@ -780,16 +970,16 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
     if (buf_size == 0 || hcnt[1] <= cap) break;
     cap = hcnt[1];  // every candidate counted: run once more with room for all of them
   }
-  k_sel_pt2<<<n_st, SBLK, 0, st>>>((const double*)d_part.p, n_items, n_st, (double*)d_pt2.p);
+  k_sel_pt2<<<n_st, SBLK, 0, st>>>((const double*)d_part.p, n_units, n_st, (double*)d_pt2.p);
   QP_CUDA(c, cudaMemcpyAsync(pt2, d_pt2.p, n_st * sizeof(double), cudaMemcpyDeviceToHost, st));
   if (per_gen) {
-    std::vector<double> part((size_t)n_items * n_st);
+    std::vector<double> part((size_t)n_units * n_st);
     QP_CUDA(c, cudaMemcpyAsync(part.data(), d_part.p, part.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     QP_CUDA(c, cudaStreamSynchronize(st));
     for (int l = 0; l < n_list; ++l)
       for (int s = 0; s < n_st; ++s) {
         double acc = 0.0;
-        for (int64_t i = item_first[l]; i < item_first[l + 1]; ++i) acc += part[(size_t)i * n_st + s];
+        for (int64_t i = unit_first[l]; i < unit_first[l + 1]; ++i) acc += part[(size_t)i * n_st + s];
         per_gen[(size_t)l * n_st + s] = acc;
       }
   }

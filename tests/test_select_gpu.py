@@ -157,3 +157,37 @@ def test_select_many_generators_per_item():
     e0 = np.array([-10.0])  # below every H_aa of this space: all denominators of one sign
     _compare(wf.select_pt2(c, e0, nd, nd, 300), o.select_pt2(c, e0, nd, nd, 300))
     wf.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_mo,n_st,n_gen", [(40, 1, 2), (67, 2, 1)])  # one and two words, few generators
+def test_select_split_items(n_mo, n_st, n_gen):
+    # all singles and many doubles of one reference: most selectors reach every
+    # entry of an item, so the items are split over several blocks (128 entries
+    # each at least) and a warp meets more single excitations than it evaluates
+    # ahead (128); the last generators' own holes give entries that nearly
+    # every selector is connected to
+    from quantum_package_gb300.sigma import Wavefunction
+    ne = 5
+    ints = G.make_integrals(n_mo, 31)
+    rng = np.random.default_rng(n_mo)
+    ref = (1 << ne) - 1
+    words = {(ref, ref)}
+    one = [ref ^ (1 << i) ^ (1 << a) for i in range(ne) for a in range(ne, n_mo)]
+    words |= {(x, ref) for x in one} | {(ref, x) for x in one}
+    while len(words) < 900:
+        x, y = rng.integers(len(one), size=2)
+        words.add((one[x], one[y]))
+    words = sorted(words, key=lambda w: (w != (ref, ref), bin(w[0] & ref).count("1") + bin(w[1] & ref).count("1"), w))
+    rest = [words[i] for i in 1 + rng.permutation(len(words) - 1)]
+    n_int = (n_mo - 1) // 64 + 1
+    dets = np.array([[[(s >> (64 * k)) & (2**64 - 1) for k in range(n_int)] for s in w]
+                     for w in [(ref, ref)] + rest], dtype=np.uint64)
+    n = len(dets)
+    c = rng.normal(size=(n_st, n)) * np.exp(-np.arange(n) / 200.0)
+    e0 = -np.arange(60.0, 60.0 + n_st)  # below every H_aa of this space
+    o = Oracle(n_mo, ne, ne, ints.h, ints.eri, dets)
+    wf = Wavefunction(n_mo, ne, ne, ints.h, ints.eri, dets)
+    n_sel = 700
+    _compare(wf.select_pt2(c, e0, n_gen, n_sel, 400), o.select_pt2(c, e0, n_gen, n_sel, 400))
+    wf.close()
