@@ -219,7 +219,7 @@ size_t qp_pool_cached(qpgpu_ctx* c) {
 void qp_pool_trim(qpgpu_ctx* c) {
   uint64_t used = 0;
   if (cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return;
-  const uint64_t spare = std::max<uint64_t>(used / 2, 64ull << 20);
+  const uint64_t spare = std::max<uint64_t>(used / 2, 256ull << 20);
   if (qp_pool_cached(c) > spare) cudaMemPoolTrimTo(c->pool, (size_t)(used + spare));
 }
 

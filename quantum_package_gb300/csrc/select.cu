@@ -112,7 +112,7 @@ struct SelArgs {
   unsigned long long* n_cand;
   uint64_t cap;
   double* cand_val;
-  u64* cand_det;             // (2 nint) per candidate
+  uint64_t* cand_at;         // its unit (high 32 bits) and entry
   int* err;
 };
 
@@ -691,8 +691,7 @@ __global__ void __launch_bounds__(SBLK, 3) k_sel_items(SelArgs A) {
     slot = __shfl_sync(grp, slot, __ffs(grp) - 1) + __popc(grp & ((1u << lane) - 1));
     if (slot < A.cap) {
       A.cand_val[slot] = mine;
-#pragma unroll
-      for (int w = 0; w < 2 * NINT; ++w) A.cand_det[slot * 2 * NINT + w] = a[w];
+      A.cand_at[slot] = (uint64_t)blockIdx.x << 32 | (unsigned)(it.e0 + e);
     }
   }
   if (next) atomicAdd(A.n_ext, next);
@@ -725,21 +724,115 @@ __global__ void __launch_bounds__(SBLK) k_sel_pt2(const double* part, int64_t n_
 }
 
 // ascending order of doubles as unsigned keys
-__global__ void k_sel_keys(const double* v, uint64_t n, unsigned long long* key, long long* idx) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v[i]);
-    key[i] = (b >> 63) ? ~b : (b | (1ull << 63));
-    idx[i] = (long long)i;
+__device__ __forceinline__ unsigned long long sel_key(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return (b >> 63) ? ~b : (b | (1ull << 63));
+}
+
+// The buffer holds a few of millions of candidates.  Two histograms of 12 key
+// bits each find the key prefix up to which at least `want` of them lie, and
+// only those are sorted (sorting all 10.1M took 0.85 ms and 320 MB).
+constexpr int SEL_BINS = 4096;
+struct SelCut {
+  unsigned long long want, below, prefix, upto;  // below: candidates before the prefix; upto: with it
+};
+
+__global__ void __launch_bounds__(SBLK) k_sel_hist(const double* v, uint64_t n, int level, const SelCut* cut,
+                                                   unsigned long long* hist) {
+  __shared__ unsigned h[SEL_BINS];
+  for (int i = threadIdx.x; i < SEL_BINS; i += SBLK) h[i] = 0;
+  __syncthreads();
+  const unsigned long long prefix = level ? cut->prefix : 0;
+  for (uint64_t i = blockIdx.x * (uint64_t)SBLK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * SBLK) {
+    const unsigned long long k = sel_key(v[i]);
+    if (level == 0)
+      atomicAdd(&h[k >> 52], 1u);
+    else if ((k >> 52) == prefix)
+      atomicAdd(&h[(k >> 40) & (SEL_BINS - 1)], 1u);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < SEL_BINS; i += SBLK)
+    if (h[i]) atomicAdd(&hist[i], (unsigned long long)h[i]);
+}
+
+// one block: the first bin that reaches `want`
+__global__ void __launch_bounds__(1024) k_sel_pick(const unsigned long long* hist, int level, SelCut* cut) {
+  __shared__ unsigned long long part[1024];
+  constexpr int PER = SEL_BINS / 1024;
+  const int t = threadIdx.x;
+  unsigned long long mine = 0;
+  for (int i = 0; i < PER; ++i) mine += hist[t * PER + i];
+  part[t] = mine;
+  __syncthreads();
+  for (int o = 1; o < 1024; o <<= 1) {
+    const unsigned long long x = t >= o ? part[t - o] : 0;
+    __syncthreads();
+    part[t] += x;
+    __syncthreads();
+  }
+  const unsigned long long want = cut->want, below = level ? cut->below : 0, prefix = level ? cut->prefix : 0;
+  __syncthreads();
+  unsigned long long at = below + part[t] - mine;
+  if (at >= want || below + part[t] < want) return;  // one thread goes on
+  for (int i = 0; i < PER; ++i) {
+    const unsigned long long c = hist[t * PER + i];
+    if (at + c >= want) {
+      cut->below = at;
+      cut->prefix = prefix << 12 | (unsigned)(t * PER + i);
+      cut->upto = at + c;
+      return;
+    }
+    at += c;
   }
 }
 
-// the head of the sorted candidates, contiguous
-__global__ void k_sel_gather(const long long* idx, uint64_t take, const double* cval, const u64* cdet, int w2,
-                             double* vals, u64* dets) {
+// keys and numbers of the candidates up to the cut (of all, without one)
+__global__ void k_sel_keys(const double* v, uint64_t n, const SelCut* cut, unsigned long long* key, uint64_t* idx,
+                           unsigned long long* count) {
+  const unsigned long long last = cut ? cut->prefix : 0;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const unsigned long long k = sel_key(v[i]);
+    uint64_t o = i;
+    if (cut) {
+      if ((k >> 40) > last) continue;
+      o = atomicAdd(count, 1ull);
+    }
+    key[o] = k;
+    idx[o] = i;
+  }
+}
+
+// the head of the sorted candidates, contiguous, as determinants
+template <int NINT>
+__global__ void k_sel_gather(const uint64_t* idx, uint64_t take, const double* cval, const uint64_t* cat,
+                             const SelItem* units, const u64* gens, int n_mo, double* vals, u64* out) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < take; i += (uint64_t)gridDim.x * blockDim.x) {
-    const long long j = idx[i];
+    const uint64_t j = idx[i];
     vals[i] = cval[j];
-    for (int w = 0; w < w2; ++w) dets[i * w2 + w] = cdet[j * w2 + w];
+    const SelItem it = units[cat[j] >> 32];
+    const int e = (int)(unsigned)cat[j];
+    const u64* g = gens + (int64_t)it.g * 2 * NINT;
+    u64 d[2 * NINT];
+    item_mask<NINT>(it, g, d);
+    // virtual orbital number v of the generator
+    auto vir = [&](int spin, int v) {
+      int o = 1;
+      for (;; ++o)
+        if (!has_orb(g, NINT, spin, o) && v-- == 0) break;
+      return o;
+    };
+    int v1 = e, v2 = 0;
+    if (it.kind == IT_SAME) {
+      tri_decode(e, v1, v2);
+    } else if (it.kind == IT_AB) {
+      int nb = n_mo;
+      for (int w = 0; w < NINT; ++w) nb -= popc64(g[NINT + w]);
+      v1 = e / nb;
+      v2 = e - v1 * nb;
+    }
+    set_orb<NINT>(d, it.kind == IT_AB ? 0 : it.spin, vir(it.kind == IT_AB ? 0 : it.spin, v1), true);
+    if (it.kind != IT_SINGLE) set_orb<NINT>(d, it.kind == IT_AB ? 1 : it.spin, vir(it.kind == IT_AB ? 1 : it.spin, v2), true);
+    for (int w = 0; w < 2 * NINT; ++w) out[i * 2 * NINT + w] = d[w];
   }
 }
 
@@ -864,8 +957,8 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   // candidates (only when a buffer is asked for): at most one per entry
   uint64_t ub = 0;
   for (const SelItem& it : items) ub += (uint64_t)(it.e1 - it.e0);
-  uint64_t cap = buf_size > 0 ? std::min<uint64_t>(ub, 1ull << 28) : 0;  // <= 10.7 GB of candidates
-  Dev d_cval{c}, d_cdet{c};
+  uint64_t cap = buf_size > 0 ? std::min<uint64_t>(ub, 1ull << 28) : 0;  // <= 4.3 GB of candidates
+  Dev d_cval{c}, d_cat{c};
   SelArgs A{};
   A.t = c->tab;
   A.dets = dets;
@@ -947,13 +1040,13 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   unsigned long long hcnt[2] = {0, 0};
   for (int attempt = 0; attempt < 2; ++attempt) {
     qp_pool_free(c, d_cval.p);
-    qp_pool_free(c, d_cdet.p);
-    d_cval.p = d_cdet.p = nullptr;
+    qp_pool_free(c, d_cat.p);
+    d_cval.p = d_cat.p = nullptr;
     QP_CUDA(c, qp_pool_alloc(c, &d_cval.p, std::max<uint64_t>(1, cap) * sizeof(double)));
-    QP_CUDA(c, qp_pool_alloc(c, &d_cdet.p, std::max<uint64_t>(1, cap) * 2 * nint * sizeof(u64)));
+    QP_CUDA(c, qp_pool_alloc(c, &d_cat.p, std::max<uint64_t>(1, cap) * sizeof(uint64_t)));
     A.cap = cap;
     A.cand_val = (double*)d_cval.p;
-    A.cand_det = (u64*)d_cdet.p;
+    A.cand_at = (uint64_t*)d_cat.p;
     QP_CUDA(c, cudaMemsetAsync(d_cnt.p, 0, 2 * sizeof(unsigned long long), st));
 #define QP_SEL_RUN(NI)                                                                                             \
   QP_CUDA(c, cudaFuncSetAttribute(k_sel_items<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));       \
@@ -989,36 +1082,65 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   if (nout > 0) {
     // sort by value on the device; the head (and any tie group crossing its
     // end) goes to the host, where equal values are put in determinant order
-    Dev kin{c}, kout{c}, vin{c}, vout{c}, tmp{c};
-    QP_CUDA(c, qp_pool_alloc(c, &kin.p, nc * 8));
-    QP_CUDA(c, qp_pool_alloc(c, &kout.p, nc * 8));
-    QP_CUDA(c, qp_pool_alloc(c, &vin.p, nc * 8));
-    QP_CUDA(c, qp_pool_alloc(c, &vout.p, nc * 8));
-    k_sel_keys<<<(unsigned)std::min<uint64_t>((nc + 255) / 256, (uint64_t)c->n_sm * 8), 256, 0, st>>>(
-        (const double*)d_cval.p, nc, (unsigned long long*)kin.p, (long long*)vin.p);
+    Dev kin{c}, kout{c}, vin{c}, vout{c}, tmp{c}, d_cut{c}, d_hist{c};
+    const unsigned grid = (unsigned)std::min<uint64_t>((nc + 255) / 256, (uint64_t)c->n_sm * 8);
+    // few candidates are sorted as they are: the cut costs 5 launches and a wait
+    const bool cut = nc >= (1u << 17) && (uint64_t)nout + 64 < nc / 8;
+    uint64_t m = nc;  // candidates to sort
+    if (cut) {
+      SelCut h{(unsigned long long)nout + 64, 0, 0, 0};
+      QP_CUDA(c, qp_pool_alloc(c, &d_cut.p, sizeof(SelCut)));
+      QP_CUDA(c, qp_pool_alloc(c, &d_hist.p, (2 * SEL_BINS + 1) * sizeof(unsigned long long)));
+      QP_CUDA(c, cudaMemcpyAsync(d_cut.p, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+      QP_CUDA(c, cudaMemsetAsync(d_hist.p, 0, (2 * SEL_BINS + 1) * sizeof(unsigned long long), st));
+      for (int level = 0; level < 2; ++level) {
+        unsigned long long* hist = (unsigned long long*)d_hist.p + level * SEL_BINS;
+        k_sel_hist<<<grid, SBLK, 0, st>>>((const double*)d_cval.p, nc, level, (const SelCut*)d_cut.p, hist);
+        k_sel_pick<<<1, 1024, 0, st>>>(hist, level, (SelCut*)d_cut.p);
+      }
+      QP_CUDA(c, cudaMemcpyAsync(&h, d_cut.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+      QP_CUDA(c, cudaStreamSynchronize(st));
+      m = h.upto;
+    }
+    QP_CUDA(c, qp_pool_alloc(c, &kin.p, m * 8));
+    QP_CUDA(c, qp_pool_alloc(c, &kout.p, m * 8));
+    QP_CUDA(c, qp_pool_alloc(c, &vin.p, m * 8));
+    QP_CUDA(c, qp_pool_alloc(c, &vout.p, m * 8));
+    k_sel_keys<<<grid, 256, 0, st>>>((const double*)d_cval.p, nc, cut ? (const SelCut*)d_cut.p : nullptr,
+                                     (unsigned long long*)kin.p, (uint64_t*)vin.p,
+                                     cut ? (unsigned long long*)d_hist.p + 2 * SEL_BINS : nullptr);
     size_t tb = 0;
     QP_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, tb, (unsigned long long*)kin.p, (unsigned long long*)kout.p,
-                                               (long long*)vin.p, (long long*)vout.p, (int64_t)nc, 0, 64, st));
+                                               (uint64_t*)vin.p, (uint64_t*)vout.p, (int64_t)m, 0, 64, st));
     QP_CUDA(c, qp_pool_alloc(c, &tmp.p, tb));
     QP_CUDA(c, cub::DeviceRadixSort::SortPairs(tmp.p, tb, (unsigned long long*)kin.p, (unsigned long long*)kout.p,
-                                               (long long*)vin.p, (long long*)vout.p, (int64_t)nc, 0, 64, st));
+                                               (uint64_t*)vin.p, (uint64_t*)vout.p, (int64_t)m, 0, 64, st));
     std::vector<unsigned long long> keys;
-    uint64_t take = std::min<uint64_t>(nc, (uint64_t)nout + 64);
+    uint64_t take = std::min<uint64_t>(m, (uint64_t)nout + 64);
     while (true) {  // grow the head until it ends past the tie group of entry nout - 1
       keys.resize(take);
       QP_CUDA(c, cudaMemcpyAsync(keys.data(), kout.p, take * 8, cudaMemcpyDeviceToHost, st));
       QP_CUDA(c, cudaStreamSynchronize(st));
-      if (take == nc || keys[take - 1] != keys[nout - 1]) break;
-      take = std::min<uint64_t>(nc, take * 2);
+      if (take == m || keys[take - 1] != keys[nout - 1]) break;
+      take = std::min<uint64_t>(m, take * 2);
     }
     std::vector<double> vals(take);
     std::vector<u64> dts(take * 2 * nint);
     Dev gv{c}, gd{c};
     QP_CUDA(c, qp_pool_alloc(c, &gv.p, take * sizeof(double)));
     QP_CUDA(c, qp_pool_alloc(c, &gd.p, take * 2 * nint * sizeof(u64)));
-    k_sel_gather<<<(unsigned)std::min<uint64_t>((take + 255) / 256, (uint64_t)c->n_sm * 8), 256, 0, st>>>(
-        (const long long*)vout.p, take, (const double*)d_cval.p, (const u64*)d_cdet.p, 2 * nint, (double*)gv.p,
-        (u64*)gd.p);
+    const unsigned ggrid = (unsigned)std::min<uint64_t>((take + 127) / 128, (uint64_t)c->n_sm * 8);
+#define QP_SEL_GATHER(NI)                                                                                           \
+  k_sel_gather<NI><<<ggrid, 128, 0, st>>>((const uint64_t*)vout.p, take, (const double*)d_cval.p,                   \
+                                          (const uint64_t*)d_cat.p, (const SelItem*)d_units.p, dets, n,             \
+                                          (double*)gv.p, (u64*)gd.p);
+    if (nint == 1) {
+      QP_SEL_GATHER(1)
+    } else {
+      QP_SEL_GATHER(2)
+    }
+#undef QP_SEL_GATHER
+    QP_CUDA(c, cudaGetLastError());
     QP_CUDA(c, cudaMemcpyAsync(vals.data(), gv.p, take * sizeof(double), cudaMemcpyDeviceToHost, st));
     QP_CUDA(c, cudaMemcpyAsync(dts.data(), gd.p, take * 2 * nint * sizeof(u64), cudaMemcpyDeviceToHost, st));
     QP_CUDA(c, cudaStreamSynchronize(st));
