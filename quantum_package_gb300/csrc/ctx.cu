@@ -486,9 +486,8 @@ int qpgpu_set_dets(qpgpu_ctx* c, const uint64_t* psi_det, int64_t n_det) {
     c->have_dets = true;
     rc = qp_build_pairs(c);
   }
-  if (rc == 0 && !c->direct) rc = qp_build_sigma_items(c, &c->items);
   if (rc == 0) rc = qp_det_features(c);
-  qp_mark(c, "sigma work items");
+  qp_mark(c, "determinant features");
   qp_report_marks(c);
   QP_CUDA(c, cudaEventRecord(e1, st));
   QP_CUDA(c, cudaEventSynchronize(e1));

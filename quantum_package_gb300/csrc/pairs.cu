@@ -36,6 +36,7 @@
 namespace {
 
 constexpr int BLK = 256;
+constexpr int SAME_BPS = 4, CLASS_C_BPS = 3;  // blocks of the scans resident on an SM, by their registers
 
 inline unsigned nblocks(int64_t n, int tpb) {
   int64_t g = (n + tpb - 1) / tpb;
@@ -86,7 +87,15 @@ struct BuildArgs {
   const int64_t* s2ptr;
   int* s2col;
   float* s2val;
-  float4* feat;         // .w: coupling strength of the row (learned step), or null
+  float4* feat;         // .w: coupling strength of the row (learned step)
+  // elements: work items (stretches of QP_SIGMA_CHUNK pairs of a row) and, for
+  // rows of several, each item's sum of squared elements
+  const int* row_nitems;
+  const int* row_item0;
+  const int* item_row;
+  const int* item_sub;
+  int64_t n_items;
+  double* item_sum2;
   const u64* det_pos;   // both strings at each bilinear position (2 NINT words)
   const u64* det_tpos;  // the same at each alpha-major position (direct sigma)
   int* err;  // set when a pass would write past its row's segment
@@ -153,7 +162,8 @@ __device__ __forceinline__ void for_rows(const BuildArgs& a, int lane, Row row) 
 // Writes the hits of one class of a row after the other.
 template <int MODE, int CLS>
 struct RowOut {
-  int64_t at = 0, room = 0;  // MODE_POOL: this warp's place in the pool and what is left of its chunk
+  int64_t at = 0, keep_at = 0;  // MODE_POOL: this warp's place in the pool and what is left of its chunk,
+  int room = 0, keep_room = 0;  // and the largest piece that the row in hand has outgrown
   int* dst = nullptr;
   int cnt = 0, cap = 0;
   __device__ __forceinline__ void begin(const BuildArgs& a, int64_t k) {
@@ -184,26 +194,44 @@ struct RowOut {
     cnt += n;
   }
   // a new chunk for a row that does not fit the rest of the current one: what
-  // the row has so far moves over
+  // the row has so far moves over, and the rows after it go on in the larger
+  // of what it leaves (given up, the pieces that the longest rows outgrew and
+  // the ends of theirs made the pool of a 1e5 or 2e5 set run full, so that the
+  // scans ran again: 0.9 of 7.2 and 1.6 of 13.5 ms)
   __device__ __forceinline__ void grow(const BuildArgs& a, int need, int lane) {
-    const int64_t size = max((int64_t)a.pool_chunk[CLS], 2 * (int64_t)need);
+    const int64_t size = min(max((int64_t)a.pool_chunk[CLS], 2 * (int64_t)need), (int64_t)INT_MAX);
     unsigned long long o = 0;
     if (lane == 0) o = atomicAdd(a.pool_next, (unsigned long long)size);
     o = __shfl_sync(0xffffffffu, o, 0);
     if (dst == nullptr || (int64_t)o + size > a.pool_cap) {  // full: go on counting
       if (lane == 0) *a.pool_full = 1;
+      if (dst) leave();
       dst = nullptr;
       at = 0;
-      room = INT64_MAX;
+      room = INT_MAX;
       return;
     }
+    leave();
     int* to = a.pool + o;
     __syncwarp();
-    for (int i = lane; i < cnt; i += 32) to[i] = dst[i];
+    for (int i0 = 0; i0 < cnt; i0 += 32 * 8) {
+      int x[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) x[q] = dst[min(i0 + 32 * q + lane, cnt - 1)];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (i0 + 32 * q + lane < cnt) to[i0 + 32 * q + lane] = x[q];
+    }
     __syncwarp();
     dst = to;
     at = (int64_t)o;
-    room = size;
+    room = (int)size;
+  }
+  __device__ __forceinline__ void leave() {
+    if (room > keep_room) {
+      keep_at = at;
+      keep_room = room;
+    }
   }
   __device__ __forceinline__ void end(const BuildArgs& a, int64_t k, int lane) {
     if (MODE == MODE_FILL) return;
@@ -216,6 +244,11 @@ struct RowOut {
       } else {
         room = 0;
       }
+      if (keep_room > room) {
+        at = keep_at;
+        room = keep_room;
+      }
+      keep_room = 0;
     }
   }
 };
@@ -239,8 +272,11 @@ __device__ __forceinline__ bool spin_flip(const u64* my, const u64* ca, const u6
 // row's alpha (beta) string with each electron removed, and the members of
 // each group are the alpha (beta) singles of the row in that column (row).
 template <int NINT, int MODE>
-__global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
+__global__ void __launch_bounds__(BLK, CLASS_C_BPS) k_class_c(BuildArgs a) {
   constexpr unsigned FULL = 0xffffffffu;
+  // steps of scanned candidates in flight (one: 0.55 instead of 0.42 ms at 1e5
+  // determinants, 19.5 instead of 19.2 at 1e6; four need two blocks of an SM: 21.2)
+  constexpr int CU = 2;
   const int lane = threadIdx.x & 31;
   RowOut<MODE, CLS_C> out;
   for_rows<MODE, CLS_C>(a, lane, [&](int64_t k) {
@@ -319,51 +355,54 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
         if (lane >= o) incl += y;
       }
       const int total = __shfl_sync(FULL, incl, 31);
-      for (int c0 = 0; c0 < total; c0 += 32) {
-        const int ci = c0 + lane;
-        int src = 0;  // first lane whose inclusive prefix exceeds ci
+      for (int c0 = 0; c0 < total; c0 += 32 * CU) {
+        int pos[CU], sln[CU];
+        u64 y[CU][NINT];  // the scanned strings: alpha of a column, beta of a row
 #pragma unroll
-        for (int st = 16; st > 0; st >>= 1) {
-          const int pr = __shfl_sync(FULL, incl, src + st - 1);
-          if (pr <= ci) src += st;
-        }
-        const int sbeg = __shfl_sync(FULL, beg, src), slen = __shfl_sync(FULL, len, src);
-        const int sinc = __shfl_sync(FULL, incl, src), sln = __shfl_sync(FULL, ln, src);
-        bool hit = false;
-        u64 ca[NINT], cb[NINT];
+        for (int q = 0; q < CU; ++q) {
+          const int ci = c0 + 32 * q + lane;
+          int src = 0;  // first lane whose inclusive prefix exceeds ci
 #pragma unroll
-        for (int w = 0; w < NINT; ++w) ca[w] = cb[w] = 0;
-        int col = 0;
-        if (ci < total) {
-          const int pos = sbeg + (ci - (sinc - slen));
-          int d = 0;
-          if (by_cols) {  // column sln (a beta single): alpha singles of the row
-#pragma unroll
-            for (int w = 0; w < NINT; ++w) {
-              ca[w] = a.alpha_pos[(int64_t)pos * NINT + w];
-              d += popc64(my[w] ^ ca[w]);
-            }
-            hit = d == 2;
-            if (hit) {
-#pragma unroll
-              for (int w = 0; w < NINT; ++w) cb[w] = a.beta[(int64_t)sln * NINT + w];
-              col = pos;
-            }
-          } else {  // row sln (an alpha single): beta singles of the row
-#pragma unroll
-            for (int w = 0; w < NINT; ++w) {
-              cb[w] = a.beta_tpos[(int64_t)pos * NINT + w];
-              d += popc64(my[NINT + w] ^ cb[w]);
-            }
-            hit = d == 2;
-            if (hit) {
-#pragma unroll
-              for (int w = 0; w < NINT; ++w) ca[w] = a.alpha[(int64_t)sln * NINT + w];
-              if (MODE != MODE_COUNT) col = a.tag_t ? (int)(QP_TAG_T | (unsigned)pos) : a.t_order[pos];
-            }
+          for (int st = 16; st > 0; st >>= 1) {
+            const int pr = __shfl_sync(FULL, incl, src + st - 1);
+            if (pr <= ci) src += st;
           }
+          const int sbeg = __shfl_sync(FULL, beg, src), slen = __shfl_sync(FULL, len, src);
+          const int sinc = __shfl_sync(FULL, incl, src);
+          sln[q] = __shfl_sync(FULL, ln, src);
+          pos[q] = ci < total ? sbeg + (ci - (sinc - slen)) : -1;
+          const u64* const str = (by_cols ? a.alpha_pos : a.beta_tpos) + (int64_t)max(pos[q], 0) * NINT;
+#pragma unroll
+          for (int w = 0; w < NINT; ++w) y[q][w] = str[w];
         }
-        step(hit, ca, cb, col);
+#pragma unroll
+        for (int q = 0; q < CU; ++q) {
+          if (c0 + 32 * q >= total) break;
+          int d = 0;
+#pragma unroll
+          for (int w = 0; w < NINT; ++w) d += popc64((by_cols ? my[w] : my[NINT + w]) ^ y[q][w]);
+          // column sln (a beta single): alpha singles of the row; row sln (an
+          // alpha single): beta singles of the row
+          const bool hit = pos[q] >= 0 && d == 2;
+          u64 ca[NINT], cb[NINT];
+#pragma unroll
+          for (int w = 0; w < NINT; ++w) ca[w] = cb[w] = 0;
+          int col = 0;
+          if (hit) {
+            const u64* const line = (by_cols ? a.beta : a.alpha) + (int64_t)sln[q] * NINT;
+#pragma unroll
+            for (int w = 0; w < NINT; ++w) {
+              const u64 z = line[w];
+              ca[w] = by_cols ? y[q][w] : z;
+              cb[w] = by_cols ? z : y[q][w];
+            }
+            if (by_cols)
+              col = pos[q];
+            else if (MODE != MODE_COUNT)
+              col = a.tag_t ? (int)(QP_TAG_T | (unsigned)pos[q]) : a.t_order[pos[q]];
+          }
+          step(hit, ca, cb, col);
+        }
       }
       unsigned kb = __ballot_sync(FULL, kl);
       while (kb) {
@@ -471,9 +510,16 @@ __global__ void __launch_bounds__(BLK, 3) k_class_c(BuildArgs a) {
 // each pair is accepted under exactly one key, whatever the hash collisions.
 // (A thread per row of a line staged in shared memory took 140 us for each
 // fill of a 5,000 determinant set, whose longest line gave 20 blocks work.)
+// A group of 64 members or more is read by itself, four steps in flight and
+// without the search for each member's group: the reference's row, one warp
+// whose groups are that long, bounds the scan (5.0 and 5.4 of 5.0 and 5.4 ms
+// at 1e6 determinants, now 3.6 and 4.0; 1.10 and 1.17 -> 0.80 and 0.71 at 2e5).
+// Groups from 32 or 128 on made no difference; registers for five blocks of an
+// SM spill (3.9 and 4.6 ms).
 template <int NINT, int MODE, int SPIN>
-__global__ void __launch_bounds__(BLK, 5) k_same(BuildArgs a) {
+__global__ void __launch_bounds__(BLK, SAME_BPS) k_same(BuildArgs a) {
   constexpr unsigned FULL = 0xffffffffu;
+  constexpr int GU = 4;  // steps of a large group in flight
   constexpr int kind = SPIN == 0 ? KT_COL2 : KT_ROW2;
   const int lane = threadIdx.x & 31;
   const KeyView kv = a.kv[kind];
@@ -510,6 +556,30 @@ __global__ void __launch_bounds__(BLK, 5) k_same(BuildArgs a) {
       out.end(a, k, lane);
       return;
     }
+    // the string at p is a partner of the row under key Kr
+    auto partner = [&](int p, const u64 (&Kr)[NINT]) {
+      u64 m[NINT];
+      int d = 0;
+#pragma unroll
+      for (int w = 0; w < NINT; ++w) {
+        const u64 y = strs[(int64_t)p * NINT + w];
+        d += popc64(x[w] ^ y);
+        m[w] = x[w] & y;
+      }
+      if (d == 2) {  // canonical key of a single: drop the lowest common electron
+        bool done = false;
+#pragma unroll
+        for (int w = 0; w < NINT; ++w)
+          if (!done && m[w]) {
+            m[w] &= m[w] - 1;
+            done = true;
+          }
+      }
+      bool eq = d == 2 || d == 4;
+#pragma unroll
+      for (int w = 0; w < NINT; ++w) eq &= m[w] == Kr[w];
+      return eq;
+    };
     for (int c0 = 0; c0 < nc; c0 += 32) {
       unsigned gs = 0, gl = 0;
       u64 K[NINT];
@@ -525,7 +595,37 @@ __global__ void __launch_bounds__(BLK, 5) k_same(BuildArgs a) {
         clear_orbital<NINT>(K, bj);
         if (!key_find(kv, key_hash<NINT>(kind, line, K, a.hmask), gs, gl)) gl = 0;
       }
-      // the members of the 32 probed groups, packed into full warp steps
+      // groups of two warp steps or more, one after the other: GU x 32 members
+      // a trip, whose loads are in flight together
+      unsigned large = __ballot_sync(FULL, gl >= 64);
+      while (large) {
+        const int L = __ffs(large) - 1;
+        large &= large - 1;
+        const int* mem = kv.mem + __shfl_sync(FULL, gs, L);
+        const int len = (int)__shfl_sync(FULL, gl, L);
+        u64 Kr[NINT];
+#pragma unroll
+        for (int w = 0; w < NINT; ++w) Kr[w] = __shfl_sync(FULL, K[w], L);
+        if (lane == L) gl = 0;
+        for (int t0 = 0; t0 < len; t0 += 32 * GU) {
+          int p[GU];
+          bool hit[GU];
+#pragma unroll
+          for (int q = 0; q < GU; ++q) {
+            const int t = t0 + 32 * q + lane;
+            p[q] = t < len ? mem[t] : -1;
+            if (t > 0 && t < len && mem[t - 1] == p[q]) p[q] = -1;  // repeated member
+          }
+#pragma unroll
+          for (int q = 0; q < GU; ++q) hit[q] = p[q] >= ls && p[q] < le && partner(p[q], Kr);
+#pragma unroll
+          for (int q = 0; q < GU; ++q) p[q] = hit[q] ? column(p[q]) : 0;
+#pragma unroll
+          for (int q = 0; q < GU; ++q)
+            if (t0 + 32 * q < len) out.put(a, hit[q], p[q], lane);
+        }
+      }
+      // the members of the other groups, packed into full warp steps
       int inc = (int)gl;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -552,31 +652,7 @@ __global__ void __launch_bounds__(BLK, 5) k_same(BuildArgs a) {
         if (mi < tot) {
           p = kv.mem[s0 + t];
           const bool dup = t > 0 && kv.mem[s0 + t - 1] == p;
-          if (!dup && p >= ls && p < le) {
-            u64 m[NINT];
-            int d = 0;
-#pragma unroll
-            for (int w = 0; w < NINT; ++w) {
-              const u64 y = strs[(int64_t)p * NINT + w];
-              d += popc64(x[w] ^ y);
-              m[w] = x[w] & y;
-            }
-            if (d == 2) {  // canonical key of a single: drop the lowest common electron
-              bool done = false;
-#pragma unroll
-              for (int w = 0; w < NINT; ++w)
-                if (!done && m[w]) {
-                  m[w] &= m[w] - 1;
-                  done = true;
-                }
-            }
-            if (d == 2 || d == 4) {
-              bool eq = true;
-#pragma unroll
-              for (int w = 0; w < NINT; ++w) eq &= m[w] == Kr[w];
-              hit = eq;
-            }
-          }
+          hit = !dup && p >= ls && p < le && partner(p, Kr);
         }
         out.put(a, hit, hit ? column(p) : 0, lane);
       }
@@ -874,25 +950,33 @@ __device__ __forceinline__ void load_det(const u64* det, int64_t p, u64 (&J)[2 *
 // the holes and particles against the reference take several times a double's
 // loads), and same-spin doubles where they are few in a trip, are deferred
 // until 32 of a kind are there (a row's own beta column is one run of its
-// ascending columns, whose trips take them at once).  The row's sum of squared elements gives the coupling feature of the learned
-// step (log10(sum_J H_IJ^2) / 4), which took a pass of its own (4.2 ms).
-// 991M pairs at 1e6 determinants: 30.8 -> 22.9 ms; bound by the integer
-// instructions of the Slater routines (about 400 a pair, 45 % issue) with the
-// L2 latency of the integrals.
+// ascending columns, whose trips take them at once).  The row's sum of squared
+// elements gives the coupling feature of the learned step
+// (log10(sum_J H_IJ^2) / 4), which took a pass of its own (4.2 ms).
+// A warp takes a stretch of QP_SIGMA_CHUNK pairs: with a warp per row the
+// reference's row, which holds up to a quarter of the determinants, ran on
+// when the others were done.  The next trip's partners are loaded ahead, for
+// which three blocks of an SM have registers (four without: 20.8 ms at 1e6).
+// 1e5 (60 MOs) / 2e5 / 1e6 determinants: 1.26 / 3.0 / 21.3 -> 0.70 / 1.75 /
+// 19.1 ms; bound by the integer instructions of the Slater routines (about 400
+// a pair, 45 % issue) with the L2 latency of the integrals.
+__device__ __forceinline__ float coupling_feature(double sum2) { return (float)(log10(sum2 + 1e-30) * 0.25); }
+
 template <int NINT>
-__global__ void __launch_bounds__(BLK, 4) k_pair_values(BuildArgs a) {
+__global__ void __launch_bounds__(BLK, 3) k_pair_values(BuildArgs a) {
   __shared__ int s_q[BLK / 32][2][DEFER];
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const int64_t warp = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5;
   const int64_t nwarp = ((int64_t)gridDim.x * BLK) >> 5;
   Deferred same{s_q[threadIdx.x >> 5][0], 0}, mono{s_q[threadIdx.x >> 5][1], 0};
-  for (int64_t k = warp; k < a.N; k += nwarp) {
+  for (int64_t it = warp; it < a.n_items; it += nwarp) {
+    const int k = a.item_row[it];
     u64 my[2 * NINT], E[2 * NINT];
     load_det<NINT>(a.det_pos, k, my);
     det_parity<NINT>(my, E);
-    const int64_t e0 = a.rowptr[k];
-    const int n = (int)(a.rowptr[k + 1] - e0);
+    const int64_t e0 = a.rowptr[k] + (int64_t)a.item_sub[it] * QP_SIGMA_CHUNK;
+    const int n = (int)min((int64_t)QP_SIGMA_CHUNK, a.rowptr[k + 1] - e0);
     double sum2 = 0.0;
     auto put = [&](int x, double v) {
       a.val64[e0 + x] = v;
@@ -932,13 +1016,20 @@ __global__ void __launch_bounds__(BLK, 4) k_pair_values(BuildArgs a) {
       return same_spin(x, J);
     };
     int j = lane < n ? a.colidx[e0 + lane] : -1;
+    int jn = lane + 32 < n ? a.colidx[e0 + lane + 32] : -1;
+    u64 Jn[2 * NINT];
+#pragma unroll
+    for (int w = 0; w < 2 * NINT; ++w) Jn[w] = 0;
+    if (j >= 0) load_det<NINT>(a.det_pos, j, Jn);
     for (int x0 = 0; x0 < n; x0 += 32) {
       const int x = x0 + lane;
-      const int jn = x + 32 < n ? a.colidx[e0 + x + 32] : -1;  // the next trip's column
+      const int jnn = x + 64 < n ? a.colidx[e0 + x + 64] : -1;  // two trips ahead
       bool is_same = false;
       u64 J[2 * NINT];
+#pragma unroll
+      for (int w = 0; w < 2 * NINT; ++w) J[w] = Jn[w];
+      if (jn >= 0) load_det<NINT>(a.det_pos, jn, Jn);
       if (j >= 0) {
-        load_det<NINT>(a.det_pos, j, J);
         bool samea = true, sameb = true;
 #pragma unroll
         for (int w = 0; w < NINT; ++w) {
@@ -956,17 +1047,31 @@ __global__ void __launch_bounds__(BLK, 4) k_pair_values(BuildArgs a) {
         if (mono.push(do_same(y), y, lt)) do_mono(mono.pop(lane));
       }
       j = jn;
+      jn = jnn;
     }
     {
       const int y = same.pop(lane);
       if (mono.push(do_same(y), y, lt)) do_mono(mono.pop(lane));
     }
     do_mono(mono.pop(lane));
-    if (a.feat) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
-      if (lane == 0) a.feat[k].w = (float)(log10(sum2 + 1e-30) * 0.25);
+    for (int o = 16; o > 0; o >>= 1) sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
+    if (lane == 0) {
+      if (a.row_nitems[k] == 1)
+        a.feat[k].w = coupling_feature(sum2);
+      else
+        a.item_sum2[it] = sum2;
     }
+  }
+}
+
+// the coupling feature of the rows of several items: their sums in item order
+__global__ void k_row_coupling(BuildArgs a, const int* multi_rows, int n) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int k = multi_rows[i];
+    double s = 0.0;
+    for (int j = 0; j < a.row_nitems[k]; ++j) s += a.item_sum2[a.row_item0[k] + j];
+    a.feat[k].w = coupling_feature(s);
   }
 }
 
@@ -1130,14 +1235,13 @@ int sort_row_columns(qpgpu_ctx* c, const BuildArgs& a) {
 }
 
 // the scans of all three classes; a pool pass runs as many blocks as are
-// resident (six per SM of the same-spin scans, three of the alpha x beta
-// one, by their registers)
+// resident
 template <int NINT, int MODE>
 void launch_scans(qpgpu_ctx* c, const BuildArgs& a) {
   cudaStream_t st = c->stream;
   const unsigned g = nblocks(c->N * 32, BLK);
-  const unsigned gs = MODE == MODE_POOL ? std::min(g, (unsigned)c->n_sm * 6) : g;
-  const unsigned gc = MODE == MODE_POOL ? std::min(g, (unsigned)c->n_sm * 3) : g;
+  const unsigned gs = MODE == MODE_POOL ? std::min(g, (unsigned)c->n_sm * SAME_BPS) : g;
+  const unsigned gc = MODE == MODE_POOL ? std::min(g, (unsigned)c->n_sm * CLASS_C_BPS) : g;
   k_same<NINT, MODE, 0><<<gs, BLK, 0, st>>>(a);
   qp_mark(c, "scan A (same beta)");
   k_same<NINT, MODE, 1><<<gs, BLK, 0, st>>>(a);
@@ -1178,16 +1282,18 @@ int build_pairs_t(qpgpu_ctx* c) {
     // room for as many pairs a row as the context's last set had (1,200 when
     // it had none; the bench system has 991 at 1e6 determinants), 0.3 of that
     // for what rows leave behind when they outgrow a chunk, and for the
-    // unfinished chunks of the warps; a pool that is too
-    // small costs its rows a second scan, one that would not fit beside the
-    // stored pairs is left out
+    // unfinished chunks of the warps; a pool that is too small costs its rows a
+    // second scan, one that would not fit beside the stored pairs is left out
     const double per_row = c->pairs_per_row > 0 ? c->pairs_per_row : 1200.0;
     const double est = per_row * (double)N;
-    // chunks: an eighth of a warp's share of about 0.3 / 0.3 / 0.6 of the pairs
+    // chunks: an eighth of a warp's share of about 0.3 / 0.3 / 0.6 of the
+    // pairs, but sixteen rows at least, as a row that does not fit the rest of
+    // a chunk takes another
     const int64_t all = nblocks(N * 32, BLK);
-    const int64_t ws = std::min<int64_t>(all, c->n_sm * 6) * (BLK / 32), wc = std::min<int64_t>(all, c->n_sm * 3) * (BLK / 32);
+    const int64_t ws = std::min<int64_t>(all, c->n_sm * SAME_BPS) * (BLK / 32);
+    const int64_t wc = std::min<int64_t>(all, c->n_sm * CLASS_C_BPS) * (BLK / 32);
     auto chunk_of = [&](double share, int64_t warps) {
-      return (int)std::min(65536.0, std::max(256.0, share * est / (8.0 * (double)warps)));
+      return (int)std::min(65536.0, std::max({256.0, share * est / (8.0 * (double)warps), 16.0 * share * per_row}));
     };
     a.pool_chunk[CLS_A] = a.pool_chunk[CLS_B] = chunk_of(0.3, ws);
     a.pool_chunk[CLS_C] = chunk_of(0.6, wc);
@@ -1306,7 +1412,20 @@ int build_pairs_t(qpgpu_ctx* c) {
   if (rc) return rc;
   qp_mark(c, "row columns sorted");
   pool.reset();
-  k_pair_values<NINT><<<nblocks(N * 32, BLK), BLK, 0, st>>>(a);
+  const int rci = qp_build_sigma_items(c, &c->items);
+  if (rci) return rci;
+  qp_mark(c, "sigma work items");
+  Scoped<double> sum2(c);
+  QP_CUDA(c, sum2.alloc((size_t)c->items.n_items));
+  a.row_nitems = c->items.row_nitems;
+  a.row_item0 = c->items.row_item0;
+  a.item_row = c->items.item_row;
+  a.item_sub = c->items.item_sub;
+  a.n_items = c->items.n_items;
+  a.item_sum2 = sum2.p;
+  k_pair_values<NINT><<<nblocks(a.n_items * 32, BLK), BLK, 0, st>>>(a);
+  if (c->items.n_multi > 0)
+    k_row_coupling<<<nblocks(c->items.n_multi, 256), 256, 0, st>>>(a, c->items.multi_rows, c->items.n_multi);
   qp_mark(c, "pair elements");
   QP_CUDA(c, cudaGetLastError());
   int herr = 0;

@@ -7,7 +7,9 @@ which the sort takes another path (a warp's registers, blocks of 2 to 16 warps,
 the segmented sort); a set whose hits do not fit the pool (sized from the
 context's previous set) gives the same pairs and sigma as a fresh context; a
 set replaced while a sigma of the old one is in flight on another stream leaves
-that sigma untouched.
+that sigma untouched.  Deletion-key groups of every length at which they are
+read another way, and rows that outgrow their chunks of the pool, give the
+oracle's pairs.
 """
 import ctypes as C
 
@@ -127,3 +129,47 @@ def test_set_replaced_under_a_running_sigma():
     wf.set_dets(q.dets)
     torch.cuda.synchronize()
     assert torch.equal(v, ref)
+
+
+def _all_pairs_match(wf, o):
+    I, J, cls = o.connected_pairs()
+    g = wf.connected_pairs()
+    np.testing.assert_array_equal(g["I"], I)
+    np.testing.assert_array_equal(g["J"], J)
+    np.testing.assert_array_equal(g["cls"], cls)
+    np.testing.assert_array_equal(g["hij"], o.pair_excitations(I, J, cls)[2])
+
+
+@pytest.mark.parametrize("spin", [0, 1])
+@pytest.mark.parametrize("n_mo,bits", [(30, 64), (70, 64), (30, 3)])
+@pytest.mark.parametrize("m", [62, 63, 64, 127, 128, 129, 200])
+def test_key_groups_of_every_length(m, n_mo, bits, spin):
+    """m strings that share a deletion key with the reference's: the group is read
+    in whole steps from 64 members on (m + 1 with the reference's own), four at a time."""
+    from quantum_package_gb300.sigma import Wavefunction
+    ne = 4
+    ref = G.reference_det(n_mo, ne, ne)
+    two = [(p, q) for p in range(ne, n_mo) for q in range(p + 1, n_mo)]
+    pick = np.random.default_rng(m).permutation(len(two))[:m]
+    dets = np.repeat(ref[None], m + 1, axis=0)
+    for k, t in enumerate(pick):
+        s = 0b0011  # two electrons of the reference stay
+        for p in two[t]:
+            s |= 1 << p
+        for w in range(ref.shape[1]):
+            dets[k + 1, spin, w] = (s >> (64 * w)) & 0xFFFFFFFFFFFFFFFF
+    ints = G.make_integrals(n_mo, 5)
+    wf = Wavefunction(n_mo, ne, ne, ints.h, ints.eri, dets, SIGMA_STORED, line_keys=(0, 0, bits))
+    _all_pairs_match(wf, Oracle(n_mo, ne, ne, ints.h, ints.eri, dets))
+
+
+@pytest.mark.parametrize("n_mo", [30, 70])
+def test_rows_that_outgrow_their_chunks(n_mo):
+    """Chunks sized from a set that is hardly connected: the star's rows move to larger ones."""
+    from quantum_package_gb300.sigma import Wavefunction
+    ne, m = 8, 3000
+    ints = G.make_integrals(n_mo, 5)
+    dets = _star(n_mo, ne, m, 41)
+    wf = Wavefunction(n_mo, ne, ne, ints.h, ints.eri, dets[:2], SIGMA_STORED, line_keys=(0, 0, 64))
+    wf.set_dets(dets)
+    _all_pairs_match(wf, Oracle(n_mo, ne, ne, ints.h, ints.eri, dets))
