@@ -201,6 +201,24 @@ void qp_pool_free(qpgpu_ctx* c, void* p) {
   if (p) cudaFreeAsync(p, c->stream);
 }
 
+int qp_fork(qpgpu_ctx* c) {
+  for (int i = 0; i < 2; ++i) {
+    if (!c->side[i]) QP_CUDA(c, cudaStreamCreateWithFlags(&c->side[i], cudaStreamNonBlocking));
+    if (!c->side_ev[i]) QP_CUDA(c, cudaEventCreateWithFlags(&c->side_ev[i], cudaEventDisableTiming));
+  }
+  QP_CUDA(c, cudaEventRecord(c->side_ev[0], c->stream));
+  for (int i = 0; i < 2; ++i) QP_CUDA(c, cudaStreamWaitEvent(c->side[i], c->side_ev[0], 0));
+  return 0;
+}
+
+int qp_join(qpgpu_ctx* c) {
+  for (int i = 0; i < 2; ++i) {
+    QP_CUDA(c, cudaEventRecord(c->side_ev[i], c->side[i]));
+    QP_CUDA(c, cudaStreamWaitEvent(c->stream, c->side_ev[i], 0));
+  }
+  return 0;
+}
+
 void qp_pool_idle(qpgpu_ctx* c) {
   int cur = -1;
   if (cudaGetDevice(&cur) == cudaSuccess && cur != c->device) cudaSetDevice(c->device);
@@ -331,6 +349,10 @@ int qpgpu_destroy(qpgpu_ctx* c) {
     if (c->h_pin) cudaFreeHost(c->h_pin);
     cudaStreamSynchronize(c->stream);
     cudaMemPoolDestroy(c->pool);
+    for (int i = 0; i < 2; ++i) {
+      if (c->side[i]) cudaStreamDestroy(c->side[i]);
+      if (c->side_ev[i]) cudaEventDestroy(c->side_ev[i]);
+    }
     cudaStreamDestroy(c->stream);
   }
   delete c;

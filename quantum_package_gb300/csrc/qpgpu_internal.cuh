@@ -534,6 +534,8 @@ struct qpgpu_ctx {
   int n_sm = 0;  // streaming multiprocessors of the device (read at create)
   cudaStream_t stream = nullptr;
   cudaMemPool_t pool = nullptr;  // see qp_pool_alloc
+  cudaStream_t side[2] = {nullptr, nullptr};  // kernels of a set-up beside those on stream (qp_fork, qp_join)
+  cudaEvent_t side_ev[2] = {nullptr, nullptr};
   std::string last_error;
 
   int n_mo = 0, na = 0, nb = 0, nint = 0;
@@ -688,6 +690,11 @@ struct Scoped {
     p = nullptr;
   }
 };
+
+// qp_fork: c->side, created on first use, wait for what c->stream has;
+// qp_join: c->stream waits for them
+int qp_fork(qpgpu_ctx* c);
+int qp_join(qpgpu_ctx* c);
 
 // entry points implemented across translation units
 int qp_build_index(qpgpu_ctx* c);      // index.cu
