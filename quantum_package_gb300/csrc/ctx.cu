@@ -201,20 +201,20 @@ void qp_pool_free(qpgpu_ctx* c, void* p) {
   if (p) cudaFreeAsync(p, c->stream);
 }
 
-int qp_fork(qpgpu_ctx* c) {
+int qp_fork(qpgpu_ctx* c, cudaStream_t st) {
   for (int i = 0; i < 2; ++i) {
     if (!c->side[i]) QP_CUDA(c, cudaStreamCreateWithFlags(&c->side[i], cudaStreamNonBlocking));
     if (!c->side_ev[i]) QP_CUDA(c, cudaEventCreateWithFlags(&c->side_ev[i], cudaEventDisableTiming));
   }
-  QP_CUDA(c, cudaEventRecord(c->side_ev[0], c->stream));
+  QP_CUDA(c, cudaEventRecord(c->side_ev[0], st));
   for (int i = 0; i < 2; ++i) QP_CUDA(c, cudaStreamWaitEvent(c->side[i], c->side_ev[0], 0));
   return 0;
 }
 
-int qp_join(qpgpu_ctx* c) {
+int qp_join(qpgpu_ctx* c, cudaStream_t st) {
   for (int i = 0; i < 2; ++i) {
     QP_CUDA(c, cudaEventRecord(c->side_ev[i], c->side[i]));
-    QP_CUDA(c, cudaStreamWaitEvent(c->stream, c->side_ev[i], 0));
+    QP_CUDA(c, cudaStreamWaitEvent(st, c->side_ev[i], 0));
   }
   return 0;
 }
@@ -381,7 +381,7 @@ int qpgpu_get_info(qpgpu_ctx* c, qpgpu_info* info) {
   if (c->have_dets) b += c->Ua + c->Ub;
   b += (int64_t)c->work_bytes;
   info->device_bytes = b;
-  info->n_split_rows = c->items.n_multi;
+  info->n_split_rows = c->direct ? 0 : c->items.n_multi;  // of the stored pairs
   info->direct_sigma = c->direct ? 1 : 0;
   info->n_keyed_lines = c->n_keyed_lines;
   return QPGPU_OK;

@@ -88,14 +88,17 @@ struct BuildArgs {
   int* s2col;
   float* s2val;
   float4* feat;         // .w: coupling strength of the row (learned step)
-  // elements: work items (stretches of QP_SIGMA_CHUNK pairs of a row) and, for
-  // rows of several, each item's sum of squared elements
+  // elements and direct sigma: work items (stretches of QP_SIGMA_CHUNK pairs of
+  // a row) and, for rows of several, each item's sum of squared elements or its
+  // shares of v and s
   const int* row_nitems;
   const int* row_item0;
   const int* item_row;
   const int* item_sub;
   int64_t n_items;
   double* item_sum2;
+  double* item_v;
+  double* item_s;
   const u64* det_pos;   // both strings at each bilinear position (2 NINT words)
   const u64* det_tpos;  // the same at each alpha-major position (direct sigma)
   int* err;  // set when a pass would write past its row's segment
@@ -1234,22 +1237,32 @@ int sort_row_columns(qpgpu_ctx* c, const BuildArgs& a) {
   return 0;
 }
 
-// the scans of all three classes, side by side: each of them ends with the
+// The scans of all three classes, side by side: each of them ends with the
 // reference's row in one warp (0.8, 0.7 and 1.1 ms at 2e5 determinants, where
-// the other rows keep the device busy for 0.3, 0.3 and 1.0).  A pool pass runs
-// as many blocks as are resident.
+// the other rows keep the device busy for 0.3, 0.3 and 1.0).  Small sets, whose
+// scans take 0.1 ms together, run them one after the other: the streams cost a
+// new context 0.28 ms.
+constexpr int64_t SIDE_BY_SIDE = 1 << 15;
 template <int NINT, int MODE>
-int launch_scans(qpgpu_ctx* c, const BuildArgs& a) {
+int launch_scans(qpgpu_ctx* c, const BuildArgs& a, unsigned gs, unsigned gc, cudaStream_t st) {
+  const bool side = c->N >= SIDE_BY_SIDE;
+  int rc = side ? qp_fork(c, st) : 0;
+  if (rc) return rc;
+  k_same<NINT, MODE, 0><<<gs, BLK, 0, st>>>(a);
+  k_same<NINT, MODE, 1><<<gs, BLK, 0, side ? c->side[0] : st>>>(a);
+  k_class_c<NINT, MODE><<<gc, BLK, 0, side ? c->side[1] : st>>>(a);
+  rc = side ? qp_join(c, st) : 0;
+  if (rc) cudaDeviceSynchronize();  // work arrays are given back on c->stream
+  return rc;
+}
+
+// the scans of a set-up; a pool pass runs as many blocks as are resident
+template <int NINT, int MODE>
+int setup_scans(qpgpu_ctx* c, const BuildArgs& a) {
   const unsigned g = nblocks(c->N * 32, BLK);
   const unsigned gs = MODE == MODE_POOL ? std::min(g, (unsigned)c->n_sm * SAME_BPS) : g;
   const unsigned gc = MODE == MODE_POOL ? std::min(g, (unsigned)c->n_sm * CLASS_C_BPS) : g;
-  int rc = qp_fork(c);
-  if (rc) return rc;
-  k_same<NINT, MODE, 0><<<gs, BLK, 0, c->stream>>>(a);
-  k_same<NINT, MODE, 1><<<gs, BLK, 0, c->side[0]>>>(a);
-  k_class_c<NINT, MODE><<<gc, BLK, 0, c->side[1]>>>(a);
-  rc = qp_join(c);
-  if (rc) cudaDeviceSynchronize();  // work arrays are given back on c->stream
+  const int rc = launch_scans<NINT, MODE>(c, a, gs, gc, c->stream);
   qp_mark(c, "pair scans");
   return rc;
 }
@@ -1315,7 +1328,7 @@ int build_pairs_t(qpgpu_ctx* c) {
       cudaGetLastError();
     }
   }
-  const int rcs = a.pool ? launch_scans<NINT, MODE_POOL>(c, a) : launch_scans<NINT, MODE_COUNT>(c, a);
+  const int rcs = a.pool ? setup_scans<NINT, MODE_POOL>(c, a) : setup_scans<NINT, MODE_COUNT>(c, a);
   if (rcs) return rcs;
   QP_CUDA(c, cudaGetLastError());
   Scoped<int64_t> tot(c), stot(c);
@@ -1377,8 +1390,7 @@ int build_pairs_t(qpgpu_ctx* c) {
     QP_CUDA(c, cudaMemcpyAsync(c->h_rowptr.data(), c->d_rowptr, (N + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
                                st));
     QP_CUDA(c, cudaGetLastError());
-    QP_CUDA(c, cudaStreamSynchronize(st));
-    return 0;
+    return qp_build_sigma_items(c, &c->items);  // waits for the stream
   }
   if (pool_alloc(c, &c->d_colidx, P) != cudaSuccess || pool_alloc(c, &c->d_val64, P) != cudaSuccess ||
       pool_alloc(c, &c->d_val32, P) != cudaSuccess || pool_alloc(c, &c->d_s2col, PS) != cudaSuccess ||
@@ -1401,7 +1413,7 @@ int build_pairs_t(qpgpu_ctx* c) {
   QP_CUDA(c, cudaMemsetAsync(err.p, 0, sizeof(int), st));
   a.err = err.p;
   if (!a.pool || full) {
-    const int rcf = launch_scans<NINT, MODE_FILL>(c, a);
+    const int rcf = setup_scans<NINT, MODE_FILL>(c, a);
     if (rcf) return rcf;
     int herr = 0;
     QP_CUDA(c, cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1445,18 +1457,21 @@ __global__ void k_alpha_major(const double* u, const int* t_order, double* uT, i
 
 // Direct sigma of the rows [row_lo, row_hi) of one chunk, after the fill
 // scans wrote their columns into pc (at rowptr[k] - col_base): one warp per
-// row, lanes over its pairs; each pair's element is evaluated as in
+// stretch of a row, lanes over its pairs; each pair's element is evaluated as in
 // k_pair_values (same routines, same arguments), multiplied by the partner's
 // coefficients (same-alpha partners, tagged with their alpha-major position,
 // read from the alpha-major copy uT, where a row's partners are contiguous),
-// and the lanes are combined in a fixed order.  The fill wrote the row's
+// and the lanes are combined in a fixed order (as are the stretches of a row,
+// k_direct_combine).  The fill wrote the row's
 // same-beta partners, then its same-alpha partners, then the alpha x beta
 // ones, so each class has a loop of its own, a same-spin partner reads only
 // the string it does not share with the row, and the single excitations of
 // both same-spin classes are deferred until 32 are there (k_pair_values).
 // NP: states padded to a power of two, so that the sums stay in registers.
 // 2e5 determinants in 120 MOs, 2 states: 7.4 -> 4.1 ms with the register-only
-// Slater routines, the loops per class and the deferred singles.
+// Slater routines, the loops per class and the deferred singles; about 1.8
+// since a warp takes a stretch of QP_SIGMA_CHUNK pairs and not a row (the
+// reference's row outlasted the others; the whole sigma 6.9 -> 4.6 ms, 4.0 with the scans side by side).
 template <int NINT, int NP>
 __global__ void __launch_bounds__(BLK, 3) k_pair_sigma(BuildArgs a, const int* __restrict__ pc) {
   __shared__ int s_q[BLK / 32][DEFER];
@@ -1466,7 +1481,9 @@ __global__ void __launch_bounds__(BLK, 3) k_pair_sigma(BuildArgs a, const int* _
   const int64_t nwarp = ((int64_t)gridDim.x * BLK) >> 5;
   const int nst = a.nst;
   Deferred mono{s_q[threadIdx.x >> 5], 0};
-  for (int64_t k = a.row_lo + warp; k < a.row_hi; k += nwarp) {
+  const int64_t it_end = a.row_item0[a.row_hi];
+  for (int64_t it = a.row_item0[a.row_lo] + warp; it < it_end; it += nwarp) {
+    const int64_t k = a.item_row[it];
     if (((k - a.row_first) % a.row_step) != 0) continue;
     u64 my[2 * NINT], E[2 * NINT];
     const int bi = a.cols[k];
@@ -1484,9 +1501,12 @@ __global__ void __launch_bounds__(BLK, 3) k_pair_sigma(BuildArgs a, const int* _
       for (int st = 0; st < NP; ++st)
         if (st < nst) s[st] = fma(v, __ldg(uj + st), s[st]);
     };
-    const int64_t e0 = a.rowptr[k];
+    const int first = a.item_sub[it] * QP_SIGMA_CHUNK;
+    const int64_t e0 = a.rowptr[k] + first;
     const int* prow = pc + (e0 - a.col_base);
-    const int n = (int)(a.rowptr[k + 1] - e0), nA = a.cnt[CLS_A][k], nB = nA + a.cnt[CLS_B][k];
+    const int n = (int)min((int64_t)QP_SIGMA_CHUNK, a.rowptr[k + 1] - e0);
+    const int ra = a.cnt[CLS_A][k] - first;  // where the classes of the row end in this stretch
+    const int nA = min(max(ra, 0), n), nB = min(max(ra + a.cnt[CLS_B][k], 0), n);
     auto do_mono = [&](int x) {
       if (x < 0) return;
       const bool beta = x >= nA;
@@ -1543,10 +1563,33 @@ __global__ void __launch_bounds__(BLK, 3) k_pair_sigma(BuildArgs a, const int* _
     const double sv = qpsig::reduce_scatter64<NP>(sacc, lane);
     const int st = lane >> SH;
     if ((lane & ((1 << SH) - 1)) == 0 && st < nst) {
-      const double uk = a.u[k * nst + st];
-      a.v[k * nst + st] = hv + a.hdiag[k] * uk;
-      a.s[k * nst + st] = sv + a.sdiag[k] * uk;
+      if (a.row_nitems[k] > 1) {
+        a.item_v[it * nst + st] = hv;
+        a.item_s[it * nst + st] = sv;
+      } else {
+        const double uk = a.u[k * nst + st];
+        a.v[k * nst + st] = hv + a.hdiag[k] * uk;
+        a.s[k * nst + st] = sv + a.sdiag[k] * uk;
+      }
     }
+  }
+}
+
+// the rows of several stretches: their shares in order, then the diagonal
+__global__ void k_direct_combine(BuildArgs a, const int* multi_rows, int n) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n * a.nst; t += gridDim.x * blockDim.x) {
+    const int64_t k = multi_rows[t / a.nst];
+    const int st = t % a.nst;
+    if (!dsel(a, k)) continue;
+    double hv = 0.0, sv = 0.0;
+    for (int j = 0; j < a.row_nitems[k]; ++j) {
+      const int64_t it = a.row_item0[k] + j;
+      hv += a.item_v[it * a.nst + st];
+      sv += a.item_s[it * a.nst + st];
+    }
+    const double uk = a.u[k * a.nst + st];
+    a.v[k * a.nst + st] = hv + a.hdiag[k] * uk;
+    a.s[k * a.nst + st] = sv + a.sdiag[k] * uk;
   }
 }
 
@@ -1584,6 +1627,14 @@ int sigma_direct_t(qpgpu_ctx* c, double* v, double* s, const double* u, const do
   a.tag_t = 1;
   a.row_first = row_first;
   a.row_step = row_step;
+  const int rci = qp_ensure_partials(c, &c->items, nst);
+  if (rci) return rci;
+  a.row_nitems = c->items.row_nitems;
+  a.row_item0 = c->items.row_item0;
+  a.item_row = c->items.item_row;
+  a.item_sub = c->items.item_sub;
+  a.item_v = c->items.pv;
+  a.item_s = c->items.ps;
   const int64_t N = c->N;
   const std::vector<int64_t>& rp = c->h_rowptr;
   int64_t clo = 0;
@@ -1600,13 +1651,14 @@ int sigma_direct_t(qpgpu_ctx* c, double* v, double* s, const double* u, const do
       const unsigned gK = nblocks((hi - lo) * 32, BLK);
       const bool marks = st == c->stream;  // QPGPU_PROFILE=1: phase times on the context stream
       if (marks) qp_mark(c, "direct: chunk start");
-      k_same<NINT, MODE_FILL, 0><<<gK, BLK, 0, st>>>(a);
-      if (marks) qp_mark(c, "direct: scan A");
-      k_same<NINT, MODE_FILL, 1><<<gK, BLK, 0, st>>>(a);
-      if (marks) qp_mark(c, "direct: scan B");
-      k_class_c<NINT, MODE_FILL><<<gK, BLK, 0, st>>>(a);
-      if (marks) qp_mark(c, "direct: scan C");
-      launch_pair_sigma<NINT>(a, c->d_direct_cols, gK, st);
+      const int rcs = launch_scans<NINT, MODE_FILL>(c, a, gK, gK, st);
+      if (rcs) return rcs;
+      if (marks) qp_mark(c, "direct: scans");
+      const int64_t items = hi - lo + (rp[hi] - rp[lo]) / QP_SIGMA_CHUNK;  // at most
+      launch_pair_sigma<NINT>(a, c->d_direct_cols, nblocks(items * 32, BLK), st);
+      if (c->items.n_multi > 0)
+        k_direct_combine<<<nblocks((int64_t)c->items.n_multi * nst, 256), 256, 0, st>>>(a, c->items.multi_rows,
+                                                                                       c->items.n_multi);
       if (marks) qp_mark(c, "direct: elements");
     }
     clo = chi;

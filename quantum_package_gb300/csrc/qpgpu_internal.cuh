@@ -534,7 +534,7 @@ struct qpgpu_ctx {
   int n_sm = 0;  // streaming multiprocessors of the device (read at create)
   cudaStream_t stream = nullptr;
   cudaMemPool_t pool = nullptr;  // see qp_pool_alloc
-  cudaStream_t side[2] = {nullptr, nullptr};  // kernels of a set-up beside those on stream (qp_fork, qp_join)
+  cudaStream_t side[2] = {nullptr, nullptr};  // kernels beside those of a call's stream (qp_fork, qp_join)
   cudaEvent_t side_ev[2] = {nullptr, nullptr};
   std::string last_error;
 
@@ -691,10 +691,10 @@ struct Scoped {
   }
 };
 
-// qp_fork: c->side, created on first use, wait for what c->stream has;
-// qp_join: c->stream waits for them
-int qp_fork(qpgpu_ctx* c);
-int qp_join(qpgpu_ctx* c);
+// qp_fork: c->side, created on first use, wait for what st has; qp_join: st
+// waits for them
+int qp_fork(qpgpu_ctx* c, cudaStream_t st);
+int qp_join(qpgpu_ctx* c, cudaStream_t st);
 
 // entry points implemented across translation units
 int qp_build_index(qpgpu_ctx* c);      // index.cu
@@ -721,6 +721,7 @@ int qp_build_pairs(qpgpu_ctx* c);      // pairs.cu
 void qp_free_dets(qpgpu_ctx* c);       // index.cu
 void qp_free_pairs(qpgpu_ctx* c);      // pairs.cu
 int qp_build_sigma_items(qpgpu_ctx* c, SigmaItems* it);  // sigma.cu
+int qp_ensure_partials(qpgpu_ctx* c, SigmaItems* it, int nst);
 // FP64 sigma without stored pairs (pairs.cu)
 int qp_sigma_direct(qpgpu_ctx* c, double* v, double* s, const double* u, int nst, cudaStream_t st, int row_lo,
                     int row_hi, int row_first, int row_step);

@@ -617,7 +617,7 @@ int qp_build_sigma_items(qpgpu_ctx* c, SigmaItems* it) {
 }
 
 // Partial-sum buffers sized for nst states.
-static int ensure_partials(qpgpu_ctx* c, SigmaItems* it, int nst) {
+int qp_ensure_partials(qpgpu_ctx* c, SigmaItems* it, int nst) {
   const size_t need = (size_t)it->n_items * nst;
   if (it->partial_cap >= need) return 0;
   dev_free(it->pv);
@@ -639,7 +639,7 @@ int qp_sigma_launch(qpgpu_ctx* c, SigmaItems* it, double* v, double* s, const do
   if (u32_ld != nst && !(u32_ld == qp_pad_states(nst) && (((uintptr_t)u32) & 31) == 0))
     return qpgpu_fail(c, QPGPU_ERR_ARG, "FP32 rows must be n_st floats apart, or padded to 4/8 and 32-byte aligned");
   if (precision == QPGPU_FP32 && !u32) return qpgpu_fail(c, QPGPU_ERR_ARG, "FP32 sigma needs u_t32");
-  int rc = ensure_partials(c, it, nst);
+  int rc = qp_ensure_partials(c, it, nst);
   if (rc) return rc;
   SigArgs a{};
   a.N = c->N;
