@@ -1305,12 +1305,14 @@ int build_pairs_t(qpgpu_ctx* c) {
     const double est = per_row * (double)N;
     // chunks: an eighth of a warp's share of about 0.3 / 0.3 / 0.6 of the
     // pairs, but sixteen rows at least, as a row that does not fit the rest of
-    // a chunk takes another
+    // a chunk takes another (of 300 pairs in a new context: with 1,200 the
+    // chunks of a 5,000 determinant set took 300 MB, 0.3 of 2.5 ms to map)
+    const double usual = c->pairs_per_row > 0 ? per_row : 300.0;
     const int64_t all = nblocks(N * 32, BLK);
     const int64_t ws = std::min<int64_t>(all, c->n_sm * SAME_BPS) * (BLK / 32);
     const int64_t wc = std::min<int64_t>(all, c->n_sm * CLASS_C_BPS) * (BLK / 32);
     auto chunk_of = [&](double share, int64_t warps) {
-      return (int)std::min(65536.0, std::max({256.0, share * est / (8.0 * (double)warps), 16.0 * share * per_row}));
+      return (int)std::min(65536.0, std::max({256.0, share * est / (8.0 * (double)warps), 16.0 * share * usual}));
     };
     a.pool_chunk[CLS_A] = a.pool_chunk[CLS_B] = chunk_of(0.3, ws);
     a.pool_chunk[CLS_C] = chunk_of(0.6, wc);
