@@ -72,6 +72,25 @@ __device__ __forceinline__ void store_row(const SigArgs& a, int64_t it, int k, i
     (sub == 0 ? a.pv : a.ps)[it * NST + st] = sum;
   }
 }
+// the same by one lane of each state, for the kernels that the FP64 pipe does
+// not bound: k_sigma32 keeps 40 instead of 48 registers (1e6 determinants x 4
+// states 2.69 -> 2.60 ms)
+template <int NST>
+__device__ __forceinline__ void store_row_lean(const SigArgs& a, int64_t it, int k, int lane, double hv, double sv,
+                                               bool has_s2) {
+  constexpr int SH = 5 - Pow2<NST>::lg;
+  const int st = lane >> SH;
+  if ((lane & ((1 << SH) - 1)) != 0 || st >= NST) return;
+  const double s2 = has_s2 ? sv : 0.0;
+  if (a.row_nitems[k] == 1) {
+    const double uk = a.u[(int64_t)k * NST + st];
+    a.v[(int64_t)k * NST + st] = fma(a.hdiag[k], uk, hv);
+    a.s[(int64_t)k * NST + st] = fma(a.sdiag[k], uk, s2);
+  } else {
+    a.pv[it * NST + st] = hv;
+    a.ps[it * NST + st] = s2;
+  }
+}
 
 
 
@@ -232,7 +251,7 @@ __global__ void __launch_bounds__(BS) k_sigma32(SigArgs a) {
       reduce_scatter_ff<NP>(sh, sl, lane, qh, ql);
       ssum = (double)qh + (double)ql;
     }
-    store_row<NST>(a, it, k, lane, hsum, ssum, has_s2);
+    store_row_lean<NST>(a, it, k, lane, hsum, ssum, has_s2);
   }
 }
 
@@ -506,7 +525,7 @@ __global__ void __launch_bounds__(128) k_sigma_ff(SigArgs a) {
       reduce_scatter_ff<NP>(sh, sl, lane, qh, ql);
       ssum = (double)qh + (double)ql;
     }
-    store_row<NST>(a, it, k, lane, hsum, ssum, has_s2);
+    store_row_lean<NST>(a, it, k, lane, hsum, ssum, has_s2);
   }
 }
 
@@ -538,10 +557,10 @@ void launch_any(const SigArgs& a, int nst, int precision, unsigned grid, cudaStr
 // Times every FP32 launch shape on this determinant set (two launches each,
 // the second timed with events on the caller's stream) and keeps the fastest
 // for n_st.  Runs once per determinant set and n_st, on the first FP32 call,
-// whose own launch follows.  A stretch of an eighth of the work items is
-// enough to tell the shapes apart (of all of them where they are few): over
-// all the items the choice cost 8 sigmas, 9.3 of the 11.3 ms of a first call
-// at 5e5 determinants x 8 states.
+// whose own launch follows.  A stretch of a quarter of the work items tells
+// the shapes apart (of 2^18 at least: on 65,536 of the 330,000 items of 3e5
+// determinants x 2 states the persistent shape lost, over all it wins by 9
+// percent).
 int tune_sigma32(qpgpu_ctx* c, SigmaItems* it, const SigArgs& all, int nst, cudaStream_t st, int slot) {
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
@@ -549,7 +568,7 @@ int tune_sigma32(qpgpu_ctx* c, SigmaItems* it, const SigArgs& all, int nst, cuda
     return qpgpu_fail(c, QPGPU_ERR_CUDA, "cudaEventCreate failed while tuning the FP32 sigma");
   }
   SigArgs a = all;
-  const int64_t n = std::min<int64_t>(all.n_items, std::max<int64_t>(all.n_items / 8, 1 << 16));
+  const int64_t n = std::min<int64_t>(all.n_items, std::max<int64_t>(all.n_items / 4, 1 << 18));
   const int64_t first = (all.n_items - n) / 2;
   a.n_items = n;
   a.item_row += first;
