@@ -50,6 +50,7 @@
 // *status.
 #include <algorithm>
 
+#include "block_ring.h"
 #include "qpgpu_internal.cuh"
 
 namespace {
@@ -894,6 +895,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
           if (c == 0 && t >= 2) ok = mbar_wait(BAR(LC_B_ACCE + buf), (uint32_t)((t >> 1) - 1) & 1u, sflag);
           if (ok) ok = mbar_wait(BAR(LC_B_FULL + s), (uint32_t)round & 1u, sflag);
           if (ok) {
+            // every read of this step's slots, which the barrier has put before
+            // this thread, comes before their next copies
+            __threadfence_block();
             *sdone = gstep + 1;
             asm volatile("tcgen05.fence::after_thread_sync;");
             const uint32_t a0 = smem_u32(adig + s * LC_ASTAGE), b0 = smem_u32(bdig + (size_t)c * LC_BCHUNK);
@@ -926,82 +930,56 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
   } else {
     // ---- load warp: blocks of tile t in order, each as one bulk copy, or by
     // the lanes when it is not whole 16-byte lines (g.lane_copies: some are not)
-    auto span = [&](int t, int b, const double*& src) -> uint32_t {
-      const int64_t R = r0 + (int64_t)t * LC_TM;
-      src = g.A + (int64_t)b * g.sA + R * nsd;
-      return (uint32_t)(min((int64_t)LC_TM, r1 - R) * nsd * 8);
-    };
-    auto whole = [](const double* src, uint32_t bytes) { return ((((uintptr_t)src) | bytes) & 15) == 0; };
-    auto expect = [&](int t) {
-      if (lane == 0) {
-        uint32_t total = 0;
-        for (int b = 0; b < nb; ++b) {
-          const double* src;
-          const uint32_t bytes = span(t, b, src);
-          if (whole(src, bytes)) total += bytes;
+    struct Io {
+      const LcArgs& g;
+      double* raw;
+      const int* sflag;
+      volatile int* sdone;
+      int64_t r0, r1;
+      int nsd, lane;
+      uint32_t rawf;  // barriers of the even and odd tiles
+      __device__ __forceinline__ uint32_t bar(int t) const { return rawf + 8u * (uint32_t)(t & 1); }
+      // bounded wait for K step `step` of the whole run to be cut
+      __device__ __forceinline__ bool cut(int step) const {
+        bool ok = false;
+        for (long long it = 0; it < OZ_WAIT_LIMIT && !ok; ++it) {
+          ok = *sdone > step;
+          if (!ok && (it & 255) == 255 && *(volatile const int*)sflag) break;
         }
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(BAR(LC_B_RAWF + (t & 1))),
-                     "r"(total)
-                     : "memory");
+        __threadfence_block();
+        return __all_sync(0xffffffffu, ok) != 0;
       }
-      __syncwarp();
-    };
-    auto copy = [&](int t, int b, int slot) {
-      const double* src;
-      const uint32_t bytes = span(t, b, src);
-      const uint32_t dst = smem_u32(raw + (size_t)slot * LC_TM * nsd);
-      if (whole(src, bytes)) {
-        if (lane == 0)
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                           dst),
-                       "l"(src), "r"(bytes), "r"(BAR(LC_B_RAWF + (t & 1)))
-                       : "memory");
-      } else {
-        for (uint32_t x = lane; x < bytes / 8; x += 32)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * x), "l"(src + x) : "memory");
-      }
-    };
-    auto finish = [&](int t) {  // the lanes' share of the tile arrives once their copies have landed
-      if (g.lane_copies)
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(BAR(LC_B_RAWF + (t & 1))) : "memory");
-    };
-    // bounded wait for K step `step` of the whole run to be cut
-    auto cut = [&](int step) {
-      bool ok = false;
-      for (long long it = 0; it < OZ_WAIT_LIMIT && !ok; ++it) {
-        ok = *sdone > step;
-        if (!ok && (it & 255) == 255 && *(volatile const int*)sflag) break;
-      }
-      __threadfence_block();
-      return __all_sync(0xffffffffu, ok) != 0;
-    };
-    int issued = 0, slot = 0;  // tiles whose copies are all on their way; next slot
-    bool ok = true;
-    for (int t = 0; t < ntile && ok; ++t) {
-      for (int b = 0; b < nb && ok; ++b) {
-        // the slot's last block: nslots blocks back, free after its last K step
-        const int old = t * nb + b - nslots;
-        if (old >= 0) {
-          const int ot = old / nb, ob = old - ot * nb;
-          ok = cut(ot * nks + ((ob + 1) * nsd - 1) / LC_KS);
-          if (!ok) break;
+      __device__ __forceinline__ void copy(int t, int b, int slot) const {
+        const int64_t R = r0 + (int64_t)t * LC_TM;
+        const double* src = g.A + (int64_t)b * g.sA + R * nsd;
+        const uint32_t bytes = (uint32_t)(min((int64_t)LC_TM, r1 - R) * nsd * 8);
+        const uint32_t dst = smem_u32(raw + (size_t)slot * LC_TM * nsd);
+        if ((((uintptr_t)src | bytes) & 15) == 0) {
+          if (lane == 0) {
+            asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar(t)), "r"(bytes)
+                         : "memory");
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                "l"(src), "r"(bytes), "r"(bar(t))
+                : "memory");
+          }
+        } else {
+          for (uint32_t x = lane; x < bytes / 8; x += 32)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * x), "l"(src + x) : "memory");
         }
-        if (b == 0) expect(t);
-        copy(t, b, slot);
-        if (++slot == nslots) slot = 0;
       }
-      if (!ok) {
-        if (lane == 0) atomicExch(sflag, 1);
-        break;
+      __device__ __forceinline__ void finish(int t) const {
+        if (lane == 0) mbar_arrive(bar(t));
+        if (g.lane_copies)  // the lanes' share of the tile arrives once their copies have landed
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar(t)) : "memory");
       }
-      finish(t);
-      issued = t + 1;
-    }
-    // the copies still in flight land before the CTA may exit
+      __device__ __forceinline__ void drain(int t) const {
+        if (lane == 0 && !mbar_drain(bar(t), (uint32_t)(t >> 1) & 1u)) atomicExch(const_cast<int*>(sflag), 1);
+      }
+    };
+    Io io{g, raw, sflag, sdone, r0, r1, nsd, lane, BAR(LC_B_RAWF)};
+    if (!block_ring_load(io, ntile, nb, nslots, nsd, nks, LC_KS) && lane == 0) atomicExch(sflag, 1);
     asm volatile("cp.async.wait_all;" ::: "memory");
-    if (lane == 0)
-      for (int t = max(0, issued - 2); t < issued; ++t)
-        if (!mbar_drain(BAR(LC_B_RAWF + (t & 1)), (uint32_t)(t >> 1) & 1u)) atomicExch(sflag, 1);
     __syncwarp();
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
