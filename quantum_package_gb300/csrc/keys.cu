@@ -255,7 +255,11 @@ int build_line_keys_t(qpgpu_ctx* c) {
   const int64_t t1_col = c->key_min_single >= 0 ? c->key_min_single : 64 * (int64_t)(c->na + 2);
   const int64_t t1_row = c->key_min_single >= 0 ? c->key_min_single : 64 * (int64_t)(c->nb + 2);
   const int64_t t2 = c->key_min_double >= 0 ? c->key_min_double : 16384;
-  const u64 hmask = qp_key_mask(c);
+  // a set keeps the bits that its tables were built with, whatever
+  // qpgpu_set_line_keys asks of the next one: the direct sigma probes them at every call
+  const int kept = qp_key_bits(c);
+  const u64 hmask = kept >= 64 ? ~0ull : (1ull << kept) - 1ull;
+  c->key_mask = hmask;
   QP_CUDA(c, pool_alloc(c, &c->d_colkey, (size_t)c->Ub));
   QP_CUDA(c, pool_alloc(c, &c->d_rowkey, (size_t)c->Ua));
   Scoped<unsigned long long> sums(c);

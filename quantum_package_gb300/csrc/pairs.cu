@@ -1163,7 +1163,7 @@ BuildArgs index_args(const qpgpu_ctx* c) {
   }
   a.colkey = c->d_colkey;
   a.rowkey = c->d_rowkey;
-  a.hmask = qp_key_mask(c);
+  a.hmask = c->key_mask;
   return a;
 }
 

@@ -582,6 +582,7 @@ struct qpgpu_ctx {
   // tables (-1: defaults), and the hash bits kept
   int64_t key_min_single = -1, key_min_double = -1;
   int key_hash_bits = 64;
+  u64 key_mask = 0;  // hash bits of the tables that the set in hand was built with
 
   // Hamiltonian in CSR over bilinear rows (columns are bilinear positions)
   bool have_pairs = false;
@@ -712,10 +713,6 @@ inline int qp_key_bits(const qpgpu_ctx* c) {
     ++b;
   }
   return std::max(1, std::min(c->key_hash_bits, b));
-}
-inline u64 qp_key_mask(const qpgpu_ctx* c) {
-  const int b = qp_key_bits(c);
-  return b >= 64 ? ~0ull : (1ull << b) - 1ull;
 }
 int qp_build_pairs(qpgpu_ctx* c);      // pairs.cu
 void qp_free_dets(qpgpu_ctx* c);       // index.cu
