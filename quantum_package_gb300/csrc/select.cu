@@ -75,6 +75,7 @@ constexpr int SEL_DTILE = 256;     // selectors staged per pass (one word of 32 
 constexpr int SEL_DWORDS = SEL_DTILE / 32;
 static_assert(SEL_DWORDS == SBLK / 32 && SBLK <= SEL_DTILE, "each warp transposes one word of staged selectors");
 constexpr int SEL_MAXST = 8;       // states
+constexpr int SEL_SUM = SBLK / 2;  // entries whose energies are summed together, and that units are cut in
 constexpr int SEL_MQ = 128;        // single-excitation elements a warp evaluates ahead
 constexpr int SEL_MG = 4;          // entries per lane they are collected from
 static_assert(SEL_DTILE <= 256 && SEL_MG <= 8, "codes of 3 + 5 + 8 bits");
@@ -89,7 +90,7 @@ struct SelItem {
   int spin;      // single / same-spin double: 0 alpha, 1 beta
   int h1, h2;    // holes (1-based); alpha-beta: h1 alpha, h2 beta
   int e0, e1;    // entry range
-  int part;      // its place in pt2_part (generators in order)
+  int part;      // first of its sums in pt2_part (generators in order)
 };
 
 struct SelArgs {
@@ -107,7 +108,7 @@ struct SelArgs {
   const double* fock;        // per listed generator: build_fock_tmp, [gl][2][n_mo + 2]
   const int* hslot;          // hash set of psi_det: det index or -1
   uint64_t hmask;
-  double* pt2_part;          // [part][n_st]
+  double* pt2_part;          // [part][n_st]: sums over SEL_SUM entries each
   unsigned long long* n_ext;
   unsigned long long* n_cand;
   uint64_t cap;
@@ -645,13 +646,11 @@ __global__ void __launch_bounds__(SBLK, 3) k_sel_items(SelArgs A) {
       }
     __syncthreads();
   }
-  // energies of this thread's entries
-  double pt[SEL_MAXST];
-#pragma unroll
-  for (int s = 0; s < SEL_MAXST; ++s) pt[s] = 0.0;
+  // energies of this thread's entries, in place of their numerators (zero for
+  // an entry that does not count)
   unsigned long long next = 0;
   for (int e = tid; e < ne; e += SBLK) {
-    const double* m = tile + (size_t)e * nst;
+    double* m = tile + (size_t)e * nst;
     unsigned long long any = 0;
     for (int s = 0; s < nst; ++s) any |= (unsigned long long)__double_as_longlong(m[s]) << 1;
     if (any == 0) continue;
@@ -670,7 +669,10 @@ __global__ void __launch_bounds__(SBLK, 3) k_sel_items(SelArgs A) {
       for (int64_t f = A.flist_off[it.gl]; f < A.flist_off[it.gl + 1] && !banned; ++f)
         banned = exc_deg<NINT>(a, A.dets + (int64_t)A.flist[f] * 2 * NINT) <= 2;
     }
-    if (banned) continue;
+    if (banned) {
+      for (int s = 0; s < nst; ++s) m[s] = 0.0;
+      continue;
+    }
     ++next;
     double haa = hp1[v1];
     if (two) haa += (hp2[v2] + tab2(pp, n, p1, p2)) - hq2[v2];
@@ -681,7 +683,7 @@ __global__ void __launch_bounds__(SBLK, 3) k_sel_items(SelArgs A) {
       double tmp = sqrt(delta * delta + val * val);
       if (delta < 0.0) tmp = -tmp;
       const double ev = 0.5 * (tmp - delta);
-      pt[s] += ev;
+      m[s] = ev;
       mine = fmin(ev, mine);
     }
     // one atomic for the lanes that are here together
@@ -695,32 +697,40 @@ __global__ void __launch_bounds__(SBLK, 3) k_sel_items(SelArgs A) {
     }
   }
   if (next) atomicAdd(A.n_ext, next);
-  // the numerator tile is free now: it holds the per-thread sums (the
-  // dynamic allocation is at least SBLK x n_st doubles)
+  // sums over SEL_SUM entries of the item each, whatever unit they are in: how
+  // a call's work is split does not show in the bits
   __syncthreads();
-  for (int s = 0; s < nst; ++s) tile[tid * nst + s] = pt[s];
-  __syncthreads();
-  if (tid < nst) {
+  const int nsum = (ne + SEL_SUM - 1) / SEL_SUM;
+  for (int x = warp; x < nsum * nst; x += SBLK / 32) {
+    const int b = x / nst, s = x - b * nst;
     double acc = 0.0;
-    for (int x = 0; x < SBLK; ++x) acc += tile[x * nst + tid];
-    A.pt2_part[(int64_t)it.part * nst + tid] = acc;
+#pragma unroll
+    for (int q = 0; q < SEL_SUM / 32; ++q) {
+      const int e = b * SEL_SUM + 32 * q + lane;
+      if (e < ne) acc += tile[(size_t)e * nst + s];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) A.pt2_part[((int64_t)it.part + b) * nst + s] = acc;
   }
 }
 
-// pt2[s] = sum over units: one CTA per state, strided partial sums combined in
-// thread order (one thread walking 3,248 items waited 193 us on its loads)
-__global__ void __launch_bounds__(SBLK) k_sel_pt2(const double* part, int64_t n_units, int nst, double* pt2) {
+// detail[l][s] = sum over the parts of listed generator l: one CTA per
+// generator and state, strided sums combined in thread order (one thread
+// walking 3,248 of them waited 193 us on its loads)
+__global__ void __launch_bounds__(SBLK) k_sel_pt2(const double* part, const int64_t* first, int nst, double* detail) {
   __shared__ double red[SBLK];
-  const int s = blockIdx.x;
+  const int l = blockIdx.x, s = blockIdx.y;
   double acc = 0.0;
-  for (int64_t i = threadIdx.x; i < n_units; i += SBLK) acc += part[i * nst + s];
+#pragma unroll 8
+  for (int64_t i = first[l] + threadIdx.x; i < first[l + 1]; i += SBLK) acc += part[i * nst + s];
   red[threadIdx.x] = acc;
   __syncthreads();
   for (int o = SBLK / 2; o > 0; o >>= 1) {
     if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) pt2[s] = red[0];
+  if (threadIdx.x == 0) detail[(int64_t)l * nst + s] = red[0];
 }
 
 // ascending order of doubles as unsigned keys
@@ -845,10 +855,11 @@ struct Dev {
 }  // namespace
 
 // The selection over the listed generators (psi_det indices, each banned by
-// every generator before it, listed or not).  pt2 (n_st) sums all of them;
-// per_gen (n_list x n_st, optional) holds each generator's share, summed over
-// its items in order.  The buffer as qpgpu_select_pt2.  Returns the number of
-// buffer entries written or a negative status.
+// every generator before it, listed or not).  pt2 (n_st) sums all of them, in
+// the order of the list; per_gen (n_list x n_st, optional) holds each
+// generator's share, summed in an order that is the generator's own.  The
+// buffer as qpgpu_select_pt2.  Returns the number of buffer entries written or
+// a negative status.
 static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const double* e0, int n_sel,
                          const std::vector<int>& gens, int buf_size, double* pt2, double* per_gen,
                          uint64_t* buf_dets, double* buf_vals, int64_t* n_ext) {
@@ -898,7 +909,7 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   }
   // device arrays
   Dev d_items{c}, d_gens{c}, d_coef{c}, d_e0{c}, d_icnt{c}, d_ioff{c}, d_ilist{c}, d_fcnt{c}, d_foff{c};
-  Dev d_flist{c}, d_fock{c}, d_slot{c}, d_part{c}, d_cnt{c}, d_err{c}, d_pt2{c}, d_wgt{c}, d_units{c};
+  Dev d_flist{c}, d_fock{c}, d_slot{c}, d_part{c}, d_cnt{c}, d_err{c}, d_pt2{c}, d_wgt{c}, d_units{c}, d_first{c};
   uint64_t hcap = 1;
   while (hcap < (uint64_t)(2 * N)) hcap <<= 1;
   QP_CUDA(c, qp_pool_alloc(c, &d_items.p, items.size() * sizeof(SelItem)));
@@ -922,7 +933,7 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   QP_CUDA(c, qp_pool_alloc(c, &d_cnt.p, 2 * sizeof(unsigned long long)));
   QP_CUDA(c, qp_pool_alloc(c, &d_err.p, sizeof(int)));
   QP_CUDA(c, cudaMemsetAsync(d_err.p, 0, sizeof(int), st));
-  QP_CUDA(c, qp_pool_alloc(c, &d_pt2.p, n_st * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_pt2.p, (size_t)n_list * n_st * sizeof(double)));
   const u64* dets = c->d_dets;
   const int* dg = (const int*)d_gens.p;
   const int hb = (int)std::min<int64_t>((N + 255) / 256, (int64_t)c->n_sm * 8);
@@ -994,49 +1005,57 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   QP_CUDA(c, cudaMemcpyAsync(wgt.data(), d_wgt.p, items.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
   QP_CUDA(c, cudaStreamSynchronize(st));
   // Units: an item whose work is above the share of a CTA is split by entries
-  // (in multiples of SPLIT_ENTRIES), and the heaviest units start first.  The
+  // (in multiples of SEL_SUM), and the heaviest units start first.  The
   // work differs by up to a hundred times between items: the call of the
   // header's example ran 8.0 ms with one CTA per item in their order, the last
   // percent of them alone in the second half of that, and 6.1 ms this way.  A
   // share is at least several times what the staging of a CTA costs; 3, 4, 6
   // and 12 shares per resident CTA took 4.4, 3.8, 3.9 and 4.3 ms.
-  constexpr int SPLIT_ENTRIES = SBLK / 2, SHARES = 4;
+  constexpr int SHARES = 4;
   double work = 0.0;
   for (float w : wgt) work += w;
   const double staging = LIST_COST * (double)ioff[n_list] / n_list;
   const double share = std::max(work / ((double)c->n_sm * 3 * SHARES), 4.0 * staging);
   std::vector<SelItem> units;
   std::vector<float> uw;
-  std::vector<int64_t> unit_first(n_list + 1, 0);
+  std::vector<int64_t> part_first(n_list + 1, 0);
+  int64_t n_parts = 0;
   for (size_t i = 0; i < items.size(); ++i) {
     SelItem it = items[i];
-    const int ne = it.e1 - it.e0, blocks = (ne + SPLIT_ENTRIES - 1) / SPLIT_ENTRIES;
+    const int ne = it.e1 - it.e0, blocks = (ne + SEL_SUM - 1) / SEL_SUM;
     const int parts = (int)std::min<double>(std::ceil(wgt[i] / share), blocks);
-    const int step = parts <= 1 ? ne : (blocks + parts - 1) / parts * SPLIT_ENTRIES;
+    const int step = parts <= 1 ? ne : (blocks + parts - 1) / parts * SEL_SUM;
     for (int a = 0; a < ne; a += step) {
       it.e0 = items[i].e0 + a;
       it.e1 = std::min(items[i].e1, it.e0 + step);
-      it.part = (int)units.size();
+      it.part = (int)(n_parts + a / SEL_SUM);
       units.push_back(it);
       uw.push_back(wgt[i] * (float)(it.e1 - it.e0) / (float)ne);
     }
-    unit_first[it.gl + 1] = (int64_t)units.size();
+    n_parts += blocks;
+    part_first[it.gl + 1] = n_parts;
   }
-  for (int l = 0; l < n_list; ++l) unit_first[l + 1] = std::max(unit_first[l + 1], unit_first[l]);
+  for (int l = 0; l < n_list; ++l) part_first[l + 1] = std::max(part_first[l + 1], part_first[l]);
   const int64_t n_units = (int64_t)units.size();
-  std::sort(units.begin(), units.end(), [&](const SelItem& x, const SelItem& y) {
-    return uw[x.part] != uw[y.part] ? uw[x.part] > uw[y.part] : x.part < y.part;
-  });
+  {
+    std::vector<int> order(n_units);
+    for (int64_t i = 0; i < n_units; ++i) order[i] = (int)i;
+    std::sort(order.begin(), order.end(), [&](int x, int y) { return uw[x] != uw[y] ? uw[x] > uw[y] : x < y; });
+    std::vector<SelItem> by_weight(n_units);
+    for (int64_t i = 0; i < n_units; ++i) by_weight[i] = units[order[i]];
+    units.swap(by_weight);
+  }
   QP_CUDA(c, qp_pool_alloc(c, &d_units.p, n_units * sizeof(SelItem)));
   QP_CUDA(c, cudaMemcpyAsync(d_units.p, units.data(), n_units * sizeof(SelItem), cudaMemcpyHostToDevice, st));
-  QP_CUDA(c, qp_pool_alloc(c, &d_part.p, (size_t)n_units * n_st * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_part.p, (size_t)n_parts * n_st * sizeof(double)));
+  QP_CUDA(c, qp_pool_alloc(c, &d_first.p, (n_list + 1) * sizeof(int64_t)));
+  QP_CUDA(c, cudaMemcpyAsync(d_first.p, part_first.data(), (n_list + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
   A.items = (const SelItem*)d_units.p;
   A.pt2_part = (double*)d_part.p;
-  // dynamic shared memory: the largest unit's numerator tile (at least the
-  // SBLK x n_st doubles of the final reduction), so that several CTAs fit an SM
+  // dynamic shared memory: the largest unit's numerator tile, so that several CTAs fit an SM
   int max_ne = 0;
   for (const SelItem& it : units) max_ne = std::max(max_ne, it.e1 - it.e0);
-  const size_t smem = (size_t)std::max(max_ne * n_st, SBLK * n_st) * sizeof(double);
+  const size_t smem = (size_t)max_ne * n_st * sizeof(double);
   unsigned long long hcnt[2] = {0, 0};
   for (int attempt = 0; attempt < 2; ++attempt) {
     qp_pool_free(c, d_cval.p);
@@ -1063,19 +1082,14 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
     if (buf_size == 0 || hcnt[1] <= cap) break;
     cap = hcnt[1];  // every candidate counted: run once more with room for all of them
   }
-  k_sel_pt2<<<n_st, SBLK, 0, st>>>((const double*)d_part.p, n_units, n_st, (double*)d_pt2.p);
-  QP_CUDA(c, cudaMemcpyAsync(pt2, d_pt2.p, n_st * sizeof(double), cudaMemcpyDeviceToHost, st));
-  if (per_gen) {
-    std::vector<double> part((size_t)n_units * n_st);
-    QP_CUDA(c, cudaMemcpyAsync(part.data(), d_part.p, part.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    QP_CUDA(c, cudaStreamSynchronize(st));
-    for (int l = 0; l < n_list; ++l)
-      for (int s = 0; s < n_st; ++s) {
-        double acc = 0.0;
-        for (int64_t i = unit_first[l]; i < unit_first[l + 1]; ++i) acc += part[(size_t)i * n_st + s];
-        per_gen[(size_t)l * n_st + s] = acc;
-      }
-  }
+  k_sel_pt2<<<dim3(n_list, n_st), SBLK, 0, st>>>((const double*)d_part.p, (const int64_t*)d_first.p, n_st,
+                                                 (double*)d_pt2.p);
+  std::vector<double> detail((size_t)n_list * n_st);
+  QP_CUDA(c, cudaMemcpyAsync(detail.data(), d_pt2.p, detail.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+  QP_CUDA(c, cudaStreamSynchronize(st));
+  for (int l = 0; l < n_list; ++l)
+    for (int s = 0; s < n_st; ++s) pt2[s] += detail[(size_t)l * n_st + s];
+  if (per_gen) std::copy(detail.begin(), detail.end(), per_gen);
   if (n_ext) *n_ext = (int64_t)hcnt[0];
   const uint64_t nc = std::min<uint64_t>(hcnt[1], cap);
   int nout = (int)std::min<uint64_t>(nc, (uint64_t)buf_size);
