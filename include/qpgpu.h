@@ -299,7 +299,11 @@ int qpgpu_mlp_train(qpgpu_ctx* ctx, int epochs, int batch, float lr, uint64_t se
  * over a work queue of (problem, row chunk) items, the Davidson algebra of all
  * problems runs in batched kernels, the device part of each iteration is
  * replayed from CUDA graphs, and the persistent kernel's launch shape is
- * autotuned on the first call.  All problems must share S_z. */
+ * autotuned on the first call.  All problems must share S_z.  The contexts must
+ * outlive the batch; once integrals or determinants of one of them are set
+ * again, qpgpu_batch_davidson gives QPGPU_ERR_STATE (make a new batch).  The
+ * Davidson storage of all problems and the graphs stay with the batch between
+ * calls, and are given back by qpgpu_batch_destroy. */
 typedef struct qpgpu_batch qpgpu_batch;
 typedef struct qpgpu_batch_stats {
   int32_t n_iter;              /* Davidson iterations (all problems advance together) */

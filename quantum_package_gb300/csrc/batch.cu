@@ -480,6 +480,7 @@ struct GraphCache {
 
 struct qpgpu_batch {
   std::vector<qpgpu_ctx*> ctx;
+  std::vector<uint64_t> set_id;  // the sets that the batch was made with
   int np = 0;
   cudaStream_t st = nullptr;
   std::string last_error;
@@ -659,6 +660,7 @@ int qpgpu_batch_create(qpgpu_ctx* const* ctxs, int n, qpgpu_batch** out) {
   int64_t base = 0;
   for (int i = 0; i < n; ++i) {
     qpgpu_ctx* c = ctxs[i];
+    B->set_id.push_back(c->set_id);
     BProb& p = B->h[i];
     std::memset(&p, 0, sizeof(BProb));
     p.N = c->N;
@@ -717,6 +719,10 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
   if (nsd < 1 || nsd > BMAXS || (prm->precision != QPGPU_FP64 && prm->precision != QPGPU_FP32) ||
       prm->preconditioner != 0)
     return bfail(B, QPGPU_ERR_ARG, "bad batch Davidson parameters (n_states_diag <= 8, diagonal step only)");
+  // the arrays of a set that has gone are other memory of its context's pool by now
+  for (int p = 0; p < np; ++p)
+    if (B->ctx[p]->set_id != B->set_id[p])
+      return bfail(B, QPGPU_ERR_STATE, "the integrals or determinants of a problem were set again after the batch was made");
   int64_t minN = INT64_MAX, maxN = 0;
   for (int p = 0; p < np; ++p) {
     if (n_states[p] < 1 || n_states[p] > nsd || dim_in[p] < B->h[p].N || !u_in[p])

@@ -373,6 +373,7 @@ void qp_free_dets(qpgpu_ctx* c) {
     *p = nullptr;
   }
   c->have_dets = false;
+  ++c->set_id;
   c->N = 0;
 }
 

@@ -547,6 +547,7 @@ struct qpgpu_ctx {
 
   // determinant set
   bool have_dets = false;
+  uint64_t set_id = 0;  // counts the sets dropped (qp_free_dets): a batch checks that its set is still there
   int64_t N = 0;
   int Ua = 0, Ub = 0;
   u64* d_dets = nullptr;       // (nint,2,N) original order
