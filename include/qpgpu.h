@@ -60,7 +60,7 @@ typedef struct qpgpu_info {
   int64_t n_s2_pairs;     /* pairs with <I|S^2|J> != 0 */
   double setup_ms;        /* device time of the last qpgpu_set_dets */
   double ref_energy;      /* ref_bitmask_energy */
-  int64_t device_bytes;   /* device memory held by the context */
+  int64_t device_bytes;   /* device memory held by the context, kept work memory included */
   int64_t n_split_rows;   /* rows whose pairs span several sigma work chunks */
   int32_t direct_sigma;   /* 1: pairs not stored, sigma enumerates them at each call */
   int32_t n_keyed_lines;  /* beta columns + alpha rows with deletion-key tables */

@@ -167,7 +167,7 @@ int check_ctx(qpgpu_ctx* c, bool need_ints, bool need_dets) {
 void free_ints(qpgpu_ctx* c) {
   double** ps[] = {&c->d_eri, &c->d_h, &c->d_jj, &c->d_kk, &c->d_ja, &c->d_bc, &c->d_bx, &c->d_fock, &c->d_eref};
   for (auto p : ps) {
-    dev_free(*p);
+    dev_free(c, *p);
     *p = nullptr;
   }
   c->have_ints = false;
@@ -175,15 +175,36 @@ void free_ints(qpgpu_ctx* c) {
 
 int ensure_work(qpgpu_ctx* c, size_t bytes) {
   if (c->work_bytes >= bytes) return 0;
-  dev_free(c->d_work);
+  dev_free(c, c->d_work);
   c->d_work = nullptr;
   c->work_bytes = 0;
-  QP_CUDA(c, cudaMalloc((void**)&c->d_work, bytes));
+  QP_CUDA(c, qp_dev_malloc(c, (void**)&c->d_work, bytes));
   c->work_bytes = bytes;
   return 0;
 }
 
 }  // namespace
+
+cudaError_t qp_dev_malloc(qpgpu_ctx* c, void** p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    return e;
+  }
+  c->dev.emplace(*p, bytes);
+  c->dev_bytes += bytes;
+  return e;
+}
+
+void dev_free(qpgpu_ctx* c, void* p) {
+  if (!p) return;
+  const auto it = c->dev.find(p);
+  if (it != c->dev.end()) {
+    c->dev_bytes -= it->second;
+    c->dev.erase(it);
+  }
+  cudaFree(p);
+}
 
 cudaError_t qp_pool_alloc(qpgpu_ctx* c, void** p, size_t bytes) {
   cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
@@ -226,6 +247,12 @@ void qp_pool_idle(qpgpu_ctx* c) {
   if (cur >= 0 && cur != c->device) cudaSetDevice(cur);
 }
 
+size_t qp_pool_reserved(qpgpu_ctx* c) {
+  uint64_t reserved = 0;
+  if (cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess) return 0;
+  return (size_t)reserved;
+}
+
 size_t qp_pool_cached(qpgpu_ctx* c) {
   uint64_t used = 0, reserved = 0;
   if (cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
@@ -254,7 +281,7 @@ void qp_report_marks(qpgpu_ctx* c) {
 }
 
 int qp_numeric_flag(qpgpu_ctx* c, cudaStream_t st, int** flag) {
-  if (!c->d_flag) QP_CUDA(c, cudaMalloc((void**)&c->d_flag, 64));
+  if (!c->d_flag) QP_CUDA(c, qp_dev_malloc(c, (void**)&c->d_flag, 64));
   QP_CUDA(c, cudaMemsetAsync(c->d_flag, 0, sizeof(int), st));
   *flag = c->d_flag;
   return 0;
@@ -339,13 +366,13 @@ int qpgpu_destroy(qpgpu_ctx* c) {
     qp_free_pairs(c);
     qp_free_dets(c);
     free_ints(c);
-    c->mlp.free_all();
-    dev_free(c->d_work);
-    dev_free(c->d_stage);
-    dev_free(c->d_ffu);
-    dev_free(c->d_direct_ut);
-    dev_free(c->d_flag);
-    dev_free(c->d_tc_scratch);
+    c->mlp.free_all(c);
+    dev_free(c, c->d_work);
+    dev_free(c, c->d_stage);
+    dev_free(c, c->d_ffu);
+    dev_free(c, c->d_direct_ut);
+    dev_free(c, c->d_flag);
+    dev_free(c, c->d_tc_scratch);
     if (c->h_pin) cudaFreeHost(c->h_pin);
     cudaStreamSynchronize(c->stream);
     cudaMemPoolDestroy(c->pool);
@@ -371,16 +398,7 @@ int qpgpu_get_info(qpgpu_ctx* c, qpgpu_info* info) {
   info->n_s2_pairs = c->P_s2;
   info->setup_ms = c->setup_ms;
   info->ref_energy = c->tab.e_ref;
-  const int64_t n = c->n_mo, N = c->N, P = c->P;
-  int64_t b = 0;
-  if (c->have_ints) b += 8 * (n * (n + 1) / 2) * (n * (n + 1) / 2 + 1) / 2 + 8 * (6 * n * n + 2 * n * n * n);
-  if (c->have_dets) b += N * (32 * c->nint + 4 * 8) + 8 * (int64_t)(c->Ua + c->Ub) * c->nint;
-  if (c->have_pairs && !c->direct) b += P * 16 + c->P_s2 * 8 + N * 28;
-  if (c->have_pairs && c->direct) b += N * 24;
-  for (int k = 0; k < KT_N; ++k) b += c->kslots[k] * (int64_t)sizeof(KeySlot) + c->kmem_n[k] * 4;
-  if (c->have_dets) b += c->Ua + c->Ub;
-  b += (int64_t)c->work_bytes;
-  info->device_bytes = b;
+  info->device_bytes = (int64_t)(qp_pool_reserved(c) + c->dev_bytes);
   info->n_split_rows = c->direct ? 0 : c->items.n_multi;  // of the stored pairs
   info->direct_sigma = c->direct ? 1 : 0;
   info->n_keyed_lines = c->n_keyed_lines;
@@ -424,11 +442,11 @@ int qpgpu_set_integrals(qpgpu_ctx* c, const double* h, const double* eri) {
   const int64_t p2 = (int64_t)n * (n + 1) / 2;
   const int64_t npk = p2 * (p2 + 1) / 2;
   cudaStream_t st = c->stream;
-  if (dev_alloc(&c->d_eri, npk) != cudaSuccess || dev_alloc(&c->d_h, (size_t)n * n) != cudaSuccess ||
-      dev_alloc(&c->d_jj, (size_t)n * n) != cudaSuccess || dev_alloc(&c->d_kk, (size_t)n * n) != cudaSuccess ||
-      dev_alloc(&c->d_ja, (size_t)n * n) != cudaSuccess || dev_alloc(&c->d_fock, (size_t)n * n) != cudaSuccess ||
-      dev_alloc(&c->d_bc, (size_t)n * n * n) != cudaSuccess || dev_alloc(&c->d_bx, (size_t)n * n * n) != cudaSuccess ||
-      dev_alloc(&c->d_eref, 1) != cudaSuccess) {
+  if (dev_alloc(c, &c->d_eri, npk) != cudaSuccess || dev_alloc(c, &c->d_h, (size_t)n * n) != cudaSuccess ||
+      dev_alloc(c, &c->d_jj, (size_t)n * n) != cudaSuccess || dev_alloc(c, &c->d_kk, (size_t)n * n) != cudaSuccess ||
+      dev_alloc(c, &c->d_ja, (size_t)n * n) != cudaSuccess || dev_alloc(c, &c->d_fock, (size_t)n * n) != cudaSuccess ||
+      dev_alloc(c, &c->d_bc, (size_t)n * n * n) != cudaSuccess || dev_alloc(c, &c->d_bx, (size_t)n * n * n) != cudaSuccess ||
+      dev_alloc(c, &c->d_eref, 1) != cudaSuccess) {
     cudaGetLastError();
     free_ints(c);
     return qpgpu_fail(c, QPGPU_ERR_NOMEM, "integral tables do not fit on the device");
@@ -626,10 +644,10 @@ int h_s2_u0_host(qpgpu_ctx* c, double* v0, double* s0, const double* u0, int n_s
   Lock l(c->mu);
   if (cols <= H_S2_PIN_DOUBLES) return h_s2_u0_pinned(c, v0, s0, u0, n_st, ld, dressed);
   if (c->stage_bytes < 3 * cols * sizeof(double)) {
-    dev_free(c->d_stage);
+    dev_free(c, c->d_stage);
     c->d_stage = nullptr;
     c->stage_bytes = 0;
-    QP_CUDA(c, cudaMalloc((void**)&c->d_stage, 3 * cols * sizeof(double)));
+    QP_CUDA(c, qp_dev_malloc(c, (void**)&c->d_stage, 3 * cols * sizeof(double)));
     c->stage_bytes = 3 * cols * sizeof(double);
   }
   double *du = c->d_stage, *dv = du + cols, *ds = du + 2 * cols;
@@ -709,10 +727,10 @@ int qpgpu_u0_h_u0(qpgpu_ctx* c, double* e_0, const double* u0, int n_st, int64_t
   Lock l(c->mu);
   PoolTrim trim{c};
   if (c->stage_bytes < 3 * cols * sizeof(double)) {
-    dev_free(c->d_stage);
+    dev_free(c, c->d_stage);
     c->d_stage = nullptr;
     c->stage_bytes = 0;
-    QP_CUDA(c, cudaMalloc((void**)&c->d_stage, 3 * cols * sizeof(double)));
+    QP_CUDA(c, qp_dev_malloc(c, (void**)&c->d_stage, 3 * cols * sizeof(double)));
     c->stage_bytes = 3 * cols * sizeof(double);
   }
   double *du = c->d_stage, *dv = du + cols, *ds = du + 2 * cols;

@@ -1013,9 +1013,9 @@ struct Dav {
     qp_pool_free(c, u32);
     qp_pool_free(c, part);
     qp_pool_free(c, small);
-    dev_free(cX);
-    dev_free(cd);
-    dev_free(cc);
+    dev_free(c, cX);
+    dev_free(c, cd);
+    dev_free(c, cc);
     qp_pool_free(c, mlpX);
     qp_pool_free(c, mlpG);
     qp_pool_free(c, Uf);
@@ -1461,9 +1461,9 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
   if (collect_every) {
     if (!c->d_detfeat) return qpgpu_fail(c, QPGPU_ERR_STATE, "no determinant features");
     const size_t nsl = (size_t)collect_max * nst;
-    if (cudaMalloc((void**)&d.cX, nsl * N * QP_MLP_IN * sizeof(float)) != cudaSuccess ||
-        cudaMalloc((void**)&d.cd, nsl * N * sizeof(float)) != cudaSuccess ||
-        cudaMalloc((void**)&d.cc, nsl * N * sizeof(float)) != cudaSuccess) {
+    if (qp_dev_malloc(c, (void**)&d.cX, nsl * N * QP_MLP_IN * sizeof(float)) != cudaSuccess ||
+        qp_dev_malloc(c, (void**)&d.cd, nsl * N * sizeof(float)) != cudaSuccess ||
+        qp_dev_malloc(c, (void**)&d.cc, nsl * N * sizeof(float)) != cudaSuccess) {
       cudaGetLastError();
       return qpgpu_fail(c, QPGPU_ERR_NOMEM, "training capture does not fit on the device");
     }
@@ -1770,9 +1770,9 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
     double* dpart = nullptr;
     double* ddot = nullptr;
     SlotScale* dsc = nullptr;
-    QP_CUDA(c, cudaMalloc((void**)&dpart, part.size() * sizeof(double)));
-    QP_CUDA(c, cudaMalloc((void**)&ddot, nslot * sizeof(double)));
-    QP_CUDA(c, cudaMalloc((void**)&dsc, nslot * sizeof(SlotScale)));
+    QP_CUDA(c, qp_dev_malloc(c, (void**)&dpart, part.size() * sizeof(double)));
+    QP_CUDA(c, qp_dev_malloc(c, (void**)&ddot, nslot * sizeof(double)));
+    QP_CUDA(c, qp_dev_malloc(c, (void**)&dsc, nslot * sizeof(SlotScale)));
     k_capture_sums<<<d.ncta, DBLK, 0, st>>>(d.U, nsd, nst, d.cd, d.cc, nslot, N, nullptr, 0, dpart);
     QP_CUDA(c, cudaMemcpyAsync(part.data(), dpart, part.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     QP_CUDA(c, cudaStreamSynchronize(st));
@@ -1804,18 +1804,18 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
     const int64_t per_slot = (N + stride - 1) / stride;
     const int64_t total = per_slot * nslot;
     float *X = nullptr, *Gt = nullptr, *Wt = nullptr;
-    QP_CUDA(c, cudaMalloc((void**)&X, total * QP_MLP_IN * sizeof(float)));
-    QP_CUDA(c, cudaMalloc((void**)&Gt, total * sizeof(float)));
-    QP_CUDA(c, cudaMalloc((void**)&Wt, total * sizeof(float)));
+    QP_CUDA(c, qp_dev_malloc(c, (void**)&X, total * QP_MLP_IN * sizeof(float)));
+    QP_CUDA(c, qp_dev_malloc(c, (void**)&Gt, total * sizeof(float)));
+    QP_CUDA(c, qp_dev_malloc(c, (void**)&Wt, total * sizeof(float)));
     k_capture_samples<<<gsz(total), DBLK, 0, st>>>(d.U, nsd, nst, d.cX, d.cd, d.cc, nslot, N, dsc, stride, per_slot, X,
                                                    Gt, Wt);
     int rc2 = qp_mlp_append(c, X, Gt, Wt, total, true);
-    cudaFree(X);
-    cudaFree(Gt);
-    cudaFree(Wt);
-    cudaFree(dpart);
-    cudaFree(ddot);
-    cudaFree(dsc);
+    dev_free(c, X);
+    dev_free(c, Gt);
+    dev_free(c, Wt);
+    dev_free(c, dpart);
+    dev_free(c, ddot);
+    dev_free(c, dsc);
     if (rc2) return rc2;
     n_new_samples = total;
   }

@@ -96,7 +96,7 @@ void qp_free_dressing(qpgpu_ctx* c) {
   Dressing& D = c->dress;
   void* ps[] = {D.ref, D.nref, D.d, D.ds, D.dii, D.hdress};
   for (void* p : ps)
-    if (p) cudaFree(p);
+    dev_free(c, p);
   D = Dressing{};
 }
 
@@ -145,9 +145,9 @@ extern "C" int qpgpu_set_dressing(qpgpu_ctx* c, int n_ref, const int32_t* idx_re
   for (int64_t j = 0; j < n_non_ref; ++j) nref[j] = inv[idx_non_ref[j]];
   Dressing& D = c->dress;
   const size_t nd = (size_t)n_ref * n_non_ref;
-  if (dev_alloc(&D.ref, n_ref + 1) != cudaSuccess || dev_alloc(&D.nref, n_non_ref + 1) != cudaSuccess ||
-      dev_alloc(&D.d, nd + 1) != cudaSuccess || dev_alloc(&D.ds, nd + 1) != cudaSuccess ||
-      dev_alloc(&D.dii, n_ref + 1) != cudaSuccess || dev_alloc(&D.hdress, N) != cudaSuccess) {
+  if (dev_alloc(c, &D.ref, n_ref + 1) != cudaSuccess || dev_alloc(c, &D.nref, n_non_ref + 1) != cudaSuccess ||
+      dev_alloc(c, &D.d, nd + 1) != cudaSuccess || dev_alloc(c, &D.ds, nd + 1) != cudaSuccess ||
+      dev_alloc(c, &D.dii, n_ref + 1) != cudaSuccess || dev_alloc(c, &D.hdress, N) != cudaSuccess) {
     cudaGetLastError();
     qp_free_dressing(c);
     return qpgpu_fail(c, QPGPU_ERR_NOMEM, "dressing does not fit on the device");

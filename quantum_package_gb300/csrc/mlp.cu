@@ -178,9 +178,9 @@ namespace {
 
 int ensure_mlp(qpgpu_ctx* c) {
   if (c->mlp.params) return 0;
-  QP_CUDA(c, dev_alloc(&c->mlp.params, QP_MLP_NPARAM));
-  QP_CUDA(c, dev_alloc(&c->mlp.adam_m, QP_MLP_NPARAM));
-  QP_CUDA(c, dev_alloc(&c->mlp.adam_v, QP_MLP_NPARAM));
+  QP_CUDA(c, dev_alloc(c, &c->mlp.params, QP_MLP_NPARAM));
+  QP_CUDA(c, dev_alloc(c, &c->mlp.adam_m, QP_MLP_NPARAM));
+  QP_CUDA(c, dev_alloc(c, &c->mlp.adam_v, QP_MLP_NPARAM));
   return 0;
 }
 
@@ -223,13 +223,13 @@ int qp_mlp_append(qpgpu_ctx* c, const float* X, const float* G, const float* W, 
   if (m.n + n > m.cap) {
     const int64_t cap = std::max<int64_t>(2 * (m.n + n), 1 << 16);
     float *nX = nullptr, *nG = nullptr, *nW = nullptr;
-    if (cudaMalloc((void**)&nX, cap * QP_MLP_IN * sizeof(float)) != cudaSuccess ||
-        cudaMalloc((void**)&nG, cap * sizeof(float)) != cudaSuccess ||
-        cudaMalloc((void**)&nW, cap * sizeof(float)) != cudaSuccess) {
+    if (qp_dev_malloc(c, (void**)&nX, cap * QP_MLP_IN * sizeof(float)) != cudaSuccess ||
+        qp_dev_malloc(c, (void**)&nG, cap * sizeof(float)) != cudaSuccess ||
+        qp_dev_malloc(c, (void**)&nW, cap * sizeof(float)) != cudaSuccess) {
       cudaGetLastError();
-      dev_free(nX);
-      dev_free(nG);
-      dev_free(nW);
+      dev_free(c, nX);
+      dev_free(c, nG);
+      dev_free(c, nW);
       return qpgpu_fail(c, QPGPU_ERR_NOMEM, "training set does not fit on the device");
     }
     if (m.n) {
@@ -238,9 +238,9 @@ int qp_mlp_append(qpgpu_ctx* c, const float* X, const float* G, const float* W, 
       QP_CUDA(c, cudaMemcpyAsync(nW, m.Wt, m.n * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
       QP_CUDA(c, cudaStreamSynchronize(c->stream));
     }
-    dev_free(m.X);
-    dev_free(m.G);
-    dev_free(m.Wt);
+    dev_free(c, m.X);
+    dev_free(c, m.G);
+    dev_free(c, m.Wt);
     m.X = nX;
     m.G = nG;
     m.Wt = nW;
@@ -337,9 +337,9 @@ int qpgpu_mlp_gradient(qpgpu_ctx* c, const float* X, const float* G, const float
   const int ncta = 256;
   int* d_idx = nullptr;
   float *d_part = nullptr, *d_grad = nullptr;
-  QP_CUDA(c, cudaMalloc((void**)&d_idx, n * sizeof(int)));
-  QP_CUDA(c, cudaMalloc((void**)&d_part, (size_t)ncta * (QP_MLP_NPARAM + 1) * sizeof(float)));
-  QP_CUDA(c, cudaMalloc((void**)&d_grad, (QP_MLP_NPARAM + 1) * sizeof(float)));
+  QP_CUDA(c, qp_dev_malloc(c, (void**)&d_idx, n * sizeof(int)));
+  QP_CUDA(c, qp_dev_malloc(c, (void**)&d_part, (size_t)ncta * (QP_MLP_NPARAM + 1) * sizeof(float)));
+  QP_CUDA(c, qp_dev_malloc(c, (void**)&d_grad, (QP_MLP_NPARAM + 1) * sizeof(float)));
   QP_CUDA(c, cudaMemcpyAsync(d_idx, idx.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
   rc = mlp_gradient(c, d_idx, (int)n, d_part, ncta, d_grad, false, 0.f);
   std::vector<float> g(QP_MLP_NPARAM + 1);
@@ -347,9 +347,9 @@ int qpgpu_mlp_gradient(qpgpu_ctx* c, const float* X, const float* G, const float
     QP_CUDA(c, cudaMemcpyAsync(g.data(), d_grad, g.size() * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
     QP_CUDA(c, cudaStreamSynchronize(c->stream));
   }
-  cudaFree(d_idx);
-  cudaFree(d_part);
-  cudaFree(d_grad);
+  dev_free(c, d_idx);
+  dev_free(c, d_part);
+  dev_free(c, d_grad);
   c->mlp.n = keep;  // the probe samples are not kept
   if (rc) return rc;
   std::memcpy(grad, g.data(), QP_MLP_NPARAM * sizeof(float));
@@ -362,14 +362,14 @@ int qpgpu_mlp_predict(qpgpu_ctx* c, const float* X, int64_t n, float* y) {
   if (!c->mlp.ready) return qpgpu_fail(c, QPGPU_ERR_STATE, "MLP not initialised");
   Lk l(c->mu);
   float *dX = nullptr, *dy = nullptr;
-  QP_CUDA(c, cudaMalloc((void**)&dX, n * QP_MLP_IN * sizeof(float)));
-  QP_CUDA(c, cudaMalloc((void**)&dy, n * sizeof(float)));
+  QP_CUDA(c, qp_dev_malloc(c, (void**)&dX, n * QP_MLP_IN * sizeof(float)));
+  QP_CUDA(c, qp_dev_malloc(c, (void**)&dy, n * sizeof(float)));
   QP_CUDA(c, cudaMemcpyAsync(dX, X, n * QP_MLP_IN * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   k_mlp_predict<<<gsz(n), 256, 0, c->stream>>>(c->mlp.params, dX, dy, n);
   cudaError_t e = cudaMemcpyAsync(y, dy, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  cudaFree(dX);
-  cudaFree(dy);
+  dev_free(c, dX);
+  dev_free(c, dy);
   if (e != cudaSuccess) return qpgpu_fail(c, QPGPU_ERR_CUDA, cudaGetErrorString(e));
   return QPGPU_OK;
 }
@@ -385,9 +385,9 @@ int qpgpu_mlp_train(qpgpu_ctx* c, int epochs, int batch, float lr, uint64_t seed
   const int ncta = 256;
   int* d_idx = nullptr;
   float *d_part = nullptr, *d_grad = nullptr;
-  QP_CUDA(c, cudaMalloc((void**)&d_idx, n * sizeof(int)));
-  QP_CUDA(c, cudaMalloc((void**)&d_part, (size_t)ncta * (QP_MLP_NPARAM + 1) * sizeof(float)));
-  QP_CUDA(c, cudaMalloc((void**)&d_grad, (QP_MLP_NPARAM + 1) * sizeof(float)));
+  QP_CUDA(c, qp_dev_malloc(c, (void**)&d_idx, n * sizeof(int)));
+  QP_CUDA(c, qp_dev_malloc(c, (void**)&d_part, (size_t)ncta * (QP_MLP_NPARAM + 1) * sizeof(float)));
+  QP_CUDA(c, qp_dev_malloc(c, (void**)&d_grad, (QP_MLP_NPARAM + 1) * sizeof(float)));
   std::vector<int> idx(n);
   std::iota(idx.begin(), idx.end(), 0);
   std::mt19937_64 gen(seed);
@@ -411,9 +411,9 @@ int qpgpu_mlp_train(qpgpu_ctx* c, int epochs, int batch, float lr, uint64_t seed
     }
   }
   QP_CUDA(c, cudaStreamSynchronize(c->stream));
-  cudaFree(d_idx);
-  cudaFree(d_part);
-  cudaFree(d_grad);
+  dev_free(c, d_idx);
+  dev_free(c, d_part);
+  dev_free(c, d_grad);
   if (loss) *loss = (float)last;
   return rc;
 }

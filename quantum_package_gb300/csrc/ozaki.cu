@@ -1191,10 +1191,10 @@ extern "C" int qpgpu_gram_tc(qpgpu_ctx* c, const double* A, int64_t lda, int m, 
   const int ncta = c->n_sm;
   const size_t need = (size_t)ncta * m * n * sizeof(double) + (size_t)(m + n + 8) * sizeof(int) + 256;
   if (c->tc_scratch_bytes < need) {
-    dev_free(c->d_tc_scratch);
+    dev_free(c, c->d_tc_scratch);
     c->d_tc_scratch = nullptr;
     c->tc_scratch_bytes = 0;
-    QP_CUDA(c, cudaMalloc(&c->d_tc_scratch, need));
+    QP_CUDA(c, qp_dev_malloc(c, &c->d_tc_scratch, need));
     c->tc_scratch_bytes = need;
   }
   double* part = (double*)c->d_tc_scratch;
@@ -1221,10 +1221,10 @@ extern "C" int qpgpu_lincomb_tc(qpgpu_ctx* c, const double* A, int64_t sA, int m
     return qpgpu_fail(c, QPGPU_ERR_ARG, "lincomb_tc: need m = nb nsd <= 128, nsd <= 16, N >= 1, ldO >= nsd, sA >= N nsd");
   std::lock_guard<std::mutex> lk(c->mu);
   if (!c->d_tc_scratch || c->tc_scratch_bytes < sizeof(int)) {
-    dev_free(c->d_tc_scratch);
+    dev_free(c, c->d_tc_scratch);
     c->d_tc_scratch = nullptr;
     c->tc_scratch_bytes = 0;
-    QP_CUDA(c, cudaMalloc(&c->d_tc_scratch, 256));
+    QP_CUDA(c, qp_dev_malloc(c, &c->d_tc_scratch, 256));
     c->tc_scratch_bytes = 256;
   }
   int* status = (int*)c->d_tc_scratch;

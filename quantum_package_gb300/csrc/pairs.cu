@@ -1679,10 +1679,10 @@ int qp_sigma_direct(qpgpu_ctx* c, double* v, double* s, const double* u, int nst
   if (row_step < 1) return qpgpu_fail(c, QPGPU_ERR_ARG, "row step must be >= 1");
   const size_t need = (size_t)c->N * nst;
   if (c->direct_ut_n < need) {
-    dev_free(c->d_direct_ut);
+    dev_free(c, c->d_direct_ut);
     c->d_direct_ut = nullptr;
     c->direct_ut_n = 0;
-    QP_CUDA(c, dev_alloc(&c->d_direct_ut, need));
+    QP_CUDA(c, dev_alloc(c, &c->d_direct_ut, need));
     c->direct_ut_n = need;
   }
   if (!c->d_direct_cols) {  // column buffer: the whole set if it fits in half the free memory
@@ -1696,8 +1696,8 @@ int qp_sigma_direct(qpgpu_ctx* c, double* v, double* s, const double* u, int nst
     // force many chunks)
     if (const char* e = getenv("QPGPU_DIRECT_CHUNK_COLS")) cap = std::min<int64_t>(cap, atoll(e) > 0 ? atoll(e) : cap);
     cap = std::max<int64_t>(cap, maxrow);
-    QP_CUDA(c, dev_alloc(&c->d_direct_cols, (size_t)std::max<int64_t>(cap, 1)));
-    QP_CUDA(c, dev_alloc(&c->d_direct_err, 1));
+    QP_CUDA(c, dev_alloc(c, &c->d_direct_cols, (size_t)std::max<int64_t>(cap, 1)));
+    QP_CUDA(c, dev_alloc(c, &c->d_direct_err, 1));
     QP_CUDA(c, cudaMemsetAsync(c->d_direct_err, 0, sizeof(int), st));
     c->direct_cols_cap = cap;
   }
@@ -1729,7 +1729,7 @@ void qp_free_pairs(qpgpu_ctx* c) {
   // grown by a sigma on the caller's stream: not from the pool
   void** up[] = {(void**)&c->d_val32lo, (void**)&c->d_direct_cols, (void**)&c->d_direct_err};
   for (auto p : up) {
-    dev_free(*p);
+    dev_free(c, *p);
     *p = nullptr;
   }
   c->direct_cols_cap = 0;

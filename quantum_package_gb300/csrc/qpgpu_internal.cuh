@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/qpgpu.h"
@@ -445,6 +446,7 @@ __device__ __forceinline__ void pair_of_combo(int c, int ne, int& i, int& j) {
 
 struct qpgpu_ctx;
 void qp_pool_free(qpgpu_ctx* c, void* p);  // ctx.cu
+void dev_free(qpgpu_ctx* c, void* p);      // ctx.cu
 
 // Rows are split into chunks of at most QP_SIGMA_CHUNK pairs, one warp each.
 #define QP_SIGMA_CHUNK 2048
@@ -470,8 +472,8 @@ struct SigmaItems {
     qp_pool_free(c, item_row);
     qp_pool_free(c, item_sub);
     qp_pool_free(c, multi_rows);
-    if (pv) cudaFree(pv);
-    if (ps) cudaFree(ps);
+    dev_free(c, pv);
+    dev_free(c, ps);
     row_nitems = row_item0 = item_row = item_sub = multi_rows = nullptr;
     pv = ps = nullptr;
     partial_cap = 0;
@@ -504,10 +506,10 @@ struct MlpState {
   float* G = nullptr;
   float* Wt = nullptr;
   int64_t n = 0, cap = 0;
-  void free_all() {
+  template <class Ctx>
+  void free_all(Ctx* c) {
     void* ps[] = {params, adam_m, adam_v, X, G, Wt};
-    for (void* p : ps)
-      if (p) cudaFree(p);
+    for (void* p : ps) dev_free(c, p);
     params = adam_m = adam_v = X = G = Wt = nullptr;
     n = cap = 0;
     adam_t = 0;
@@ -534,6 +536,8 @@ struct qpgpu_ctx {
   int n_sm = 0;  // streaming multiprocessors of the device (read at create)
   cudaStream_t stream = nullptr;
   cudaMemPool_t pool = nullptr;  // see qp_pool_alloc
+  std::unordered_map<void*, size_t> dev;  // arrays beside the pool (qp_dev_malloc) and their bytes
+  size_t dev_bytes = 0;                   // all of them together
   cudaStream_t side[2] = {nullptr, nullptr};  // kernels beside those of a call's stream (qp_fork, qp_join)
   cudaEvent_t side_ev[2] = {nullptr, nullptr};
   std::string last_error;
@@ -645,12 +649,11 @@ int qpgpu_fail(qpgpu_ctx* c, int code, const std::string& msg);
       return qpgpu_fail((c), QPGPU_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
   } while (0)
 
+// cudaMalloc, counted in the context (dev_free takes it off)
+cudaError_t qp_dev_malloc(qpgpu_ctx* c, void** p, size_t bytes);
 template <class T>
-inline cudaError_t dev_alloc(T** p, size_t count) {
-  return cudaMalloc((void**)p, count * sizeof(T) + 16);
-}
-inline void dev_free(void* p) {
-  if (p) cudaFree(p);
+inline cudaError_t dev_alloc(qpgpu_ctx* c, T** p, size_t count) {
+  return qp_dev_malloc(c, (void**)p, count * sizeof(T) + 16);
 }
 
 // Memory of a determinant set and of the work arrays of one call comes from a
@@ -668,7 +671,8 @@ inline void dev_free(void* p) {
 cudaError_t qp_pool_alloc(qpgpu_ctx* c, void** p, size_t bytes);
 void qp_pool_idle(qpgpu_ctx* c);
 void qp_pool_trim(qpgpu_ctx* c);
-size_t qp_pool_cached(qpgpu_ctx* c);  // reserved bytes that are not in use
+size_t qp_pool_reserved(qpgpu_ctx* c);  // bytes that the pool holds on the device
+size_t qp_pool_cached(qpgpu_ctx* c);    // those of them that are not in use
 struct PoolTrim {  // trims when a call ends
   qpgpu_ctx* c;
   ~PoolTrim() { qp_pool_trim(c); }

@@ -639,12 +639,12 @@ int qp_build_sigma_items(qpgpu_ctx* c, SigmaItems* it) {
 int qp_ensure_partials(qpgpu_ctx* c, SigmaItems* it, int nst) {
   const size_t need = (size_t)it->n_items * nst;
   if (it->partial_cap >= need) return 0;
-  dev_free(it->pv);
-  dev_free(it->ps);
+  dev_free(c, it->pv);
+  dev_free(c, it->ps);
   it->pv = it->ps = nullptr;
   it->partial_cap = 0;
-  QP_CUDA(c, dev_alloc(&it->pv, need));
-  QP_CUDA(c, dev_alloc(&it->ps, need));
+  QP_CUDA(c, dev_alloc(c, &it->pv, need));
+  QP_CUDA(c, dev_alloc(c, &it->ps, need));
   it->partial_cap = need;
   return 0;
 }
@@ -740,16 +740,16 @@ int qp_sigma_ff(qpgpu_ctx* c, SigmaItems* it, double* v, double* s, const double
   if (c->direct) return qp_sigma_direct(c, v, s, u, nst, st, row_lo, row_hi, row_first, row_step);
   const int64_t N = c->N;
   if (!c->d_val32lo) {  // once per determinant set
-    QP_CUDA(c, dev_alloc(&c->d_val32lo, c->P));
+    QP_CUDA(c, dev_alloc(c, &c->d_val32lo, c->P));
     k_lo_parts<<<gsz(c->P, 256), 256, 0, st>>>(c->d_val64, c->d_val32, c->d_val32lo, c->P);
   }
   const int ld = qp_pad_states(nst);
   const size_t half = ((size_t)N * ld + 63) / 64 * 64;  // keeps lo 256-byte aligned
   if (c->ffu_floats < 2 * half) {
-    dev_free(c->d_ffu);
+    dev_free(c, c->d_ffu);
     c->d_ffu = nullptr;
     c->ffu_floats = 0;
-    QP_CUDA(c, dev_alloc(&c->d_ffu, 2 * half));
+    QP_CUDA(c, dev_alloc(c, &c->d_ffu, 2 * half));
     c->ffu_floats = 2 * half;
   }
   float* hi = c->d_ffu;
