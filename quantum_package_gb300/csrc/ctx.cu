@@ -434,6 +434,7 @@ int qpgpu_set_integrals(qpgpu_ctx* c, const double* h, const double* eri) {
       if (h[i + (size_t)j * n] != h[j + (size_t)i * n])
         return qpgpu_fail(c, QPGPU_ERR_ARG, "h_pq must be symmetric");
   qp_pool_idle(c);
+  PoolTrim trim{c};  // the set that goes
   c->items.free_all(c);
   qp_free_dressing(c);
   qp_free_pairs(c);

@@ -1,9 +1,10 @@
 """Device memory that a context keeps: what qpgpu_info reports is what the
-device has given.
+device has given, and a determinant set that goes gives its memory back.
 
 Bars: the reported bytes of a context are those by which the device's free
 memory changed, to 4 MiB an allocation of the driver's granularity (2 MiB) for
-each of its larger arrays.
+each of its larger arrays; after qpgpu_set_integrals drops the set of 2e5
+determinants the context holds its integral tables and at most 256 MiB.
 """
 import pytest
 
@@ -44,3 +45,14 @@ def test_reported_bytes(warm, mode):
     assert abs(wf.info()["device_bytes"] - held) <= 80 * MIB, (wf.info()["device_bytes"], held)
     wf.close()
     assert before - _free() <= 4 * MIB
+
+
+def test_new_integrals_give_the_set_back(warm):
+    from quantum_package_gb300.sigma import Wavefunction
+    p = G.make_problem(2, n_det=200_000)
+    before = _free()
+    wf = Wavefunction.from_problem(p, SIGMA_STORED)
+    assert before - _free() > 1500 * MIB  # the stored pairs
+    wf.set_integrals(p.ints.h, p.ints.eri)
+    assert before - _free() <= (256 + 128) * MIB
+    wf.close()
