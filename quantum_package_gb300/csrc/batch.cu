@@ -650,8 +650,8 @@ int qpgpu_batch_create(qpgpu_ctx* const* ctxs, int n, qpgpu_batch** out) {
   B->np = n;
   B->sm_count = ctxs[0]->n_sm;
   if (cudaStreamCreateWithFlags(&B->st, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc((void**)&B->d_counter, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc((void**)&B->d, n * sizeof(BProb)) != cudaSuccess) {
+      qp_device_malloc(ctxs[0]->device, (void**)&B->d_counter, sizeof(unsigned long long)) != cudaSuccess ||
+      qp_device_malloc(ctxs[0]->device, (void**)&B->d, n * sizeof(BProb)) != cudaSuccess) {
     cudaGetLastError();
     delete B;
     return QPGPU_ERR_CUDA;
@@ -781,7 +781,7 @@ int qpgpu_batch_davidson(qpgpu_batch* B, double* const* u_in, const int64_t* dim
       cudaFree(B->slab);
       B->slab = nullptr;
       B->slab_bytes = 0;
-      if (cudaMalloc((void**)&B->slab, off) != cudaSuccess) {
+      if (qp_device_malloc(B->ctx[0]->device, (void**)&B->slab, off) != cudaSuccess) {
         cudaGetLastError();
         return bfail(B, QPGPU_ERR_NOMEM, "batch Davidson storage does not fit on the device");
       }

@@ -185,12 +185,56 @@ int ensure_work(qpgpu_ctx* c, size_t bytes) {
 
 }  // namespace
 
-cudaError_t qp_dev_malloc(qpgpu_ctx* c, void** p, size_t bytes) {
-  const cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) {
-    *p = nullptr;
-    return e;
+namespace {
+struct Pools {  // of all contexts of the process
+  std::mutex mu;
+  std::vector<std::pair<int, cudaMemPool_t>> v;  // device, pool
+};
+Pools& pools() {
+  static Pools* p = new Pools;  // contexts may go after the statics
+  return *p;
+}
+
+// the context's memory limit (environment QPGPU_MEMORY_LIMIT) does not allow
+// this many bytes more in the pool / beside it
+bool over_limit(qpgpu_ctx* c, size_t pool_more, size_t dev_more) {
+  if (c->memory_limit == 0) return false;
+  const size_t reserved = qp_pool_reserved(c), used = reserved - qp_pool_cached(c);
+  return std::max(reserved, used + pool_more) + c->dev_bytes + dev_more > c->memory_limit;
+}
+}  // namespace
+
+void qp_give_back(int device) {
+  int cur = -1;
+  if (cudaGetDevice(&cur) == cudaSuccess && cur != device) cudaSetDevice(device);
+  cudaDeviceSynchronize();  // a block whose free is still queued cannot go
+  {
+    std::lock_guard<std::mutex> l(pools().mu);
+    for (auto& p : pools().v)
+      if (p.first == device) cudaMemPoolTrimTo(p.second, 0);
   }
+  if (cur >= 0 && cur != device) cudaSetDevice(cur);
+}
+
+cudaError_t qp_device_malloc(int device, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    qp_give_back(device);
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
+
+cudaError_t qp_dev_malloc(qpgpu_ctx* c, void** p, size_t bytes) {
+  *p = nullptr;
+  if (over_limit(c, 0, bytes)) {
+    qp_give_back(c->device);
+    if (over_limit(c, 0, bytes)) return cudaErrorMemoryAllocation;
+  }
+  const cudaError_t e = qp_device_malloc(c->device, p, bytes);
+  if (e != cudaSuccess) return e;
   c->dev.emplace(*p, bytes);
   c->dev_bytes += bytes;
   return e;
@@ -207,12 +251,12 @@ void dev_free(qpgpu_ctx* c, void* p) {
 }
 
 cudaError_t qp_pool_alloc(qpgpu_ctx* c, void** p, size_t bytes) {
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
-  if (e != cudaSuccess) {  // cached blocks may hold the memory that is missing
+  cudaError_t e = cudaErrorMemoryAllocation;
+  if (!over_limit(c, bytes, 0)) e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+  if (e != cudaSuccess) {  // blocks cached here or by another context may be the memory that is missing
     cudaGetLastError();
-    cudaStreamSynchronize(c->stream);
-    cudaMemPoolTrimTo(c->pool, 0);
-    e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+    qp_give_back(c->device);
+    if (!over_limit(c, bytes, 0)) e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
   }
   if (e != cudaSuccess) *p = nullptr;
   return e;
@@ -325,6 +369,8 @@ int qpgpu_create(int n_mo, int n_alpha, int n_beta, int n_int, qpgpu_ctx** out) 
   {
     const char* pe = getenv("QPGPU_PROFILE");
     c->profile = pe && pe[0] == '1';
+    const char* ml = getenv("QPGPU_MEMORY_LIMIT");  // device bytes that a context may hold
+    if (ml && atoll(ml) > 0) c->memory_limit = (size_t)atoll(ml);
   }
   if (cudaGetDevice(&c->device) != cudaSuccess || cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
@@ -351,6 +397,8 @@ int qpgpu_create(int n_mo, int n_alpha, int n_beta, int n_int, qpgpu_ctx** out) 
       delete c;
       return QPGPU_ERR_CUDA;
     }
+    std::lock_guard<std::mutex> l(pools().mu);
+    pools().v.emplace_back(c->device, c->pool);
   }
   *out = c;
   return QPGPU_OK;
@@ -375,6 +423,11 @@ int qpgpu_destroy(qpgpu_ctx* c) {
     dev_free(c, c->d_tc_scratch);
     if (c->h_pin) cudaFreeHost(c->h_pin);
     cudaStreamSynchronize(c->stream);
+    {
+      std::lock_guard<std::mutex> l(pools().mu);
+      auto& v = pools().v;
+      v.erase(std::remove(v.begin(), v.end(), std::make_pair(c->device, c->pool)), v.end());
+    }
     cudaMemPoolDestroy(c->pool);
     for (int i = 0; i < 2; ++i) {
       if (c->side[i]) cudaStreamDestroy(c->side[i]);

@@ -538,6 +538,7 @@ struct qpgpu_ctx {
   cudaMemPool_t pool = nullptr;  // see qp_pool_alloc
   std::unordered_map<void*, size_t> dev;  // arrays beside the pool (qp_dev_malloc) and their bytes
   size_t dev_bytes = 0;                   // all of them together
+  size_t memory_limit = 0;                // bytes the context may hold (environment QPGPU_MEMORY_LIMIT; 0: no limit)
   cudaStream_t side[2] = {nullptr, nullptr};  // kernels beside those of a call's stream (qp_fork, qp_join)
   cudaEvent_t side_ev[2] = {nullptr, nullptr};
   std::string last_error;
@@ -649,7 +650,12 @@ int qpgpu_fail(qpgpu_ctx* c, int code, const std::string& msg);
       return qpgpu_fail((c), QPGPU_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
   } while (0)
 
-// cudaMalloc, counted in the context (dev_free takes it off)
+// qp_give_back: every pool of the process on the device returns what is not in
+// use.  An allocation that fails, in a pool or by cudaMalloc, is tried again
+// after it: cudaMalloc does not see what a pool keeps mapped.
+void qp_give_back(int device);
+cudaError_t qp_device_malloc(int device, void** p, size_t bytes);
+// the same, counted in the context (dev_free takes it off)
 cudaError_t qp_dev_malloc(qpgpu_ctx* c, void** p, size_t bytes);
 template <class T>
 inline cudaError_t dev_alloc(qpgpu_ctx* c, T** p, size_t count) {
@@ -666,8 +672,7 @@ inline cudaError_t dev_alloc(qpgpu_ctx* c, T** p, size_t count) {
 // now.  qp_pool_trim() at the end of a call bounds what the pool keeps
 // beyond the live bytes to half of those (at least 256 MiB, which the work
 // arrays of a selection over 1e7 entries fit: mapping and unmapping them at
-// each call took 1.2 of its 6.2 ms), and an allocation
-// that fails is tried again after the pool has given back all it can.
+// each call took 1.2 of its 6.2 ms).
 cudaError_t qp_pool_alloc(qpgpu_ctx* c, void** p, size_t bytes);
 void qp_pool_idle(qpgpu_ctx* c);
 void qp_pool_trim(qpgpu_ctx* c);
