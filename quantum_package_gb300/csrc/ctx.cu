@@ -195,12 +195,23 @@ Pools& pools() {
   return *p;
 }
 
+// bytes that a pool holds and are not in use
+size_t pool_cached(cudaMemPool_t pool) {
+  uint64_t used = 0, reserved = 0;
+  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess)
+    return 0;
+  return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
 // the context's memory limit (environment QPGPU_MEMORY_LIMIT) does not allow
-// this many bytes more in the pool / beside it
-bool over_limit(qpgpu_ctx* c, size_t pool_more, size_t dev_more) {
+// this many bytes more in the pool / beside it, on top of what the pool holds
+// (after a give-back, which leaves whole pages of 32 MiB: of what it uses)
+bool over_limit(qpgpu_ctx* c, size_t pool_more, size_t dev_more, bool given_back) {
   if (c->memory_limit == 0) return false;
-  const size_t reserved = qp_pool_reserved(c), used = reserved - qp_pool_cached(c);
-  return std::max(reserved, used + pool_more) + c->dev_bytes + dev_more > c->memory_limit;
+  const size_t reserved = qp_pool_reserved(c), used = reserved - pool_cached(c->pool);
+  const size_t held = given_back ? used + pool_more : std::max(reserved, used + pool_more);
+  return held + c->dev_bytes + dev_more > c->memory_limit;
 }
 }  // namespace
 
@@ -216,6 +227,22 @@ void qp_give_back(int device) {
   if (cur >= 0 && cur != device) cudaSetDevice(cur);
 }
 
+cudaError_t qp_free_bytes(qpgpu_ctx* c, size_t* fr, size_t* total) {
+  const cudaError_t e = cudaMemGetInfo(fr, total);
+  if (e != cudaSuccess) return e;
+  {
+    std::lock_guard<std::mutex> l(pools().mu);
+    for (auto& p : pools().v)
+      if (p.first == c->device) *fr += pool_cached(p.second);
+  }
+  if (c->memory_limit) {
+    const size_t held = qp_pool_reserved(c) - pool_cached(c->pool) + c->dev_bytes;
+    *total = std::min(*total, c->memory_limit);
+    *fr = std::min(*fr, c->memory_limit > held ? c->memory_limit - held : 0);
+  }
+  return cudaSuccess;
+}
+
 cudaError_t qp_device_malloc(int device, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) {
@@ -229,9 +256,9 @@ cudaError_t qp_device_malloc(int device, void** p, size_t bytes) {
 
 cudaError_t qp_dev_malloc(qpgpu_ctx* c, void** p, size_t bytes) {
   *p = nullptr;
-  if (over_limit(c, 0, bytes)) {
+  if (over_limit(c, 0, bytes, false)) {
     qp_give_back(c->device);
-    if (over_limit(c, 0, bytes)) return cudaErrorMemoryAllocation;
+    if (over_limit(c, 0, bytes, true)) return cudaErrorMemoryAllocation;
   }
   const cudaError_t e = qp_device_malloc(c->device, p, bytes);
   if (e != cudaSuccess) return e;
@@ -252,11 +279,11 @@ void dev_free(qpgpu_ctx* c, void* p) {
 
 cudaError_t qp_pool_alloc(qpgpu_ctx* c, void** p, size_t bytes) {
   cudaError_t e = cudaErrorMemoryAllocation;
-  if (!over_limit(c, bytes, 0)) e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+  if (!over_limit(c, bytes, 0, false)) e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
   if (e != cudaSuccess) {  // blocks cached here or by another context may be the memory that is missing
     cudaGetLastError();
     qp_give_back(c->device);
-    if (!over_limit(c, bytes, 0)) e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+    if (!over_limit(c, bytes, 0, true)) e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
   }
   if (e != cudaSuccess) *p = nullptr;
   return e;
@@ -297,19 +324,11 @@ size_t qp_pool_reserved(qpgpu_ctx* c) {
   return (size_t)reserved;
 }
 
-size_t qp_pool_cached(qpgpu_ctx* c) {
-  uint64_t used = 0, reserved = 0;
-  if (cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
-      cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess)
-    return 0;
-  return reserved > used ? (size_t)(reserved - used) : 0;
-}
-
 void qp_pool_trim(qpgpu_ctx* c) {
   uint64_t used = 0;
   if (cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return;
   const uint64_t spare = std::max<uint64_t>(used / 2, 256ull << 20);
-  if (qp_pool_cached(c) > spare) cudaMemPoolTrimTo(c->pool, (size_t)(used + spare));
+  if (pool_cached(c->pool) > spare) cudaMemPoolTrimTo(c->pool, (size_t)(used + spare));
 }
 
 void qp_report_marks(qpgpu_ctx* c) {

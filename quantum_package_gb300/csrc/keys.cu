@@ -169,8 +169,7 @@ int build_table(qpgpu_ctx* c, int kind, unsigned char* lflags, int nlines, int64
   // scans when that would take more than half of the free memory or the
   // member offsets would not fit 32 bits
   size_t fr = 0, total = 0;
-  QP_CUDA(c, cudaMemGetInfo(&fr, &total));
-  fr += qp_pool_cached(c);
+  QP_CUDA(c, qp_free_bytes(c, &fr, &total));
   const double need = 26.0 * (double)E + 12.0 * (double)N;
   if (E >= (int64_t)INT_MAX || need > 0.5 * (double)fr) {
     k_clear_flag<<<grid_n(nlines), TPB, 0, st>>>(lflags, nlines, bit);

@@ -1293,14 +1293,14 @@ int build_pairs_t(qpgpu_ctx* c) {
   a.s2rec_next = ctr.p + 5;
   qp_mark(c, "pair setup");
   size_t fr = 0, total = 0;
-  QP_CUDA(c, cudaMemGetInfo(&fr, &total));
-  fr += qp_pool_cached(c);
+  QP_CUDA(c, qp_free_bytes(c, &fr, &total));
   if (c->sigma_mode != QPGPU_SIGMA_DIRECT) {
     // room for as many pairs a row as the context's last set had (1,200 when
     // it had none; the bench system has 991 at 1e6 determinants), 0.3 of that
     // for what rows leave behind when they outgrow a chunk, and for the
     // unfinished chunks of the warps; a pool that is too small costs its rows a
     // second scan, one that would not fit beside the stored pairs is left out
+    // (or given up, once their number is known)
     const double per_row = c->pairs_per_row > 0 ? c->pairs_per_row : 1200.0;
     const double est = per_row * (double)N;
     // chunks: an eighth of a warp's share of about 0.3 / 0.3 / 0.6 of the
@@ -1328,6 +1328,9 @@ int build_pairs_t(qpgpu_ctx* c) {
       for (int q = 0; q < 3; ++q) a.pos[q] = pos.p + q * N;
     } else {
       cudaGetLastError();
+      pool.reset();
+      pos.reset();
+      s2rec.reset();
     }
   }
   const int rcs = a.pool ? setup_scans<NINT, MODE_POOL>(c, a) : setup_scans<NINT, MODE_COUNT>(c, a);
@@ -1352,21 +1355,28 @@ int build_pairs_t(qpgpu_ctx* c) {
   QP_CUDA(c, cudaStreamSynchronize(st));
   const int64_t P = c->P, PS = c->P_s2;
   c->pairs_per_row = (double)P / (double)N;
+  // stored pairs (16 B each, S^2 pairs 8 B) or the direct sigma: forced by
+  // qpgpu_set_sigma_mode, else direct when the stored pairs would leave less
+  // than 1/16 of the device memory free
+  const double need = 16.0 * (double)P + 8.0 * (double)PS + 28.0 * (double)N, margin = (double)total / 16.0;
+  bool direct = c->sigma_mode == QPGPU_SIGMA_DIRECT;
+  if (c->sigma_mode == QPGPU_SIGMA_AUTO) direct = need + margin > (double)fr;
+  c->direct = direct;
+  // a set with more pairs than the pool was sized for may fit the device, but
+  // not beside the pool: its rows are then scanned a second time
+  const double hits = 4.0 * (double)a.pool_cap + 24.0 * (double)N + 16.0 * (double)a.s2rec_cap;
+  if (a.pool && (direct || need + margin + hits > (double)fr)) {
+    pool.reset();
+    pos.reset();
+    s2rec.reset();
+    a.pool = nullptr;
+  }
   if (a.pool && PS > a.s2rec_cap) {  // not all spin-flip pairs recorded: class C again, for every row
     QP_CUDA(c, cudaMemsetAsync(a.pos[CLS_C], 0xff, (size_t)N * sizeof(int64_t), st));
     full = 1;
     a.write_s2 = 1;
   }
   if (!a.pool) a.write_s2 = 1;
-  // stored pairs (16 B each, S^2 pairs 8 B) or the direct sigma: forced by
-  // qpgpu_set_sigma_mode, else direct when the stored pairs would leave less
-  // than 1/16 of the device memory free
-  bool direct = c->sigma_mode == QPGPU_SIGMA_DIRECT;
-  if (c->sigma_mode == QPGPU_SIGMA_AUTO) {
-    const double need = 16.0 * (double)P + 8.0 * (double)PS + 28.0 * (double)N;
-    direct = need + (double)total / 16.0 > (double)fr;
-  }
-  c->direct = direct;
   QP_CUDA(c, pool_alloc(c, &c->d_hdiag, N));
   QP_CUDA(c, pool_alloc(c, &c->d_sdiag, N));
   QP_CUDA(c, pool_alloc(c, &c->d_hdiag32, N));
@@ -1687,8 +1697,7 @@ int qp_sigma_direct(qpgpu_ctx* c, double* v, double* s, const double* u, int nst
   }
   if (!c->d_direct_cols) {  // column buffer: the whole set if it fits in half the free memory
     size_t fr = 0, total = 0;
-    QP_CUDA(c, cudaMemGetInfo(&fr, &total));
-    fr += qp_pool_cached(c);
+    QP_CUDA(c, qp_free_bytes(c, &fr, &total));
     int64_t maxrow = 0;
     for (int64_t k = 0; k < c->N; ++k) maxrow = std::max(maxrow, c->h_rowptr[k + 1] - c->h_rowptr[k]);
     int64_t cap = std::min<int64_t>(c->P, (int64_t)(fr / 2 / sizeof(int)));

@@ -654,6 +654,9 @@ int qpgpu_fail(qpgpu_ctx* c, int code, const std::string& msg);
 // use.  An allocation that fails, in a pool or by cudaMalloc, is tried again
 // after it: cudaMalloc does not see what a pool keeps mapped.
 void qp_give_back(int device);
+// what can still be allocated: free on the device or unused in a pool, within
+// the context's limit; and the device's (or the limit's) size
+cudaError_t qp_free_bytes(qpgpu_ctx* c, size_t* fr, size_t* total);
 cudaError_t qp_device_malloc(int device, void** p, size_t bytes);
 // the same, counted in the context (dev_free takes it off)
 cudaError_t qp_dev_malloc(qpgpu_ctx* c, void** p, size_t bytes);
@@ -677,7 +680,6 @@ cudaError_t qp_pool_alloc(qpgpu_ctx* c, void** p, size_t bytes);
 void qp_pool_idle(qpgpu_ctx* c);
 void qp_pool_trim(qpgpu_ctx* c);
 size_t qp_pool_reserved(qpgpu_ctx* c);  // bytes that the pool holds on the device
-size_t qp_pool_cached(qpgpu_ctx* c);    // those of them that are not in use
 struct PoolTrim {  // trims when a call ends
   qpgpu_ctx* c;
   ~PoolTrim() { qp_pool_trim(c); }
