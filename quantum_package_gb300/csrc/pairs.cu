@@ -202,7 +202,7 @@ struct RowOut {
   // the ends of theirs made the pool of a 1e5 or 2e5 set run full, so that the
   // scans ran again: 0.9 of 7.2 and 1.6 of 13.5 ms)
   __device__ __forceinline__ void grow(const BuildArgs& a, int need, int lane) {
-    const int64_t size = min(max((int64_t)a.pool_chunk[CLS], 2 * (int64_t)need), (int64_t)INT_MAX);
+    const int64_t size = min(max((int64_t)a.pool_chunk[CLS], 2 * (int64_t)need), a.N);  // a row holds fewer than N
     unsigned long long o = 0;
     if (lane == 0) o = atomicAdd(a.pool_next, (unsigned long long)size);
     o = __shfl_sync(0xffffffffu, o, 0);
@@ -1306,13 +1306,17 @@ int build_pairs_t(qpgpu_ctx* c) {
     // chunks: an eighth of a warp's share of about 0.3 / 0.3 / 0.6 of the
     // pairs, but sixteen rows at least, as a row that does not fit the rest of
     // a chunk takes another (of 300 pairs in a new context: with 1,200 the
-    // chunks of a 5,000 determinant set took 300 MB, 0.3 of 2.5 ms to map)
+    // chunks of a 5,000 determinant set took 300 MB, 0.3 of 2.5 ms to map), and
+    // a row's most at most: the 3 N^2 entries that bound the pool are then a
+    // chunk of each class for every row (a 900 determinant set, whose warps have
+    // a row each, found it full and was scanned twice)
     const double usual = c->pairs_per_row > 0 ? per_row : 300.0;
     const int64_t all = nblocks(N * 32, BLK);
     const int64_t ws = std::min<int64_t>(all, c->n_sm * SAME_BPS) * (BLK / 32);
     const int64_t wc = std::min<int64_t>(all, c->n_sm * CLASS_C_BPS) * (BLK / 32);
     auto chunk_of = [&](double share, int64_t warps) {
-      return (int)std::min(65536.0, std::max({256.0, share * est / (8.0 * (double)warps), 16.0 * share * usual}));
+      return (int)std::min({65536.0, (double)N,
+                            std::max({256.0, share * est / (8.0 * (double)warps), 16.0 * share * usual})});
     };
     a.pool_chunk[CLS_A] = a.pool_chunk[CLS_B] = chunk_of(0.3, ws);
     a.pool_chunk[CLS_C] = chunk_of(0.6, wc);
