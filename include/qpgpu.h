@@ -66,6 +66,15 @@ typedef struct qpgpu_info {
   int32_t n_keyed_lines;  /* beta columns + alpha rows with deletion-key tables */
 } qpgpu_info;
 
+/* Device memory.  A context keeps work memory between calls: beyond what is in
+ * use up to half of that (256 MiB at least) in a pool of its own, and staging
+ * arrays as large as its largest call needed; device_bytes counts both.  An
+ * allocation that fails is tried again after all contexts of the process have
+ * given back what they do not use.  The environment variable
+ * QPGPU_MEMORY_LIMIT (bytes, read by qpgpu_create) bounds what a context
+ * holds; a set whose pairs do not fit it is treated as one that does not fit
+ * the device. */
+
 /* Context for one orbital space; replaces the IRPF90 providers N_int,
  * elec_alpha_num, elec_beta_num, mo_tot_num (src/Bitmask/bitmasks.irp.f:3-15).
  * n_int must be (n_mo-1)/64+1 and at most 2 (n_mo <= 128).  n_alpha >= n_beta
@@ -101,12 +110,13 @@ int qpgpu_set_sigma_mode(qpgpu_ctx* ctx, int mode);
  * pairs, and so sigma, are the same either way; only the work changes (a few
  * heavy lines carry most of the scan work of large sets).  -1 keeps a default
  * (min_single 64 (n_elec + 2), min_double 16384); INT64_MAX turns tables off.
- * hash_bits (1..64, default 64) keeps the low bits of the key hashes only, to
- * test that colliding keys still give the exact pairs; below 64,
+ * hash_bits (1..64) keeps the low bits of the key hashes only, to test that
+ * colliding keys still give the exact pairs; the default, 64, keeps 12 bits
+ * more than the number of keys of the largest possible table has.  Below 64,
  * qpgpu_set_dets refuses (QPGPU_ERR_ARG) a table of more than 2^22 keys,
  * whose merged groups would make the scans quadratic.  Tables that would
  * take more than half of the free device memory are left out.  Takes effect
- * at the next qpgpu_set_dets. */
+ * at the next qpgpu_set_dets; the set in hand keeps its tables. */
 int qpgpu_set_line_keys(qpgpu_ctx* ctx, int64_t min_single, int64_t min_double, int hash_bits);
 
 /* u_0_H_u_0 (src/Davidson/diagonalization_hs2.irp.f:446-484), the psi_energy

@@ -365,7 +365,7 @@ void qp_free_dets(qpgpu_ctx* c) {
   qp_free_line_keys(c);
   void** ps[] = {(void**)&c->d_dets, (void**)&c->d_alpha, (void**)&c->d_beta, (void**)&c->d_rows,
                  (void**)&c->d_cols, (void**)&c->d_order, (void**)&c->d_pos, (void**)&c->d_col_loc, (void**)&c->d_t_order,
-                 (void**)&c->d_t_cols, (void**)&c->d_row_loc, (void**)&c->d_sa_ptr, (void**)&c->d_sa_idx,
+                 (void**)&c->d_row_loc, (void**)&c->d_sa_ptr, (void**)&c->d_sa_idx,
                  (void**)&c->d_sb_ptr, (void**)&c->d_sb_idx, (void**)&c->d_cost_a, (void**)&c->d_cost_b,
                  (void**)&c->d_detfeat, (void**)&c->d_alpha_pos, (void**)&c->d_beta_tpos};
   for (auto p : ps) {
@@ -422,7 +422,6 @@ int qp_build_index(qpgpu_ctx* c) {
   k_seg_starts<<<grid_for(N), TPB, 0, st>>>(c->d_cols, c->d_col_loc, N, Ub);
   // alpha-major (transposed) order over bilinear positions: key = alpha_id * Ub + beta_id
   QP_CUDA(c, pool_alloc(c, &c->d_t_order, N));
-  QP_CUDA(c, pool_alloc(c, &c->d_t_cols, N));
   QP_CUDA(c, pool_alloc(c, &c->d_row_loc, (size_t)Ua + 1));
   {
     Scoped<u64> key(c);
@@ -436,7 +435,6 @@ int qp_build_index(qpgpu_ctx* c) {
     Scoped<int> trows(c);
     QP_CUDA(c, trows.alloc(N));
     k_gather_int<<<grid_for(N), TPB, 0, st>>>(c->d_rows, c->d_t_order, trows.p, N);
-    k_gather_int<<<grid_for(N), TPB, 0, st>>>(c->d_cols, c->d_t_order, c->d_t_cols, N);
     k_seg_starts<<<grid_for(N), TPB, 0, st>>>(trows.p, c->d_row_loc, N, Ua);
   }
   // spin strings in scan order: the pair kernels read the strings of a

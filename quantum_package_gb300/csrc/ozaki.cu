@@ -241,8 +241,6 @@ __device__ __forceinline__ void oz_flush1(uint32_t taddr, int sh, long long (&ac
   for (int j = 0; j < OZ_N; ++j) acc[j] += (long long)__float2int_rn(__uint_as_float(v[j])) << sh;
 }
 
-// digit planes of one chunk: task (column, group of RPT rows) writes RPT
-// rows of one column into each of the 8 planes of stage (sa, sb)
 // RPT rows of one column (rows wcol doubles apart, nr of them real) into each
 // of the 8 planes, `tile` bytes apart
 template <int RPT>
@@ -1021,7 +1019,6 @@ __global__ void __launch_bounds__(256) k_col_maxexp(const double* X, int nblk, i
   }
 }
 
-// out[p] = sum over CTAs c = 0, 1, ... of partial[c][p], in that order
 // The CTAs' partial sums of one entry per thread, added in the CTAs' order.
 // Bound by the latency of the loads, so OZ_RED_AHEAD of them are in flight
 // at a time and the entries are spread over one warp per block.

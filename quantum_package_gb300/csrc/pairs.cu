@@ -17,7 +17,7 @@
 // Stored pairs.  The scans run once: each warp writes the hits of its rows
 // into chunks of a pool and counts them.  k_sort_rows then moves each row's
 // hits to their place in the CSR, ascending, and k_pair_values evaluates the
-// elements.  At 1e6 determinants the scans take 29 ms (68 ms as a count and a
+// elements.  At 1e6 determinants the scans take 26 ms (68 ms as a count and a
 // fill pass).  Rows that found the pool full are scanned a second time and write
 // straight into the CSR; without a pool that is every row.
 //
@@ -52,7 +52,6 @@ struct BuildArgs {
   const int* cols;
   const int* col_loc;
   const int* t_order;
-  const int* t_cols;
   const int* row_loc;
   const u64* alpha_pos;  // alpha string at each bilinear position
   const u64* beta_tpos;  // beta string at each alpha-major position
@@ -101,7 +100,7 @@ struct BuildArgs {
   double* item_s;
   const u64* det_pos;   // both strings at each bilinear position (2 NINT words)
   const u64* det_tpos;  // the same at each alpha-major position (direct sigma)
-  int* err;  // set when a pass would write past its row's segment
+  int* err;  // set when a fill of the CSR would write past its row's segment (direct sigma: null)
   // direct sigma (k_pair_sigma): v, s = H u, S^2 u for the selected rows, u (N, nst)
   const double* u;
   const double* uT;  // u in alpha-major order: same-alpha partners are contiguous there
@@ -190,7 +189,7 @@ struct RowOut {
         if (dst) dst[o] = col;
       } else if (o < cap) {
         dst[o] = col;
-      } else {
+      } else if (a.err) {
         atomicOr(a.err, 1 << CLS);
       }
     }
@@ -1140,7 +1139,6 @@ BuildArgs index_args(const qpgpu_ctx* c) {
   a.cols = c->d_cols;
   a.col_loc = c->d_col_loc;
   a.t_order = c->d_t_order;
-  a.t_cols = c->d_t_cols;
   a.row_loc = c->d_row_loc;
   a.alpha_pos = c->d_alpha_pos;
   a.beta_tpos = c->d_beta_tpos;
@@ -1239,9 +1237,10 @@ int sort_row_columns(qpgpu_ctx* c, const BuildArgs& a) {
 
 // The scans of all three classes, side by side: each of them ends with the
 // reference's row in one warp (0.8, 0.7 and 1.1 ms at 2e5 determinants, where
-// the other rows keep the device busy for 0.3, 0.3 and 1.0).  Small sets, whose
-// scans take 0.1 ms together, run them one after the other: the streams cost a
-// new context 0.28 ms.
+// the other rows keep the device busy for 0.3, 0.3 and 1.0).  A whole set-up
+// takes 6.2 ms side by side and 6.8 one after the other at 1e5 determinants,
+// 3.54 and 3.69 at 32,768, 2.31 and 2.34 at 5,000: below the line the gain is
+// under 0.15 ms, and a context that holds only small sets has no streams.
 constexpr int64_t SIDE_BY_SIDE = 1 << 15;
 template <int NINT, int MODE>
 int launch_scans(qpgpu_ctx* c, const BuildArgs& a, unsigned gs, unsigned gc, cudaStream_t st) {
@@ -1639,7 +1638,6 @@ int sigma_direct_t(qpgpu_ctx* c, double* v, double* s, const double* u, const do
   a.det_pos = c->d_det_pos;
   a.det_tpos = c->d_det_tpos;
   a.colidx = c->d_direct_cols;
-  a.err = c->d_direct_err;
   a.tag_t = 1;
   a.row_first = row_first;
   a.row_step = row_step;
@@ -1710,8 +1708,6 @@ int qp_sigma_direct(qpgpu_ctx* c, double* v, double* s, const double* u, int nst
     if (const char* e = getenv("QPGPU_DIRECT_CHUNK_COLS")) cap = std::min<int64_t>(cap, atoll(e) > 0 ? atoll(e) : cap);
     cap = std::max<int64_t>(cap, maxrow);
     QP_CUDA(c, dev_alloc(c, &c->d_direct_cols, (size_t)std::max<int64_t>(cap, 1)));
-    QP_CUDA(c, dev_alloc(c, &c->d_direct_err, 1));
-    QP_CUDA(c, cudaMemsetAsync(c->d_direct_err, 0, sizeof(int), st));
     c->direct_cols_cap = cap;
   }
   k_alpha_major<<<nblocks((int64_t)need, 256), 256, 0, st>>>(u, c->d_t_order, c->d_direct_ut, c->N, nst);
@@ -1740,7 +1736,7 @@ void qp_free_pairs(qpgpu_ctx* c) {
     *p = nullptr;
   }
   // grown by a sigma on the caller's stream: not from the pool
-  void** up[] = {(void**)&c->d_val32lo, (void**)&c->d_direct_cols, (void**)&c->d_direct_err};
+  void** up[] = {(void**)&c->d_val32lo, (void**)&c->d_direct_cols};
   for (auto p : up) {
     dev_free(c, *p);
     *p = nullptr;

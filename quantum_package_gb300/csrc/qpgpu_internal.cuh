@@ -564,7 +564,6 @@ struct qpgpu_ctx {
   int* d_pos = nullptr;        // original index -> bilinear position
   int* d_col_loc = nullptr;    // (U_b+1) first bilinear position of each beta column
   int* d_t_order = nullptr;    // alpha-major position -> bilinear position
-  int* d_t_cols = nullptr;     // alpha-major position -> beta id
   int* d_row_loc = nullptr;    // (U_a+1) first alpha-major position of each alpha row
   u64* d_alpha_pos = nullptr;  // (N, nint) alpha string at each bilinear position (coalesced scans)
   u64* d_beta_tpos = nullptr;  // (N, nint) beta string at each alpha-major position
@@ -603,7 +602,6 @@ struct qpgpu_ctx {
   std::vector<int64_t> h_rowptr;      // direct sigma: row starts (host)
   int* d_direct_cols = nullptr;       // direct sigma: columns of one chunk of rows
   int64_t direct_cols_cap = 0;
-  int* d_direct_err = nullptr;
   double pairs_per_row = 0.0;         // of the last set (sizes the next set-up's pool of hits)
   int64_t P = 0;
   int64_t* d_rowptr = nullptr;  // N+1

@@ -114,7 +114,6 @@ struct SelArgs {
   uint64_t cap;
   double* cand_val;
   uint64_t* cand_at;         // its unit (high 32 bits) and entry
-  int* err;
 };
 
 template <int NINT>
@@ -909,7 +908,7 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   }
   // device arrays
   Dev d_items{c}, d_gens{c}, d_coef{c}, d_e0{c}, d_icnt{c}, d_ioff{c}, d_ilist{c}, d_fcnt{c}, d_foff{c};
-  Dev d_flist{c}, d_fock{c}, d_slot{c}, d_part{c}, d_cnt{c}, d_err{c}, d_pt2{c}, d_wgt{c}, d_units{c}, d_first{c};
+  Dev d_flist{c}, d_fock{c}, d_slot{c}, d_part{c}, d_cnt{c}, d_pt2{c}, d_wgt{c}, d_units{c}, d_first{c};
   uint64_t hcap = 1;
   while (hcap < (uint64_t)(2 * N)) hcap <<= 1;
   QP_CUDA(c, qp_pool_alloc(c, &d_items.p, items.size() * sizeof(SelItem)));
@@ -931,8 +930,6 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   QP_CUDA(c, qp_pool_alloc(c, &d_icnt.p, (n_list + 1) * sizeof(int64_t)));
   QP_CUDA(c, qp_pool_alloc(c, &d_fcnt.p, (n_list + 1) * sizeof(int64_t)));
   QP_CUDA(c, qp_pool_alloc(c, &d_cnt.p, 2 * sizeof(unsigned long long)));
-  QP_CUDA(c, qp_pool_alloc(c, &d_err.p, sizeof(int)));
-  QP_CUDA(c, cudaMemsetAsync(d_err.p, 0, sizeof(int), st));
   QP_CUDA(c, qp_pool_alloc(c, &d_pt2.p, (size_t)n_list * n_st * sizeof(double)));
   const u64* dets = c->d_dets;
   const int* dg = (const int*)d_gens.p;
@@ -987,7 +984,6 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
   A.hmask = hcap - 1;
   A.n_ext = (unsigned long long*)d_cnt.p;
   A.n_cand = (unsigned long long*)d_cnt.p + 1;
-  A.err = (int*)d_err.p;
 #define QP_SEL_WEIGH(NI)                                                                                           \
   k_sel_lists<NI><<<n_list, SBLK, 0, st>>>(dets, dg, n_list, n_sel, 0, 1, nullptr, (const int64_t*)d_ioff.p,       \
                                            (int*)d_ilist.p);                                                       \

@@ -394,22 +394,14 @@ inline unsigned gsz(int64_t n, int tpb) {
   return (unsigned)g;
 }
 
-// FP32 launch shapes tried by the tuner: kernel variant, CTA size and grid
-// policy (0: one warp per work item; n: a persistent grid of n CTAs per SM)
-struct Sig32Shape {
-  bool pipe;
-  int bs, ctas_per_sm;
-};
-constexpr Sig32Shape kSig32Shapes[] = {{false, 256, 0}, {false, 128, 0}, {false, 64, 0}, {true, 256, 0}};
-constexpr int kNSig32Shapes = sizeof(kSig32Shapes) / sizeof(kSig32Shapes[0]);
+// FP32 launch shapes tried by the tuner, one warp per work item: CTA size, the
+// last one with the next trip's loads ahead
+constexpr int kSig32Block[] = {256, 128, 64, 256};
+constexpr int kNSig32Shapes = sizeof(kSig32Block) / sizeof(kSig32Block[0]);
 
 template <int NST, int LD, bool V8>
-void launch_sigma32_ld(const SigArgs& a, int variant, cudaStream_t st, int n_sm) {
-  const Sig32Shape sh = kSig32Shapes[variant];
-  int64_t g = (a.n_items * 32 + sh.bs - 1) / sh.bs;
-  if (sh.ctas_per_sm) g = std::min<int64_t>(g, (int64_t)sh.ctas_per_sm * n_sm);
-  g = std::max<int64_t>(1, std::min<int64_t>(g, 65535LL * 32));
-  const unsigned grid = (unsigned)g;
+void launch_sigma32_ld(const SigArgs& a, int variant, cudaStream_t st) {
+  const unsigned grid = gsz(a.n_items * 32, kSig32Block[variant]);
   switch (variant) {
     case 1: k_sigma32<NST, false, 128, LD, V8><<<grid, 128, 0, st>>>(a); break;
     case 2: k_sigma32<NST, false, 64, LD, V8><<<grid, 64, 0, st>>>(a); break;
@@ -421,12 +413,12 @@ void launch_sigma32_ld(const SigArgs& a, int variant, cudaStream_t st, int n_sm)
 // dense rows (u32_ld == NST) or rows padded to 4 / 8 floats; rows of 8 floats
 // on a 32-byte aligned array are read with one 256-bit load each
 template <int NST>
-void launch_sigma32(const SigArgs& a, int variant, cudaStream_t st, int n_sm) {
+void launch_sigma32(const SigArgs& a, int variant, cudaStream_t st) {
   constexpr int P = Pow2<NST>::v;
   const bool a32 = ((uintptr_t)a.u32 & 31) == 0;
   if constexpr (P == 8) {
     if (a.u32_ld == 8 && a32) {
-      launch_sigma32_ld<NST, 8, true>(a, variant, st, n_sm);
+      launch_sigma32_ld<NST, 8, true>(a, variant, st);
       return;
     }
     if constexpr (NST == 8) {
@@ -438,11 +430,11 @@ void launch_sigma32(const SigArgs& a, int variant, cudaStream_t st, int n_sm) {
   }
   if constexpr (P != NST && P == 4) {
     if (a.u32_ld == 4) {
-      launch_sigma32_ld<NST, 4, false>(a, variant, st, n_sm);
+      launch_sigma32_ld<NST, 4, false>(a, variant, st);
       return;
     }
   }
-  if constexpr (NST != 8) launch_sigma32_ld<NST, NST, false>(a, variant, st, n_sm);
+  if constexpr (NST != 8) launch_sigma32_ld<NST, NST, false>(a, variant, st);
 }
 
 // Float-float sigma: elements h = vh + vl and coefficients u = uh + ul as
@@ -530,37 +522,39 @@ __global__ void __launch_bounds__(128) k_sigma_ff(SigArgs a) {
 }
 
 template <int NST>
-void launch_sigma(const SigArgs& a, int precision, unsigned grid, cudaStream_t st, int n_sm, int variant) {
+void launch_sigma(const SigArgs& a, int precision, unsigned grid, cudaStream_t st, int variant) {
   constexpr int P = Pow2<NST>::v;
   if (precision == QPGPU_FF) {
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((a.n_items * 32 + 127) / 128, 65535LL * 32));
     k_sigma_ff<NST, P><<<g, 128, 0, st>>>(a);
   } else if (precision == QPGPU_FP32)
-    launch_sigma32<NST>(a, variant < 0 ? 0 : variant, st, n_sm);
+    launch_sigma32<NST>(a, variant < 0 ? 0 : variant, st);
   else
     k_sigma64<NST><<<grid, SBLK, 0, st>>>(a);
 }
 
-void launch_any(const SigArgs& a, int nst, int precision, unsigned grid, cudaStream_t st, int n_sm, int variant) {
+void launch_any(const SigArgs& a, int nst, int precision, unsigned grid, cudaStream_t st, int variant) {
   switch (nst) {
-    case 1: launch_sigma<1>(a, precision, grid, st, n_sm, variant); break;
-    case 2: launch_sigma<2>(a, precision, grid, st, n_sm, variant); break;
-    case 3: launch_sigma<3>(a, precision, grid, st, n_sm, variant); break;
-    case 4: launch_sigma<4>(a, precision, grid, st, n_sm, variant); break;
-    case 5: launch_sigma<5>(a, precision, grid, st, n_sm, variant); break;
-    case 6: launch_sigma<6>(a, precision, grid, st, n_sm, variant); break;
-    case 7: launch_sigma<7>(a, precision, grid, st, n_sm, variant); break;
-    default: launch_sigma<8>(a, precision, grid, st, n_sm, variant); break;
+    case 1: launch_sigma<1>(a, precision, grid, st, variant); break;
+    case 2: launch_sigma<2>(a, precision, grid, st, variant); break;
+    case 3: launch_sigma<3>(a, precision, grid, st, variant); break;
+    case 4: launch_sigma<4>(a, precision, grid, st, variant); break;
+    case 5: launch_sigma<5>(a, precision, grid, st, variant); break;
+    case 6: launch_sigma<6>(a, precision, grid, st, variant); break;
+    case 7: launch_sigma<7>(a, precision, grid, st, variant); break;
+    default: launch_sigma<8>(a, precision, grid, st, variant); break;
   }
 }
 
 // Times every FP32 launch shape on this determinant set (two launches each,
 // the second timed with events on the caller's stream) and keeps the fastest
 // for n_st.  Runs once per determinant set and n_st, on the first FP32 call,
-// whose own launch follows.  A stretch of a quarter of the work items tells
-// the shapes apart (of 2^18 at least: on 65,536 of the 330,000 items of 3e5
-// determinants x 2 states the persistent shape lost, over all it wins by 9
-// percent).
+// whose own launch follows.  A stretch of a quarter of the work items (2^18 at
+// least) tells the shapes apart: at 3e5, 5e5 and 1e6 determinants with 1, 2, 3,
+// 4 and 8 states its fastest shape is the one of all items or within 0.5
+// percent of it (65,536 items: within 3 percent).  No shape is the best
+// everywhere: loads one trip ahead win with 2 states (0.321 against 0.345 ms at
+// 3e5, 2.18 against 2.26 at 1e6) and cost 20 percent with 8.
 int tune_sigma32(qpgpu_ctx* c, SigmaItems* it, const SigArgs& all, int nst, cudaStream_t st, int slot) {
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
@@ -578,9 +572,9 @@ int tune_sigma32(qpgpu_ctx* c, SigmaItems* it, const SigArgs& all, int nst, cuda
   int best = 0;
   float best_ms = 1e30f;
   for (int v = 0; v < kNSig32Shapes; ++v) {
-    launch_any(a, nst, QPGPU_FP32, 1, st, c->n_sm, v);
+    launch_any(a, nst, QPGPU_FP32, 1, st, v);
     cudaEventRecord(e0, st);
-    launch_any(a, nst, QPGPU_FP32, 1, st, c->n_sm, v);
+    launch_any(a, nst, QPGPU_FP32, 1, st, v);
     cudaEventRecord(e1, st);
     if (cudaEventSynchronize(e1) != cudaSuccess) break;
     float ms = 0.f;
@@ -696,7 +690,7 @@ int qp_sigma_launch(qpgpu_ctx* c, SigmaItems* it, double* v, double* s, const do
     rc = tune_sigma32(c, it, a, nst, st, slot);
     if (rc) return rc;
   }
-  launch_any(a, nst, precision, grid, st, c->n_sm, it->sig32_variant[slot]);
+  launch_any(a, nst, precision, grid, st, it->sig32_variant[slot]);
   if (it->n_multi > 0)
     k_sigma_combine<<<gsz((int64_t)it->n_multi * nst, 256), 256, 0, st>>>(a, it->multi_rows, it->row_item0,
                                                                          it->n_multi, nst);
@@ -846,7 +840,7 @@ extern "C" int qpgpu_sigma_bilinear_noalloc(qpgpu_ctx* c, double* v_t, double* s
   a.row_step = 1;
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   const unsigned grid = gsz(it->n_items * 32, SBLK);
-  launch_any(a, n_st, precision, grid, st, c->n_sm, it->sig32_variant[n_st]);
+  launch_any(a, n_st, precision, grid, st, it->sig32_variant[n_st]);
   if (it->n_multi > 0)
     k_sigma_combine<<<gsz((int64_t)it->n_multi * n_st, 256), 256, 0, st>>>(a, it->multi_rows, it->row_item0,
                                                                           it->n_multi, n_st);
