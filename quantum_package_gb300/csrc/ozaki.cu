@@ -937,34 +937,50 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
       int nsd, lane;
       uint32_t rawf;  // barriers of the even and odd tiles
       __device__ __forceinline__ uint32_t bar(int t) const { return rawf + 8u * (uint32_t)(t & 1); }
-      // bounded wait for K step `step` of the whole run to be cut
-      __device__ __forceinline__ bool cut(int step) const {
-        bool ok = false;
-        for (long long it = 0; it < OZ_WAIT_LIMIT && !ok; ++it) {
-          ok = *sdone > step;
-          if (!ok && (it & 255) == 255 && *(volatile const int*)sflag) break;
+      // bounded wait for K step `step` of the whole run to be cut: the steps cut, 0 when it gave up
+      __device__ __forceinline__ int cut(int step) const {
+        int done = 0;
+        for (long long it = 0; it < OZ_WAIT_LIMIT; ++it) {
+          done = *sdone;
+          if (done > step || ((it & 255) == 255 && *(volatile const int*)sflag)) break;
         }
         __threadfence_block();
-        return __all_sync(0xffffffffu, ok) != 0;
+        done = __reduce_min_sync(0xffffffffu, done);
+        return done > step ? done : 0;
       }
-      __device__ __forceinline__ void copy(int t, int b, int slot) const {
+      // a lane per block: one bulk copy, or by all lanes when the block is not whole 16-byte lines
+      __device__ __forceinline__ void copy(int t, int b, int n, int slot) const {
         const int64_t R = r0 + (int64_t)t * LC_TM;
-        const double* src = g.A + (int64_t)b * g.sA + R * nsd;
         const uint32_t bytes = (uint32_t)(min((int64_t)LC_TM, r1 - R) * nsd * 8);
-        const uint32_t dst = smem_u32(raw + (size_t)slot * LC_TM * nsd);
-        if ((((uintptr_t)src | bytes) & 15) == 0) {
-          if (lane == 0) {
-            asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar(t)), "r"(bytes)
+        const double* const src0 = g.A + (int64_t)b * g.sA + R * nsd;
+        const uint32_t dst0 = smem_u32(raw + (size_t)slot * LC_TM * nsd), step = (uint32_t)(LC_TM * nsd * 8);
+        for (int i0 = 0; i0 < n; i0 += 32) {
+          const int i = i0 + lane;
+          const double* const src = src0 + (int64_t)i * g.sA;
+          const bool whole = i < n && (((uintptr_t)src | bytes) & 15) == 0;
+          const unsigned bulk = __ballot_sync(0xffffffffu, whole);
+          if (lane == 0 && bulk)
+            asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar(t)),
+                         "r"((uint32_t)__popc(bulk) * bytes)
                          : "memory");
+          __syncwarp();
+          if (whole)
             asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                    dst0 + (uint32_t)i * step),
                 "l"(src), "r"(bytes), "r"(bar(t))
                 : "memory");
+          const unsigned all = n - i0 >= 32 ? 0xffffffffu : (1u << (n - i0)) - 1u;
+          for (unsigned rest = all & ~bulk; rest; rest &= rest - 1) {
+            const int k = i0 + __ffs(rest) - 1;
+            const double* const from = src0 + (int64_t)k * g.sA;
+            for (uint32_t x = lane; x < bytes / 8; x += 32)
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst0 + (uint32_t)k * step + 8u * x),
+                           "l"(from + x)
+                           : "memory");
           }
-        } else {
-          for (uint32_t x = lane; x < bytes / 8; x += 32)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * x), "l"(src + x) : "memory");
         }
+        __syncwarp();
       }
       __device__ __forceinline__ void finish(int t) const {
         if (lane == 0) mbar_arrive(bar(t));

@@ -34,6 +34,7 @@ struct Model {
   std::vector<Copy> flight;
   std::vector<int> slot_tile, slot_block;
   int cut_steps = 0;        // K steps cut so far
+  int ahead = 0, rnd = 1, finished = 0;
   void complete(int i) {
     if (pending[i] == 0 && tx[i] == 0) { ++phase[i]; pending[i] = 1; }
   }
@@ -48,17 +49,24 @@ struct Model {
       if (flight[k].tile == t) land(k);
   }
   // the consumers: a tile's steps are cut in order once its phase is complete
-  bool cut(int step) {
-    if (waits++ == give_up) return false;
-    while (cut_steps <= step) {
+  int cut(int step) {
+    if (waits++ == give_up) return 0;
+    while (cut_steps <= step || ahead > 0) {  // up to `ahead` steps more, as far as the tiles have been started
+      if (cut_steps > step && ahead-- <= 0) break;
       const int t = cut_steps / nks;
+      if (t >= ntile || (cut_steps > step && t >= finished)) break;
       land_tile(t);
-      if (phase[t & 1] <= t / 2) { bad |= 1; return false; }  // would wait for ever
+      if (phase[t & 1] <= t / 2) { bad |= 1; return 0; }  // would wait for ever
       ++cut_steps;
     }
-    return true;
+    ahead = rnd = (rnd * 5 + 3) % 8;
+    return cut_steps;
   }
-  void copy(int t, int b, int slot) {
+  void copy(int t, int b, int n, int slot) {
+    if (n < 1 || b + n > nb) { bad |= 64; return; }
+    for (int i = 0; i < n; ++i) copy1(t, b + i, slot + i);
+  }
+  void copy1(int t, int b, int slot) {
     if (slot < 0 || slot >= nslots) { bad |= 2; return; }
     if (slot_tile[slot] >= 0) {
       const int last = slot_tile[slot] * nks + ((slot_block[slot] + 1) * nsd - 1) / ks;
@@ -74,6 +82,7 @@ struct Model {
   void finish(int t) {
     if (phase[t & 1] != t / 2 || pending[t & 1] == 0) { bad |= 16; return; }
     pending[t & 1] = 0;
+    finished = t + 1;
     complete(t & 1);
   }
   void drain(int t) {
@@ -85,8 +94,8 @@ struct Model {
 int main() {
   long runs = 0;
   for (int nsd : {1, 2, 3, 4, 5, 8, 16})
-    for (int nb : {1, 2, 3, 7, 8})
-      for (int nslots = nb; nslots <= 2 * nb; ++nslots)
+    for (int nb : {1, 2, 3, 7, 8, 17, 40})
+      for (int nslots = nb; nslots <= 2 * nb; nslots += nb > 8 ? 5 : 1)
         for (int ntile : {0, 1, 2, 3, 5})
           for (int eager : {0, 1})
             for (int give_up = -1; give_up <= ntile * nb; ++give_up) {
