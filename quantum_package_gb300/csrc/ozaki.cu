@@ -104,6 +104,7 @@ struct OzArgs {
   int nraw;        // raw stages in the ring
   int raw_stride;  // doubles per raw stage
   int rpt;         // rows per splitting task: 2, 4 or 8
+  int nsw;         // splitting warps that have tasks
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
   }
   if (tid == 0) {
     for (int s = 0; s < OZ_MAXST; ++s) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(BAR(OZ_B_FULL, s)), "r"(OZ_SPLIT / 32));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(BAR(OZ_B_FULL, s)), "r"(g.nsw));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(BAR(OZ_B_EMPTY, s)));
     }
     for (int b = 0; b < OZ_NBUF; ++b) {
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
     }
     for (int r = 0; r < OZ_MAXRAW; ++r) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(BAR(OZ_B_RAWF, r)));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(BAR(OZ_B_RAWE, r)), "r"(OZ_SPLIT / 32));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(BAR(OZ_B_RAWE, r)), "r"(g.nsw));
     }
     asm volatile("fence.mbarrier_init.release.cluster;");
     *sflag = 0;
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_gram_oz(OzArgs g) {
     // digit stage s and raw stage rs of the chunk, and the parities of their uses
     int s = 0, rs = 0;
     uint32_t sp = 0, rp = 0;
-    for (int c = 0; c < nchunks; ++c) {
+    for (int c = 0; c < nchunks && warp < g.nsw; ++c) {
       // chunk c's raw rows have landed; the MMAs of chunk c - nst are done with digit stage s
       bool ok = mbar_wait(BAR(OZ_B_RAWF, rs), rp, sflag);
       if (ok && c >= nst) ok = mbar_wait(BAR(OZ_B_EMPTY, s), sp ^ 1u, sflag);
@@ -1119,18 +1120,13 @@ void qp_gram_oz(const double* A, int64_t sA, int m, int nsdA, int ldA, const dou
   g.nst = rawfit(3) >= 2 ? 3 : 2;
   g.nraw = std::max(1, std::min(OZ_MAXRAW, rawfit(g.nst)));
   const int smem = g.nst * g.stage + g.nraw * g.raw_stride * 8 + OZ_TAB;
-  // rows per splitting task: the fewest rows per thread on the longest
-  // thread's path (more, narrower stores only where that gains)
-  int best = 1 << 30;
-  g.rpt = 8;
-  for (int r : {8, 4, 2}) {
-    const int ntask = rw * (OZ_KC / r);
-    const int cost = (ntask + OZ_SPLIT - 1) / OZ_SPLIT * r * 4 + (8 / r);
-    if (cost < best) {
-      best = cost;
-      g.rpt = r;
-    }
-  }
+  // rows per splitting task, by what each measured over 2 to 144 columns: wide
+  // tasks need the fewest stores, narrow ones the shortest chain when a chunk
+  // leaves most splitting threads without one.  1e6 rows, 2 / 4 / 8 rows: 4 + 4
+  // columns 250 / 256 / 260 us, 8 + 4 281 / 270 / 270, 8 + 8 292 / 280 / 281,
+  // 16 + 1 309 / 305 / 281, 48 + 4 448 / 412 / 378, 128 + 16 874 / 768 / 702
+  g.rpt = rw <= 8 ? 2 : rw <= 16 ? 4 : 8;
+  g.nsw = std::min(OZ_SPLIT / 32, (rw * (OZ_KC / g.rpt) + 31) / 32);
   k_gram_oz<<<ncta, OZ_THREADS, smem, st>>>(g);
 }
 
