@@ -931,12 +931,14 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
     // the lanes when it is not whole 16-byte lines (g.lane_copies: some are not)
     struct Io {
       const LcArgs& g;
-      double* raw;
       const int* sflag;
       volatile int* sdone;
       int64_t r0, r1;
       int nsd, lane;
       uint32_t rawf;  // barriers of the even and odd tiles
+      uint32_t dst0;  // first slot
+      const double* tile;  // first block of the tile being loaded, and the bytes of its blocks
+      uint32_t bytes;
       __device__ __forceinline__ uint32_t bar(int t) const { return rawf + 8u * (uint32_t)(t & 1); }
       // bounded wait for K step `step` of the whole run to be cut: the steps cut, 0 when it gave up
       __device__ __forceinline__ int cut(int step) const {
@@ -949,39 +951,43 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
         done = __reduce_min_sync(0xffffffffu, done);
         return done > step ? done : 0;
       }
-      // a lane per block: one bulk copy, or by all lanes when the block is not whole 16-byte lines
-      __device__ __forceinline__ void copy(int t, int b, int n, int slot) const {
+      __device__ __forceinline__ void begin(int t) {
         const int64_t R = r0 + (int64_t)t * LC_TM;
-        const uint32_t bytes = (uint32_t)(min((int64_t)LC_TM, r1 - R) * nsd * 8);
-        const double* const src0 = g.A + (int64_t)b * g.sA + R * nsd;
-        const uint32_t dst0 = smem_u32(raw + (size_t)slot * LC_TM * nsd), step = (uint32_t)(LC_TM * nsd * 8);
-        for (int i0 = 0; i0 < n; i0 += 32) {
-          const int i = i0 + lane;
-          const double* const src = src0 + (int64_t)i * g.sA;
-          const bool whole = i < n && (((uintptr_t)src | bytes) & 15) == 0;
-          const unsigned bulk = __ballot_sync(0xffffffffu, whole);
-          if (lane == 0 && bulk)
-            asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar(t)),
-                         "r"((uint32_t)__popc(bulk) * bytes)
-                         : "memory");
+        tile = g.A + R * nsd;
+        bytes = (uint32_t)(min((int64_t)LC_TM, r1 - R) * nsd * 8);
+      }
+      // one bulk copy a block, started by a lane each when there are many, or by
+      // all lanes when the block is not whole 16-byte lines
+      __device__ __forceinline__ void copy(int t, int b, int n, int slot) const {
+        const uint32_t step = (uint32_t)(LC_TM * nsd * 8);
+        const double* src = tile + (int64_t)b * g.sA;
+        uint32_t dst = dst0 + (uint32_t)slot * step;
+        if (n >= 8 && !g.lane_copies) {
+          if (lane == 0) expect(t, (uint32_t)n * bytes);
           __syncwarp();
-          if (whole)
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    dst0 + (uint32_t)i * step),
-                "l"(src), "r"(bytes), "r"(bar(t))
-                : "memory");
-          const unsigned all = n - i0 >= 32 ? 0xffffffffu : (1u << (n - i0)) - 1u;
-          for (unsigned rest = all & ~bulk; rest; rest &= rest - 1) {
-            const int k = i0 + __ffs(rest) - 1;
-            const double* const from = src0 + (int64_t)k * g.sA;
+          for (int i = lane; i < n; i += 32) bulk(t, dst + (uint32_t)i * step, src + (int64_t)i * g.sA);
+          __syncwarp();
+          return;
+        }
+        for (int i = 0; i < n; ++i, src += g.sA, dst += step) {
+          if (!g.lane_copies || (((uintptr_t)src | bytes) & 15) == 0) {
+            if (lane == 0) {
+              expect(t, bytes);
+              bulk(t, dst, src);
+            }
+          } else {
             for (uint32_t x = lane; x < bytes / 8; x += 32)
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst0 + (uint32_t)k * step + 8u * x),
-                           "l"(from + x)
-                           : "memory");
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * x), "l"(src + x) : "memory");
           }
         }
-        __syncwarp();
+      }
+      __device__ __forceinline__ void expect(int t, uint32_t n) const {
+        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar(t)), "r"(n) : "memory");
+      }
+      __device__ __forceinline__ void bulk(int t, uint32_t dst, const double* src) const {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                     "l"(src), "r"(bytes), "r"(bar(t))
+                     : "memory");
       }
       __device__ __forceinline__ void finish(int t) const {
         if (lane == 0) mbar_arrive(bar(t));
@@ -992,8 +998,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) k_lincomb_oz(LcArgs g) {
         if (lane == 0 && !mbar_drain(bar(t), (uint32_t)(t >> 1) & 1u)) atomicExch(const_cast<int*>(sflag), 1);
       }
     };
-    Io io{g, raw, sflag, sdone, r0, r1, nsd, lane, BAR(LC_B_RAWF)};
-    if (!block_ring_load(io, ntile, nb, nslots, nsd, nks, LC_KS) && lane == 0) atomicExch(sflag, 1);
+    Io io{g, sflag, sdone, r0, r1, nsd, lane, BAR(LC_B_RAWF), smem_u32(raw), nullptr, 0};
+    if (!block_ring_load<LC_KS>(io, ntile, nb, nslots, nsd, nks) && lane == 0) atomicExch(sflag, 1);
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
   }

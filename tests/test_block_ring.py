@@ -62,7 +62,13 @@ struct Model {
     ahead = rnd = (rnd * 5 + 3) % 8;
     return cut_steps;
   }
+  int begun = -1;
+  void begin(int t) {
+    if (t != begun + 1) bad |= 128;
+    begun = t;
+  }
   void copy(int t, int b, int n, int slot) {
+    if (t != begun) bad |= 128;
     if (n < 1 || b + n > nb) { bad |= 64; return; }
     for (int i = 0; i < n; ++i) copy1(t, b + i, slot + i);
   }
@@ -93,7 +99,7 @@ struct Model {
 
 int main() {
   long runs = 0;
-  for (int nsd : {1, 2, 3, 4, 5, 8, 16})
+  for (int nsd : {1, 2, 3, 4, 5, 7, 8, 11, 15, 16})
     for (int nb : {1, 2, 3, 7, 8, 17, 40})
       for (int nslots = nb; nslots <= 2 * nb; nslots += nb > 8 ? 5 : 1)
         for (int ntile : {0, 1, 2, 3, 5})
@@ -105,7 +111,7 @@ int main() {
               m.bytes_of_block = 128L * nsd * 8;
               m.slot_tile.assign(nslots, -1);
               m.slot_block.assign(nslots, -1);
-              const bool ok = block_ring_load(m, ntile, nb, nslots, nsd, m.nks, m.ks);
+              const bool ok = block_ring_load<16>(m, ntile, nb, nslots, nsd, m.nks);
               const bool gave_up = give_up >= 0 && m.waits > give_up;
               ++runs;
               if (m.bad || !m.flight.empty() || ok == gave_up) {
