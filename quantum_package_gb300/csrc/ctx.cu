@@ -187,8 +187,13 @@ int ensure_work(qpgpu_ctx* c, size_t bytes) {
 
 namespace {
 struct Pools {  // of all contexts of the process
+  struct Pool {
+    int device;
+    cudaMemPool_t pool;
+    cudaStream_t stream;  // the one it is used on
+  };
   std::mutex mu;
-  std::vector<std::pair<int, cudaMemPool_t>> v;  // device, pool
+  std::vector<Pool> v;
 };
 Pools& pools() {
   static Pools* p = new Pools;  // contexts may go after the statics
@@ -218,11 +223,13 @@ bool over_limit(qpgpu_ctx* c, size_t pool_more, size_t dev_more, bool given_back
 void qp_give_back(int device) {
   int cur = -1;
   if (cudaGetDevice(&cur) == cudaSuccess && cur != device) cudaSetDevice(device);
-  cudaDeviceSynchronize();  // a block whose free is still queued cannot go
   {
     std::lock_guard<std::mutex> l(pools().mu);
     for (auto& p : pools().v)
-      if (p.first == device) cudaMemPoolTrimTo(p.second, 0);
+      if (p.device == device) {
+        cudaStreamSynchronize(p.stream);  // a block whose free is still queued cannot go
+        cudaMemPoolTrimTo(p.pool, 0);
+      }
   }
   if (cur >= 0 && cur != device) cudaSetDevice(cur);
 }
@@ -233,7 +240,7 @@ cudaError_t qp_free_bytes(qpgpu_ctx* c, size_t* fr, size_t* total) {
   {
     std::lock_guard<std::mutex> l(pools().mu);
     for (auto& p : pools().v)
-      if (p.first == c->device) *fr += pool_cached(p.second);
+      if (p.device == c->device) *fr += pool_cached(p.pool);
   }
   if (c->memory_limit) {
     const size_t held = qp_pool_reserved(c) - pool_cached(c->pool) + c->dev_bytes;
@@ -312,9 +319,18 @@ int qp_join(qpgpu_ctx* c, cudaStream_t st) {
 }
 
 void qp_pool_idle(qpgpu_ctx* c) {
+  if (!c->have_dets) return;
   int cur = -1;
   if (cudaGetDevice(&cur) == cudaSuccess && cur != c->device) cudaSetDevice(c->device);
-  cudaDeviceSynchronize();
+  // cudaFree waits for the device, as it did for each array of a set.  Unlike
+  // cudaDeviceSynchronize it leaves a capture on another thread alone.
+  void* p = nullptr;
+  if (cudaMalloc(&p, 1) == cudaSuccess) {
+    cudaFree(p);
+  } else {
+    cudaGetLastError();
+    cudaDeviceSynchronize();
+  }
   if (cur >= 0 && cur != c->device) cudaSetDevice(cur);
 }
 
@@ -417,7 +433,7 @@ int qpgpu_create(int n_mo, int n_alpha, int n_beta, int n_int, qpgpu_ctx** out) 
       return QPGPU_ERR_CUDA;
     }
     std::lock_guard<std::mutex> l(pools().mu);
-    pools().v.emplace_back(c->device, c->pool);
+    pools().v.push_back({c->device, c->pool, c->stream});
   }
   *out = c;
   return QPGPU_OK;
@@ -445,7 +461,7 @@ int qpgpu_destroy(qpgpu_ctx* c) {
     {
       std::lock_guard<std::mutex> l(pools().mu);
       auto& v = pools().v;
-      v.erase(std::remove(v.begin(), v.end(), std::make_pair(c->device, c->pool)), v.end());
+      v.erase(std::remove_if(v.begin(), v.end(), [&](const Pools::Pool& p) { return p.pool == c->pool; }), v.end());
     }
     cudaMemPoolDestroy(c->pool);
     for (int i = 0; i < 2; ++i) {

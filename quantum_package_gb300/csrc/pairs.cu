@@ -1251,7 +1251,10 @@ int launch_scans(qpgpu_ctx* c, const BuildArgs& a, unsigned gs, unsigned gc, cud
   k_same<NINT, MODE, 1><<<gs, BLK, 0, side ? c->side[0] : st>>>(a);
   k_class_c<NINT, MODE><<<gc, BLK, 0, side ? c->side[1] : st>>>(a);
   rc = side ? qp_join(c, st) : 0;
-  if (rc) cudaDeviceSynchronize();  // work arrays are given back on c->stream
+  if (rc) {  // work arrays are given back on c->stream
+    cudaStreamSynchronize(c->side[0]);
+    cudaStreamSynchronize(c->side[1]);
+  }
   return rc;
 }
 

@@ -649,7 +649,8 @@ int qpgpu_fail(qpgpu_ctx* c, int code, const std::string& msg);
   } while (0)
 
 // qp_give_back: every pool of the process on the device returns what is not in
-// use.  An allocation that fails, in a pool or by cudaMalloc, is tried again
+// use, once its own stream is idle (not the device: a capture on another thread
+// would be lost).  An allocation that fails, in a pool or by cudaMalloc, is tried again
 // after it: cudaMalloc does not see what a pool keeps mapped.
 void qp_give_back(int device);
 // what can still be allocated: free on the device or unused in a pool, within
