@@ -1728,7 +1728,9 @@ extern "C" int qpgpu_davidson_hs2(qpgpu_ctx* c, double* u_in, int64_t dim_in, do
       // the next block is orthonormalised while the norms travel; when they
       // end the cycle or the run its block is not read
       if (iter < itermax - 1 && n_sigma < max_sigma) {
+        prof.mark(DavProf::STEP);
         orthonormalise(d, iter, ffalg);
+        prof.mark(DavProf::ORTHO);
         ortho_done = true;
       }
       QP_CUDA(c, cudaEventSynchronize(norms_ready.e));
