@@ -33,8 +33,8 @@
 //  * the last warp streams the raw FP64 rows of each chunk into a ring of raw
 //    stages (cp.async.bulk per operand block, completing on rawfull[r]; a
 //    block whose rows are strided or unaligned is copied by the warp's lanes);
-//  * warps 0-11 cut the chunk into digit planes (stores of 2, 4 or 8 rows of
-//    one column), free the raw stage (rawempty[r]) and fill digit stage s
+//  * warps 0-11 (those that have tasks) cut the chunk into digit planes (stores of
+//    2, 4 or 8 rows of one column), free the raw stage (rawempty[r]) and fill digit stage s
 //    (full[s]);
 //  * one warp issues the chunk's 16 MMAs once full[s] completes and commits
 //    them to empty[s] and, at the end of a window, to accf[b]; the windows

@@ -95,7 +95,7 @@ __device__ __forceinline__ void store_row_lean(const SigArgs& a, int64_t it, int
 
 
 constexpr int UNR = 4;    // FP64 sigma: pairs per lane per loop trip
-constexpr int UNR32 = 4;  // FP32 sigma: more independent loads in flight (latency bound)
+constexpr int UNR32 = 4;  // FP32 sigma
 
 // FP64 sigma.  From 3 states on it is bound by the FP64 pipe: an instruction of
 // a warp takes 64 cycles of its scheduler's pipe, against one for the integer
@@ -170,11 +170,13 @@ __device__ __forceinline__ void accumulate32(const SigArgs& a, const int (&col)[
 // lanes are combined as float-float pairs, and only the owner lane of each
 // state converts to FP64 and adds the FP64 diagonal term.
 //
-// The kernel is bound by load latency (each coefficient gather waits on its
-// column index).  With PIPE the next trip's (column, value) pairs are loaded
-// one trip ahead of the current trip's gathers, at the price of registers,
-// hence occupancy; which launch shape hides the latency best depends on the
-// row lengths, so it is chosen by timing (tune_sigma32).  Every shape gives
+// The kernel is bound by the L1TEX data pipe, at 76-81 percent of its peak with
+// 4 and 8 states: a wavefront for each distinct 32-byte sector of a coefficient
+// gather (2e5 x 8: 309 us; 1e6 x 8: 3.45 ms, with 8 instead of 4 gathers in
+// flight 3.52).  With PIPE the next trip's (column, value) pairs are loaded one
+// trip ahead of the current trip's gathers, at the price of registers, hence
+// occupancy; which launch shape keeps that pipe fed best depends on the row
+// lengths, so it is chosen by timing (tune_sigma32).  Every shape gives
 // bit-identical sums: each lane sees the same pairs in the same order.
 template <int NST, bool PIPE, int BS, int LD, bool V8>
 __global__ void __launch_bounds__(BS) k_sigma32(SigArgs a) {
