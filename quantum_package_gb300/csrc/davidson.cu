@@ -345,8 +345,9 @@ inline int gram_stage_width(int m, int nsd, int nbc) {
   for (int y = 0; y < ny; ++y) w = std::max(w, gram_tile(m, nsd, nbc, y).nblk * nsd + nbc);
   return w;
 }
+constexpr int GRAMF_SMEM = 72 * 1024;  // two stages
 inline int gram_rows_per_stage(int width) {
-  const int T = (72 * 1024 / (2 * (int)sizeof(float2) * width)) / 32 * 32;
+  const int T = (GRAMF_SMEM / (2 * (int)sizeof(float2) * width)) / 32 * 32;
   return std::max(32, std::min(T, 256));
 }
 
@@ -1158,10 +1159,11 @@ int gram_ff(Dav& d, const float2* A, int m, const float2* B, int nbc, double* ou
   const size_t smem = (size_t)2 * T * width * sizeof(float2);
   const bool two = nbc == 2 * d.nsd;
   if (!two && nbc != d.nsd) return -1;
-  // opted in at every launch (the attribute belongs to the current device),
-  // and for every size: the 48 KB default counts the static red[] too
+  // opted in at every launch (the attribute belongs to the current device), for
+  // the largest size: another thread may set it before this one launches
 #define QP_GRAMF_LAUNCH(NB, NS)                                                                        \
-  cudaFuncSetAttribute(k_gram_ff<NB, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
+  cudaFuncSetAttribute(k_gram_ff<NB, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,                 \
+                       std::max((int)smem, GRAMF_SMEM));                                               \
   cudaFuncSetAttribute(k_gram_ff<NB, NS>, cudaFuncAttributePreferredSharedMemoryCarveout,              \
                        cudaSharedmemCarveoutMaxShared);                                                \
   k_gram_ff<NB, NS><<<grid, DBLK, smem, d.st>>>(A, m, d.sUf, B, d.N, d.rows_per_cta, T, d.part, skip);

@@ -1063,8 +1063,10 @@ static int run_selection(qpgpu_ctx* c, const double* coef, int n_st, const doubl
     A.cand_val = (double*)d_cval.p;
     A.cand_at = (uint64_t*)d_cat.p;
     QP_CUDA(c, cudaMemsetAsync(d_cnt.p, 0, 2 * sizeof(unsigned long long), st));
+    // (the attribute is for the largest size: another thread may set it before this one launches)
 #define QP_SEL_RUN(NI)                                                                                             \
-  QP_CUDA(c, cudaFuncSetAttribute(k_sel_items<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));       \
+  QP_CUDA(c, cudaFuncSetAttribute(k_sel_items<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize,                    \
+                                  SEL_TILE * (int)sizeof(double)));                                                \
   k_sel_items<NI><<<(unsigned)n_units, SBLK, smem, st>>>(A);
     if (nint == 1) {
       QP_SEL_RUN(1)
