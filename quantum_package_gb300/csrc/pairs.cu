@@ -960,8 +960,8 @@ __device__ __forceinline__ void load_det(const u64* det, int64_t p, u64 (&J)[2 *
 // when the others were done.  The next trip's partners are loaded ahead, for
 // which three blocks of an SM have registers (four without: 20.8 ms at 1e6).
 // 1e5 (60 MOs) / 2e5 / 1e6 determinants: 1.26 / 3.0 / 21.3 -> 0.70 / 1.75 /
-// 19.1 ms; bound by the integer instructions of the Slater routines (about 400
-// a pair, 45 % issue) with the L2 latency of the integrals.
+// 19.1 ms; bound by the Slater routines (about 400 integer instructions a pair,
+// 42 percent issue, FP64 pipe at 62) with the L2 latency of the integrals.
 __device__ __forceinline__ float coupling_feature(double sum2) { return (float)(log10(sum2 + 1e-30) * 0.25); }
 
 template <int NINT>
